@@ -1,0 +1,271 @@
+// Softmax attention of two tiles of 128 rows per CTA on the fifth-generation tensor cores: what the prompt kernels share.
+// A kernel brings the queries into shared memory and gives the copies of a block of keys and values, the scores' form and
+// the mask; here are the order of the matrix instructions, the ring and the softmax.
+//
+// Roles of the 384 threads:
+//     warps 0..3, 4..7   softmax of tile 0, of tile 1: thread r holds row r = lane r of tensor memory
+//     warp 8             matrix instructions, per block j of KEYS keys and tile m
+//                            O_m[128 x vdim] += P_m(j) . V(j)   P_m from tensor memory, V read MN-major as its rows lie
+//                            S_m[128 x KEYS]  = Q_m . K(j + 1)^T
+//                        While the tensor cores work on one tile, the other tile's threads do their softmax.
+//     warp 9             TMA: two blocks of K, `nv` of V in flight
+// Tensor memory: S_m at column 128 m (P_m over its first KEYS / 2 columns), O_m at 256 + 128 m.  S_m(j + 1) is issued behind
+// O_m += P_m(j) . V(j), whose operand it overwrites: matrix instructions of one thread execute in order.  The barrier of
+// S_m(j) therefore also says that O_m is complete up to block j - 1, so a row may be rescaled without a wait of its own.
+//
+// Blocks of 128 keys: an instruction with N = 64 takes 32 cycles and its operands 48 cycles of shared memory (A 4 KiB, B 2 KiB
+// at 128 B a cycle); with N = 128 both take 64.  Per tile and block of 128 keys, 128 columns: 1024 cycles of matrix instructions and
+// 1024 of the special-function units (16 exponentials a cycle).
+// Every wait is bounded; the caller reports `abort` and frees tensor memory.
+#pragma once
+
+#include "ktk_umma.cuh"
+
+namespace ktk {
+
+constexpr int kFlThreads = 384;             // warps 10 and 11 only complete the warpgroup whose registers go to the softmax
+constexpr int kFlTmemCols = 512;
+constexpr int kFlColO = 256;
+constexpr int kFlQTile = kUmRows * 128;      // [128 rows][64 columns]
+constexpr float kFlSlack = 8.0f;             // the exponentials' reference moves when a maximum is 2^8 above it
+constexpr int kFlMaxSmem = 225 * 1024;       // dynamic; the barriers are static
+
+// Registers: 384 threads start with 168 each (64512 of the SM's); the softmax holds a row of scores, so its two warpgroups go
+// to 200 and the third to 104: 256 * 200 + 128 * 104 = 64512.  Every warp of a warpgroup calls the one of its role.
+__device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 200;"); }
+__device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 104;"); }
+
+// -inf where no key has been seen: the exponentials then refer to 0
+__device__ __forceinline__ float reference_or_zero(float m) { return m == -INFINITY ? 0.0f : m; }
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// S complete, P in place, O complete (tile) | K, V landed, K, V read out (buffer)
+struct FlashShared {
+    uint64_t s[2], p[2], o[2], k[2], v[2], kfree[2], vfree[2];
+    uint32_t tmem;
+    int abort;
+    __device__ __forceinline__ void init() {             // one thread
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&s[i], 1);
+            mbar_init(&p[i], 4);
+            mbar_init(&o[i], 1);
+            mbar_init(&k[i], 1);
+            mbar_init(&v[i], 1);
+            mbar_init(&kfree[i], 1);
+            mbar_init(&vfree[i], 1);
+        }
+        abort = 0;
+        mbar_init_fence();
+    }
+};
+
+template <int KEYS, int VC> struct Flash {
+    static constexpr int kTile = KEYS * 128;             // [KEYS keys][64 columns]
+    static constexpr int kVBuf = VC * kTile;
+    FlashShared& sh;
+    uint8_t *q, *k, *v;                                  // [tile][chunk] | [buffer][chunk] | [buffer][chunk]
+    int q_chunks, k_chunks;                              // 64-column chunks of a tile's queries, of a block of K
+    int nv;                                              // buffers of V: 1 or 2
+    int blocks0, blocks1;                                // blocks that each tile sees
+
+    __device__ __forceinline__ Flash(FlashShared& shared, uint8_t* smem, int qc, int kc, int v_bufs, int b0, int b1)
+        : sh(shared), q(smem), k(smem + 2 * qc * kFlQTile), v(k + 2 * kc * kTile), q_chunks(qc), k_chunks(kc), nv(v_bufs),
+          blocks0(b0), blocks1(b1) {}
+    __host__ __device__ static constexpr int bytes(int qc, int kc, int v_bufs) {
+        return 2 * qc * kFlQTile + 2 * kc * kTile + v_bufs * kVBuf;
+    }
+    // the second buffer of V where shared memory holds it
+    __host__ __device__ static constexpr int v_buffers(int qc, int kc) { return bytes(qc, kc, 2) + 1024 <= kFlMaxSmem ? 2 : 1; }
+
+    __device__ __forceinline__ int blocks() const { return blocks0 > blocks1 ? blocks0 : blocks1; }
+    __device__ __forceinline__ int blocks_of(int m) const { return m ? blocks1 : blocks0; }
+    __device__ __forceinline__ int v_buf(int blk) const { return blk & (nv - 1); }
+    __device__ __forceinline__ uint32_t v_phase(int blk) const { return (uint32_t)(blk >> (nv - 1)) & 1u; }
+
+    // ---- matrix instructions, by a converged warp.  steps(c): 16-column steps of chunk c; k_off: bytes between the keys of
+    // the two tiles in a buffer of K (0: the same keys); vcols: columns of V, a multiple of 16
+    template <class Steps> __device__ __forceinline__ void issue(Steps steps, int k_off, int vcols) {
+        const uint32_t tmem = sh.tmem;
+        const uint32_t idesc_s = umma_idesc(KEYS, false), idesc_o = umma_idesc(vcols, true);
+        const uint64_t q_desc = umma_desc(smem_u32(q), 0, 1024), k_desc = umma_desc(smem_u32(k), 0, 1024);
+        const uint64_t v_desc = umma_desc(smem_u32(v), kTile, 1024);
+        const int n = blocks();
+        auto scores = [&](int m, int blk) {
+            const uint64_t qa = umma_desc_at(q_desc, m * q_chunks * kFlQTile);
+            const uint64_t ka = umma_desc_at(k_desc, (blk & 1) * k_chunks * kTile + m * k_off);
+            if (elect_one()) {
+                for (int c = 0; c < q_chunks; ++c) {
+                    const int n_steps = steps(c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < n_steps)
+                            umma_f16(tmem + m * 128, umma_desc_at(qa, c * kFlQTile + i * 32), umma_desc_at(ka, c * kTile + i * 32),
+                                     idesc_s, (c > 0 || i > 0) ? 1u : 0u);
+                }
+                umma_commit(&sh.s[m]);
+            }
+            __syncwarp();
+        };
+        auto wait = [&](uint64_t* bar, uint32_t parity) {
+            if (!mbar_wait_all(bar, parity, &sh.abort)) return false;
+            tc_fence_after();
+            return true;
+        };
+        if (n == 0 || !wait(&sh.k[0], 0)) return;
+        if (blocks0 > 0) scores(0, 0);
+        if (blocks1 > 0) scores(1, 0);
+        if (elect_one()) umma_commit(&sh.kfree[0]);
+        __syncwarp();
+        for (int j = 0; j < n; ++j) {
+            const bool more = j + 1 < n;
+            if (!wait(&sh.v[v_buf(j)], v_phase(j))) return;
+            const uint64_t va = umma_desc_at(v_desc, v_buf(j) * kVBuf);
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const int mine = blocks_of(m);
+                if (j < mine) {
+                    if (!wait(&sh.p[m], j & 1)) return;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int i = 0; i < KEYS / 16; ++i)
+                            umma_f16_ts(tmem + kFlColO + m * 128, tmem + m * 128 + i * 8, umma_desc_at(va, i * (16 * 128)), idesc_o,
+                                        (j > 0 || i > 0) ? 1u : 0u);
+                        if (j + 1 == mine) umma_commit(&sh.o[m]);
+                    }
+                    __syncwarp();
+                }
+                if (m == 1) {
+                    if (elect_one()) umma_commit(&sh.vfree[v_buf(j)]);
+                    __syncwarp();
+                }
+                if (m == 0 && more && !wait(&sh.k[(j + 1) & 1], ((j + 1) >> 1) & 1)) return;
+                if (j + 1 < mine) scores(m, j + 1);
+                if (m == 1 && more) {
+                    if (elect_one()) umma_commit(&sh.kfree[(j + 1) & 1]);
+                    __syncwarp();
+                }
+            }
+        }
+    }
+
+    // ---- copies, by a converged warp.  load_k(blk, dst, bar), load_v(blk, dst, bar): tell the barrier the bytes and start the copies
+    template <class LoadK, class LoadV> __device__ __forceinline__ void copy(LoadK load_k, LoadV load_v) {
+        const int n = blocks();
+        int k_issued = 0, v_issued = 0;
+        auto more_k = [&] {
+            load_k(k_issued, k + (k_issued & 1) * k_chunks * kTile, &sh.k[k_issued & 1]);
+            ++k_issued;
+        };
+        bool alive = true;
+        if (n > 0) more_k();
+        if (n > 1) more_k();
+        for (int j = 0; j < n && alive; ++j) {
+            // V over that of block j - nv, then K of block j + 2 over that of block j
+            alive = j < nv || mbar_wait_all(&sh.vfree[v_buf(j)], v_phase(j) ^ 1u, &sh.abort);
+            if (!alive) break;
+            load_v(j, v + v_buf(j) * kVBuf, &sh.v[v_buf(j)]);
+            ++v_issued;
+            if (j + 2 < n) {
+                alive = mbar_wait_all(&sh.kfree[j & 1], (j >> 1) & 1, &sh.abort);
+                if (alive) more_k();
+            }
+        }
+        if (!alive) {                                    // the copies in flight still write shared memory
+            volatile int never = 0;
+            for (int i = k_issued > 2 ? k_issued - 2 : 0; i < k_issued; ++i) mbar_wait(&sh.k[i & 1], (i >> 1) & 1, &never);
+            for (int i = v_issued > nv ? v_issued - nv : 0; i < v_issued; ++i) mbar_wait(&sh.v[v_buf(i)], v_phase(i), &never);
+        }
+    }
+
+    // ---- softmax of tile m, by its four warps (thread `row`).  prepare(s, j): the scores of block j, masked ones -inf;
+    // the exponents are s f (FIXED: s) against m_ref.  clear(j): whether rows of V(j) that hold no key have been cleared.
+    // Returns whether O is complete.
+    template <bool FIXED, class Prepare, class Clear>
+    __device__ __forceinline__ bool softmax(int m, float f, float& m_ref, float& l_run, Prepare prepare, Clear clear) {
+        const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+        const uint32_t my = sh.tmem + ((uint32_t)(warp * 32) << 16), s_at = my + m * 128, o_at = my + kFlColO + m * 128;
+        const int mine = blocks_of(m);
+        for (int j = 0; j < mine; ++j) {
+            if (!mbar_wait_all(&sh.s[m], j & 1, &sh.abort)) return false;
+            tc_fence_after();
+            float s[KEYS];
+            tmem_load(s_at, s);
+            prepare(s, j);
+            float base = 0.0f;
+            if (!FIXED) {
+                float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+                for (int c = 4; c < KEYS - 4; c += 8)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) mx[i] = max3(mx[i], s[c + i], s[c + 4 + i]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], s[KEYS - 4 + i]);
+                const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * f;
+                float alpha = 1.0f;
+                if (top > m_ref + (j == 0 ? 0.0f : kFlSlack)) {
+                    alpha = ex2(m_ref - top);
+                    m_ref = top;
+                    l_run *= alpha;
+                }
+                base = -reference_or_zero(m_ref);
+                if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {     // warp-uniform: the loads and stores are warp-wide
+#pragma unroll
+                    for (int c = 0; c < VC * 64; c += 16) {
+                        float o[16];
+                        tmem_ld16(o_at + c, o);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] *= alpha;
+                        tmem_st16(o_at + c, o);
+                    }
+                }
+            }
+            const uint64_t f2 = pack2(f, f), b2 = pack2(base, base);
+            uint64_t sum[2] = {0, 0};
+#pragma unroll
+            for (int h = 0; h < KEYS; h += 64) {
+                uint32_t packed[32];
+#pragma unroll
+                for (int c = 0; c < 32; ++c) {
+                    float x = s[h + 2 * c], y = s[h + 2 * c + 1];
+                    if (!FIXED) unpack2(fma2(pack2(x, y), f2, b2), x, y);
+                    x = ex2(x);
+                    y = ex2(y);
+                    sum[c & 1] = add2(sum[c & 1], pack2(x, y));
+                    packed[c] = pack_bf16(x, y);
+                }
+                tmem_st32_u32(s_at + h / 2, packed);
+            }
+            float a, b;
+            unpack2(add2(sum[0], sum[1]), a, b);
+            l_run += a + b;
+            tmem_st_wait();
+            clear(j);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.p[m]);
+        }
+        if (mine > 0 && !mbar_wait_all(&sh.o[m], 0, &sh.abort)) return false;
+        tc_fence_after();
+        return true;
+    }
+
+    // Zeros over the rows of V(j) without a key (has_key(row)), by the first tile that sees the block
+    template <class HasKey> __device__ __forceinline__ void clear_rows(int m, int j, HasKey has_key) {
+        if (m != (j < blocks0 ? 0 : 1)) return;
+        const int r = threadIdx.x & (kUmRows - 1);
+        if (r < KEYS && !has_key(r)) {
+            mbar_wait_fast(&sh.v[v_buf(j)], v_phase(j), &sh.abort);          // a wait that ran out ends the next block
+#pragma unroll
+            for (int c = 0; c < VC * 8; ++c)
+                *reinterpret_cast<uint4*>(v + v_buf(j) * kVBuf + (c >> 3) * kTile + swz(r, c & 7)) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async();
+    }
+};
+
+}  // namespace ktk

@@ -21,11 +21,6 @@ struct PrefillUmmaParams {
     int32_t* status;
 };
 
-// Descriptor of the V operand (MN-major: 64 keys x 128 B rows per 64-dim tile, 128-byte swizzle): byte distance
-// between the two 64-dim tiles, and between groups of eight keys.
-constexpr uint32_t kUmVLbo = 64 * 128;
-constexpr uint32_t kUmVSbo = 1024;
-
 int launch_prefill_umma(const PrefillUmmaParams& p, int max_new_tokens, cudaStream_t st);
 
 }  // namespace ktk
