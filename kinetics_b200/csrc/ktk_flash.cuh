@@ -16,6 +16,8 @@
 // Blocks of 128 keys: an instruction with N = 64 takes 32 cycles and its operands 48 cycles of shared memory (A 4 KiB, B 2 KiB
 // at 128 B a cycle); with N = 128 both take 64.  Per tile and block of 128 keys, 128 columns: 1024 cycles of matrix instructions and
 // 1024 of the special-function units (16 exponentials a cycle).
+// The exponentials of one warp come at 12 cycles each instead of 8 (latencies), those of two at 10.  Two threads to a row (16 softmax
+// warps) and a polynomial on the FMA pipes for a part of the exponentials were not faster; over seconds the power limit binds.
 // Every wait is bounded; the caller reports `abort` and frees tensor memory.
 #pragma once
 
@@ -27,7 +29,7 @@ constexpr int kFlThreads = 384;             // warps 10 and 11 only complete the
 constexpr int kFlTmemCols = 512;
 constexpr int kFlColO = 256;
 constexpr int kFlQTile = kUmRows * 128;      // [128 rows][64 columns]
-constexpr float kFlSlack = 8.0f;             // the exponentials' reference moves when a maximum is 2^8 above it
+constexpr float kFlMost = 1073741824.0f;     // 2^30: the exponentials' reference moves when half a block's sum is above it
 constexpr int kFlMaxSmem = 225 * 1024;       // dynamic; the barriers are static
 
 // Registers: 384 threads start with 168 each (64512 of the SM's); the softmax holds a row of scores, so its two warpgroups go
@@ -44,15 +46,17 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-// S complete, P in place, O complete (tile) | K, V landed, K, V read out (buffer)
+// S complete, the halves of P in place, O complete up to the first half of a block, O complete (tile) | K, V landed, K, V read out (buffer)
 struct FlashShared {
-    uint64_t s[2], p[2], o[2], k[2], v[2], kfree[2], vfree[2];
+    uint64_t s[2], p[2], p_rest[2], o_half[2], o[2], k[2], v[2], kfree[2], vfree[2];
     uint32_t tmem;
     int abort;
     __device__ __forceinline__ void init() {             // one thread
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s[i], 1);
             mbar_init(&p[i], 4);
+            mbar_init(&p_rest[i], 4);
+            mbar_init(&o_half[i], 1);
             mbar_init(&o[i], 1);
             mbar_init(&k[i], 1);
             mbar_init(&v[i], 1);
@@ -66,6 +70,7 @@ struct FlashShared {
 
 template <int KEYS, int VC> struct Flash {
     static constexpr int kTile = KEYS * 128;             // [KEYS keys][64 columns]
+    static constexpr int kHalf = KEYS / 2;
     static constexpr int kVBuf = VC * kTile;
     FlashShared& sh;
     uint8_t *q, *k, *v;                                  // [tile][chunk] | [buffer][chunk] | [buffer][chunk]
@@ -123,27 +128,32 @@ template <int KEYS, int VC> struct Flash {
         __syncwarp();
         for (int j = 0; j < n; ++j) {
             const bool more = j + 1 < n;
-            if (!wait(&sh.v[v_buf(j)], v_phase(j))) return;
+            // both copies before the probabilities, which are what the tensor cores are short of
+            if (!wait(&sh.v[v_buf(j)], v_phase(j)) || (more && !wait(&sh.k[(j + 1) & 1], ((j + 1) >> 1) & 1))) return;
             const uint64_t va = umma_desc_at(v_desc, v_buf(j) * kVBuf);
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const int mine = blocks_of(m);
                 if (j < mine) {
-                    if (!wait(&sh.p[m], j & 1)) return;
-                    if (elect_one()) {
+                    // the first half of the block's keys while the threads work on the second
 #pragma unroll
-                        for (int i = 0; i < KEYS / 16; ++i)
-                            umma_f16_ts(tmem + kFlColO + m * 128, tmem + m * 128 + i * 8, umma_desc_at(va, i * (16 * 128)), idesc_o,
-                                        (j > 0 || i > 0) ? 1u : 0u);
-                        if (j + 1 == mine) umma_commit(&sh.o[m]);
+                    for (int part = 0; part < 2; ++part) {
+                        if (!wait(part ? &sh.p_rest[m] : &sh.p[m], j & 1)) return;
+                        if (elect_one()) {
+#pragma unroll
+                            for (int i = part * (kHalf / 16); i < (part + 1) * (kHalf / 16); ++i)
+                                umma_f16_ts(tmem + kFlColO + m * 128, tmem + m * 128 + i * 8, umma_desc_at(va, i * (16 * 128)), idesc_o,
+                                            (j > 0 || i > 0) ? 1u : 0u);
+                            if (part == 0) umma_commit(&sh.o_half[m]);
+                            else if (j + 1 == mine) umma_commit(&sh.o[m]);
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
                 }
                 if (m == 1) {
                     if (elect_one()) umma_commit(&sh.vfree[v_buf(j)]);
                     __syncwarp();
                 }
-                if (m == 0 && more && !wait(&sh.k[(j + 1) & 1], ((j + 1) >> 1) & 1)) return;
                 if (j + 1 < mine) scores(m, j + 1);
                 if (m == 1 && more) {
                     if (elect_one()) umma_commit(&sh.kfree[(j + 1) & 1]);
@@ -182,38 +192,77 @@ template <int KEYS, int VC> struct Flash {
         }
     }
 
-    // ---- softmax of tile m, by its four warps (thread `row`).  prepare(s, j): the scores of block j, masked ones -inf;
-    // the exponents are s f (FIXED: s) against m_ref.  clear(j): whether rows of V(j) that hold no key have been cleared.
-    // Returns whether O is complete.
-    template <bool FIXED, class Prepare, class Clear>
-    __device__ __forceinline__ bool softmax(int m, float f, float& m_ref, float& l_run, Prepare prepare, Clear clear) {
+    // ---- softmax of tile m, by its four warps (thread `row`).  prepare(s, j): the scores of block j, masked ones -inf; returns
+    // whether form(x, y) is still to be applied to every pair of them.  The exponents are s f (FIXED: s) against m_ref.
+    // clear(j): rows of V(j) that hold no key.  Returns whether O is complete.
+    //
+    // The reference is the sink or the first block's maximum, and stays: exponentials, their bf16 and the sums have the range of
+    // fp32, and a common factor changes none of their relative roundings.  It moves only where half a block's sum passes 2^30
+    // (or is infinite), so no other block's maximum has to be searched: that cost 500 of a block's 3400 cycles.
+    // The halves of a block are handed over one by one: 521 us for the prompt of 8192 tokens and 32 heads without that, 498 with it.
+    template <bool FIXED, class Prepare, class Form, class Clear>
+    __device__ __forceinline__ bool softmax(int m, float f, float& m_ref, float& l_run, Prepare prepare, Form form, Clear clear) {
         const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
         const uint32_t my = sh.tmem + ((uint32_t)(warp * 32) << 16), s_at = my + m * 128, o_at = my + kFlColO + m * 128;
+        const uint64_t f2 = pack2(f, f);
         const int mine = blocks_of(m);
         for (int j = 0; j < mine; ++j) {
             if (!mbar_wait_all(&sh.s[m], j & 1, &sh.abort)) return false;
             tc_fence_after();
             float s[KEYS];
             tmem_load(s_at, s);
-            prepare(s, j);
-            float base = 0.0f;
-            if (!FIXED) {
-                float mx[4] = {s[0], s[1], s[2], s[3]};
+            const bool raw = prepare(s, j);
+            float base = FIXED ? 0.0f : -reference_or_zero(m_ref);
+            uint32_t packed[kHalf / 2];
+            uint64_t sum[2] = {0, 0};
+            auto pair = [&](int from, int c, bool formed) {
+                float x = s[from + 2 * c], y = s[from + 2 * c + 1];
+                if (formed) form(x, y);
+                if (!FIXED) unpack2(fma2(pack2(x, y), f2, pack2(base, base)), x, y);
+                x = ex2(x);
+                y = ex2(y);
+                sum[c & 1] = add2(sum[c & 1], pack2(x, y));
+                packed[c] = pack_bf16(x, y);
+            };
+            auto half = [&](int from) {
+                sum[0] = sum[1] = 0;
+                if (FIXED && raw) {
 #pragma unroll
-                for (int c = 4; c < KEYS - 4; c += 8)
+                    for (int c = 0; c < kHalf / 2; ++c) pair(from, c, true);
+                } else {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) mx[i] = max3(mx[i], s[c + i], s[c + 4 + i]);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], s[KEYS - 4 + i]);
-                const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * f;
-                float alpha = 1.0f;
-                if (top > m_ref + (j == 0 ? 0.0f : kFlSlack)) {
-                    alpha = ex2(m_ref - top);
-                    m_ref = top;
-                    l_run *= alpha;
+                    for (int c = 0; c < kHalf / 2; ++c) pair(from, c, false);
                 }
+            };
+            auto total = [&] {
+                float a, b;
+                unpack2(add2(sum[0], sum[1]), a, b);
+                return a + b;
+            };
+            auto hand_over = [&](int from, uint64_t* bar) {
+                tmem_store(s_at + from / 2, packed);
+                l_run += total();
+                tmem_st_wait();
+                if (from == 0) clear(j);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar);
+            };
+            // another reference, no lower than the exponents of columns from ..: O and the sum so far follow it
+            auto move = [&](int from, bool mine_moves, bool has_o) {
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int c = 0; c < KEYS; c += 8)
+                    if (c >= from)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) mx[i] = max3(mx[i], s[c + i], s[c + 4 + i]);
+                const float top = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]) * f;
+                const bool moves = mine_moves && top > m_ref;
+                const float alpha = moves ? ex2(m_ref - top) : 1.0f;
+                if (moves) m_ref = top;
                 base = -reference_or_zero(m_ref);
-                if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {     // warp-uniform: the loads and stores are warp-wide
+                l_run *= alpha;
+                if (has_o) {
 #pragma unroll
                     for (int c = 0; c < VC * 64; c += 16) {
                         float o[16];
@@ -223,31 +272,26 @@ template <int KEYS, int VC> struct Flash {
                         tmem_st16(o_at + c, o);
                     }
                 }
+            };
+            // the votes: tensor memory is read and written by whole warps
+            if (!FIXED && __any_sync(0xffffffffu, m_ref == -INFINITY)) move(0, m_ref == -INFINITY, j > 0);
+            half(0);
+            if (!FIXED) {
+                const bool over = total() > kFlMost;
+                if (__any_sync(0xffffffffu, over)) { move(0, over, j > 0); half(0); }
             }
-            const uint64_t f2 = pack2(f, f), b2 = pack2(base, base);
-            uint64_t sum[2] = {0, 0};
-#pragma unroll
-            for (int h = 0; h < KEYS; h += 64) {
-                uint32_t packed[32];
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    float x = s[h + 2 * c], y = s[h + 2 * c + 1];
-                    if (!FIXED) unpack2(fma2(pack2(x, y), f2, b2), x, y);
-                    x = ex2(x);
-                    y = ex2(y);
-                    sum[c & 1] = add2(sum[c & 1], pack2(x, y));
-                    packed[c] = pack_bf16(x, y);
+            hand_over(0, &sh.p[m]);
+            half(kHalf);
+            if (!FIXED) {
+                const bool over = total() > kFlMost;
+                if (__any_sync(0xffffffffu, over)) {
+                    if (!mbar_wait_all(&sh.o_half[m], j & 1, &sh.abort)) return false;
+                    tc_fence_after();
+                    move(kHalf, over, true);
+                    half(kHalf);
                 }
-                tmem_st32_u32(s_at + h / 2, packed);
             }
-            float a, b;
-            unpack2(add2(sum[0], sum[1]), a, b);
-            l_run += a + b;
-            tmem_st_wait();
-            clear(j);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.p[m]);
+            hand_over(kHalf, &sh.p_rest[m]);
         }
         if (mine > 0 && !mbar_wait_all(&sh.o[m], 0, &sh.abort)) return false;
         tc_fence_after();

@@ -6,7 +6,7 @@
 // group) pairs.  Both tiles share every block of 128 keys (eight pages, 16-row x 128-byte boxes under the 128-byte swizzle, which
 // is the operand layout tcgen05.mma reads).  The softmax and the order of the matrix instructions: ktk_flash.cuh.
 // Bound by the chain of a tile's block: matrix instructions, softmax, matrix instructions.  8192 tokens, 32 heads over 8 kv
-// heads: 531 us (1035 TFLOP/s), 880 us with one tile per CTA, blocks of 64 keys and two CTAs per SM.
+// heads: 510 us (1078 TFLOP/s), 880 us with one tile per CTA, blocks of 64 keys and two CTAs per SM.
 #include "ktk_decode_mma.cuh"
 #include "ktk_flash.cuh"
 #include "ktk_prefill_umma.cuh"
@@ -137,6 +137,7 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
                     for (int c = 0; c < kPageSize; ++c) s[c] = c < sp.first_fill ? s[c] : -INFINITY;
                 }
             }
+            return false;
         };
         // the rows of V that hold no key: pages that are not read, the places of a page that is not full
         auto clear = [&](int j) {
@@ -148,7 +149,7 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
             });
         };
         float m_ref = -INFINITY, l_run = 0.0f;
-        const bool done = fl.softmax<false>(tile, p.scale_log2, m_ref, l_run, prepare, clear);
+        const bool done = fl.softmax<false>(tile, p.scale_log2, m_ref, l_run, prepare, [](float&, float&) {}, clear);
         if (done && fl.blocks_of(tile) > 0) {
             const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
             const uint32_t o_at = sh.tmem + ((uint32_t)((warp & 3) * 32) << 16) + kFlColO + tile * 128;

@@ -5,7 +5,7 @@
 // One CTA per (head, two tiles of 128 tokens): both tiles share every block of keys (128; 64 where the queries of a wide head
 // leave shared memory for no more) that comes in by TMA: the unrotated columns of the head, then the shared rotated ones.  The
 // softmax and the order of the matrix instructions: ktk_flash.cuh; the exponents' reference starts at the sink.
-// 8192 tokens, 32 heads of 128 + 64 and 128 columns: 609 us (1128 TFLOP/s), 899 us with blocks of 64 keys.  Heads are walked
+// 8192 tokens, 32 heads of 128 + 64 and 128 columns: 590 us (1164 TFLOP/s), 899 us with blocks of 64 keys.  Heads are walked
 // in groups whose keys and values fit L2, so that the CTAs left for the end are short ones.
 #include "../ktk_flash.cuh"
 #include "ktl_score.cuh"
@@ -120,11 +120,13 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bu
         const int tile_min_vis = base + tok0 + tile * kUmRows + 1;
         float m_ref = p.sink ? p.sink[head] * kLog2eF : -INFINITY, l_run = p.sink ? 1.0f : 0.0f;
         const bool done = fl.template softmax<false>(tile, a.scale * kLog2eF, m_ref, l_run, [&](float (&s)[KEYS], int j) {
-            if ((j + 1) * KEYS <= tile_min_vis) return;                // every row of the tile sees the whole block
-            const int lim = vis - j * KEYS;
+            if ((j + 1) * KEYS > tile_min_vis) {                       // some row of the tile does not see the whole block
+                const int lim = vis - j * KEYS;
 #pragma unroll
-            for (int c = 0; c < KEYS; ++c) s[c] = c < lim ? s[c] : -INFINITY;
-        }, [](int) {});
+                for (int c = 0; c < KEYS; ++c) s[c] = c < lim ? s[c] : -INFINITY;
+            }
+            return false;
+        }, [](float&, float&) {}, [](int) {});
         if (done && fl.blocks_of(tile) > 0) {
             float g = l_run > 0.0f ? 1.0f / l_run : 0.0f;
             if (row_on && p.gate) g *= sigmoid_f(__bfloat162float(p.gate[(int64_t)tok * p.gate_stride + head]));

@@ -6,7 +6,7 @@
 // ktk_flash.cuh are the two maps, each with keys of its own; a block is 128 keys of both maps and their values.
 // With a softcap the exponentials have a fixed reference (ktl_score.cuh): nothing is ever rescaled.  Without one (or
 // with a large one) the reference follows the running maximum in jumps.
-// Bound by what the softmax issues: 8192 tokens, 16 heads of 2 x 64 and 128 columns, softcap: 659 us, 792 us with blocks of
+// Bound by what the softmax issues: 8192 tokens, 16 heads of 2 x 64 and 128 columns, softcap: 523 us, 792 us with blocks of
 // 64 keys.
 #include "../ktk_flash.cuh"
 #include "ktl_score.cuh"
@@ -128,6 +128,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
         exact.set(factor, capped ? a.softcap : 1.0f);
         const int tile_min_vis = base_pos + tok0 + 1;
         auto prepare = [&](float (&v)[kAuKeys], int j) {
+            const bool masked = (j + 1) * kAuKeys > tile_min_vis;      // some row of the tile does not see the whole block
             if (capped) {
                 float mx[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -135,9 +136,11 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
 #pragma unroll
                     for (int i = 0; i < 4; ++i) mx[i] = max3(mx[i], fabsf(v[c + i]), fabsf(v[c + 4 + i]));
                 // rows without a token and keys behind a row's own hold stale numbers: they decide the branch at most
-                if (__any_sync(0xffffffffu, !(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) <= poly.limit))) {
+                if (__any_sync(0xffffffffu, !(max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]) <= poly.limit))) {
 #pragma unroll
                     for (int c = 0; c < kAuKeys; ++c) v[c] = exact(v[c]);
+                } else if (FIXED && !masked) {
+                    return true;                                       // beside the exponentials
                 } else {
 #pragma unroll
                     for (int c = 0; c < kAuKeys; c += 2) poly.two(v[c], v[c + 1]);
@@ -146,17 +149,18 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
 #pragma unroll
                 for (int c = 0; c < kAuKeys; ++c) v[c] *= plain;
             }
-            if ((j + 1) * kAuKeys > tile_min_vis) {                    // some row of the tile does not see the whole block
+            if (masked) {
                 const int lim = vis - j * kAuKeys;
 #pragma unroll
                 for (int c = 0; c < kAuKeys; ++c) v[c] = c < lim ? v[c] : -INFINITY;
             }
+            return false;
         };
         auto clear = [&](int j) {                                      // the last block: rows of V without a key
             if ((j + 1) * kAuKeys > seen) fl.clear_rows(map, j, [&](int r) { return j * kAuKeys + r < seen; });
         };
         float m_ref = -INFINITY, l_run = 0.0f;
-        fl.template softmax<FIXED>(map, 1.0f, m_ref, l_run, prepare, clear);
+        fl.template softmax<FIXED>(map, 1.0f, m_ref, l_run, prepare, [&](float& x, float& y) { poly.two(x, y); }, clear);
         // ---- o = O_1 / l_1 - lambda O_2 / l_2, unit norm: warps 0..3 the first half of the columns, 4..7 the second.
         // Row sums go over the queries, which each map's last block has read.
         float* row_l = reinterpret_cast<float*>(fl.q + map * DC * kFlQTile);

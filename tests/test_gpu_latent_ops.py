@@ -130,6 +130,40 @@ def test_expanded_attention(cuda_device, heads, dim, rot_dim, vdim):
         assert (got[:, :, vdim:] == 0).all()
 
 
+@pytest.mark.parametrize("sink", [-300.0, 0.0, 300.0])
+@pytest.mark.parametrize("dim", [128, 192])
+def test_expanded_scores_far_from_the_sink(cuda_device, dim, sink):
+    """Scores that grow by hundreds along the keys, against sinks far under and over them: the exponentials' reference starts at
+    the sink.  Bound: as in test_expanded_attention."""
+    from kinetics_b200 import layer_ops as lo, ops
+    from kinetics_b200.layer_ops import LatentSpec, Rotation
+    heads, rot_dim, vdim, rank, n = 2, 64, 64, 48, 400
+    spec = LatentSpec(heads, dim, rot_dim, vdim, rank, (dim + rot_dim) ** -0.5, Rotation(rot_dim, 1e4))
+    g = torch.Generator().manual_seed(dim)
+    factor = torch.ones(n)
+    factor[150:160], factor[200:204], factor[300:330] = 30.0, 90.0, 150.0
+    q = torch.randn(n, heads, dim + rot_dim, generator=g)
+    keys, rot = torch.randn(n, heads, dim, generator=g) * factor[:, None, None], torch.randn(n, rot_dim, generator=g)
+    values = torch.randn(n, heads, vdim, generator=g)
+    kv = torch.cat((keys.reshape(n, -1), values.reshape(n, -1)), dim=1)
+    put = lambda t: t.to(BF).to(cuda_device)
+    proj = put(torch.cat((q.reshape(n, -1), torch.zeros(n, spec.proj_cols - spec.q_cols)), dim=1))
+    proj[:, spec.gate_col:spec.gate_col + heads] = 1.0
+    status = ops.new_status(cuda_device)
+    lat = torch.cat((torch.zeros(n, rank), rot), dim=1)
+    got = lo.expanded_attention(proj, put(kv), put(lat), spec, torch.full((heads,), sink, device=cuda_device),
+                                proj[:, spec.gate_col:], status)
+    ops.raise_on_status(status)
+    got = got.view(n, heads, vdim).double().cpu()
+    r64 = lambda t: t.to(BF).double()
+    for h in range(heads):
+        s = (r64(q[:, h, :dim]) @ r64(keys[:, h]).t() + r64(q[:, h, dim:]) @ r64(rot).t()) * spec.scale
+        want = plain.sigmoid(torch.ones(1, 1, dtype=torch.float64)) * \
+            (plain.sink_softmax(s, torch.tensor(sink, dtype=torch.float64), 0) @ r64(values[:, h]))
+        err = (got[:, h] - want).pow(2).mean(-1).sqrt()
+        assert err.max() < 3e-2, (h, float(err.max()))
+
+
 @pytest.mark.parametrize("dtype", [F32, BF])
 def test_append_rotates_and_normalises(cuda_device, dtype):
     from kinetics_b200 import layer_ops as lo, ops

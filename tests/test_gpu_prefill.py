@@ -122,3 +122,32 @@ def test_prefill_on_block_and_tile_edges(cuda_device, variant, G, sink):
         lo, hi = int(q_indptr[b]), int(q_indptr[b + 1])
         ref = _reference(q[lo:hi].float(), k[b, :, :lens[b]].to(cuda_device), v[b, :, :lens[b]].to(cuda_device), G)
         torch.testing.assert_close(out[lo:hi].float(), ref, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("G,sink,grow", [(4, 0, (0.1, 40.0, 200.0)), (1, 4, (1.0, 1.0, 90.0)), (2, 0, (60.0, 0.1, 30.0))])
+def test_prefill_scores_that_outgrow_their_reference(cuda_device, G, sink, grow):
+    """The exponentials' reference is the first block's maximum until a half block's sum passes 2^30: scores that grow by far
+    more in the first half of a block of 128 keys, in its second half, in the block of the row itself; and that shrink.
+
+    Bound: operands are the reference's own bf16 values, products of 128 columns are summed in fp32, so a score of up to about
+    1000 is off by a few 1e-4, a weight by that share; bf16 weights add 2^-9 of each value: 2e-2, as in the other cases."""
+    from kinetics_b200 import ops
+    Hkv, hist, n = 2, 330, 200
+    total = hist + n
+    g = torch.Generator().manual_seed(7 + G)
+    factor = torch.full((total,), grow[0])
+    factor[140:170] = grow[1]                                # first half of the second block
+    factor[230:236] = grow[2]                                # second half of it
+    factor[hist + 20:hist + 90] = grow[2]                    # among the new tokens
+    k = (torch.randn(1, Hkv, total, 128, generator=g) * factor[:, None]).to(torch.bfloat16).float()
+    v = torch.randn(1, Hkv, total, 128, generator=g).to(torch.bfloat16).float()
+    d = to_dev(paged_state(k, v, [total], torch.bfloat16, seed=3, sink=sink), cuda_device)
+    q = torch.randn(n, Hkv * G, 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    q_indptr = torch.tensor([0, n], dtype=torch.int32, device=cuda_device)
+    status = ops.new_status(cuda_device)
+    view = ops.PageView(sink_tokens=sink, local_tokens=1) if sink else None
+    out = ops.prefill_attention(q, q_indptr, n, d["kv_cache"], d["kv_indices"], d["kv_indptr"], d["kv_last_page_len"],
+                                status=status, view=view)
+    ops.raise_on_status(status)
+    ref = _reference(q.float(), k[0].to(cuda_device), v[0].to(cuda_device), G)
+    torch.testing.assert_close(out.float(), ref, rtol=2e-2, atol=2e-2)
