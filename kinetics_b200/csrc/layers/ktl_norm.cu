@@ -1,6 +1,13 @@
 // The residual stream between two sublayers in one pass over each row: the previous sublayer's output (summed over
 // its parts) is normalised and added, the new stream normalised for the next sublayer.  The stream and everything
-// computed here is fp32; one CTA per row, the row in registers, 8 elements per access.
+// computed here is fp32; a CTA has one row at a time in registers, 8 elements per access.
+//
+// Bound by DRAM for prompts, by its chain of reductions unless other rows are on their way meanwhile: a CTA walks rows and has
+// the next row's stream and output in flight (one part; several parts of a row are in flight together).  8192 rows of 2048
+// columns, 201 MB: 54 us with a CTA per row, 48 us so; with the eight parts of 64 routed experts 95 and 81 us.  More rows in
+// flight through fewer registers (spills) or with fewer threads to a row were slower.
+#include <type_traits>
+
 #include "../ktk_vec.cuh"
 #include "ktk_layers.h"
 
@@ -8,6 +15,9 @@ namespace ktk {
 
 constexpr int kRnThreads = 256;
 constexpr int kRnMaxVec = 8;      // 8 x 8 elements per thread: rows of up to 16384 columns
+// CTAs of full width that an SM holds; rows of more than 4096 columns leave no registers for the next one: a CTA for each
+__host__ __device__ constexpr int rn_resident(int nv) { return nv <= 1 ? 3 : nv <= 2 ? 2 : 1; }
+__host__ __device__ constexpr bool rn_walks(int nv) { return nv <= 2; }
 
 struct ResidualNormParams {
     const int64_t* tokens;
@@ -23,26 +33,52 @@ struct ResidualNormParams {
     void* h;
     float eps;
     int center, cols, stride;
+    int64_t rows;
     int32_t* zero;
     int zero_n;
     int32_t* status;
 };
 
-__device__ __forceinline__ float row_sum(float v, float* part) {
-    v = warp_sum_f(v);
-    const int warps = blockDim.x >> 5;
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float t = 0.0f;
-    for (int i = 0; i < warps; ++i) t += part[i];
-    __syncthreads();
-    return t;
-}
+// Sum over the CTA.  `part` has room for two sums, taken in turns: who writes one of them again has met everybody at the
+// barrier of the other.
+struct RowParts {
+    float* part;
+    int turn = 0;
+    __device__ __forceinline__ void clear() {
+        static_assert(kRnThreads == 256, "two vectors of four sums");
+        // places of absent warps: nobody else writes them, and the first sum's barrier is in front of their first reading
+        if (threadIdx.x < 2 * (kRnThreads / 32) && threadIdx.x % (kRnThreads / 32) >= blockDim.x / 32) part[threadIdx.x] = 0.0f;
+    }
+    __device__ __forceinline__ float sum(float v) {
+        float* p = part + turn * (kRnThreads / 32);
+        turn ^= 1;
+        v = warp_sum_f(v);
+        if ((threadIdx.x & 31) == 0) p[threadIdx.x >> 5] = v;
+        __syncthreads();
+        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+        return ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+    }
+};
+
+// 8 elements as they lie in memory
+template <typename T> struct Raw8;
+template <> struct Raw8<float> {
+    float4 a, b;
+    __device__ __forceinline__ void load(const float* p) { a = *reinterpret_cast<const float4*>(p); b = *(reinterpret_cast<const float4*>(p) + 1); }
+    __device__ __forceinline__ void get(float (&f)[8]) const {
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    }
+};
+template <> struct Raw8<__nv_bfloat16> {
+    uint4 a;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { a = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ void get(float (&f)[8]) const { unpack8(a, f); }
+};
 
 // v <- norm(v; w, b), in registers; elements past `cols` are zero before and after (their w and b are)
 template <int NV>
 __device__ __forceinline__ void norm_regs(float (&v)[NV][8], const float* w, const float* b, float eps, bool center,
-                                          int cols, int nvec, float* part) {
+                                          int cols, int nvec, RowParts& part) {
     float c = 0.0f;
     if (center) {
         float s = 0.0f;
@@ -50,7 +86,7 @@ __device__ __forceinline__ void norm_regs(float (&v)[NV][8], const float* w, con
         for (int i = 0; i < NV; ++i)
 #pragma unroll
             for (int e = 0; e < 8; ++e) s += v[i][e];
-        c = row_sum(s, part) / (float)cols;
+        c = part.sum(s) / (float)cols;
     }
     float ss = 0.0f;
 #pragma unroll
@@ -60,7 +96,7 @@ __device__ __forceinline__ void norm_regs(float (&v)[NV][8], const float* w, con
         for (int e = 0; e < 8; ++e)
             if (k + e < cols) { const float d = v[i][e] - c; ss += d * d; }
     }
-    const float inv = 1.0f / sqrtf(row_sum(ss, part) / (float)cols + eps);
+    const float inv = 1.0f / sqrtf(part.sum(ss) / (float)cols + eps);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int k = threadIdx.x + i * blockDim.x;
@@ -74,72 +110,94 @@ __device__ __forceinline__ void norm_regs(float (&v)[NV][8], const float* w, con
     }
 }
 
-template <typename T, int NV>
-__global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const ResidualNormParams p) {
-    __shared__ float part[kRnThreads / 32];
-    const int64_t r = blockIdx.x;
+// TOKENS: the stream starts as embedding rows
+template <typename T, int NV, bool TOKENS>
+__global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_kernel(const ResidualNormParams p) {
+    using Stream = typename std::conditional<TOKENS, T, float>::type;
+    __shared__ __align__(16) float part_s[2 * (kRnThreads / 32)];
+    RowParts part{part_s};
+    part.clear();
     const int nvec = p.stride / 8;
     if (p.zero != nullptr && blockIdx.x == 0)
         for (int i = threadIdx.x; i < p.zero_n; i += blockDim.x) p.zero[i] = 0;
-    float x[NV][8];
-    float* xrow = p.x + r * p.stride;
-    int64_t tok = 0;
-    if (p.tokens != nullptr) {
-        tok = p.tokens[r];
-        if (tok < 0 || tok >= p.vocab) {
-            if (threadIdx.x == 0) report(p.status, KTK_STATUS_BAD_TABLE);
-            tok = 0;
+    const bool one = p.y != nullptr && p.parts == 1;
+    auto token = [&](int64_t r) -> int64_t {
+        if (!TOKENS || r >= p.rows) return 0;
+        const int64_t t = p.tokens[r];
+        if (t >= 0 && t < p.vocab) return t;
+        if (threadIdx.x == 0) report(p.status, KTK_STATUS_BAD_TABLE);
+        return 0;
+    };
+    Raw8<Stream> xr[NV];
+    Raw8<T> yr[NV];
+    auto fetch = [&](int64_t r, int64_t tok) {
+        if (r >= p.rows) return;
+        const Stream* from = TOKENS ? (const Stream*)p.embed + tok * p.stride : (const Stream*)p.x + r * p.stride;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int k = threadIdx.x + i * blockDim.x;
+            if (k >= nvec) continue;
+            xr[i].load(from + k * 8);
+            if (one) yr[i].load((const T*)p.y + r * p.stride + k * 8);
         }
-    }
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int k = threadIdx.x + i * blockDim.x;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[i][e] = 0.0f;
-        if (k < nvec) {
-            if (p.tokens != nullptr) {
-                Vec8<T>::load((const T*)p.embed + tok * p.stride + k * 8, x[i]);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[i][e] *= p.embed_scale;
-            } else Vec8<float>::load(xrow + k * 8, x[i]);
-        }
-    }
-    if (p.y != nullptr) {
-        float y[NV][8];
-        const T* yrow = (const T*)p.y + r * p.parts * p.stride;
+    };
+    int64_t r = blockIdx.x;
+    fetch(r, token(r));
+    int64_t ahead = rn_walks(NV) ? token(r + gridDim.x) : 0;
+    for (; r < p.rows; r += gridDim.x) {
+        float x[NV][8], y[NV][8];
+        float* xrow = p.x + r * p.stride;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int k = threadIdx.x + i * blockDim.x;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) y[i][e] = 0.0f;
-            if (k < nvec)
+            for (int e = 0; e < 8; ++e) x[i][e] = y[i][e] = 0.0f;
+            if (k >= nvec) continue;
+            xr[i].get(x[i]);
+            if (TOKENS) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[i][e] *= p.embed_scale;
+            }
+            if (one) {
+                yr[i].get(y[i]);
+            } else if (p.y != nullptr) {
+                const T* yk = (const T*)p.y + r * p.parts * p.stride + k * 8;
+#pragma unroll 4
                 for (int j = 0; j < p.parts; ++j) {
                     float t[8];
-                    Vec8<T>::load(yrow + (int64_t)j * p.stride + k * 8, t);
+                    Vec8<T>::load(yk + (int64_t)j * p.stride, t);
 #pragma unroll
                     for (int e = 0; e < 8; ++e) y[i][e] += t[e];
                 }
+            }
         }
-        if (p.post_w != nullptr) norm_regs<NV>(y, p.post_w, p.post_b, p.eps, p.center != 0, p.cols, nvec, part);
-#pragma unroll
-        for (int i = 0; i < NV; ++i)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) x[i][e] += p.mult * y[i][e];
-    }
-    if (p.y != nullptr || p.tokens != nullptr) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int k = threadIdx.x + i * blockDim.x;
-            if (k < nvec) Vec8<float>::store(xrow + k * 8, x[i]);
+        if (rn_walks(NV)) {
+            fetch(r + gridDim.x, ahead);
+            ahead = token(r + 2 * (int64_t)gridDim.x);
         }
-    }
-    if (p.h != nullptr) {
-        if (p.pre_w != nullptr) norm_regs<NV>(x, p.pre_w, p.pre_b, p.eps, p.center != 0, p.cols, nvec, part);
+        if (p.y != nullptr) {
+            if (p.post_w != nullptr) norm_regs<NV>(y, p.post_w, p.post_b, p.eps, p.center != 0, p.cols, nvec, part);
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int k = threadIdx.x + i * blockDim.x;
-            if (k < nvec) Vec8<T>::store((T*)p.h + r * p.stride + k * 8, x[i]);
+            for (int i = 0; i < NV; ++i)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[i][e] += p.mult * y[i][e];
         }
+        if (TOKENS || p.y != nullptr) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const int k = threadIdx.x + i * blockDim.x;
+                if (k < nvec) Vec8<float>::store(xrow + k * 8, x[i]);
+            }
+        }
+        if (p.h != nullptr) {
+            if (p.pre_w != nullptr) norm_regs<NV>(x, p.pre_w, p.pre_b, p.eps, p.center != 0, p.cols, nvec, part);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const int k = threadIdx.x + i * blockDim.x;
+                if (k < nvec) Vec8<T>::store((T*)p.h + r * p.stride + k * 8, x[i]);
+            }
+        }
+        if (!rn_walks(NV)) break;
     }
 }
 
@@ -148,11 +206,14 @@ static int residual_norm_launch(const ResidualNormParams& p, int64_t rows, cudaS
     const int nvec = p.stride / 8;
     const int threads = nvec >= kRnThreads ? kRnThreads : (nvec + 31) / 32 * 32;
     const int nv = (nvec + threads - 1) / threads;
-    const unsigned grid = (unsigned)rows;
-    if (nv <= 1) residual_norm_kernel<T, 1><<<grid, threads, 0, st>>>(p);
-    else if (nv <= 2) residual_norm_kernel<T, 2><<<grid, threads, 0, st>>>(p);
-    else if (nv <= 4) residual_norm_kernel<T, 4><<<grid, threads, 0, st>>>(p);
-    else residual_norm_kernel<T, kRnMaxVec><<<grid, threads, 0, st>>>(p);
+    // a row per CTA; beyond what the SMs hold the CTAs walk
+    const int64_t most = (int64_t)sm_count() * rn_resident(nv) * (kRnThreads / threads);
+    const unsigned grid = (unsigned)(rows < most || !rn_walks(nv) ? rows : most);
+    auto kernel = nv <= 1 ? (p.tokens ? residual_norm_kernel<T, 1, true> : residual_norm_kernel<T, 1, false>)
+                : nv <= 2 ? (p.tokens ? residual_norm_kernel<T, 2, true> : residual_norm_kernel<T, 2, false>)
+                : nv <= 4 ? (p.tokens ? residual_norm_kernel<T, 4, true> : residual_norm_kernel<T, 4, false>)
+                          : (p.tokens ? residual_norm_kernel<T, kRnMaxVec, true> : residual_norm_kernel<T, kRnMaxVec, false>);
+    kernel<<<grid, threads, 0, st>>>(p);
     KTK_CUDA_TRY(cudaGetLastError(), "ktk_residual_norm");
     return KTK_OK;
 }
@@ -186,7 +247,7 @@ extern "C" int ktk_residual_norm(const int64_t* tokens, const void* embed, int64
                          (uintptr_t)pre_w | (uintptr_t)pre_b | (uintptr_t)h;
     if ((al & 15u) != 0) { set_error("%s: pointers must be 16-byte aligned", who); return KTK_ERR_ARG; }
     const ResidualNormParams p{tokens, embed, vocab, embed_scale, x, y, parts, post_w, post_b, mult, pre_w, pre_b, h, eps,
-                               center, cols, stride, zero, zero ? zero_n : 0, status};
+                               center, cols, stride, rows, zero, zero ? zero_n : 0, status};
     return dtype == KTK_F32 ? residual_norm_launch<float>(p, rows, (cudaStream_t)stream)
                             : residual_norm_launch<__nv_bfloat16>(p, rows, (cudaStream_t)stream);
 }
