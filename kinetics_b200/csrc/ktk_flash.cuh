@@ -33,9 +33,11 @@ constexpr float kFlMost = 1073741824.0f;     // 2^30: the exponentials' referenc
 constexpr int kFlMaxSmem = 225 * 1024;       // dynamic; the barriers are static
 
 // Registers: 384 threads start with 168 each (64512 of the SM's); the softmax holds a row of scores, so its two warpgroups go
-// to 200 and the third to 104: 256 * 200 + 128 * 104 = 64512.  Every warp of a warpgroup calls the one of its role.
+// to 200 and the third to 104: 256 * 200 + 128 * 104 = 64512.  All warps of a warpgroup have to execute the same instruction:
+// each stands once in a kernel, on a branch that whole warpgroups take, and the third one's roles part behind it.
 __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 200;"); }
 __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 104;"); }
+constexpr int kFlSoftmaxWarps = 8;
 
 // -inf where no key has been seen: the exponentials then refer to 0
 __device__ __forceinline__ float reference_or_zero(float m) { return m == -INFINITY ? 0.0f : m; }

@@ -84,45 +84,44 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
     __syncthreads();
     tc_fence_after();
 
-    if (warp == 8) {
+    if (warp >= kFlSoftmaxWarps) {
         fewer_registers();
-        fl.issue([](int) { return 4; }, 0, kHeadDim);
-    } else if (warp == 9) {
-        fewer_registers();
-        // lane i < 8: page i of a block; entries are read one block ahead of their first use
-        auto entry = [&](int blk) {
-            const int e = blk * kPuPages + lane;
-            return lane < kPuPages && e < n_need ? p.kv_indices[sp.start + e] : -1;
-        };
-        int at[3] = {entry(0), entry(1), entry(2)}, first = 0;        // of blocks first, first + 1, first + 2
-        auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
-            while (first + 2 < blk || (which && first < blk)) {
-                at[0] = at[1];
-                at[1] = at[2];
-                ++first;
-                at[2] = entry(first + 2);
-            }
-            const int pg = blk == first ? at[0] : (blk == first + 1 ? at[1] : at[2]);
-            const bool on = pg >= 0 && pg < p.num_pages;
-            if (which == 0 && !on && lane < kPuPages && blk * kPuPages + lane < n_need) report(p.status, KTK_STATUS_BAD_PAGE);
-            const uint32_t pages = __popc(__ballot_sync(0xffffffffu, on));
-            if (lane == 0) {
-                if (pages) mbar_arrive_expect_tx(bar, pages * (2u * kPageSize * 128u));
-                else mbar_arrive(bar);
-            }
-            __syncwarp();
-            if (on) {
-                const int z = pg * (2 * kPageSize) + which * kPageSize;      // token row of slot 0
-                tma_load_3d(dst + lane * (kPageSize * 128), &kv_map, bar, 0, h, z);
-                tma_load_3d(dst + PrefillFlash::kTile + lane * (kPageSize * 128), &kv_map, bar, 64, h, z);
-            }
-            __syncwarp();
-        };
-        if (lane == 0) prefetch_tensormap(&kv_map);
-        fl.copy([&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); },
-                [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); });
-    } else if (warp >= 10) {
-        fewer_registers();
+        if (warp == 8) {
+            fl.issue([](int) { return 4; }, 0, kHeadDim);
+        } else if (warp == 9) {
+            // lane i < 8: page i of a block; entries are read one block ahead of their first use
+            auto entry = [&](int blk) {
+                const int e = blk * kPuPages + lane;
+                return lane < kPuPages && e < n_need ? p.kv_indices[sp.start + e] : -1;
+            };
+            int at[3] = {entry(0), entry(1), entry(2)}, first = 0;        // of blocks first, first + 1, first + 2
+            auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
+                while (first + 2 < blk || (which && first < blk)) {
+                    at[0] = at[1];
+                    at[1] = at[2];
+                    ++first;
+                    at[2] = entry(first + 2);
+                }
+                const int pg = blk == first ? at[0] : (blk == first + 1 ? at[1] : at[2]);
+                const bool on = pg >= 0 && pg < p.num_pages;
+                if (which == 0 && !on && lane < kPuPages && blk * kPuPages + lane < n_need) report(p.status, KTK_STATUS_BAD_PAGE);
+                const uint32_t pages = __popc(__ballot_sync(0xffffffffu, on));
+                if (lane == 0) {
+                    if (pages) mbar_arrive_expect_tx(bar, pages * (2u * kPageSize * 128u));
+                    else mbar_arrive(bar);
+                }
+                __syncwarp();
+                if (on) {
+                    const int z = pg * (2 * kPageSize) + which * kPageSize;      // token row of slot 0
+                    tma_load_3d(dst + lane * (kPageSize * 128), &kv_map, bar, 0, h, z);
+                    tma_load_3d(dst + PrefillFlash::kTile + lane * (kPageSize * 128), &kv_map, bar, 64, h, z);
+                }
+                __syncwarp();
+            };
+            if (lane == 0) prefetch_tensormap(&kv_map);
+            fl.copy([&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); },
+                    [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); });
+        }
     } else {
         more_registers();
         const int tile_min_vis = base_pos + tok0 + tile * tpc + 1;

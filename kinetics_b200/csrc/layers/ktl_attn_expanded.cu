@@ -79,42 +79,41 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bu
     __syncthreads();
     tc_fence_after();
 
-    if (warp == 8) {
+    if (warp >= kFlSoftmaxWarps) {
         fewer_registers();
-        const int ksteps = (a.dim_stride + 15) / 16, rsteps = (a.rot_stride + 15) / 16;
-        fl.issue([&](int c) { return c < nc ? (ksteps - 4 * c < 4 ? ksteps - 4 * c : 4)
-                                            : (rsteps - 4 * (c - nc) < 4 ? rsteps - 4 * (c - nc) : 4); },
-                 0, (a.vdim_stride + 15) / 16 * 16);
-    } else if (warp == 9) {
-        fewer_registers();
-        if (elect_one()) {
-            prefetch_tensormap(&k_map);
-            prefetch_tensormap(&r_map);
-            prefetch_tensormap(&v_map);
-        }
-        __syncwarp();
-        // columns and tokens outside come as zeros
-        fl.copy(
-            [&](int blk, uint8_t* dst, uint64_t* bar) {
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(bar, (uint32_t)(dc * F::kTile));
-                    for (int c = 0; c < dc; ++c) {
-                        if (c < nc) tma_load_3d(dst + c * F::kTile, &k_map, bar, c * 64, head, blk * KEYS);
-                        else tma_load_3d(dst + c * F::kTile, &r_map, bar, (c - nc) * 64, 0, blk * KEYS);
+        if (warp == 8) {
+            const int ksteps = (a.dim_stride + 15) / 16, rsteps = (a.rot_stride + 15) / 16;
+            fl.issue([&](int c) { return c < nc ? (ksteps - 4 * c < 4 ? ksteps - 4 * c : 4)
+                                                : (rsteps - 4 * (c - nc) < 4 ? rsteps - 4 * (c - nc) : 4); },
+                     0, (a.vdim_stride + 15) / 16 * 16);
+        } else if (warp == 9) {
+            if (elect_one()) {
+                prefetch_tensormap(&k_map);
+                prefetch_tensormap(&r_map);
+                prefetch_tensormap(&v_map);
+            }
+            __syncwarp();
+            // columns and tokens outside come as zeros
+            fl.copy(
+                [&](int blk, uint8_t* dst, uint64_t* bar) {
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(bar, (uint32_t)(dc * F::kTile));
+                        for (int c = 0; c < dc; ++c) {
+                            if (c < nc) tma_load_3d(dst + c * F::kTile, &k_map, bar, c * 64, head, blk * KEYS);
+                            else tma_load_3d(dst + c * F::kTile, &r_map, bar, (c - nc) * 64, 0, blk * KEYS);
+                        }
                     }
-                }
-                __syncwarp();
-            },
-            [&](int blk, uint8_t* dst, uint64_t* bar) {
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(bar, (uint32_t)F::kVBuf);
-#pragma unroll
-                    for (int c = 0; c < VC; ++c) tma_load_3d(dst + c * F::kTile, &v_map, bar, c * 64, head, blk * KEYS);
-                }
-                __syncwarp();
-            });
-    } else if (warp >= 10) {
-        fewer_registers();
+                    __syncwarp();
+                },
+                [&](int blk, uint8_t* dst, uint64_t* bar) {
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(bar, (uint32_t)F::kVBuf);
+    #pragma unroll
+                        for (int c = 0; c < VC; ++c) tma_load_3d(dst + c * F::kTile, &v_map, bar, c * 64, head, blk * KEYS);
+                    }
+                    __syncwarp();
+                });
+        }
     } else {
         more_registers();
         const int tile_min_vis = base + tok0 + tile * kUmRows + 1;

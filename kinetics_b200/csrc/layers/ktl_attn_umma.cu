@@ -78,45 +78,44 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     __syncthreads();
     tc_fence_after();
 
-    if (warp == 8) {
+    if (warp >= kFlSoftmaxWarps) {
         fewer_registers();
-        const int ksteps = (a.dim_stride + 15) / 16;
-        fl.issue([&](int c) { return ksteps - 4 * c < 4 ? ksteps - 4 * c : 4; }, DC * F::kTile, (a.vdim_stride + 15) / 16 * 16);
-    } else if (warp == 9) {
-        fewer_registers();
-        // a box is a page of one head (of one map); lane i: page i of a block
-        const int pages = kAuKeys / ps, box = ps * 128;
-        auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
-            const int tok = blk * kAuKeys + lane * ps;
-            const int64_t pg = lane < pages && tok < seen ? p.t.kv_indices[s.start + tok / ps] : -1;
-            const bool on = pg >= 0 && pg < p.t.num_pages;
-            if (lane < pages && tok < seen && !on) report(p.status, KTK_STATUS_BAD_PAGE);
-            const uint32_t n = __popc(__ballot_sync(0xffffffffu, on));
+        if (warp == 8) {
+            const int ksteps = (a.dim_stride + 15) / 16;
+            fl.issue([&](int c) { return ksteps - 4 * c < 4 ? ksteps - 4 * c : 4; }, DC * F::kTile, (a.vdim_stride + 15) / 16 * 16);
+        } else if (warp == 9) {
+            // a box is a page of one head (of one map); lane i: page i of a block
+            const int pages = kAuKeys / ps, box = ps * 128;
+            auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
+                const int tok = blk * kAuKeys + lane * ps;
+                const int64_t pg = lane < pages && tok < seen ? p.t.kv_indices[s.start + tok / ps] : -1;
+                const bool on = pg >= 0 && pg < p.t.num_pages;
+                if (lane < pages && tok < seen && !on) report(p.status, KTK_STATUS_BAD_PAGE);
+                const uint32_t n = __popc(__ballot_sync(0xffffffffu, on));
+                if (lane == 0) {
+                    if (n) mbar_arrive_expect_tx(bar, n * (uint32_t)((which ? VC : 2 * DC) * box));
+                    else mbar_arrive(bar);
+                }
+                __syncwarp();
+                if (on && which) {
+    #pragma unroll
+                    for (int c = 0; c < VC; ++c)
+                        tma_load_3d(dst + c * F::kTile + lane * box, &v_map, bar, c * 64, 0, (int)(pg * a.kv_heads) + kvh);
+                } else if (on) {
+    #pragma unroll
+                    for (int mc = 0; mc < 2 * DC; ++mc)
+                        tma_load_3d(dst + mc * F::kTile + lane * box, &k_map, bar, (mc % DC) * 64, 0,
+                                    (int)(pg * (2 * a.kv_heads)) + kvh * 2 + mc / DC);
+                }
+                __syncwarp();
+            };
             if (lane == 0) {
-                if (n) mbar_arrive_expect_tx(bar, n * (uint32_t)((which ? VC : 2 * DC) * box));
-                else mbar_arrive(bar);
+                prefetch_tensormap(&k_map);
+                prefetch_tensormap(&v_map);
             }
-            __syncwarp();
-            if (on && which) {
-#pragma unroll
-                for (int c = 0; c < VC; ++c)
-                    tma_load_3d(dst + c * F::kTile + lane * box, &v_map, bar, c * 64, 0, (int)(pg * a.kv_heads) + kvh);
-            } else if (on) {
-#pragma unroll
-                for (int mc = 0; mc < 2 * DC; ++mc)
-                    tma_load_3d(dst + mc * F::kTile + lane * box, &k_map, bar, (mc % DC) * 64, 0,
-                                (int)(pg * (2 * a.kv_heads)) + kvh * 2 + mc / DC);
-            }
-            __syncwarp();
-        };
-        if (lane == 0) {
-            prefetch_tensormap(&k_map);
-            prefetch_tensormap(&v_map);
+            fl.copy([&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); },
+                    [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); });
         }
-        fl.copy([&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); },
-                [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); });
-    } else if (warp >= 10) {
-        fewer_registers();
     } else {
         more_registers();
         const float factor = a.scale * query_temperature(a.temp_coef, a.temp_every, vis > 0 ? vis - 1 : 0);
