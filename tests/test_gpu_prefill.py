@@ -126,7 +126,7 @@ def test_prefill_on_block_and_tile_edges(cuda_device, variant, G, sink):
 
 @pytest.mark.parametrize("G,sink,grow", [(4, 0, (0.1, 40.0, 200.0)), (1, 4, (1.0, 1.0, 90.0)), (2, 0, (60.0, 0.1, 30.0))])
 def test_prefill_scores_that_outgrow_their_reference(cuda_device, G, sink, grow):
-    """The exponentials' reference is the first block's maximum until a half block's sum passes 2^30: scores that grow by far
+    """The exponentials' reference is the first block's maximum until a half block's sum passes 2^8: scores that grow by far
     more in the first half of a block of 128 keys, in its second half, in the block of the row itself; and that shrink.
 
     Bound: operands are the reference's own bf16 values, products of 128 columns are summed in fp32, so a score of up to about
@@ -151,3 +151,45 @@ def test_prefill_scores_that_outgrow_their_reference(cuda_device, G, sink, grow)
     ops.raise_on_status(status)
     ref = _reference(q.float(), k[0].to(cuda_device), v[0].to(cuda_device), G)
     torch.testing.assert_close(out.float(), ref, rtol=2e-2, atol=2e-2)
+
+
+def _attend_exponents(dev, exponents, v, n, G=4):
+    """Attention of the last n tokens over keys whose weights are 2^exponent for every query: q = (1, 2^-8, 0, ..), k = (whole
+    part, 256 times the rest, 0, ..), both exact in bf16; sm_scale = ln 2."""
+    from kinetics_b200 import ops
+    e = torch.tensor(exponents)
+    k = torch.zeros(1, 1, len(exponents), 128)
+    k[0, 0, :, 0], k[0, 0, :, 1] = e.floor(), (e - e.floor()) * 256
+    assert torch.equal(k.to(torch.bfloat16).float(), k)
+    d = to_dev(paged_state(k, v, [len(exponents)], torch.bfloat16, seed=3), dev)
+    q = torch.zeros(n, G, 128, dtype=torch.bfloat16, device=dev)
+    q[..., 0], q[..., 1] = 1.0, 2.0 ** -8
+    status = ops.new_status(dev)
+    out = ops.prefill_attention(q, torch.tensor([0, n], dtype=torch.int32, device=dev), n, d["kv_cache"], d["kv_indices"],
+                                d["kv_indptr"], d["kv_last_page_len"], sm_scale=math.log(2.0), status=status)
+    ops.raise_on_status(status)
+    return out.float().cpu()
+
+
+#: 2^0.005615 = 1.0039: half way between two bf16 numbers, so that a weight of that mantissa is off by 2^-8 of itself in bf16
+HALF_WAY = 1.4375 / 256
+
+
+@pytest.mark.parametrize("at", [5, 100, 140, 200, 396])
+def test_prefill_a_key_that_outweighs_all_others(cuda_device, at):
+    """Its weight is 2^28 of the others': the row is its value, whose bf16 form the result is to the bit (400 others change it by
+    less than 2^-19 of their size)."""
+    exponents = [0.0] * 400
+    exponents[at] = 28.0 + HALF_WAY
+    v = torch.randn(1, 1, 400, 128, generator=torch.Generator().manual_seed(at)).to(torch.bfloat16).float()
+    v += v.sign() * 0.5                                      # no value so small that the others matter in its last bit
+    v = v.to(torch.bfloat16).float()
+    out = _attend_exponents(cuda_device, exponents, v, 4)
+    assert torch.equal(out, v[0, 0, at].expand_as(out))
+
+
+def test_prefill_values_near_the_end_of_the_range(cuda_device):
+    """Values of 2^104 behind scores that grow by 22: 8192 keys of weight 2^8 leave 2^107."""
+    v = torch.full((1, 1, 400, 128), 2.0 ** 104)
+    out = _attend_exponents(cuda_device, [0.0] * 150 + [22.0] * 100 + [0.0] * 150, v, 4)
+    assert torch.equal(out, torch.full_like(out, 2.0 ** 104))
