@@ -198,10 +198,10 @@ template <int KEYS, int VC> struct Flash {
     // whether form(x, y) is still to be applied to every pair of them.  The exponents are s f (FIXED: s) against m_ref.
     // clear(j): rows of V(j) that hold no key.  Returns whether O is complete.
     //
-    // The reference is the sink or the first block's maximum, and stays while no half block's sum passes 2^8 (or is infinite); then
-    // it is that half's maximum.  So no other block's maximum has to be searched, which cost 500 of a block's 3400 cycles.  A weight
-    // of 2^8 or more becomes 1, which bf16 holds exactly: the row of a key that outweighs all others is that key's value.  And
-    // |O| <= 2^8 max|V| per 64 keys: 8192 keys leave |V| 2^113 (1e34) of the range of fp32.
+    // The reference is the larger of the sink and the first block's maximum, and stays while no half block's sum passes 2^8 (or is
+    // infinite); then it is that half's maximum.  So no other block's maximum has to be searched, which cost 500 of a block's 3400
+    // cycles.  A weight of 2^8 or more becomes 1, which bf16 holds exactly: the row of a key that outweighs all others is that
+    // key's value.  And |O| <= 2^8 max|V| per 64 keys: 8192 keys leave |V| 2^113 (1e34) of the range of fp32.
     // The halves of a block are handed over one by one: 521 us for the prompt of 8192 tokens and 32 heads without that, 498 with it.
     template <bool FIXED, class Prepare, class Form, class Clear>
     __device__ __forceinline__ bool softmax(int m, float f, float& m_ref, float& l_run, Prepare prepare, Form form, Clear clear) {
@@ -277,7 +277,7 @@ template <int KEYS, int VC> struct Flash {
                 }
             };
             // the votes: tensor memory is read and written by whole warps
-            if (!FIXED && __any_sync(0xffffffffu, m_ref == -INFINITY)) move(0, m_ref == -INFINITY, j > 0);
+            if (!FIXED && (j == 0 || __any_sync(0xffffffffu, m_ref == -INFINITY))) move(0, j == 0 || m_ref == -INFINITY, j > 0);
             half(0);
             if (!FIXED) {
                 const bool over = total() > kFlMost;

@@ -1,5 +1,7 @@
 """Attention over rows that all heads share (value = first columns of the key), its append step and the linear
 recurrence on the GPU, each against its plain formula: sizes, page sizes, far keys, edges, portions, splits."""
+import math
+
 import pytest
 import torch
 
@@ -162,6 +164,45 @@ def test_expanded_scores_far_from_the_sink(cuda_device, dim, sink):
             (plain.sink_softmax(s, torch.tensor(sink, dtype=torch.float64), 0) @ r64(values[:, h]))
         err = (got[:, h] - want).pow(2).mean(-1).sqrt()
         assert err.max() < 3e-2, (h, float(err.max()))
+
+
+def _expand_exponents(dev, exponents, values, n, dim, sink_exponent=0.0):
+    """Attention of the last n tokens, one head of dim + 64 columns, over keys whose weights are 2^exponent for every query, beside
+    a sink of 2^sink_exponent: q = (1, 2^-8, 0, ..), k = (whole part, 256 times the rest, 0, ..), both exact in bf16."""
+    from kinetics_b200 import layer_ops as lo, ops
+    from kinetics_b200.layer_ops import LatentSpec, Rotation
+    spec, e, ln2 = LatentSpec(1, dim, 64, 128, 48, math.log(2.0), Rotation(64, 1e4)), torch.tensor(exponents), math.log(2.0)
+    proj = torch.zeros(n, spec.proj_cols, dtype=BF, device=dev)
+    proj[:, 0], proj[:, 1] = 1.0, 2.0 ** -8
+    kv = torch.zeros(len(exponents), dim + 128)
+    kv[:, 0], kv[:, 1], kv[:, dim:] = e.floor(), (e - e.floor()) * 256, values
+    assert torch.equal(kv.to(BF).float(), kv)
+    status = ops.new_status(dev)
+    out = lo.expanded_attention(proj, kv.to(BF).to(dev), torch.zeros(len(exponents), 48 + 64, dtype=BF, device=dev), spec,
+                                torch.tensor([sink_exponent * ln2], device=dev), None, status)
+    ops.raise_on_status(status)
+    return out.view(n, 128).double().cpu()
+
+
+@pytest.mark.parametrize("at,dim", [(3, 128), (60, 128), (100, 128), (3, 192), (60, 192)])
+def test_expanded_key_above_the_sink(cuda_device, at, dim):
+    """One key of the first block outweighs the other keys by 2^40 and the sink by 2^7: the row is its value by 1 / (1 + 2^-7).
+    Bound: the nearest bf16 number of a value within 2^-15 of it (fp32 sums, the sink's exponential; rounding is monotonic); a weight
+    of half-way mantissa would be off by 2^-8 in bf16, as much as an ulp of the result."""
+    exponents = [-33.0] * 400
+    exponents[at] = 7.0 + 1.4375 / 256
+    values = torch.randn(400, 128, generator=torch.Generator().manual_seed(at)).to(BF).float()
+    out = _expand_exponents(cuda_device, exponents, values, 4, dim)
+    want = values[at].double() / (1.0 + 2.0 ** -exponents[at])
+    ends = torch.stack([(want * (1 + d)).to(BF).double() for d in (-2.0 ** -15, 2.0 ** -15)])
+    assert ((out >= ends.amin(0)) & (out <= ends.amax(0))).all(), float(((out - want) / want).abs().max())
+
+
+@pytest.mark.parametrize("dim", [128, 192])
+def test_expanded_values_near_the_end_of_the_range(cuda_device, dim):
+    """Values of 2^104 behind scores 22 above the sink: the sums of weighted values stay in the range of fp32."""
+    out = _expand_exponents(cuda_device, [22.0] * 400, torch.full((400, 128), 2.0 ** 104), 4, dim)
+    assert torch.equal(out, torch.full_like(out, 2.0 ** 104))
 
 
 @pytest.mark.parametrize("dtype", [F32, BF])
