@@ -277,7 +277,8 @@ template <int KEYS, int VC> struct Flash {
                 }
             };
             // the votes: tensor memory is read and written by whole warps
-            if (!FIXED && (j == 0 || __any_sync(0xffffffffu, m_ref == -INFINITY))) move(0, j == 0 || m_ref == -INFINITY, j > 0);
+            // Rows that have seen no key hold an O of zeros.
+            if (!FIXED && (j == 0 || __any_sync(0xffffffffu, m_ref == -INFINITY))) move(0, j == 0 || m_ref == -INFINITY, false);
             half(0);
             if (!FIXED) {
                 const bool over = total() > kFlMost;

@@ -199,6 +199,31 @@ def test_scores_beyond_the_polynomial_range(cuda_device):
         _close(*_run(cuda_device, spec, [200, 90], None, 64, MMA, torch.bfloat16, strength=strength), torch.bfloat16)
 
 
+@pytest.mark.parametrize("vdim", [64, 128])
+@pytest.mark.parametrize("cap", [0.0, 90.0])
+@pytest.mark.parametrize("first, n, grown, maps", [(60, 100, (130, 150), (0, 1)), (60, 100, (130, 150), (1,)), (330, 200, (192, 200), (0,)),
+                                                   (330, 200, (140, 236), (0, 1)), (0, 300, (128, 290), (1,))])
+def test_scores_that_outgrow_their_reference(cuda_device, vdim, cap, first, n, grown, maps):
+    """Without a softcap below 60 the exponentials' reference moves where half a block's sum passes 2^8.  Keys that grow thirtyfold in
+    the first half of a later block, in its second half, over blocks, in one of the two maps; the first cases' tile has rows without
+    a token, whose first block is masked.  Bound: that of the other prompts (bf16 probabilities and outputs of size one)."""
+    from kinetics_b200 import layer_ops as lo, ops
+    spec, total = _spec(2, 2, 64, vdim, cap=cap), first + n
+    g = torch.Generator().manual_seed(first + vdim)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    q, k, v = rnd(n, 2, 2, 64), 0.2 * rnd(total, 2, 2, 64), rnd(total, 2, vdim).to(torch.bfloat16).float()
+    for m in maps:
+        k[grown[0]:grown[1], :, m] *= 30.0
+    q, k = q.to(torch.bfloat16).float(), k.to(torch.bfloat16).float()
+    case = PagedCase([k], [v], torch.bfloat16, 64, cuda_device)
+    indptr = torch.tensor([0, n], dtype=torch.int32, device=cuda_device)
+    status = ops.new_status(cuda_device)
+    got = lo.paged_attention(pad_q(q, cuda_device, torch.bfloat16), case.k, case.v, case.table, spec, indptr, n, variant=UMMA,
+                             status=status).view(n, 2, vdim).cpu().double()
+    assert int(status.item()) == 0
+    _close(got, plain_attention(q, k, v, spec, first), torch.bfloat16)
+
+
 def test_a_sequence_alone_and_in_a_batch_and_cut_differently(cuda_device):
     # the same rows, computed in other company, other portions and other pages
     from kinetics_b200 import layer_ops as lo
