@@ -78,11 +78,12 @@ template <int KEYS, int VC> struct Flash {
     uint8_t *q, *k, *v;                                  // [tile][chunk] | [buffer][chunk] | [buffer][chunk]
     int q_chunks, k_chunks;                              // 64-column chunks of a tile's queries, of a block of K
     int nv;                                              // buffers of V: 1 or 2
-    int blocks0, blocks1;                                // blocks that each tile sees
+    int keys0, keys1;                                    // key columns up to the last one that some row of each tile sees
+    int blocks0, blocks1;                                // blocks that hold them
 
-    __device__ __forceinline__ Flash(FlashShared& shared, uint8_t* smem, int qc, int kc, int v_bufs, int b0, int b1)
+    __device__ __forceinline__ Flash(FlashShared& shared, uint8_t* smem, int qc, int kc, int v_bufs, int n0, int n1)
         : sh(shared), q(smem), k(smem + 2 * qc * kFlQTile), v(k + 2 * kc * kTile), q_chunks(qc), k_chunks(kc), nv(v_bufs),
-          blocks0(b0), blocks1(b1) {}
+          keys0(n0), keys1(n1), blocks0((n0 + KEYS - 1) / KEYS), blocks1((n1 + KEYS - 1) / KEYS) {}
     __host__ __device__ static constexpr int bytes(int qc, int kc, int v_bufs) {
         return 2 * qc * kFlQTile + 2 * kc * kTile + v_bufs * kVBuf;
     }
@@ -137,6 +138,8 @@ template <int KEYS, int VC> struct Flash {
             for (int m = 0; m < 2; ++m) {
                 const int mine = blocks_of(m);
                 if (j < mine) {
+                    // values behind the last key that the tile sees are left out: 0 times one that is not finite is not 0
+                    const int n_steps = ((m ? keys1 : keys0) - j * KEYS + 15) / 16;
                     // the first half of the block's keys while the threads work on the second
 #pragma unroll
                     for (int part = 0; part < 2; ++part) {
@@ -144,8 +147,9 @@ template <int KEYS, int VC> struct Flash {
                         if (elect_one()) {
 #pragma unroll
                             for (int i = part * (kHalf / 16); i < (part + 1) * (kHalf / 16); ++i)
-                                umma_f16_ts(tmem + kFlColO + m * 128, tmem + m * 128 + i * 8, umma_desc_at(va, i * (16 * 128)), idesc_o,
-                                            (j > 0 || i > 0) ? 1u : 0u);
+                                if (i < n_steps)
+                                    umma_f16_ts(tmem + kFlColO + m * 128, tmem + m * 128 + i * 8, umma_desc_at(va, i * (16 * 128)),
+                                                idesc_o, (j > 0 || i > 0) ? 1u : 0u);
                             if (part == 0) umma_commit(&sh.o_half[m]);
                             else if (j + 1 == mine) umma_commit(&sh.o[m]);
                         }

@@ -45,16 +45,16 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
         return;
     }
     const int shift = kPageSize - sp.first_fill;    // slots of the first page that never hold a token
-    int blocks[2], n_need = 0;                      // blocks of each tile; pages that the last row sees
+    int keys[2], n_need = 0;                        // key columns of each tile; pages that the last row sees
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
         const int t0 = tok0 + m * tpc, t1 = t0 + tpc < n_new ? t0 + tpc : n_new;
-        blocks[m] = 0;
+        keys[m] = 0;
         if (t0 < n_new) {
             int unused;
             pages_for(base_pos + t1, sp.first_fill, n_need, unused);
             if (n_need > sp.n_pages) n_need = sp.n_pages;
-            blocks[m] = (n_need + kPuPages - 1) / kPuPages;
+            keys[m] = n_need * kPageSize;
         }
     }
 
@@ -64,7 +64,7 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
     const bool row_on = warp < 8 && my_tok < n_new;
     const int vis = row_on ? base_pos + my_tok + 1 : 0;     // keys at positions < vis are seen
 
-    Flash<kPuKeys, kHeadDim / 64> fl(sh, sm, 2, 2, kPuBufs, blocks[0], blocks[1]);
+    Flash<kPuKeys, kHeadDim / 64> fl(sh, sm, 2, 2, kPuBufs, keys[0], keys[1]);
     if (tid == 0) sh.init();
     if (warp < 8) {
         // Q row -> two swizzled chunks (zeros for rows past the last new token)

@@ -48,18 +48,18 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bu
     const int head = head0 + at % here;
     const int tok0 = (pairs - 1 - at / here) * 2 * kUmRows;
     const int base = p.total - p.n;
-    int blocks[2];                                      // key blocks of each tile
+    int keys[2];                                        // keys of each tile
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
         const int t0 = tok0 + m * kUmRows, t1 = t0 + kUmRows < p.n ? t0 + kUmRows : p.n;
-        blocks[m] = t0 < p.n ? (base + t1 + KEYS - 1) / KEYS : 0;
+        keys[m] = t0 < p.n ? base + t1 : 0;
     }
     const int tile = warp >> 2, row = tid & (kUmRows - 1);
     const int tok = tok0 + tile * kUmRows + row;
     const bool row_on = warp < 8 && tok < p.n;
     const int vis = row_on ? base + tok + 1 : 0;        // keys at positions < vis are seen
 
-    F fl(sh, sm, dc, dc, v_bufs, blocks[0], blocks[1]);
+    F fl(sh, sm, dc, dc, v_bufs, keys[0], keys[1]);
     if (tid == 0) sh.init();
     if (warp < 8) {
         const __nv_bfloat16* src = p.q + (int64_t)(row_on ? tok : 0) * p.q_stride + (int64_t)head * (a.dim_stride + a.rot_stride);

@@ -50,7 +50,6 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     }
     const int tok_hi = (tok0 + tpc < n_new ? tok0 + tpc : n_new) - 1;
     const int seen = base_pos + tok_hi + 1;             // keys the tile's last row sees
-    const int n_blocks = (seen + kAuKeys - 1) / kAuKeys;
     const int ps = p.t.page_size;
 
     const int map = warp >> 2, row = tid & (kUmRows - 1);
@@ -58,7 +57,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     const bool row_on = warp < 8 && row / group < tpc && my_tok < n_new;
     const int vis = row_on ? base_pos + my_tok + 1 : 0; // keys at positions < vis are seen
 
-    F fl(sh, sm, DC, 2 * DC, kBufs, n_blocks, n_blocks);
+    F fl(sh, sm, DC, 2 * DC, kBufs, seen, seen);
     if (tid == 0) sh.init();
     if (warp < 8) {
         const uint4* src = reinterpret_cast<const uint4*>(

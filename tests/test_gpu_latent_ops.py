@@ -176,7 +176,7 @@ def _expand_exponents(dev, exponents, values, n, dim, sink_exponent=0.0):
     proj[:, 0], proj[:, 1] = 1.0, 2.0 ** -8
     kv = torch.zeros(len(exponents), dim + 128)
     kv[:, 0], kv[:, 1], kv[:, dim:] = e.floor(), (e - e.floor()) * 256, values
-    assert torch.equal(kv.to(BF).float(), kv)
+    assert torch.equal(kv[:, :dim].to(BF).float(), kv[:, :dim])
     status = ops.new_status(dev)
     out = lo.expanded_attention(proj, kv.to(BF).to(dev), torch.zeros(len(exponents), 48 + 64, dtype=BF, device=dev), spec,
                                 torch.tensor([sink_exponent * ln2], device=dev), None, status)
@@ -203,6 +203,20 @@ def test_expanded_values_near_the_end_of_the_range(cuda_device, dim):
     """Values of 2^104 behind scores 22 above the sink: the sums of weighted values stay in the range of fp32."""
     out = _expand_exponents(cuda_device, [22.0] * 400, torch.full((400, 128), 2.0 ** 104), 4, dim)
     assert torch.equal(out, torch.full_like(out, 2.0 ** 104))
+
+
+@pytest.mark.parametrize("dim", [128, 192])
+def test_expanded_rows_of_a_tile_are_free_of_later_values(cuda_device, dim):
+    """A value that is not finite spoils the rows that see its key, and may spoil those of their tile of 128 tokens before it.
+    Rows of the tile in front stay what they are without it: 10 keys of history put its last one inside a block."""
+    values = torch.randn(266, 128, generator=torch.Generator().manual_seed(dim)).to(BF).float()
+    clean = _expand_exponents(cuda_device, [0.0] * 266, values, 256, dim)
+    for at in (144, 200, 265):
+        spoilt = values.clone()
+        spoilt[at, ::2], spoilt[at, 1::2] = float("inf"), float("nan")
+        out = _expand_exponents(cuda_device, [0.0] * 266, spoilt, 256, dim)
+        assert torch.equal(out[:128], clean[:128])
+        assert not torch.isfinite(out[at - 10:]).any()
 
 
 @pytest.mark.parametrize("dtype", [F32, BF])

@@ -193,3 +193,20 @@ def test_prefill_values_near_the_end_of_the_range(cuda_device):
     v = torch.full((1, 1, 400, 128), 2.0 ** 104)
     out = _attend_exponents(cuda_device, [0.0] * 150 + [22.0] * 100 + [0.0] * 150, v, 4)
     assert torch.equal(out, torch.full_like(out, 2.0 ** 104))
+
+
+@pytest.mark.parametrize("G", [1, 4, 8])
+def test_prefill_rows_of_a_tile_are_free_of_later_values(cuda_device, G):
+    """A value that is not finite spoils the rows that see its key, and may spoil those of their tile of 128 / G tokens before it,
+    whose weight for it is 0.  Rows of the tiles in front stay what they are without it."""
+    tile = 128 // G
+    n = 3 * tile
+    v = torch.randn(1, 1, n, 128, generator=torch.Generator().manual_seed(G)).to(torch.bfloat16).float()
+    clean = _attend_exponents(cuda_device, [0.0] * n, v, n, G)
+    for at in (tile, tile + tile // 2, 2 * tile):
+        spoilt = v.clone()
+        spoilt[0, 0, at, ::2], spoilt[0, 0, at, 1::2] = float("inf"), float("nan")
+        out = _attend_exponents(cuda_device, [0.0] * n, spoilt, n, G)
+        ahead = at // tile * tile
+        assert torch.equal(out[:ahead], clean[:ahead])
+        assert not torch.isfinite(out[at:]).any()
