@@ -2,10 +2,10 @@
 // its parts) is normalised and added, the new stream normalised for the next sublayer.  The stream and everything
 // computed here is fp32; a CTA has one row at a time in registers, 8 elements per access.
 //
-// Bound by DRAM for prompts, by its chain of reductions unless other rows are on their way meanwhile: a CTA walks rows and has
-// the next row's stream and output in flight (one part; several parts of a row are in flight together).  8192 rows of 2048
-// columns, 201 MB: 54 us with a CTA per row, 48 us so; with the eight parts of 64 routed experts 95 and 81 us.  More rows in
-// flight through fewer registers (spills) or with fewer threads to a row were slower.
+// Bound by DRAM for prompts, by its chain of reductions for few rows: one barrier per sum.  8192 rows of 2048 columns in bf16, 201 MB:
+// 60 us with two barriers per sum, 54 with one, 51 where CTAs walk rows with the next one in flight; eight parts 94, 88.  What keeps
+// rows in flight otherwise is the number of CTAs that the registers allow (rn_resident): half as many, for the registers of a row
+// ahead, made eight parts of 4096 columns 211 us instead of 167, of 5120 columns 178 for 112 (3000 rows).
 #include <type_traits>
 
 #include "../ktk_vec.cuh"
@@ -15,9 +15,12 @@ namespace ktk {
 
 constexpr int kRnThreads = 256;
 constexpr int kRnMaxVec = 8;      // 8 x 8 elements per thread: rows of up to 16384 columns
-// CTAs of full width that an SM holds; rows of more than 4096 columns leave no registers for the next one: a CTA for each
-__host__ __device__ constexpr int rn_resident(int nv) { return nv <= 1 ? 3 : nv <= 2 ? 2 : 1; }
-__host__ __device__ constexpr bool rn_walks(int nv) { return nv <= 2; }
+// CTAs of full width that an SM's registers have to hold: where each takes a row, and of those that walk rows
+__host__ __device__ constexpr int rn_resident(int nv) { return nv <= 1 ? 4 : nv <= 2 ? 3 : nv <= 4 ? 2 : 1; }
+constexpr int kRnWalkers = 3;
+// CTAs walk from this many rows each: 3000 rows of 2048 bf16 columns 19.7 us with a CTA per row and 20.0 with walkers, 8192 rows 54.3
+// and 50.9.  Not rows of fewer warps (1024 columns: 23.4 and 24.3), of fp32 (61.3 and 62.4) or of several parts.
+constexpr int kRnWalkRows = 8;
 
 struct ResidualNormParams {
     const int64_t* tokens;
@@ -110,9 +113,9 @@ __device__ __forceinline__ void norm_regs(float (&v)[NV][8], const float* w, con
     }
 }
 
-// TOKENS: the stream starts as embedding rows
-template <typename T, int NV, bool TOKENS>
-__global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_kernel(const ResidualNormParams p) {
+// TOKENS: the stream starts as embedding rows.  WALK: the CTA walks rows, the next one in flight
+template <typename T, int NV, bool TOKENS, bool WALK>
+__global__ void __launch_bounds__(kRnThreads, WALK ? kRnWalkers : rn_resident(NV)) residual_norm_kernel(const ResidualNormParams p) {
     using Stream = typename std::conditional<TOKENS, T, float>::type;
     __shared__ __align__(16) float part_s[2 * (kRnThreads / 32)];
     RowParts part{part_s};
@@ -120,7 +123,6 @@ __global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_ker
     const int nvec = p.stride / 8;
     if (p.zero != nullptr && blockIdx.x == 0)
         for (int i = threadIdx.x; i < p.zero_n; i += blockDim.x) p.zero[i] = 0;
-    const bool one = p.y != nullptr && p.parts == 1;
     auto token = [&](int64_t r) -> int64_t {
         if (!TOKENS || r >= p.rows) return 0;
         const int64_t t = p.tokens[r];
@@ -128,22 +130,27 @@ __global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_ker
         if (threadIdx.x == 0) report(p.status, KTK_STATUS_BAD_TABLE);
         return 0;
     };
-    Raw8<Stream> xr[NV];
-    Raw8<T> yr[NV];
-    auto fetch = [&](int64_t r, int64_t tok) {
+    auto stream_row = [&](int64_t r, int64_t tok) {
+        return TOKENS ? (const Stream*)p.embed + tok * p.stride : (const Stream*)p.x + r * p.stride;
+    };
+    Raw8<Stream> xr[WALK ? NV : 1];
+    Raw8<T> yr[WALK ? NV : 1];
+    auto fetch = [&](int64_t r, int64_t tok) {             // WALK
         if (r >= p.rows) return;
-        const Stream* from = TOKENS ? (const Stream*)p.embed + tok * p.stride : (const Stream*)p.x + r * p.stride;
+        const Stream* from = stream_row(r, tok);
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int k = threadIdx.x + i * blockDim.x;
             if (k >= nvec) continue;
-            xr[i].load(from + k * 8);
-            if (one) yr[i].load((const T*)p.y + r * p.stride + k * 8);
+            xr[WALK ? i : 0].load(from + k * 8);
+            if (p.y != nullptr) yr[WALK ? i : 0].load((const T*)p.y + r * p.stride + k * 8);
         }
     };
-    int64_t r = blockIdx.x;
-    fetch(r, token(r));
-    int64_t ahead = rn_walks(NV) ? token(r + gridDim.x) : 0;
+    int64_t r = blockIdx.x, ahead = token(r);
+    if (WALK) {
+        fetch(r, ahead);
+        ahead = token(r + gridDim.x);
+    }
     for (; r < p.rows; r += gridDim.x) {
         float x[NV][8], y[NV][8];
         float* xrow = p.x + r * p.stride;
@@ -151,27 +158,35 @@ __global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_ker
         for (int i = 0; i < NV; ++i) {
             const int k = threadIdx.x + i * blockDim.x;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[i][e] = y[i][e] = 0.0f;
+            for (int e = 0; e < 8; ++e) x[i][e] = 0.0f;
             if (k >= nvec) continue;
-            xr[i].get(x[i]);
+            if (!WALK) xr[0].load(stream_row(r, ahead) + k * 8);
+            xr[WALK ? i : 0].get(x[i]);
             if (TOKENS) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) x[i][e] *= p.embed_scale;
             }
-            if (one) {
-                yr[i].get(y[i]);
-            } else if (p.y != nullptr) {
-                const T* yk = (const T*)p.y + r * p.parts * p.stride + k * 8;
-#pragma unroll 4
-                for (int j = 0; j < p.parts; ++j) {
-                    float t[8];
-                    Vec8<T>::load(yk + (int64_t)j * p.stride, t);
+        }
+        if (p.y != nullptr) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) y[i][e] += t[e];
+            for (int i = 0; i < NV; ++i) {
+                const int k = threadIdx.x + i * blockDim.x;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) y[i][e] = 0.0f;
+                if (k >= nvec) continue;
+                if (WALK) {
+                    yr[i].get(y[i]);
+                } else {
+                    for (int j = 0; j < p.parts; ++j) {
+                        float t[8];
+                        Vec8<T>::load((const T*)p.y + (r * p.parts + j) * p.stride + k * 8, t);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) y[i][e] += t[e];
+                    }
                 }
             }
         }
-        if (rn_walks(NV)) {
+        if (WALK) {
             fetch(r + gridDim.x, ahead);
             ahead = token(r + 2 * (int64_t)gridDim.x);
         }
@@ -197,23 +212,28 @@ __global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_ker
                 if (k < nvec) Vec8<T>::store((T*)p.h + r * p.stride + k * 8, x[i]);
             }
         }
-        if (!rn_walks(NV)) break;
+        if (!WALK) break;
     }
 }
 
-template <typename T>
-static int residual_norm_launch(const ResidualNormParams& p, int64_t rows, cudaStream_t st) {
+template <typename T, bool TOKENS>
+static int residual_norm_launch(const ResidualNormParams& p, cudaStream_t st) {
     const int nvec = p.stride / 8;
     const int threads = nvec >= kRnThreads ? kRnThreads : (nvec + 31) / 32 * 32;
     const int nv = (nvec + threads - 1) / threads;
-    // a row per CTA; beyond what the SMs hold the CTAs walk
-    const int64_t most = (int64_t)sm_count() * rn_resident(nv) * (kRnThreads / threads);
-    const unsigned grid = (unsigned)(rows < most || !rn_walks(nv) ? rows : most);
-    auto kernel = nv <= 1 ? (p.tokens ? residual_norm_kernel<T, 1, true> : residual_norm_kernel<T, 1, false>)
-                : nv <= 2 ? (p.tokens ? residual_norm_kernel<T, 2, true> : residual_norm_kernel<T, 2, false>)
-                : nv <= 4 ? (p.tokens ? residual_norm_kernel<T, 4, true> : residual_norm_kernel<T, 4, false>)
-                          : (p.tokens ? residual_norm_kernel<T, kRnMaxVec, true> : residual_norm_kernel<T, kRnMaxVec, false>);
-    kernel<<<grid, threads, 0, st>>>(p);
+    const int64_t walkers = (int64_t)sm_count() * kRnWalkers;
+    if constexpr (sizeof(T) == 2) {
+        if (threads == kRnThreads && nv == 1 && p.parts == 1 && p.rows >= kRnWalkRows * walkers) {
+            residual_norm_kernel<T, 1, TOKENS, true><<<(unsigned)walkers, threads, 0, st>>>(p);
+            KTK_CUDA_TRY(cudaGetLastError(), "ktk_residual_norm");
+            return KTK_OK;
+        }
+    }
+    auto kernel = nv <= 1 ? residual_norm_kernel<T, 1, TOKENS, false>
+                : nv <= 2 ? residual_norm_kernel<T, 2, TOKENS, false>
+                : nv <= 4 ? residual_norm_kernel<T, 4, TOKENS, false>
+                          : residual_norm_kernel<T, kRnMaxVec, TOKENS, false>;
+    kernel<<<(unsigned)p.rows, threads, 0, st>>>(p);
     KTK_CUDA_TRY(cudaGetLastError(), "ktk_residual_norm");
     return KTK_OK;
 }
@@ -248,6 +268,7 @@ extern "C" int ktk_residual_norm(const int64_t* tokens, const void* embed, int64
     if ((al & 15u) != 0) { set_error("%s: pointers must be 16-byte aligned", who); return KTK_ERR_ARG; }
     const ResidualNormParams p{tokens, embed, vocab, embed_scale, x, y, parts, post_w, post_b, mult, pre_w, pre_b, h, eps,
                                center, cols, stride, rows, zero, zero ? zero_n : 0, status};
-    return dtype == KTK_F32 ? residual_norm_launch<float>(p, rows, (cudaStream_t)stream)
-                            : residual_norm_launch<__nv_bfloat16>(p, rows, (cudaStream_t)stream);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (dtype == KTK_F32) return tokens ? residual_norm_launch<float, true>(p, st) : residual_norm_launch<float, false>(p, st);
+    return tokens ? residual_norm_launch<__nv_bfloat16, true>(p, st) : residual_norm_launch<__nv_bfloat16, false>(p, st);
 }

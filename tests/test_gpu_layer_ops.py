@@ -43,6 +43,53 @@ def test_residual_norm(cuda_device, dtype, cols):
     torch.testing.assert_close(xd[:, :cols].cpu(), embed[tokens.cpu()] + mult * y.sum(1), rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cols", [40, 1000, 2041, 2048, 4090, 5120, 9000])
+def test_residual_norm_over_many_rows(cuda_device, dtype, cols):
+    """More rows than the SMs hold CTAs, one over a whole number of times; bf16 rows of 1793 to 2048 columns are walked, with the
+    next row in flight: every row against fp64, with one, two and four sums per row, and a bad token among the last."""
+    from kinetics_b200 import layer_ops as lo, ops
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    rows, S, eps, mult = 3 * sms * 8 + 3 * sms + 1, lo.pad8(cols), 1e-4, 0.3
+    g = torch.Generator(device=cuda_device).manual_seed(cols)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
+    pad = lambda t: torch.nn.functional.pad(t, (0, S - cols)).contiguous()
+    x0, w1, b1, w2, b2 = rnd(rows, cols) + 2.0, *(rnd(cols) for _ in range(4))
+    tol = dict(rtol=1e-5, atol=2e-5) if dtype == torch.float32 else dict(rtol=1e-2, atol=1e-2)
+
+    def norm(v, w, b, center):
+        v = v - v.mean(1, keepdim=True) if center else v
+        return v / (v.square().mean(1, keepdim=True) + eps).sqrt() * w.double() + (0 if b is None else b.double())
+
+    for parts in (1, 3):
+        y = (rnd(rows, parts, cols) - 1.0).to(dtype)
+        for post, pre, center in (((w1, b1), (w2, b2), True), ((w1, None), (w2, None), False), (None, (w2, b2), False),
+                                  ((w1, b1), None, True)):
+            x, h = pad(x0), torch.empty(rows, S, dtype=dtype, device=cuda_device)
+            given = lambda n: None if n is None else tuple(None if t is None else pad(t) for t in n)
+            lo.residual_norm(x, None if pre is None else h, cols, eps, pre=given(pre), y=pad(y), parts=parts, post=given(post),
+                             mult=mult, center=center)
+            want = y.double().sum(1)
+            want = x0.double() + mult * (want if post is None else norm(want, *post, center))
+            torch.testing.assert_close(x[:, :cols].double(), want, rtol=1e-5, atol=2e-5)
+            assert x[:, cols:].abs().sum() == 0
+            if pre is not None:
+                torch.testing.assert_close(h[:, :cols].double(), norm(want, *pre, center), **tol)
+                assert h[:, cols:].float().abs().sum() == 0
+    # embedding rows; a token outside the vocabulary is reported and read as the first row
+    embed, status = rnd(97, cols).to(dtype), ops.new_status(cuda_device)
+    tokens = torch.randint(0, 97, (rows,), generator=g, device=cuda_device)
+    x, h = torch.empty(rows, S, device=cuda_device), torch.empty(rows, S, dtype=dtype, device=cuda_device)
+    for bad in (False, True):
+        ids = tokens.clone()
+        if bad:
+            tokens[rows - 2], ids[rows - 2] = 97, 0
+        lo.residual_norm(x, h, cols, eps, pre=(pad(w2), None), tokens=tokens, embed=pad(embed), center=False, status=status)
+        assert int(status.item()) == (2 if bad else 0)
+        assert torch.equal(x[:, :cols], embed[ids].float())
+        torch.testing.assert_close(h[:, :cols].double(), norm(embed[ids].double(), w2, None, False), **tol)
+
+
 def test_residual_norm_reports_a_token_outside_the_vocabulary(cuda_device):
     from kinetics_b200 import layer_ops as lo, ops
     x = torch.empty(1, 8, device=cuda_device)
@@ -201,8 +248,9 @@ def test_scores_beyond_the_polynomial_range(cuda_device):
 
 @pytest.mark.parametrize("vdim", [64, 128])
 @pytest.mark.parametrize("cap", [0.0, 90.0])
-@pytest.mark.parametrize("first, n, grown, maps", [(60, 100, (130, 150), (0, 1)), (60, 100, (130, 150), (1,)), (330, 200, (192, 200), (0,)),
-                                                   (330, 200, (140, 236), (0, 1)), (0, 300, (128, 290), (1,))])
+@pytest.mark.parametrize("first, n, grown, maps", [(60, 100, (130, 150), (0, 1)), (60, 100, (130, 150), (1,)),
+                                                   (330, 200, (192, 200), (0,)), (330, 200, (140, 236), (0, 1)),
+                                                   (0, 300, (128, 290), (1,))])
 def test_scores_that_outgrow_their_reference(cuda_device, vdim, cap, first, n, grown, maps):
     """Without a softcap below 60 the exponentials' reference moves where half a block's sum passes 2^8.  Keys that grow thirtyfold in
     the first half of a later block, in its second half, over blocks, in one of the two maps; the first cases' tile has rows without
