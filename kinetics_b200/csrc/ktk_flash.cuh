@@ -8,7 +8,7 @@
 //                            O_m[128 x vdim] += P_m(j) . V(j)   P_m from tensor memory, V read MN-major as its rows lie
 //                            S_m[128 x KEYS]  = Q_m . K(j + 1)^T
 //                        While the tensor cores work on one tile, the other tile's threads do their softmax.
-//     warp 9             TMA: two blocks of K, `nv` of V in flight
+//     warp 9             TMA: NK blocks of K, `nv` of V in flight
 // Tensor memory: S_m at column 128 m (P_m over its first KEYS / 2 columns), O_m at 256 + 128 m.  S_m(j + 1) is issued behind
 // O_m += P_m(j) . V(j), whose operand it overwrites: matrix instructions of one thread execute in order.  The barrier of
 // S_m(j) therefore also says that O_m is complete up to block j - 1, so a row may be rescaled without a wait of its own.
@@ -20,6 +20,8 @@
 // warps) and a polynomial on the FMA pipes for a part of the exponentials were not faster; over seconds the power limit binds.
 // Every wait is bounded; the caller reports `abort` and frees tensor memory.
 #pragma once
+
+#include <type_traits>
 
 #include "ktk_umma.cuh"
 
@@ -70,7 +72,8 @@ struct FlashShared {
     }
 };
 
-template <int KEYS, int VC> struct Flash {
+// NK: buffers of K, 1 or 2
+template <int KEYS, int VC, int NK = 2> struct Flash {
     static constexpr int kTile = KEYS * 128;             // [KEYS keys][64 columns]
     static constexpr int kHalf = KEYS / 2;
     static constexpr int kVBuf = VC * kTile;
@@ -81,17 +84,20 @@ template <int KEYS, int VC> struct Flash {
     int keys0, keys1;                                    // key columns up to the last one that some row of each tile sees
     int blocks0, blocks1;                                // blocks that hold them
 
-    __device__ __forceinline__ Flash(FlashShared& shared, uint8_t* smem, int qc, int kc, int v_bufs, int n0, int n1)
-        : sh(shared), q(smem), k(smem + 2 * qc * kFlQTile), v(k + 2 * kc * kTile), q_chunks(qc), k_chunks(kc), nv(v_bufs),
-          keys0(n0), keys1(n1), blocks0((n0 + KEYS - 1) / KEYS), blocks1((n1 + KEYS - 1) / KEYS) {}
-    __host__ __device__ static constexpr int bytes(int qc, int kc, int v_bufs) {
-        return 2 * qc * kFlQTile + 2 * kc * kTile + v_bufs * kVBuf;
+    __device__ __forceinline__ Flash(FlashShared& shared, uint8_t* smem, int qc, int kc, int n0, int n1)
+        : sh(shared), q(smem), k(smem + 2 * qc * kFlQTile), v(k + NK * kc * kTile), q_chunks(qc), k_chunks(kc),
+          nv(v_buffers(qc, kc)), keys0(n0), keys1(n1), blocks0((n0 + KEYS - 1) / KEYS), blocks1((n1 + KEYS - 1) / KEYS) {}
+    // with 1 KiB to align it; the second buffer of V where shared memory holds it
+    __host__ __device__ static constexpr int bytes_of(int qc, int kc, int v_bufs) {
+        return 2 * qc * kFlQTile + NK * kc * kTile + v_bufs * kVBuf + 1024;
     }
-    // the second buffer of V where shared memory holds it
-    __host__ __device__ static constexpr int v_buffers(int qc, int kc) { return bytes(qc, kc, 2) + 1024 <= kFlMaxSmem ? 2 : 1; }
+    __host__ __device__ static constexpr int v_buffers(int qc, int kc) { return bytes_of(qc, kc, 2) <= kFlMaxSmem ? 2 : 1; }
+    __host__ __device__ static constexpr int bytes(int qc, int kc) { return bytes_of(qc, kc, v_buffers(qc, kc)); }
 
     __device__ __forceinline__ int blocks() const { return blocks0 > blocks1 ? blocks0 : blocks1; }
     __device__ __forceinline__ int blocks_of(int m) const { return m ? blocks1 : blocks0; }
+    __device__ __forceinline__ int k_buf(int blk) const { return blk & (NK - 1); }
+    __device__ __forceinline__ uint32_t k_phase(int blk) const { return (uint32_t)(blk >> (NK - 1)) & 1u; }
     __device__ __forceinline__ int v_buf(int blk) const { return blk & (nv - 1); }
     __device__ __forceinline__ uint32_t v_phase(int blk) const { return (uint32_t)(blk >> (nv - 1)) & 1u; }
 
@@ -105,7 +111,7 @@ template <int KEYS, int VC> struct Flash {
         const int n = blocks();
         auto scores = [&](int m, int blk) {
             const uint64_t qa = umma_desc_at(q_desc, m * q_chunks * kFlQTile);
-            const uint64_t ka = umma_desc_at(k_desc, (blk & 1) * k_chunks * kTile + m * k_off);
+            const uint64_t ka = umma_desc_at(k_desc, k_buf(blk) * k_chunks * kTile + m * k_off);
             if (elect_one()) {
                 for (int c = 0; c < q_chunks; ++c) {
                     const int n_steps = steps(c);
@@ -124,6 +130,27 @@ template <int KEYS, int VC> struct Flash {
             tc_fence_after();
             return true;
         };
+        // O_m += P_m(j) . V(j), the first half of the block's keys while the threads work on the second.  Not `whole`, a tile's last
+        // block: values behind the last key that the tile sees are left out, for 0 times one that is not finite is not 0.
+        auto products = [&](auto whole, int m, int j) {
+            const int n_steps = whole ? KEYS / 16 : ((m ? keys1 : keys0) - j * KEYS + 15) / 16;
+            const uint64_t va = umma_desc_at(v_desc, v_buf(j) * kVBuf);
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                if (!wait(part ? &sh.p_rest[m] : &sh.p[m], j & 1)) return false;
+                if (elect_one()) {
+#pragma unroll
+                    for (int i = part * (kHalf / 16); i < (part + 1) * (kHalf / 16); ++i)
+                        if (whole || i < n_steps)
+                            umma_f16_ts(tmem + kFlColO + m * 128, tmem + m * 128 + i * 8, umma_desc_at(va, i * (16 * 128)), idesc_o,
+                                        (j > 0 || i > 0) ? 1u : 0u);
+                    if (part == 0) umma_commit(&sh.o_half[m]);
+                    else if (j + 1 == blocks_of(m)) umma_commit(&sh.o[m]);
+                }
+                __syncwarp();
+            }
+            return true;
+        };
         if (n == 0 || !wait(&sh.k[0], 0)) return;
         if (blocks0 > 0) scores(0, 0);
         if (blocks1 > 0) scores(1, 0);
@@ -131,38 +158,25 @@ template <int KEYS, int VC> struct Flash {
         __syncwarp();
         for (int j = 0; j < n; ++j) {
             const bool more = j + 1 < n;
-            // both copies before the probabilities, which are what the tensor cores are short of
-            if (!wait(&sh.v[v_buf(j)], v_phase(j)) || (more && !wait(&sh.k[(j + 1) & 1], ((j + 1) >> 1) & 1))) return;
-            const uint64_t va = umma_desc_at(v_desc, v_buf(j) * kVBuf);
+            // V, and K of the next block, before the probabilities, which are what the tensor cores are short of; an only buffer of
+            // K is filled later
+            if (!wait(&sh.v[v_buf(j)], v_phase(j)) || (more && NK > 1 && !wait(&sh.k[k_buf(j + 1)], k_phase(j + 1)))) return;
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const int mine = blocks_of(m);
                 if (j < mine) {
-                    // values behind the last key that the tile sees are left out: 0 times one that is not finite is not 0
-                    const int n_steps = ((m ? keys1 : keys0) - j * KEYS + 15) / 16;
-                    // the first half of the block's keys while the threads work on the second
-#pragma unroll
-                    for (int part = 0; part < 2; ++part) {
-                        if (!wait(part ? &sh.p_rest[m] : &sh.p[m], j & 1)) return;
-                        if (elect_one()) {
-#pragma unroll
-                            for (int i = part * (kHalf / 16); i < (part + 1) * (kHalf / 16); ++i)
-                                if (i < n_steps)
-                                    umma_f16_ts(tmem + kFlColO + m * 128, tmem + m * 128 + i * 8, umma_desc_at(va, i * (16 * 128)),
-                                                idesc_o, (j > 0 || i > 0) ? 1u : 0u);
-                            if (part == 0) umma_commit(&sh.o_half[m]);
-                            else if (j + 1 == mine) umma_commit(&sh.o[m]);
-                        }
-                        __syncwarp();
-                    }
+                    if (!(j + 1 < mine ? products(std::true_type{}, m, j) : products(std::false_type{}, m, j))) return;
                 }
                 if (m == 1) {
                     if (elect_one()) umma_commit(&sh.vfree[v_buf(j)]);
                     __syncwarp();
                 }
-                if (j + 1 < mine) scores(m, j + 1);
+                if (j + 1 < mine) {
+                    if (NK == 1 && !wait(&sh.k[0], k_phase(j + 1))) return;
+                    scores(m, j + 1);
+                }
                 if (m == 1 && more) {
-                    if (elect_one()) umma_commit(&sh.kfree[(j + 1) & 1]);
+                    if (elect_one()) umma_commit(&sh.kfree[k_buf(j + 1)]);
                     __syncwarp();
                 }
             }
@@ -174,26 +188,26 @@ template <int KEYS, int VC> struct Flash {
         const int n = blocks();
         int k_issued = 0, v_issued = 0;
         auto more_k = [&] {
-            load_k(k_issued, k + (k_issued & 1) * k_chunks * kTile, &sh.k[k_issued & 1]);
+            load_k(k_issued, k + k_buf(k_issued) * k_chunks * kTile, &sh.k[k_buf(k_issued)]);
             ++k_issued;
         };
         bool alive = true;
         if (n > 0) more_k();
-        if (n > 1) more_k();
+        if (n > 1 && NK > 1) more_k();
         for (int j = 0; j < n && alive; ++j) {
-            // V over that of block j - nv, then K of block j + 2 over that of block j
+            // V over that of block j - nv, then K of block j + NK over that of block j
             alive = j < nv || mbar_wait_all(&sh.vfree[v_buf(j)], v_phase(j) ^ 1u, &sh.abort);
             if (!alive) break;
             load_v(j, v + v_buf(j) * kVBuf, &sh.v[v_buf(j)]);
             ++v_issued;
-            if (j + 2 < n) {
-                alive = mbar_wait_all(&sh.kfree[j & 1], (j >> 1) & 1, &sh.abort);
+            if (j + NK < n) {
+                alive = mbar_wait_all(&sh.kfree[k_buf(j)], k_phase(j), &sh.abort);
                 if (alive) more_k();
             }
         }
         if (!alive) {                                    // the copies in flight still write shared memory
             volatile int never = 0;
-            for (int i = k_issued > 2 ? k_issued - 2 : 0; i < k_issued; ++i) mbar_wait(&sh.k[i & 1], (i >> 1) & 1, &never);
+            for (int i = k_issued > NK ? k_issued - NK : 0; i < k_issued; ++i) mbar_wait(&sh.k[k_buf(i)], k_phase(i), &never);
             for (int i = v_issued > nv ? v_issued - nv : 0; i < v_issued; ++i) mbar_wait(&sh.v[v_buf(i)], v_phase(i), &never);
         }
     }

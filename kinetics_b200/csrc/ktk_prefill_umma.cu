@@ -16,8 +16,7 @@ namespace ktk {
 constexpr int kPuKeys = 128;
 constexpr int kPuPages = kPuKeys / kPageSize;             // of a block
 using PrefillFlash = Flash<kPuKeys, kHeadDim / 64>;
-constexpr int kPuBufs = PrefillFlash::v_buffers(2, 2);
-constexpr int kPuSmem = PrefillFlash::bytes(2, 2, kPuBufs) + 1024;
+constexpr int kPuSmem = PrefillFlash::bytes(2, 2);
 
 // TILE_MAJOR: the grid is (kv heads, sequences, tile pairs), so that the tiles with the longest history come first over all
 // heads and sequences; otherwise (tile pairs, kv heads, sequences), for more than 65535 pairs
@@ -64,7 +63,7 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
     const bool row_on = warp < 8 && my_tok < n_new;
     const int vis = row_on ? base_pos + my_tok + 1 : 0;     // keys at positions < vis are seen
 
-    Flash<kPuKeys, kHeadDim / 64> fl(sh, sm, 2, 2, kPuBufs, keys[0], keys[1]);
+    PrefillFlash fl(sh, sm, 2, 2, keys[0], keys[1]);
     if (tid == 0) sh.init();
     if (warp < 8) {
         // Q row -> two swizzled chunks (zeros for rows past the last new token)

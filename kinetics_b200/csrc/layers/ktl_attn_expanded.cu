@@ -2,9 +2,8 @@
 // of its own, one rotated key part for all heads; a sink in the denominator, a gate on the output.  bf16 on the
 // fifth-generation tensor cores, fp32 scores and sums.
 //
-// One CTA per (head, two tiles of 128 tokens): both tiles share every block of keys (128; 64 where the queries of a wide head
-// leave shared memory for no more) that comes in by TMA: the unrotated columns of the head, then the shared rotated ones.  The
-// softmax and the order of the matrix instructions: ktk_flash.cuh; the exponents' reference starts at the sink.
+// One CTA per (head, two tiles of 128 tokens): both tiles share every block of 128 keys that comes in by TMA: the unrotated columns
+// of the head, then the shared rotated ones.  The softmax and the order of the matrix instructions: ktk_flash.cuh.
 // 8192 tokens, 32 heads of 128 + 64 and 128 columns: 590 us (1164 TFLOP/s), 899 us with blocks of 64 keys.  Heads are walked
 // in groups whose keys and values fit L2, so that the CTAs left for the end are short ones.
 #include "../ktk_flash.cuh"
@@ -12,6 +11,7 @@
 
 namespace ktk {
 
+constexpr int kAeKeys = 128;
 constexpr int kAeMaxChunks = 4;               // of the key: 64 columns each
 constexpr int64_t kAeGroupBytes = 48 << 20;   // keys and values that the CTAs of a wave share through L2 (126 MB)
 
@@ -28,13 +28,13 @@ struct ExpandedParams {
 };
 
 // heads_per: heads whose tiles are walked together, those with the longest history first
-template <int VC, int KEYS>
+template <int VC, int NK>
 __global__ void __launch_bounds__(kFlThreads, 1)
-attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bufs, const __grid_constant__ CUtensorMap k_map,
+attn_expanded_kernel(const ExpandedParams p, const int heads_per, const __grid_constant__ CUtensorMap k_map,
                      const __grid_constant__ CUtensorMap r_map, const __grid_constant__ CUtensorMap v_map) {
     extern __shared__ uint8_t ae_raw[];
     __shared__ __align__(8) FlashShared sh;
-    using F = Flash<KEYS, VC>;
+    using F = Flash<kAeKeys, VC, NK>;
     const ktk_latent& a = p.a;
     const int nc = (a.dim_stride + 63) / 64, dc = nc + (a.rot_stride + 63) / 64;     // chunks of a key
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ae_raw) + 1023) & ~uintptr_t(1023));
@@ -59,7 +59,7 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bu
     const bool row_on = warp < 8 && tok < p.n;
     const int vis = row_on ? base + tok + 1 : 0;        // keys at positions < vis are seen
 
-    F fl(sh, sm, dc, dc, v_bufs, keys[0], keys[1]);
+    F fl(sh, sm, dc, dc, keys[0], keys[1]);
     if (tid == 0) sh.init();
     if (warp < 8) {
         const __nv_bfloat16* src = p.q + (int64_t)(row_on ? tok : 0) * p.q_stride + (int64_t)head * (a.dim_stride + a.rot_stride);
@@ -99,8 +99,8 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bu
                     if (elect_one()) {
                         mbar_arrive_expect_tx(bar, (uint32_t)(dc * F::kTile));
                         for (int c = 0; c < dc; ++c) {
-                            if (c < nc) tma_load_3d(dst + c * F::kTile, &k_map, bar, c * 64, head, blk * KEYS);
-                            else tma_load_3d(dst + c * F::kTile, &r_map, bar, (c - nc) * 64, 0, blk * KEYS);
+                            if (c < nc) tma_load_3d(dst + c * F::kTile, &k_map, bar, c * 64, head, blk * kAeKeys);
+                            else tma_load_3d(dst + c * F::kTile, &r_map, bar, (c - nc) * 64, 0, blk * kAeKeys);
                         }
                     }
                     __syncwarp();
@@ -109,7 +109,7 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bu
                     if (elect_one()) {
                         mbar_arrive_expect_tx(bar, (uint32_t)F::kVBuf);
     #pragma unroll
-                        for (int c = 0; c < VC; ++c) tma_load_3d(dst + c * F::kTile, &v_map, bar, c * 64, head, blk * KEYS);
+                        for (int c = 0; c < VC; ++c) tma_load_3d(dst + c * F::kTile, &v_map, bar, c * 64, head, blk * kAeKeys);
                     }
                     __syncwarp();
                 });
@@ -118,11 +118,11 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const int v_bu
         more_registers();
         const int tile_min_vis = base + tok0 + tile * kUmRows + 1;
         float m_ref = p.sink ? p.sink[head] * kLog2eF : -INFINITY, l_run = p.sink ? 1.0f : 0.0f;
-        const bool done = fl.template softmax<false>(tile, a.scale * kLog2eF, m_ref, l_run, [&](float (&s)[KEYS], int j) {
-            if ((j + 1) * KEYS > tile_min_vis) {                       // some row of the tile does not see the whole block
-                const int lim = vis - j * KEYS;
+        const bool done = fl.template softmax<false>(tile, a.scale * kLog2eF, m_ref, l_run, [&](float (&s)[kAeKeys], int j) {
+            if ((j + 1) * kAeKeys > tile_min_vis) {                       // some row of the tile does not see the whole block
+                const int lim = vis - j * kAeKeys;
 #pragma unroll
-                for (int c = 0; c < KEYS; ++c) s[c] = c < lim ? s[c] : -INFINITY;
+                for (int c = 0; c < kAeKeys; ++c) s[c] = c < lim ? s[c] : -INFINITY;
             }
             return false;
         }, [](float&, float&) {}, [](int) {});
@@ -175,13 +175,13 @@ gather_rows_kernel(const uint4* __restrict__ pages, uint4* __restrict__ out, con
 
 static int chunks_of(const ktk_latent& a) { return (a.dim_stride + 63) / 64 + (a.rot_stride + 63) / 64; }
 
-template <int VC, int KEYS>
+template <int VC, int NK>
 static int expanded_launch(const ExpandedParams& p, const __nv_bfloat16* kv, const __nv_bfloat16* rows, cudaStream_t st) {
     const char* who = "ktk_expanded_attention";
     const ktk_latent& a = p.a;
     const uint64_t H = a.heads, line = H * (a.dim_stride + a.vdim_stride) * 2, row = (uint64_t)(a.rank_stride + a.rot_stride) * 2;
     CUtensorMap km, rm, vm;
-    const uint32_t box[3] = {64, 1, KEYS};
+    const uint32_t box[3] = {64, 1, kAeKeys};
     // innermost first: columns of a head, heads, tokens
     const uint64_t kd[3] = {(uint64_t)a.dim_stride, H, (uint64_t)p.total}, ks[2] = {(uint64_t)a.dim_stride * 2, line};
     const uint64_t vd[3] = {(uint64_t)a.vdim_stride, H, (uint64_t)p.total}, vs[2] = {(uint64_t)a.vdim_stride * 2, line};
@@ -194,13 +194,13 @@ static int expanded_launch(const ExpandedParams& p, const __nv_bfloat16* kv, con
         rc = make_tensor_map_3d(&rm, rows + a.rank_stride, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rd, rs, box,
                                 CU_TENSOR_MAP_SWIZZLE_128B, who);
     if (rc != KTK_OK) return rc;
-    const int dc = chunks_of(a), bufs = Flash<KEYS, VC>::v_buffers(dc, dc), smem = Flash<KEYS, VC>::bytes(dc, dc, bufs) + 1024;
+    const int dc = chunks_of(a), smem = Flash<kAeKeys, VC, NK>::bytes(dc, dc);
     const int64_t pairs = ((int64_t)p.n + 2 * kUmRows - 1) / (2 * kUmRows), per_head = (int64_t)p.total * (a.dim_stride + a.vdim_stride) * 2;
     int64_t heads_per = kAeGroupBytes / per_head;
     heads_per = heads_per < 1 ? 1 : (heads_per > a.heads ? a.heads : heads_per);
-    auto kernel = attn_expanded_kernel<VC, KEYS>;
+    auto kernel = attn_expanded_kernel<VC, NK>;
     KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), who);
-    kernel<<<(unsigned)(pairs * a.heads), kFlThreads, smem, st>>>(p, (int)heads_per, bufs, km, rm, vm);
+    kernel<<<(unsigned)(pairs * a.heads), kFlThreads, smem, st>>>(p, (int)heads_per, km, rm, vm);
     KTK_CUDA_TRY(cudaGetLastError(), who);
     return KTK_OK;
 }
@@ -253,8 +253,10 @@ extern "C" int ktk_expanded_attention(const void* q, int64_t q_stride, int64_t r
     }
     const ExpandedParams p{*shape, (const __nv_bfloat16*)q, q_stride, (int)rows, (int)total, sink, (const __nv_bfloat16*)gate,
                            gate_stride, (__nv_bfloat16*)o, status};
+    // Queries of four chunks leave room for one buffer of K: the next block comes in during the softmax of this one.  4000 keys, 32
+    // CTAs: 121 us with blocks of 64 keys and two buffers.
     const bool wide = chunks_of(*shape) > 3;
-    auto launch = shape->vdim_stride <= 64 ? (wide ? expanded_launch<1, 64> : expanded_launch<1, 128>)
-                                           : (wide ? expanded_launch<2, 64> : expanded_launch<2, 128>);
+    auto launch = shape->vdim_stride <= 64 ? (wide ? expanded_launch<1, 1> : expanded_launch<1, 2>)
+                                           : (wide ? expanded_launch<2, 1> : expanded_launch<2, 2>);
     return launch(p, (const __nv_bfloat16*)kv, (const __nv_bfloat16*)latents, (cudaStream_t)stream);
 }

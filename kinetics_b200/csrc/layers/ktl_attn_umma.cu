@@ -32,7 +32,6 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     extern __shared__ uint8_t au_raw[];
     __shared__ __align__(8) FlashShared sh;
     using F = Flash<kAuKeys, VC>;
-    constexpr int kBufs = F::v_buffers(DC, 2 * DC);
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(au_raw) + 1023) & ~uintptr_t(1023));
 
     const ktk_attn& a = p.a;
@@ -57,7 +56,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     const bool row_on = warp < 8 && row / group < tpc && my_tok < n_new;
     const int vis = row_on ? base_pos + my_tok + 1 : 0; // keys at positions < vis are seen
 
-    F fl(sh, sm, DC, 2 * DC, kBufs, seen, seen);
+    F fl(sh, sm, DC, 2 * DC, seen, seen);
     if (tid == 0) sh.init();
     if (warp < 8) {
         const uint4* src = reinterpret_cast<const uint4*>(
@@ -215,7 +214,7 @@ template <int DC, int VC, bool FIXED> static int umma_launch(const AttnParams& p
     const int rc = make_cache_maps(p, &km, &vm, (uint32_t)p.t.page_size, who);
     if (rc != KTK_OK) return rc;
     using F = Flash<kAuKeys, VC>;
-    constexpr int smem = F::bytes(DC, 2 * DC, F::v_buffers(DC, 2 * DC)) + 1024;
+    constexpr int smem = F::bytes(DC, 2 * DC);
     const int tpc = kUmRows / (p.a.heads / p.a.kv_heads);
     const unsigned tiles = (unsigned)(((int64_t)p.max_new + tpc - 1) / tpc), heads = (unsigned)p.a.kv_heads, batch = (unsigned)p.t.batch;
     const bool tile_major = tiles <= 65535;

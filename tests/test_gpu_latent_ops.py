@@ -90,7 +90,7 @@ def test_sinks_of_every_size(cuda_device):
 
 
 # heads, dim, rot_dim, vdim
-EXPANDED = [(4, 128, 64, 128), (3, 32, 32, 32), (2, 40, 8, 72), (1, 192, 64, 128), (5, 64, 128, 16), (2, 24, 16, 100)]
+EXPANDED = [(4, 128, 64, 128), (3, 32, 32, 32), (2, 40, 8, 72), (1, 192, 64, 128), (2, 192, 64, 40), (5, 64, 128, 16), (2, 24, 16, 100)]
 
 
 @pytest.mark.parametrize("heads,dim,rot_dim,vdim", EXPANDED)
@@ -184,7 +184,7 @@ def _expand_exponents(dev, exponents, values, n, dim, sink_exponent=0.0):
     return out.view(n, 128).double().cpu()
 
 
-@pytest.mark.parametrize("at,dim", [(3, 128), (60, 128), (100, 128), (3, 192), (60, 192)])
+@pytest.mark.parametrize("at,dim", [(3, 128), (60, 128), (100, 128), (3, 192), (60, 192), (100, 192)])
 def test_expanded_key_above_the_sink(cuda_device, at, dim):
     """One key of the first block outweighs the other keys by 2^40 and the sink by 2^7: the row is its value by 1 / (1 + 2^-7).
     Bound: the nearest bf16 number of a value within 2^-15 of it (fp32 sums, the sink's exponential; rounding is monotonic); a weight
