@@ -101,9 +101,31 @@ template <int KEYS, int VC, int NK = 2> struct Flash {
     __device__ __forceinline__ int v_buf(int blk) const { return blk & (nv - 1); }
     __device__ __forceinline__ uint32_t v_phase(int blk) const { return (uint32_t)(blk >> (nv - 1)) & 1u; }
 
+    // ---- queries of tile m, by its four warps.  piece(row, chunk, i): where 16 bytes of the row lie, the i-th of 64 columns, or
+    // null for zeros.  Eight lanes to a row's 128 bytes: a lane for each row took 32
+    // lines per access, 1 us per tile.
+    template <class Piece> __device__ __forceinline__ void queries(int m, Piece piece) {
+        const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, at = lane & 7;
+        uint8_t* dst = q + m * q_chunks * kFlQTile;
+#pragma unroll 2
+        for (int c = 0; c < q_chunks; ++c) {
+            uint4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint4* src = piece(warp * 32 + i * 4 + (lane >> 3), c, at);
+                v[i] = src ? __ldg(src) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                *reinterpret_cast<uint4*>(dst + c * kFlQTile + swz(warp * 32 + i * 4 + (lane >> 3), at)) = v[i];
+        }
+        fence_proxy_async();
+    }
+
     // ---- matrix instructions, by a converged warp.  steps(c): 16-column steps of chunk c; k_off: bytes between the keys of
-    // the two tiles in a buffer of K (0: the same keys); vcols: columns of V, a multiple of 16
-    template <class Steps> __device__ __forceinline__ void issue(Steps steps, int k_off, int vcols) {
+    // the two tiles in a buffer of K (0: the same keys); vcols: columns of V, a multiple of 16; CLEARED: the rows of V
+    // behind the last key that a tile sees are zeros
+    template <bool CLEARED = false, class Steps> __device__ __forceinline__ void issue(Steps steps, int k_off, int vcols) {
         const uint32_t tmem = sh.tmem;
         const uint32_t idesc_s = umma_idesc(KEYS, false), idesc_o = umma_idesc(vcols, true);
         const uint64_t q_desc = umma_desc(smem_u32(q), 0, 1024), k_desc = umma_desc(smem_u32(k), 0, 1024);
@@ -165,7 +187,7 @@ template <int KEYS, int VC, int NK = 2> struct Flash {
             for (int m = 0; m < 2; ++m) {
                 const int mine = blocks_of(m);
                 if (j < mine) {
-                    if (!(j + 1 < mine ? products(std::true_type{}, m, j) : products(std::false_type{}, m, j))) return;
+                    if (!(CLEARED || j + 1 < mine ? products(std::true_type{}, m, j) : products(std::false_type{}, m, j))) return;
                 }
                 if (m == 1) {
                     if (elect_one()) umma_commit(&sh.vfree[v_buf(j)]);

@@ -66,16 +66,13 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
     PrefillFlash fl(sh, sm, 2, 2, keys[0], keys[1]);
     if (tid == 0) sh.init();
     if (warp < 8) {
-        // Q row -> two swizzled chunks (zeros for rows past the last new token)
-        const uint4* src = reinterpret_cast<const uint4*>(
-            (const __nv_bfloat16*)p.q + ((int64_t)(q0 + (row_on ? my_tok : 0)) * Hq + my_head) * kHeadDim);
-        uint8_t* dst = fl.q + tile * 2 * kFlQTile;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            const uint4 v = row_on ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(dst + (c >> 3) * kFlQTile + swz(row, c & 7)) = v;
-        }
-        fence_proxy_async();
+        const int shift_g = 31 - __clz(G);              // 1, 2, 4 or 8
+        fl.queries(tile, [&](int r, int chunk, int i) -> const uint4* {
+            const int t = tok0 + tile * tpc + (r >> shift_g);
+            if (t >= n_new) return nullptr;
+            return reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.q + ((int64_t)(q0 + t) * Hq + h * G + (r & (G - 1))) * kHeadDim) +
+                   chunk * 8 + i;
+        });
     } else if (warp == 8) {
         tmem_alloc(&sh.tmem, kFlTmemCols);
     }

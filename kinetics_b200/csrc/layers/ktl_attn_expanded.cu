@@ -62,16 +62,14 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const __grid_c
     F fl(sh, sm, dc, dc, keys[0], keys[1]);
     if (tid == 0) sh.init();
     if (warp < 8) {
-        const __nv_bfloat16* src = p.q + (int64_t)(row_on ? tok : 0) * p.q_stride + (int64_t)head * (a.dim_stride + a.rot_stride);
-        uint8_t* dst = fl.q + tile * dc * kFlQTile;
-        for (int c = 0; c < dc * 8; ++c) {
-            const bool rot = c >= nc * 8;
-            const int col = (rot ? c - nc * 8 : c) * 8, size = rot ? a.rot_stride : a.dim_stride;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (row_on && col < size) v = *reinterpret_cast<const uint4*>(src + (rot ? a.dim_stride : 0) + col);
-            *reinterpret_cast<uint4*>(dst + (c >> 3) * kFlQTile + swz(row, c & 7)) = v;
-        }
-        fence_proxy_async();
+        fl.queries(tile, [&](int r, int chunk, int i) -> const uint4* {
+            const int t = tok0 + tile * kUmRows + r;
+            const bool rot = chunk >= nc;
+            const int col = (rot ? chunk - nc : chunk) * 64 + i * 8;
+            if (t >= p.n || col >= (rot ? a.rot_stride : a.dim_stride)) return nullptr;
+            return reinterpret_cast<const uint4*>(p.q + t * p.q_stride + (int64_t)head * (a.dim_stride + a.rot_stride) +
+                                                  (rot ? a.dim_stride : 0) + col);
+        });
     } else if (warp == 8) {
         tmem_alloc(&sh.tmem, kFlTmemCols);
     }

@@ -59,16 +59,12 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     F fl(sh, sm, DC, 2 * DC, seen, seen);
     if (tid == 0) sh.init();
     if (warp < 8) {
-        const uint4* src = reinterpret_cast<const uint4*>(
-            (const __nv_bfloat16*)p.q + (int64_t)(q0 + (row_on ? my_tok : 0)) * p.q_stride +
-            ((int64_t)(row_on ? my_head : 0) * 2 + map) * a.dim_stride);
-        uint8_t* dst = fl.q + map * DC * kFlQTile;
-#pragma unroll
-        for (int c = 0; c < DC * 8; ++c) {
-            const uint4 v = row_on && c * 8 < a.dim_stride ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(dst + (c >> 3) * kFlQTile + swz(row, c & 7)) = v;
-        }
-        fence_proxy_async();
+        fl.queries(map, [&](int r, int chunk, int i) -> const uint4* {
+            const int t = tok0 + r / group, col = chunk * 64 + i * 8;
+            if (r / group >= tpc || t >= n_new || col >= a.dim_stride) return nullptr;
+            return reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.q + (int64_t)(q0 + t) * p.q_stride +
+                                                  ((int64_t)(kvh * group + r % group) * 2 + map) * a.dim_stride + col);
+        });
     } else if (warp == 8) {
         tmem_alloc(&sh.tmem, kFlTmemCols);
     }
@@ -80,7 +76,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
         fewer_registers();
         if (warp == 8) {
             const int ksteps = (a.dim_stride + 15) / 16;
-            fl.issue([&](int c) { return ksteps - 4 * c < 4 ? ksteps - 4 * c : 4; }, DC * F::kTile, (a.vdim_stride + 15) / 16 * 16);
+            fl.template issue<true>([&](int c) { return ksteps - 4 * c < 4 ? ksteps - 4 * c : 4; }, DC * F::kTile, (a.vdim_stride + 15) / 16 * 16);
         } else if (warp == 9) {
             // a box is a page of one head (of one map); lane i: page i of a block
             const int pages = kAuKeys / ps, box = ps * 128;
