@@ -292,7 +292,7 @@ extern "C" int ktk_prefill_attention(const void* q, const int32_t* q_indptr, int
             PrefillUmmaParams u;
             u.q = q; u.o = o; u.cache = kv_cache; u.q_indptr = q_indptr; u.kv_indices = kv_indices;
             u.kv_indptr = kv_indptr; u.kv_last_page_len = kv_last_page_len; u.page_count = view.page_count;
-            u.sink_tokens = view.sink_tokens; u.batch = s->batch; u.Hkv = s->num_kv_heads; u.G = G;
+            u.sink_tokens = view.sink_tokens; u.batch = s->batch; u.total_new = total_new_tokens; u.Hkv = s->num_kv_heads; u.G = G;
             u.num_pages = s->num_pages; u.scale_log2 = sm_scale * kLog2e; u.status = status;
             return launch_prefill_umma(u, max_new_tokens, st);
         }

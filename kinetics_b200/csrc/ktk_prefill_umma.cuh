@@ -16,11 +16,13 @@ struct PrefillUmmaParams {
     const int32_t* page_count;
     int sink_tokens;
     int batch, Hkv, G;
+    int64_t total_new;
+    int tiles;                 // of a CTA: 1 or 2 (set by launch_prefill_umma)
     int64_t num_pages;
     float scale_log2;
     int32_t* status;
 };
 
-int launch_prefill_umma(const PrefillUmmaParams& p, int max_new_tokens, cudaStream_t st);
+int launch_prefill_umma(PrefillUmmaParams p, int max_new_tokens, cudaStream_t st);
 
 }  // namespace ktk

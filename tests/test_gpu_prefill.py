@@ -124,15 +124,16 @@ def test_prefill_on_block_and_tile_edges(cuda_device, variant, G, sink):
         torch.testing.assert_close(out[lo:hi].float(), ref, rtol=2e-2, atol=2e-2)
 
 
-@pytest.mark.parametrize("G,sink,grow", [(4, 0, (0.1, 40.0, 200.0)), (1, 4, (1.0, 1.0, 90.0)), (2, 0, (60.0, 0.1, 30.0))])
-def test_prefill_scores_that_outgrow_their_reference(cuda_device, G, sink, grow):
+@pytest.mark.parametrize("G,sink,grow,n", [(4, 0, (0.1, 40.0, 200.0), 200), (1, 4, (1.0, 1.0, 90.0), 200), (2, 0, (60.0, 0.1, 30.0), 200),
+                                           (8, 4, (0.1, 40.0, 200.0), 1300)])
+def test_prefill_scores_that_outgrow_their_reference(cuda_device, G, sink, grow, n):
     """The exponentials' reference is the first block's maximum until a half block's sum passes 2^8: scores that grow by far
     more in the first half of a block of 128 keys, in its second half, in the block of the row itself; and that shrink.
 
     Bound: operands are the reference's own bf16 values, products of 128 columns are summed in fp32, so a score of up to about
     1000 is off by a few 1e-4, a weight by that share; bf16 weights add 2^-9 of each value: 2e-2, as in the other cases."""
     from kinetics_b200 import ops
-    Hkv, hist, n = 2, 330, 200
+    Hkv, hist = 2, 330                                       # the last case: more tiles than SMs, two to a CTA
     total = hist + n
     g = torch.Generator().manual_seed(7 + G)
     factor = torch.full((total,), grow[0])
@@ -195,18 +196,42 @@ def test_prefill_values_near_the_end_of_the_range(cuda_device):
     assert torch.equal(out, torch.full_like(out, 2.0 ** 104))
 
 
-@pytest.mark.parametrize("G", [1, 4, 8])
-def test_prefill_rows_of_a_tile_are_free_of_later_values(cuda_device, G):
+@pytest.mark.parametrize("G,tiles", [(1, 3), (4, 3), (8, 3), (4, 0), (8, 0)])
+def test_prefill_rows_of_a_tile_are_free_of_later_values(cuda_device, G, tiles):
     """A value that is not finite spoils the rows that see its key, and may spoil those of their tile of 128 / G tokens before it,
-    whose weight for it is 0.  Rows of the tiles in front stay what they are without it."""
-    tile = 128 // G
-    n = 3 * tile
+    whose weight for it is 0.  Rows of the tiles in front stay what they are without it.  tiles 0: more than SMs, two to a CTA."""
+    tile, tiles = 128 // G, tiles or torch.cuda.get_device_properties(cuda_device).multi_processor_count + 3
+    n = tiles * tile
     v = torch.randn(1, 1, n, 128, generator=torch.Generator().manual_seed(G)).to(torch.bfloat16).float()
     clean = _attend_exponents(cuda_device, [0.0] * n, v, n, G)
-    for at in (tile, tile + tile // 2, 2 * tile):
+    for at in (tile, tile + tile // 2, 2 * tile, n - tile - 1):
         spoilt = v.clone()
         spoilt[0, 0, at, ::2], spoilt[0, 0, at, 1::2] = float("inf"), float("nan")
         out = _attend_exponents(cuda_device, [0.0] * n, spoilt, n, G)
         ahead = at // tile * tile
         assert torch.equal(out[:ahead], clean[:ahead])
         assert not torch.isfinite(out[at:]).any()
+
+
+@pytest.mark.parametrize("more", [-1, 0, 1, 17])
+def test_prefill_with_about_as_many_tiles_as_sms(cuda_device, more):
+    """A CTA takes one tile where all tiles find an SM, two otherwise: tiles of 16 tokens on either side of that, in one sequence
+    and over several with an empty one.  Bound: as in the other cases."""
+    from kinetics_b200 import ops
+    G, tokens = 8, 16 * (torch.cuda.get_device_properties(cuda_device).multi_processor_count + more) - 3
+    for new in ([tokens], [0, tokens // 2, 1, tokens - tokens // 2 - 1]):
+        lens = [n + (5 if n else 0) for n in new]
+        g = torch.Generator().manual_seed(tokens)
+        k = torch.randn(len(new), 1, max(lens), 128, generator=g).to(torch.bfloat16).float()
+        v = torch.randn(len(new), 1, max(lens), 128, generator=g).to(torch.bfloat16).float()
+        d = to_dev(paged_state(k, v, lens, torch.bfloat16, seed=5), cuda_device)
+        q = torch.randn(sum(new), G, 128, generator=g).to(torch.bfloat16).to(cuda_device)
+        indptr = torch.tensor([sum(new[:i]) for i in range(len(new) + 1)], dtype=torch.int32, device=cuda_device)
+        status = ops.new_status(cuda_device)
+        out = ops.prefill_attention(q, indptr, max(new), d["kv_cache"], d["kv_indices"], d["kv_indptr"], d["kv_last_page_len"],
+                                    status=status)
+        ops.raise_on_status(status)
+        for b, n in enumerate(new):
+            lo = int(indptr[b])
+            ref = _reference(q[lo:lo + n].float(), k[b, :, :lens[b]].to(cuda_device), v[b, :, :lens[b]].to(cuda_device), G)
+            torch.testing.assert_close(out[lo:lo + n].float(), ref, rtol=2e-2, atol=2e-2)
