@@ -205,26 +205,30 @@ template <int KEYS, int VC, int NK = 2> struct Flash {
         }
     }
 
-    // ---- copies, by a converged warp.  load_k(blk, dst, bar), load_v(blk, dst, bar): tell the barrier the bytes and start the copies
+    // ---- copies, by a converged warp.  load_k(blk, dst, bar), load_v(blk, dst, bar): tell the barrier the bytes and start the
+    // copies.  The first ones start when the barriers are set up, while the other warps bring in the queries.
+    template <class LoadK, class LoadV> __device__ __forceinline__ void first_copies(LoadK load_k, LoadV load_v) {
+        load_k(0, k, &sh.k[0]);
+        load_v(0, v, &sh.v[0]);
+        if (NK > 1 && blocks() > 1) load_k(1, k + k_chunks * kTile, &sh.k[1]);
+    }
     template <class LoadK, class LoadV> __device__ __forceinline__ void copy(LoadK load_k, LoadV load_v) {
         const int n = blocks();
-        int k_issued = 0, v_issued = 0;
-        auto more_k = [&] {
-            load_k(k_issued, k + k_buf(k_issued) * k_chunks * kTile, &sh.k[k_buf(k_issued)]);
-            ++k_issued;
-        };
+        int k_issued = n < NK ? n : NK, v_issued = 1;
         bool alive = true;
-        if (n > 0) more_k();
-        if (n > 1 && NK > 1) more_k();
         for (int j = 0; j < n && alive; ++j) {
             // V over that of block j - nv, then K of block j + NK over that of block j
-            alive = j < nv || mbar_wait_all(&sh.vfree[v_buf(j)], v_phase(j) ^ 1u, &sh.abort);
-            if (!alive) break;
-            load_v(j, v + v_buf(j) * kVBuf, &sh.v[v_buf(j)]);
-            ++v_issued;
+            if (j > 0) {
+                alive = j < nv || mbar_wait_all(&sh.vfree[v_buf(j)], v_phase(j) ^ 1u, &sh.abort);
+                if (!alive) break;
+                load_v(j, v + v_buf(j) * kVBuf, &sh.v[v_buf(j)]);
+                ++v_issued;
+            }
             if (j + NK < n) {
                 alive = mbar_wait_all(&sh.kfree[k_buf(j)], k_phase(j), &sh.abort);
-                if (alive) more_k();
+                if (!alive) break;
+                load_k(k_issued, k + k_buf(k_issued) * k_chunks * kTile, &sh.k[k_buf(k_issued)]);
+                ++k_issued;
             }
         }
         if (!alive) {                                    // the copies in flight still write shared memory
@@ -242,7 +246,8 @@ template <int KEYS, int VC, int NK = 2> struct Flash {
     // infinite); then it is that half's maximum.  So no other block's maximum has to be searched, which cost 500 of a block's 3400
     // cycles.  A weight of 2^8 or more becomes 1, which bf16 holds exactly: the row of a key that outweighs all others is that
     // key's value.  And |O| <= 2^8 max|V| per 64 keys: 8192 keys leave |V| 2^113 (1e34) of the range of fp32.
-    // The halves of a block are handed over one by one: 521 us for the prompt of 8192 tokens and 32 heads without that, 498 with it.
+    // The halves of a block are handed over one by one: the prompt of 8192 tokens and 32 heads takes 521 us without that, 498 with
+    // it (two builds of one comparison).
     template <bool FIXED, class Prepare, class Form, class Clear>
     __device__ __forceinline__ bool softmax(int m, float f, float& m_ref, float& l_run, Prepare prepare, Form form, Clear clear) {
         const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;

@@ -64,17 +64,56 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
     const int vis = row_on ? base_pos + my_tok + 1 : 0;     // keys at positions < vis are seen
 
     PrefillFlash fl(sh, sm, 2, 2, keys[0], keys[1]);
-    if (tid == 0) sh.init();
+    // warp 9.  Lane i < 8: page i of a block; entries are read one block ahead of their first use
+    auto entry = [&](int blk) {
+        const int e = blk * kPuPages + lane;
+        return lane < kPuPages && e < n_need ? p.kv_indices[sp.start + e] : -1;
+    };
+    int at[3], first = 0;                           // of blocks first, first + 1, first + 2
+    auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
+        while (first + 2 < blk || (which && first < blk)) {
+            at[0] = at[1];
+            at[1] = at[2];
+            ++first;
+            at[2] = entry(first + 2);
+        }
+        const int pg = blk == first ? at[0] : (blk == first + 1 ? at[1] : at[2]);
+        const bool on = pg >= 0 && pg < p.num_pages;
+        if (which == 0 && !on && lane < kPuPages && blk * kPuPages + lane < n_need) report(p.status, KTK_STATUS_BAD_PAGE);
+        const uint32_t pages = __popc(__ballot_sync(0xffffffffu, on));
+        if (lane == 0) {
+            if (pages) mbar_arrive_expect_tx(bar, pages * (2u * kPageSize * 128u));
+            else mbar_arrive(bar);
+        }
+        __syncwarp();
+        if (on) {
+            const int z = pg * (2 * kPageSize) + which * kPageSize;      // token row of slot 0
+            tma_load_3d(dst + lane * (kPageSize * 128), &kv_map, bar, 0, h, z);
+            tma_load_3d(dst + PrefillFlash::kTile + lane * (kPageSize * 128), &kv_map, bar, 64, h, z);
+        }
+        __syncwarp();
+    };
+    auto load_k = [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); };
+    auto load_v = [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); };
     if (warp < 8) {
         const int shift_g = 31 - __clz(G);              // 1, 2, 4 or 8
         if (fl.blocks_of(tile) > 0) fl.queries(tile, [&](int r, int chunk, int i) -> const uint4* {
             const int t = tok0 + tile * tpc + (r >> shift_g);
             if (t >= n_new) return nullptr;
-            return reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.q + ((int64_t)(q0 + t) * Hq + h * G + (r & (G - 1))) * kHeadDim) +
-                   chunk * 8 + i;
+            const int64_t q_row = (int64_t)(q0 + t) * Hq + h * G + (r & (G - 1));
+            return reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.q + q_row * kHeadDim) + chunk * 8 + i;
         });
     } else if (warp == 8) {
         tmem_alloc(&sh.tmem, kFlTmemCols);
+    } else if (warp == 9) {
+        if (lane == 0) {
+            prefetch_tensormap(&kv_map);
+            sh.init();
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) at[i] = entry(i);
+        __syncwarp();
+        fl.first_copies(load_k, load_v);
     }
     tc_fence_before();
     __syncthreads();
@@ -85,38 +124,7 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
         if (warp == 8) {
             fl.issue([](int) { return 4; }, 0, kHeadDim);
         } else if (warp == 9) {
-            // lane i < 8: page i of a block; entries are read one block ahead of their first use
-            auto entry = [&](int blk) {
-                const int e = blk * kPuPages + lane;
-                return lane < kPuPages && e < n_need ? p.kv_indices[sp.start + e] : -1;
-            };
-            int at[3] = {entry(0), entry(1), entry(2)}, first = 0;        // of blocks first, first + 1, first + 2
-            auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
-                while (first + 2 < blk || (which && first < blk)) {
-                    at[0] = at[1];
-                    at[1] = at[2];
-                    ++first;
-                    at[2] = entry(first + 2);
-                }
-                const int pg = blk == first ? at[0] : (blk == first + 1 ? at[1] : at[2]);
-                const bool on = pg >= 0 && pg < p.num_pages;
-                if (which == 0 && !on && lane < kPuPages && blk * kPuPages + lane < n_need) report(p.status, KTK_STATUS_BAD_PAGE);
-                const uint32_t pages = __popc(__ballot_sync(0xffffffffu, on));
-                if (lane == 0) {
-                    if (pages) mbar_arrive_expect_tx(bar, pages * (2u * kPageSize * 128u));
-                    else mbar_arrive(bar);
-                }
-                __syncwarp();
-                if (on) {
-                    const int z = pg * (2 * kPageSize) + which * kPageSize;      // token row of slot 0
-                    tma_load_3d(dst + lane * (kPageSize * 128), &kv_map, bar, 0, h, z);
-                    tma_load_3d(dst + PrefillFlash::kTile + lane * (kPageSize * 128), &kv_map, bar, 64, h, z);
-                }
-                __syncwarp();
-            };
-            if (lane == 0) prefetch_tensormap(&kv_map);
-            fl.copy([&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); },
-                    [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); });
+            fl.copy(load_k, load_v);
         }
     } else {
         more_registers();

@@ -60,7 +60,25 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const __grid_c
     const int vis = row_on ? base + tok + 1 : 0;        // keys at positions < vis are seen
 
     F fl(sh, sm, dc, dc, keys[0], keys[1]);
-    if (tid == 0) sh.init();
+    // warp 9; columns and tokens outside come as zeros
+    auto load_k = [&](int blk, uint8_t* dst, uint64_t* bar) {
+        if (elect_one()) {
+            mbar_arrive_expect_tx(bar, (uint32_t)(dc * F::kTile));
+            for (int c = 0; c < dc; ++c) {
+                if (c < nc) tma_load_3d(dst + c * F::kTile, &k_map, bar, c * 64, head, blk * kAeKeys);
+                else tma_load_3d(dst + c * F::kTile, &r_map, bar, (c - nc) * 64, 0, blk * kAeKeys);
+            }
+        }
+        __syncwarp();
+    };
+    auto load_v = [&](int blk, uint8_t* dst, uint64_t* bar) {
+        if (elect_one()) {
+            mbar_arrive_expect_tx(bar, (uint32_t)F::kVBuf);
+#pragma unroll
+            for (int c = 0; c < VC; ++c) tma_load_3d(dst + c * F::kTile, &v_map, bar, c * 64, head, blk * kAeKeys);
+        }
+        __syncwarp();
+    };
     if (warp < 8) {
         fl.queries(tile, [&](int r, int chunk, int i) -> const uint4* {
             const int t = tok0 + tile * kUmRows + r;
@@ -72,6 +90,15 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const __grid_c
         });
     } else if (warp == 8) {
         tmem_alloc(&sh.tmem, kFlTmemCols);
+    } else if (warp == 9) {
+        if (elect_one()) {
+            prefetch_tensormap(&k_map);
+            prefetch_tensormap(&r_map);
+            prefetch_tensormap(&v_map);
+            sh.init();
+        }
+        __syncwarp();
+        fl.first_copies(load_k, load_v);
     }
     tc_fence_before();
     __syncthreads();
@@ -85,32 +112,7 @@ attn_expanded_kernel(const ExpandedParams p, const int heads_per, const __grid_c
                                                 : (rsteps - 4 * (c - nc) < 4 ? rsteps - 4 * (c - nc) : 4); },
                      0, (a.vdim_stride + 15) / 16 * 16);
         } else if (warp == 9) {
-            if (elect_one()) {
-                prefetch_tensormap(&k_map);
-                prefetch_tensormap(&r_map);
-                prefetch_tensormap(&v_map);
-            }
-            __syncwarp();
-            // columns and tokens outside come as zeros
-            fl.copy(
-                [&](int blk, uint8_t* dst, uint64_t* bar) {
-                    if (elect_one()) {
-                        mbar_arrive_expect_tx(bar, (uint32_t)(dc * F::kTile));
-                        for (int c = 0; c < dc; ++c) {
-                            if (c < nc) tma_load_3d(dst + c * F::kTile, &k_map, bar, c * 64, head, blk * kAeKeys);
-                            else tma_load_3d(dst + c * F::kTile, &r_map, bar, (c - nc) * 64, 0, blk * kAeKeys);
-                        }
-                    }
-                    __syncwarp();
-                },
-                [&](int blk, uint8_t* dst, uint64_t* bar) {
-                    if (elect_one()) {
-                        mbar_arrive_expect_tx(bar, (uint32_t)F::kVBuf);
-    #pragma unroll
-                        for (int c = 0; c < VC; ++c) tma_load_3d(dst + c * F::kTile, &v_map, bar, c * 64, head, blk * kAeKeys);
-                    }
-                    __syncwarp();
-                });
+            fl.copy(load_k, load_v);
         }
     } else {
         more_registers();

@@ -5,7 +5,7 @@
 // One CTA per (sequence, kv head, tile of 128 (token, head of the group) rows).  A row exists once per map: the two tiles of
 // ktk_flash.cuh are the two maps, each with keys of its own; a block is 128 keys of both maps and their values.
 // With a softcap the exponentials have a fixed reference (ktl_score.cuh): nothing is ever rescaled.  Without one (or
-// with a large one) the reference follows the running maximum in jumps.
+// with a large one) the reference is the first block's maximum until half a block's sum passes 2^8 (ktk_flash.cuh).
 // Bound by what the softmax issues: 8192 tokens, 16 heads of 2 x 64 and 128 columns, softcap: 523 us, 792 us with blocks of
 // 64 keys.
 #include "../ktk_flash.cuh"
@@ -57,7 +57,33 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     const int vis = row_on ? base_pos + my_tok + 1 : 0; // keys at positions < vis are seen
 
     F fl(sh, sm, DC, 2 * DC, seen, seen);
-    if (tid == 0) sh.init();
+    // warp 9.  A box is a page of one head (of one map); lane i: page i of a block
+    const int pages = kAuKeys / ps, box = ps * 128;
+    auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
+        const int tok = blk * kAuKeys + lane * ps;
+        const int64_t pg = lane < pages && tok < seen ? p.t.kv_indices[s.start + tok / ps] : -1;
+        const bool on = pg >= 0 && pg < p.t.num_pages;
+        if (lane < pages && tok < seen && !on) report(p.status, KTK_STATUS_BAD_PAGE);
+        const uint32_t n = __popc(__ballot_sync(0xffffffffu, on));
+        if (lane == 0) {
+            if (n) mbar_arrive_expect_tx(bar, n * (uint32_t)((which ? VC : 2 * DC) * box));
+            else mbar_arrive(bar);
+        }
+        __syncwarp();
+        if (on && which) {
+    #pragma unroll
+            for (int c = 0; c < VC; ++c)
+                tma_load_3d(dst + c * F::kTile + lane * box, &v_map, bar, c * 64, 0, (int)(pg * a.kv_heads) + kvh);
+        } else if (on) {
+    #pragma unroll
+            for (int mc = 0; mc < 2 * DC; ++mc)
+                tma_load_3d(dst + mc * F::kTile + lane * box, &k_map, bar, (mc % DC) * 64, 0,
+                            (int)(pg * (2 * a.kv_heads)) + kvh * 2 + mc / DC);
+        }
+        __syncwarp();
+    };
+    auto load_k = [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); };
+    auto load_v = [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); };
     if (warp < 8) {
         fl.queries(map, [&](int r, int chunk, int i) -> const uint4* {
             const int t = tok0 + r / group, col = chunk * 64 + i * 8;
@@ -67,6 +93,14 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
         });
     } else if (warp == 8) {
         tmem_alloc(&sh.tmem, kFlTmemCols);
+    } else if (warp == 9) {
+        if (lane == 0) {
+            prefetch_tensormap(&k_map);
+            prefetch_tensormap(&v_map);
+            sh.init();
+        }
+        __syncwarp();
+        fl.first_copies(load_k, load_v);
     }
     tc_fence_before();
     __syncthreads();
@@ -78,37 +112,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
             const int ksteps = (a.dim_stride + 15) / 16;
             fl.template issue<true>([&](int c) { return ksteps - 4 * c < 4 ? ksteps - 4 * c : 4; }, DC * F::kTile, (a.vdim_stride + 15) / 16 * 16);
         } else if (warp == 9) {
-            // a box is a page of one head (of one map); lane i: page i of a block
-            const int pages = kAuKeys / ps, box = ps * 128;
-            auto load = [&](int blk, int which, uint8_t* dst, uint64_t* bar) {
-                const int tok = blk * kAuKeys + lane * ps;
-                const int64_t pg = lane < pages && tok < seen ? p.t.kv_indices[s.start + tok / ps] : -1;
-                const bool on = pg >= 0 && pg < p.t.num_pages;
-                if (lane < pages && tok < seen && !on) report(p.status, KTK_STATUS_BAD_PAGE);
-                const uint32_t n = __popc(__ballot_sync(0xffffffffu, on));
-                if (lane == 0) {
-                    if (n) mbar_arrive_expect_tx(bar, n * (uint32_t)((which ? VC : 2 * DC) * box));
-                    else mbar_arrive(bar);
-                }
-                __syncwarp();
-                if (on && which) {
-    #pragma unroll
-                    for (int c = 0; c < VC; ++c)
-                        tma_load_3d(dst + c * F::kTile + lane * box, &v_map, bar, c * 64, 0, (int)(pg * a.kv_heads) + kvh);
-                } else if (on) {
-    #pragma unroll
-                    for (int mc = 0; mc < 2 * DC; ++mc)
-                        tma_load_3d(dst + mc * F::kTile + lane * box, &k_map, bar, (mc % DC) * 64, 0,
-                                    (int)(pg * (2 * a.kv_heads)) + kvh * 2 + mc / DC);
-                }
-                __syncwarp();
-            };
-            if (lane == 0) {
-                prefetch_tensormap(&k_map);
-                prefetch_tensormap(&v_map);
-            }
-            fl.copy([&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); },
-                    [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); });
+            fl.copy(load_k, load_v);
         }
     } else {
         more_registers();
