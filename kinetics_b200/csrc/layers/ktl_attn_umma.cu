@@ -24,8 +24,8 @@ __device__ __forceinline__ void st_row16(__nv_bfloat16* d, const float* o, float
     *reinterpret_cast<uint4*>(d) = v;
 }
 
-// TILE_MAJOR: the grid is (kv heads, sequences, tiles), so that the tiles with the longest history come first over all heads and
-// sequences; otherwise (tiles, kv heads, sequences), for more than 65535 tiles
+// TILE_MAJOR: the grid is (kv heads, sequences, tiles), so that the last tiles of all heads and sequences, which see most of their own
+// sequence, come first; otherwise (tiles, kv heads, sequences), for more than 65535 tiles
 template <int DC, int VC, bool FIXED, bool TILE_MAJOR>
 __global__ void __launch_bounds__(kFlThreads, 1)
 attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map) {
@@ -85,11 +85,12 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map, 
     auto load_k = [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 0, dst, bar); };
     auto load_v = [&](int blk, uint8_t* dst, uint64_t* bar) { load(blk, 1, dst, bar); };
     if (warp < 8) {
+        const int per = (65536 + group - 1) / group;            // r / group = r per / 65536 for r (group - 1) < 65536
         fl.queries(map, [&](int r, int chunk, int i) -> const uint4* {
-            const int t = tok0 + r / group, col = chunk * 64 + i * 8;
-            if (r / group >= tpc || t >= n_new || col >= a.dim_stride) return nullptr;
+            const int at = r * per >> 16, t = tok0 + at, col = chunk * 64 + i * 8;
+            if (at >= tpc || t >= n_new || col >= a.dim_stride) return nullptr;
             return reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.q + (int64_t)(q0 + t) * p.q_stride +
-                                                  ((int64_t)(kvh * group + r % group) * 2 + map) * a.dim_stride + col);
+                                                  ((int64_t)(kvh * group + r - at * group) * 2 + map) * a.dim_stride + col);
         });
     } else if (warp == 8) {
         tmem_alloc(&sh.tmem, kFlTmemCols);
