@@ -288,7 +288,7 @@ template <int KEYS, int VC, int NK = 2> struct Flash {
                 return a + b;
             };
             auto hand_over = [&](int from, uint64_t* bar) {
-                tmem_store(s_at + from / 2, packed);
+                tmem_st32_u32(s_at + from / 2, packed);
                 l_run += total();
                 tmem_st_wait();
                 if (from == 0) clear(j);

@@ -105,12 +105,6 @@ __device__ __forceinline__ void tmem_load(uint32_t taddr, float (&v)[128]) {
           "=f"(v[120]), "=f"(v[121]), "=f"(v[122]), "=f"(v[123]), "=f"(v[124]), "=f"(v[125]), "=f"(v[126]), "=f"(v[127])
         : "r"(taddr), "r"(taddr + 32), "r"(taddr + 64), "r"(taddr + 96));
 }
-__device__ __forceinline__ void tmem_load(uint32_t taddr, float (&v)[64]) {
-    float lo[32], hi[32];
-    tmem_ld64(taddr, lo, hi);
-#pragma unroll
-    for (int i = 0; i < 32; ++i) { v[i] = lo[i]; v[32 + i] = hi[i]; }
-}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -138,15 +132,6 @@ __device__ __forceinline__ void tmem_st32_u32(uint32_t taddr, const uint32_t (&v
           "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
           "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
           "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&v)[32]) { tmem_st32_u32(taddr, v); }
-__device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
