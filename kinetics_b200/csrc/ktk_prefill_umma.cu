@@ -6,7 +6,7 @@
 // group) pairs.  Both tiles share every block of 128 keys (eight pages, 16-row x 128-byte boxes under the 128-byte swizzle, which
 // is the operand layout tcgen05.mma reads).  The softmax and the order of the matrix instructions: ktk_flash.cuh.
 // Bound by the chain of a tile's block: matrix instructions, softmax, matrix instructions.  8192 tokens, 32 heads over 8 kv
-// heads: 510 us (1078 TFLOP/s), 880 us with one tile per CTA, blocks of 64 keys and two CTAs per SM.
+// heads: 489 us (1124 TFLOP/s), 855 us with one tile per CTA, blocks of 64 keys and two CTAs per SM.
 #include "ktk_decode_mma.cuh"
 #include "ktk_flash.cuh"
 #include "ktk_prefill_umma.cuh"
@@ -18,8 +18,8 @@ constexpr int kPuPages = kPuKeys / kPageSize;             // of a block
 using PrefillFlash = Flash<kPuKeys, kHeadDim / 64>;
 constexpr int kPuSmem = PrefillFlash::bytes(2, 2);
 
-// TILE_MAJOR: the grid is (kv heads, sequences, tile pairs), so that the tiles with the longest history come first over all
-// heads and sequences; otherwise (tile pairs, kv heads, sequences), for more than 65535 pairs
+// TILE_MAJOR: the grid is (kv heads, sequences, tile pairs), so that the last tiles of all heads and sequences, which see most of
+// their own sequence, come first (not the longest histories of sequences that differ); otherwise (tile pairs, kv heads, sequences), for more than 65535 pairs
 template <bool TILE_MAJOR>
 __global__ void __launch_bounds__(kFlThreads, 1)
 prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorMap kv_map) {
