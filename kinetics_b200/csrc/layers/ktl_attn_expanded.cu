@@ -4,7 +4,7 @@
 //
 // One CTA per (head, two tiles of 128 tokens): both tiles share every block of 128 keys that comes in by TMA: the unrotated columns
 // of the head, then the shared rotated ones.  The softmax and the order of the matrix instructions: ktk_flash.cuh.
-// 8192 tokens, 32 heads of 128 + 64 and 128 columns: 590 us (1164 TFLOP/s), 899 us with blocks of 64 keys.  Heads are walked
+// 8192 tokens, 32 heads of 128 + 64 and 128 columns in a model: 694 us (990 TFLOP/s), 899 us with blocks of 64 keys.  Heads are walked
 // in groups whose keys and values fit L2, so that the CTAs left for the end are short ones.
 #include "../ktk_flash.cuh"
 #include "ktl_score.cuh"
