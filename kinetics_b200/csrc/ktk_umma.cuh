@@ -186,6 +186,17 @@ template <> struct RowPairs<8> {
     }
 };
 
+// 32 lanes of tensor memory, 32 columns, as two RowPairs<4> (lanes 0..15 in r[0 .. 15], 16..31 in r[16 .. 31]): both loads in
+// flight before the one wait
+__device__ __forceinline__ void tmem_ld_rows32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr), "r"(taddr + (16u << 16)));
+}
+
 // One lane of a converged warp.  The issuing warps run their loops with all lanes and pick the lane only around the
 // instructions themselves: descriptors and barrier addresses can then stay in uniform registers, which is what the
 // tcgen05 instructions take; from a branch on the lane number every operand has to be moved there first.

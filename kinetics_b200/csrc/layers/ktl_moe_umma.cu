@@ -1,16 +1,20 @@
 // The experts' matrix products on the fifth-generation tensor cores, for prompts and for decode steps alike.
 //
 // The weights are the M operand and the routed rows the N operand: D[128 weight rows x N rows] += A[128 x 64] . B^T[64
-// x N].  A work item is one tile of up to 256 rows of an expert and a block of 128 weight rows: stage 0 has the gate
-// and the up row of an inner column side by side, so gating needs one exchange between neighbouring lanes.  N
+// x N].  A work item is one tile of up to 256 rows of an expert and a block of 128 weight rows (stage 0: the gate and
+// the up rows of 64 inner columns, which the copy brings as eight gates, eight ups, and so on).  N
 // follows the tile's row count, and the ring's stages shrink with the rows a tile can have: a decode step with a few
 // rows per expert keeps many weight tiles in flight and moves little else.  Persistent CTAs; the item list follows
 // from the experts' row counts, which each CTA reads and scans itself.  Roles:
 //     loading warp      weight tiles by TMA; stage 1 also the rows, which lie in place
 //     gathering warps   stage 0: the bucket's rows of h, 16 bytes per cp.async, into the layout of the operand
 //     issuing warp      4 x tcgen05.mma per ring stage, accumulators double-buffered in tensor memory (2 x 256 columns)
-//     warps 0..3        epilogue of the previous item: tcgen05.ld, activation or routing weight, bf16 stores to the
-//                       rows' places
+//     warps 0..3        epilogue of the previous item: activation or routing weight, bf16 rows to their places.  The
+//                       accumulators hold the output transposed: 16x256b loads give them as 8 x 8 fragments, gate and up
+//                       of a column in one thread, which stmatrix.trans lays down as rows that leave in 16-byte pieces.
+//                       Lanes that swapped neighbours and stored 2 or 4 bytes each held the tensor cores up: 8192 rows,
+//                       8 of 64 experts, 2048 -> 768 columns 415 + 247 us (stages 0 and 1), 381 + 195 this way, 354 + 165
+//                       without any epilogue.
 // Full tiles (prompts) run on pairs of CTAs (cta_group::2): 256 weight rows x 256 routed rows per item, each CTA with its
 // half of both in shared memory, which takes a third off the traffic from L2.  The second CTA's issuing warp tells the
 // first one's when its part of a stage has landed.
@@ -58,6 +62,7 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
         acc_full[2], acc_free[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_flag;
+    __shared__ __align__(16) uint8_t staged[4][2048];        // a warp's 32 routed rows on their way out
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(mu_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int N = STAGE == 0 ? 2 * p.m.ff_stride : p.m.width_stride;       // weight rows
@@ -132,7 +137,8 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
                 uint8_t* st = ring + s * stage_bytes;
                 if (elect_one()) {
                     mbar_arrive_expect_tx(&full[s], bytes);
-                    tma_load_3d(st, &w_map, &full[s], k * kMuK, it.wrow, it.e);
+                    if (STAGE == 0) tma_load_5d(st, &w_map, &full[s], k * kMuK, 0, 0, it.wrow / 16, it.e);
+                    else tma_load_3d(st, &w_map, &full[s], k * kMuK, it.wrow, it.e);
                     for (int i = 0; i < boxes; ++i)
                         tma_load_3d(st + kMuABytes + i * kMuBox * 128, &in_map, &full[s], k * kMuK, row + i * kMuBox, 0);
                 }
@@ -255,7 +261,8 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
         // ---------------- epilogue ----------------
         const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);
         __nv_bfloat16* out = (__nv_bfloat16*)p.out;
-        const bool odd = lane & 1;
+        const int out_cols = STAGE == 0 ? p.m.ff_stride : p.m.width_stride;
+        const uint32_t st = smem_u32(staged[warp]);
         int j = 0;
         for (int w = unit; w < work; w += num_units) {
             const Item it = item(w);
@@ -275,31 +282,56 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
             const bool ok = mbar_wait_fast(&acc_full[buf], (j >> 1) & 1, &abort_flag);
             if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after();
-            const int wrow = it.wrow + warp * 32 + (lane & ~1);              // weight row of the even lane of the two
+            // first column of the output that this warp's 32 weight rows give
+            const int col0 = STAGE == 0 ? (it.wrow >> 1) + warp * 16 : it.wrow + warp * 32;
 #pragma unroll
             for (int ch = 0; ch < kMuRows / 32; ++ch) {
                 const int c0 = ch * 32;
                 if (c0 >= it.n) break;                       // uniform for the CTA
-                float v[32];
-                tmem_ld32(lanes + buf * 256 + c0, v);
-                // neighbouring lanes hold neighbouring weight rows: the even lane takes row i of the tile, the odd i + 1
+                uint32_t v[32];                              // [16 weight rows][8 routed rows]: an 8 x 8 matrix per two registers
+                tmem_ld_rows32(lanes + buf * 256 + c0, v);
+                if (STAGE == 0) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
-                    const float first = odd ? got : v[i], second = odd ? v[i + 1] : got;
-                    const int row = c0 + i + odd;
-                    if (STAGE == 0) {                        // gate and up of inner column wrow / 2
-                        const float act = gated<true>(first, second, p.m.limit, p.m.slope, p.m.shift);
-                        if (row < it.n && wrow < N)
-                            out[(int64_t)(plan.first_row[it.e] + it.r0 + row) * p.m.ff_stride + (wrow >> 1)] =
-                                __float2bfloat16_rn(act);
-                    } else {
-                        const int64_t dst = __shfl_sync(0xffffffffu, entry[ch], i + odd);
-                        const float f = __shfl_sync(0xffffffffu, weight[ch], i + odd);
-                        if (row < it.n && wrow < N)
-                            *reinterpret_cast<uint32_t*>(out + dst * N + wrow) = pack_bf16(first * f, second * f);
+                    for (int k = 0; k < 4; k += 2) {
+                        uint32_t m[4];                       // (routed rows 8 (k + i / 2) .., inner columns 8 (i % 2) ..)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const uint32_t* x = v + 16 * (i & 1) + 4 * (k + (i >> 1));      // gate, gate, up, up
+                            m[i] = pack_bf16(
+                                gated<true>(__uint_as_float(x[0]), __uint_as_float(x[2]), p.m.limit, p.m.slope, p.m.shift),
+                                gated<true>(__uint_as_float(x[1]), __uint_as_float(x[3]), p.m.limit, p.m.slope, p.m.shift));
+                        }
+                        const int row = 8 * (k + (lane >> 4)) + (lane & 7), chunk = (lane >> 3) & 1;
+                        stmatrix_x4_trans(st + row * 32 + ((chunk ^ ((row >> 2) & 1)) << 4), m);
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float w0 = __shfl_sync(0xffffffffu, weight[ch], 8 * k + 2 * (lane & 3));
+                        const float w1 = __shfl_sync(0xffffffffu, weight[ch], 8 * k + 2 * (lane & 3) + 1);
+                        uint32_t m[4];                       // (routed rows 8 k .., weight rows 8 i ..)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const uint32_t* x = v + 16 * (i >> 1) + 4 * k + 2 * (i & 1);
+                            m[i] = pack_bf16(__uint_as_float(x[0]) * w0, __uint_as_float(x[1]) * w1);
+                        }
+                        const int row = 8 * k + (lane & 7), chunk = lane >> 3;
+                        stmatrix_x4_trans(st + row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4), m);
                     }
                 }
+                __syncwarp();
+                constexpr int kPieces = STAGE == 0 ? 2 : 4;  // 16-byte pieces of a row
+#pragma unroll
+                for (int i = 0; i < kPieces; ++i) {
+                    const int row = lane / kPieces + i * (32 / kPieces), chunk = lane % kPieces;
+                    const int place = STAGE == 0 ? chunk ^ ((row >> 2) & 1) : chunk ^ ((row >> 1) & 3);
+                    const uint4 x = *reinterpret_cast<const uint4*>(staged[warp] + row * (kPieces * 16) + place * 16);
+                    const int64_t dst = STAGE == 0 ? plan.first_row[it.e] + it.r0 + c0 + row
+                                                   : __shfl_sync(0xffffffffu, entry[ch], row);
+                    const int col = col0 + chunk * 8;
+                    if (c0 + row < it.n && col < out_cols) *reinterpret_cast<uint4*>(out + dst * out_cols + col) = x;
+                }
+                __syncwarp();
             }
             tc_fence_before();
             __syncwarp();
@@ -329,10 +361,18 @@ template <int STAGE> static int moe_umma(const MoeParams& p, cudaStream_t st) {
     const uint64_t K = STAGE == 0 ? p.m.width_stride : p.m.ff_stride;
     const int64_t routed = p.rows * p.m.top;
     CUtensorMap w_map, in_map;
-    const uint64_t wd[3] = {K, N, (uint64_t)p.m.experts}, ws[2] = {K * 2, K * N * 2};
-    const uint32_t wb[3] = {kMuK, kUmRows, 1};
-    int rc = make_tensor_map_3d(&w_map, p.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B,
-                                who);
+    int rc;
+    if (STAGE == 0) {
+        // Rows 16 b + 2 j + i of the matrix (i: gate, up) come as rows 16 b + 8 i + j of the operand: of every 16 lanes of
+        // the accumulators the first eight then hold the gates, the others the ups, as the epilogue's registers want them.
+        const uint64_t wd[5] = {K, 8, 2, N / 16, (uint64_t)p.m.experts}, ws[4] = {K * 4, K * 2, K * 32, K * N * 2};
+        const uint32_t wb[5] = {kMuK, 8, 2, kUmRows / 16, 1};
+        rc = make_tensor_map(&w_map, p.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B, who);
+    } else {
+        const uint64_t wd[3] = {K, N, (uint64_t)p.m.experts}, ws[2] = {K * 2, K * N * 2};
+        const uint32_t wb[3] = {kMuK, kUmRows, 1};
+        rc = make_tensor_map_3d(&w_map, p.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B, who);
+    }
     if (rc != KTK_OK) return rc;
     const uint64_t id[3] = {K, (uint64_t)(STAGE == 0 ? p.rows : routed), 1}, is[2] = {K * 2, K * id[1] * 2};
     const uint32_t ib[3] = {kMuK, kMuBox, 1};
