@@ -81,7 +81,9 @@ extern "C" int ktk_kv_append(const void* proj, int64_t row_stride, int64_t k_col
 }
 
 extern "C" int32_t ktk_paged_attention_splits(const ktk_attn* shape, int32_t batch, int32_t new_rows, int64_t max_keys) {
-    if (attn_shared_supported(*shape)) return attn_shared_splits(*shape, batch, new_rows, max_keys);
+    if (attn_shared_supported(*shape))
+        return new_rows == 0 && attn_shared_balanced(*shape, batch, max_keys) ? KTK_SPLITS_BALANCED
+                                                                              : attn_shared_splits(*shape, batch, new_rows, max_keys);
     if (new_rows > 0) return 1;
     return attn_decode_supported(*shape) ? attn_decode_splits(*shape, batch, max_keys) : 1;
 }
@@ -126,7 +128,9 @@ extern "C" int ktk_paged_attention(const void* q, int64_t q_stride, const int32_
         return KTK_ERR_UNSUPPORTED;
     }
     if (variant != KTK_VARIANT_SIMT && can_shared) {
-        if (p.splits <= 0) p.splits = attn_shared_splits(*shape, table->batch, new_indptr ? max_new : 0, 1 << 20);
+        const bool balanced = splits == KTK_SPLITS_BALANCED && !new_indptr &&
+                              workspace_bytes >= attn_shared_workspace(*shape, rows, splits) && workspace;
+        if (p.splits <= 0 && !balanced) p.splits = attn_shared_splits(*shape, table->batch, new_indptr ? max_new : 0, 1 << 20);
         const size_t need = attn_shared_workspace(*shape, rows, p.splits);
         if (need && (!workspace || workspace_bytes < need)) {
             set_error("%s: workspace of %zu bytes needed, got %zu", who, need, workspace ? workspace_bytes : (size_t)0);

@@ -140,6 +140,7 @@ int make_cache_maps(const AttnParams& p, struct CUtensorMap_st* k_map, struct CU
 int launch_attn_decode(const AttnParams& p, cudaStream_t st);
 bool attn_umma_supported(const ktk_attn& a);
 bool attn_shared_supported(const ktk_attn& a);
+bool attn_shared_balanced(const ktk_attn& a, int batch, int64_t max_keys);
 int32_t attn_shared_splits(const ktk_attn& a, int batch, int new_rows, int64_t max_keys);
 size_t attn_shared_workspace(const ktk_attn& a, int64_t rows, int splits);
 int launch_attn_shared(const AttnParams& p, cudaStream_t st);

@@ -34,14 +34,6 @@ constexpr int kMuTmemCols = 512;
 constexpr int kMuGatherers = 128;                  // threads
 constexpr int kMuBox = 32;                         // rows per TMA box of the rows in place
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {      // bytes 16, or 0: zeros
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-// arrives on the barrier when all cp.async of this thread so far have landed (one of the barrier's expected arrivals)
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // Position in a ring of `stages` stages: advanced by one, without a division.
 struct RingPos {
     int stage = 0;

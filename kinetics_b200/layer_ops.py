@@ -14,7 +14,7 @@ import torch
 
 from . import _lib
 from ._lib import VARIANT_AUTO, check_layers
-from .ops import _cuda, _dtype_code, _launched, _ptr, _stream
+from .ops import SPLITS_BALANCED, _cuda, _dtype_code, _launched, _ptr, _stream
 
 MAX_EXPERTS = 1024
 
@@ -268,6 +268,7 @@ def kv_append(proj, k_col: int, v_col: int, k_pages, v_pages, table: PageTable, 
 
 
 def attention_splits(spec: AttentionSpec, batch: int, max_keys: int, dtype, new_rows: int = 0) -> int:
+    """Parts that a sequence's keys are best cut into, or SPLITS_BALANCED: all sequences' page lists into equal parts."""
     a = spec.c(_lib.KTK_BF16 if dtype == torch.bfloat16 else _lib.KTK_F32)
     return int(_lib.load_layers().ktk_paged_attention_splits(ctypes.byref(a), batch, new_rows, max_keys))
 
@@ -295,7 +296,8 @@ def paged_attention(proj, k_pages, v_pages, table: PageTable, spec: AttentionSpe
     rows = proj.shape[0]
     if out is None:
         out = torch.empty(rows, spec.o_cols, dtype=proj.dtype, device=proj.device)
-    if splits > 1 and workspace is None:
+    cut = splits > 1 or splits == SPLITS_BALANCED
+    if cut and workspace is None:
         need = attention_workspace(spec, rows, splits, proj.dtype)
         if need:
             workspace = torch.empty(need, dtype=torch.uint8, device=proj.device)
@@ -304,7 +306,7 @@ def paged_attention(proj, k_pages, v_pages, table: PageTable, spec: AttentionSpe
         _ptr(proj), proj.shape[1], _ptr(new_indptr), rows, max_new, _ptr(k_pages), _ptr(v_pages), ctypes.byref(t),
         _ptr(sink), None if gate is None else gate.data_ptr(), 0 if gate is None else gate.stride(0), _ptr(out),
         _ptr(workspace), wsb, splits, variant, ctypes.byref(a), _ptr(status), _stream()))
-    _launched(2 if splits > 1 else 1)
+    _launched(2 if cut else 1)
     return out
 
 

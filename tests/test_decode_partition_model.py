@@ -89,3 +89,25 @@ def test_csr_entries():
         assert all(all(x == 1 for x in cv) for cv in covered.values())
         # lists without entries own no position: the combine pass writes their zero rows separately
         assert set(out) == {k for k, _, n, _ in units if n > 0}
+
+
+def test_rows_shared_by_all_heads():
+    """csrc/layers/ktl_attn_shared.cu, balanced: positions are page-list entries, chunks whole tiles of 64 tokens; the joining
+    pass reads the second slot of the CTA that a cut sequence starts in, then the first slot of those behind it."""
+    rng = random.Random(3)
+    for _ in range(1500):
+        ps, ctas = rng.choice([16, 32, 64]), rng.choice([1, 2, 9, 148])
+        ns = [rng.choice([1, 2, rng.randint(1, 90)]) for _ in range(rng.randint(1, 12))]
+        per = 64 // ps
+        total = sum(ns)
+        chunk = max(-(-(-(-total // ctas)) // per) * per, 4 * per)
+        units, pos = [], 0
+        for b, n in enumerate(ns):
+            units.append((b, pos, n, n))
+            pos += n
+        out, slots, covered = _walk(units, total, chunk, ctas)
+        assert not slots and len(out) == len(ns)
+        assert all(all(x == 1 for x in cv) for cv in covered.values())
+        for b, start, n, _ in units:                         # what the joining pass derives from the table alone
+            c0, pieces = start // chunk, (start + n - 1) // chunk - start // chunk + 1
+            assert (pieces == 1) == (out[b] == "direct") and c0 + pieces - 1 < ctas and pieces <= 256

@@ -53,6 +53,29 @@ def test_decode_rows(cuda_device, heads, cols, vdim):
             assert err < (1e-5 if dtype == F32 else 1.2e-2), (ps, splits, lens[i], err)
 
 
+# lengths: pieces of one to three tiles; more sequences than CTAs, some of one page; one sequence over every CTA
+BALANCED = [([1, 63, 64, 65, 200, 777, 2000], 64), ([1 + (37 * i) % 130 for i in range(400)], 16), ([70000], 32),
+            ([3000, 1, 9000, 16, 17, 5000] * 4, 64)]
+
+
+@pytest.mark.parametrize("heads,cols,vdim", [(16, 576, 512), (3, 72, 56), (70, 96, 8), (40, 264, 200)])
+@pytest.mark.parametrize("lens,ps", BALANCED)
+def test_decode_rows_balanced(cuda_device, heads, cols, vdim, lens, ps):
+    """The page lists cut over all sequences.  Bound: as in test_decode_rows."""
+    from kinetics_b200 import ops
+    spec = _spec(heads, cols, vdim, 1.1 / cols ** 0.5)
+    parts = [pointed_rows(n, n - 1, heads, cols, [0, 1, n // 2, 63, 64, n - 1], i, strength=8.0) for i, n in enumerate(lens)]
+    pages = RowPages([k for _, k in parts], BF, ps, cuda_device, 1)
+    g = torch.Generator().manual_seed(2)
+    sink, gate = 2.0 * torch.randn(heads, generator=g), torch.randn(len(lens), heads, generator=g)
+    got = _attend(cuda_device, spec, torch.cat([x for x, _ in parts]), pages, BF, sink, gate, None, 1, 0, ops.SPLITS_BALANCED)
+    r = lambda t: t.to(BF).double()
+    for i in list(range(len(lens)))[::1 + len(lens) // 40]:
+        q, k = parts[i]
+        want = plain_rows(r(q), r(k), vdim, spec.scale, sink.double(), r(gate[i:i + 1]), lens[i] - 1)
+        assert rms(got[i:i + 1] - want) / rms(want) < 1.2e-2, (i, lens[i])
+
+
 @pytest.mark.parametrize("heads,cols,vdim", SIZES)
 def test_portions(cuda_device, heads, cols, vdim):
     for seed, (ps, total, new, dtype) in enumerate([(64, 300, 300, BF), (16, 130, 2, BF), (64, 65, 3, BF), (32, 513, 70, BF),
