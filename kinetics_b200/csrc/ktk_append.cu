@@ -67,17 +67,27 @@ __device__ __forceinline__ int token_slot(int pos, int sink_tokens) {
     return pos < sink_tokens ? pos : (pos - sink_tokens) % kPageSize;
 }
 
+// E consecutive elements in one access
+template <typename T, int E> struct Piece { T x[E]; };
+template <> struct __align__(16) Piece<__nv_bfloat16, 8> { __nv_bfloat16 x[8]; };
+template <> struct __align__(8) Piece<__nv_bfloat16, 4> { __nv_bfloat16 x[4]; };
+template <> struct __align__(16) Piece<float, 4> { float x[4]; };
+constexpr int kAtWarps = 4, kAtBatch = 4;
+
 // Several tokens per sequence (prefill, chunked append): token j of the packed k / v belongs to the
 // sequence b with append_indptr[b] <= j < append_indptr[b+1] and is the (j - append_indptr[b])-th of the
-// sequence's n_app newest tokens.  grid (tokens, Hkv), one thread per head-dim element.
-template <typename T>
-__global__ void __launch_bounds__(kHeadDim)
-append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ append_indptr,
+// sequence's n_app newest tokens.  A warp per token, all heads, E elements per access (16 bytes; 1 element where a pointer is
+// not aligned) and kAtBatch of keys and of values in flight: bound by DRAM.  8192 tokens of 8 heads: 40 us with a CTA per token and
+// head, an element per thread.
+template <typename T, int E>
+__global__ void __launch_bounds__(kAtWarps * 32)
+append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ append_indptr, int total,
                      int B, T* __restrict__ cache, const int32_t* __restrict__ kv_indices,
                      const int32_t* __restrict__ kv_indptr, const int32_t* __restrict__ kv_last_page_len,
                      const int32_t* __restrict__ page_count, int sink_tokens, int Hkv, int64_t num_pages,
                      int32_t* status) {
-    const int j = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
+    const int j = blockIdx.x * kAtWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (j >= total) return;
     // the sequence that owns token j: last b with append_indptr[b] <= j
     int lo = 0, hi = B;
     while (hi - lo > 1) {
@@ -91,28 +101,39 @@ append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int
     const int n_pages = page_count ? page_count[b] : kv_indptr[b + 1] - beg;
     const int last = (n_pages > 0) ? kv_last_page_len[b] : 0;
     if (n_pages <= 0 || last < 1 || last > kPageSize) {
-        if (d == 0) report(status, KTK_STATUS_BAD_TABLE);
+        if (lane == 0) report(status, KTK_STATUS_BAD_TABLE);
         return;
     }
     const int pos = seq_tokens(n_pages, last, sink_tokens) - n_app + (j - a0);
     if (pos < 0) {
-        if (d == 0) report(status, KTK_STATUS_BAD_TABLE);
+        if (lane == 0) report(status, KTK_STATUS_BAD_TABLE);
         return;
     }
     const int64_t page = kv_indices[beg + token_page(pos, sink_tokens)];
     if (page < 0 || page >= num_pages) {
-        if (d == 0) report(status, KTK_STATUS_BAD_PAGE);
+        if (lane == 0) report(status, KTK_STATUS_BAD_PAGE);
         return;
     }
-    const int64_t row = (int64_t)Hkv * kHeadDim;
-    T* kp = cache + ((page * 2) * kPageSize + token_slot(pos, sink_tokens)) * row + (int64_t)h * kHeadDim + d;
-    const int64_t src = ((int64_t)j * Hkv + h) * kHeadDim + d;
-    kp[0] = k[src];
-    kp[kPageSize * row] = v[src];
+    using P = Piece<T, E>;
+    const int64_t row = (int64_t)Hkv * (kHeadDim / E);           // pieces of a token
+    P* kp = reinterpret_cast<P*>(cache) + ((page * 2) * kPageSize + token_slot(pos, sink_tokens)) * row;
+    P* vp = kp + kPageSize * row;
+    const P* ks = reinterpret_cast<const P*>(k) + j * row;
+    const P* vs = reinterpret_cast<const P*>(v) + j * row;
+    for (int64_t i0 = lane; i0 < row; i0 += 32 * kAtBatch) {
+        P kk[kAtBatch], vv[kAtBatch];
+#pragma unroll
+        for (int i = 0; i < kAtBatch; ++i)
+            if (i0 + 32 * i < row) { kk[i] = ks[i0 + 32 * i]; vv[i] = vs[i0 + 32 * i]; }
+#pragma unroll
+        for (int i = 0; i < kAtBatch; ++i)
+            if (i0 + 32 * i < row) { kp[i0 + 32 * i] = kk[i]; vp[i0 + 32 * i] = vv[i]; }
+    }
 }
 
-// grid (B, Hkv, Z): CTA z rebuilds the summaries of logical pages z, z+Z, ...
-template <typename T>
+// grid (B, Hkv, Z): a CTA rebuilds the summaries of E logical pages at a time, E elements of one per thread with all its tokens'
+// keys in flight (512 pages of 8 heads, all touched by one prompt: 15 us with an element per thread, 9 with eight).
+template <typename T, int E>
 __global__ void __launch_bounds__(kHeadDim)
 build_summaries_kernel(const T* __restrict__ cache, T* __restrict__ summaries,
                        int64_t summary_stride, const int32_t* __restrict__ kv_indices,
@@ -120,18 +141,20 @@ build_summaries_kernel(const T* __restrict__ cache, T* __restrict__ summaries,
                        const int32_t* __restrict__ kv_last_page_len, const int32_t* __restrict__ page_count,
                        const int32_t* __restrict__ slot_index, const int32_t* __restrict__ append_indptr,
                        int sink_tokens, int Hkv, int64_t num_pages, int32_t* status) {
-    const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
+    constexpr int kCols = kHeadDim / E;                          // threads of a page
+    using P = Piece<T, E>;
+    const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x % kCols, mine = threadIdx.x / kCols;
     const int beg = kv_indptr[b];
     const int n_pages = page_count ? page_count[b] : kv_indptr[b + 1] - beg;
     const int srow_b = slot_index ? slot_index[b] : b;
     if (n_pages <= 0) return;
     const int last = kv_last_page_len[b];
     if (last < 1 || last > kPageSize || n_pages > summary_stride) {
-        if (d == 0 && blockIdx.z == 0) report(status, KTK_STATUS_BAD_TABLE);
+        if (threadIdx.x == 0 && blockIdx.z == 0) report(status, KTK_STATUS_BAD_TABLE);
         return;
     }
-    const int64_t row = (int64_t)Hkv * kHeadDim;
-    T* sbase = summaries + ((int64_t)srow_b * Hkv + h) * summary_stride * kHeadDim + d;
+    const int64_t row = (int64_t)Hkv * kCols;
+    P* sbase = reinterpret_cast<P*>(summaries) + ((int64_t)srow_b * Hkv + h) * summary_stride * kCols + d;
     // after an append of several tokens only the pages they touched need a new summary
     int first = 0;
     if (append_indptr != nullptr) {
@@ -140,7 +163,7 @@ build_summaries_kernel(const T* __restrict__ cache, T* __restrict__ summaries,
         const int len = seq_tokens(n_pages, last, sink_tokens);
         first = token_page(len - n_app < 0 ? 0 : len - n_app, sink_tokens);
     }
-    for (int p = first + blockIdx.z; p < n_pages; p += gridDim.z) {
+    for (int64_t p = first + (int64_t)blockIdx.z * E + mine; p < n_pages; p += (int64_t)gridDim.z * E) {
         const int64_t page = kv_indices[beg + p];
         if (page < 0 || page >= num_pages) {
             if (d == 0) report(status, KTK_STATUS_BAD_PAGE);
@@ -148,15 +171,20 @@ build_summaries_kernel(const T* __restrict__ cache, T* __restrict__ summaries,
         }
         // a sink page (logical 0 under a view) holds sink_tokens keys unless it is also the last page
         const int c = (p == n_pages - 1) ? last : ((p == 0 && sink_tokens > 0) ? sink_tokens : kPageSize);
-        const T* kpage = cache + (page * 2) * kPageSize * row + (int64_t)h * kHeadDim + d;
-        float x[kPageSize];
-#pragma unroll
-        for (int t = 0; t < kPageSize; ++t) x[t] = (t < c) ? to_f32(kpage[t * row]) : 0.0f;
-        float acc = 0.0f;
+        const P* kpage = reinterpret_cast<const P*>(cache) + (page * 2) * kPageSize * row + (int64_t)h * kCols + d;
+        P x[kPageSize], out;
 #pragma unroll
         for (int t = 0; t < kPageSize; ++t)
-            if (t < c) acc = __fadd_rn(acc, x[t]);
-        sbase[(int64_t)p * kHeadDim] = from_f32<T>(__fdiv_rn(acc, (float)c));
+            if (t < c) x[t] = kpage[t * row];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            float acc = 0.0f;                                    // token by token, as the one-token append sums
+#pragma unroll
+            for (int t = 0; t < kPageSize; ++t)
+                if (t < c) acc = __fadd_rn(acc, to_f32(x[t].x[e]));
+            out.x[e] = from_f32<T>(__fdiv_rn(acc, (float)c));
+        }
+        sbase[p * kCols] = out;
     }
 }
 
@@ -241,15 +269,33 @@ static int build_impl(const void* cache, void* summaries, int64_t summary_stride
                       const int32_t* kv_indices, const int32_t* kv_indptr,
                       const int32_t* kv_last_page_len, const View& view, const ktk_shape* s, int32_t* status,
                       cudaStream_t st, const int32_t* append_indptr = nullptr) {
-    const int64_t bh = (int64_t)s->batch * s->num_kv_heads;
-    int z = (int)((8LL * sm_count() + bh - 1) / bh);
-    if (z < 1) z = 1;
-    if (z > 64) z = 64;
-    dim3 grid(s->batch, s->num_kv_heads, z);
-    build_summaries_kernel<T><<<grid, kHeadDim, 0, st>>>(
+    // CTAs for all pages a list can have, no more than keep the device busy; four elements a thread, whose 16 tokens fit more warps
+    // than those of eight
+    constexpr int kPiece = 4;
+    const bool aligned = ((((uintptr_t)cache) | (uintptr_t)summaries) & 15u) == 0;
+    const int64_t bh = (int64_t)s->batch * s->num_kv_heads, each = aligned ? kPiece : 1;
+    int64_t z = (16LL * sm_count() + bh - 1) / bh;
+    if (z > (summary_stride + each - 1) / each) z = (summary_stride + each - 1) / each;
+    dim3 grid(s->batch, s->num_kv_heads, (unsigned)(z < 1 ? 1 : z));
+    auto kernel = aligned ? build_summaries_kernel<T, kPiece> : build_summaries_kernel<T, 1>;
+    kernel<<<grid, kHeadDim, 0, st>>>(
         (const T*)cache, (T*)summaries, summary_stride, kv_indices, kv_indptr, kv_last_page_len,
         view.page_count, view.slot_index, append_indptr, view.sink_tokens, s->num_kv_heads, s->num_pages, status);
     KTK_CUDA_TRY(cudaGetLastError(), "ktk_build_summaries");
+    return KTK_OK;
+}
+
+template <typename T>
+static int append_tokens_impl(const void* k, const void* v, const int32_t* append_indptr, int64_t total, void* cache,
+                              const int32_t* kv_indices, const int32_t* kv_indptr, const int32_t* kv_last_page_len, const View& view,
+                              const ktk_shape* s, int32_t* status, cudaStream_t st) {
+    constexpr int kPiece = 16 / (int)sizeof(T);
+    const bool aligned = (((uintptr_t)k | (uintptr_t)v | (uintptr_t)cache) & 15u) == 0;
+    auto kernel = aligned ? append_tokens_kernel<T, kPiece> : append_tokens_kernel<T, 1>;
+    kernel<<<(unsigned)((total + kAtWarps - 1) / kAtWarps), kAtWarps * 32, 0, st>>>(
+        (const T*)k, (const T*)v, append_indptr, (int)total, s->batch, (T*)cache, kv_indices, kv_indptr, kv_last_page_len,
+        view.page_count, view.sink_tokens, s->num_kv_heads, s->num_pages, status);
+    KTK_CUDA_TRY(cudaGetLastError(), "ktk_append_tokens");
     return KTK_OK;
 }
 
@@ -341,17 +387,12 @@ extern "C" int ktk_append_tokens(const void* k, const void* v, const int32_t* ap
     }
     const View view = make_view(view_in);
     cudaStream_t st = (cudaStream_t)stream;
-    dim3 grid((unsigned)total_tokens, shape->num_kv_heads);
-    if (shape->dtype == KTK_F32)
-        append_tokens_kernel<float><<<grid, kHeadDim, 0, st>>>(
-            (const float*)k, (const float*)v, append_indptr, shape->batch, (float*)kv_cache, kv_indices, kv_indptr,
-            kv_last_page_len, view.page_count, view.sink_tokens, shape->num_kv_heads, shape->num_pages, status);
-    else
-        append_tokens_kernel<__nv_bfloat16><<<grid, kHeadDim, 0, st>>>(
-            (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, append_indptr, shape->batch, (__nv_bfloat16*)kv_cache,
-            kv_indices, kv_indptr, kv_last_page_len, view.page_count, view.sink_tokens, shape->num_kv_heads,
-            shape->num_pages, status);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_append_tokens");
+    rc = shape->dtype == KTK_F32
+             ? append_tokens_impl<float>(k, v, append_indptr, total_tokens, kv_cache, kv_indices, kv_indptr, kv_last_page_len, view,
+                                         shape, status, st)
+             : append_tokens_impl<__nv_bfloat16>(k, v, append_indptr, total_tokens, kv_cache, kv_indices, kv_indptr,
+                                                 kv_last_page_len, view, shape, status, st);
+    if (rc != KTK_OK) return rc;
     if (summaries == nullptr) return KTK_OK;
     if (shape->dtype == KTK_F32)
         return build_impl<float>(kv_cache, summaries, summary_stride, kv_indices, kv_indptr, kv_last_page_len, view,

@@ -575,3 +575,33 @@ def test_append_tokens_chunks_bit_exact(cuda_device, dtype, sink):
         npg = st_after["npages"][b]
         assert torch.equal(_bits(got[b, :, first:npg]), _bits(want_summ[b, :, first:npg]))
         assert not got[b, :, :first].any()               # pages in front of the chunk keep their summaries
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("Hkv", [1, 9])
+def test_append_tokens_by_pieces_bit_exact(cuda_device, dtype, shift, Hkv):
+    # a token's heads in less and in more than one batch of 16-byte pieces; tensors that start between two of them
+    ops = _ops()
+    lens = [300, 16, 1]
+    q, k, v = random_case(7, len(lens), Hkv, 1, lens, dtype)
+    st = paged_state(k, v, lens, dtype, seed=3, fill=0.0)
+    pack = lambda x: torch.cat([x[b, :, :n].transpose(0, 1) for b, n in enumerate(lens)]).to(dtype).contiguous()
+
+    def placed(t):
+        whole = torch.zeros(t.numel() + shift, dtype=t.dtype, device=cuda_device)
+        whole[shift:] = t.reshape(-1).to(cuda_device)
+        return whole[shift:].view(t.shape)
+
+    ai = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32)
+    d = to_dev(st, cuda_device)
+    cache = placed(torch.zeros_like(st["kv_cache"]))
+    summ = placed(torch.zeros(len(lens), Hkv, st["summary_stride"], 128, dtype=dtype))
+    status = ops.new_status(cuda_device)
+    ops.append_tokens(placed(pack(k)), placed(pack(v)), ai.to(cuda_device), cache, summ, d["kv_indices"], d["kv_indptr"],
+                      d["kv_last_page_len"], status=status)
+    ops.raise_on_status(status)
+    assert torch.equal(_bits(cache.cpu()), _bits(st["kv_cache"]))
+    want = oracle.summaries_v(st["kv_cache"], st["kv_indices"], st["kv_indptr"], st["kv_last_page_len"], st["summary_stride"], 0)
+    for b, n in enumerate(st["npages"]):
+        assert torch.equal(_bits(summ.cpu()[b, :, :n]), _bits(want[b, :, :n]))
