@@ -1,25 +1,28 @@
 // Decode attention of one new token per sequence over a paged cache with free head sizes (up to 128), two softmax maps
 // per head over shared values: bf16 tensor cores (mma.m16n8k16), TMA-staged pages.
 //
-// One CTA per (sequence, kv head and up to 8 of its query heads, split of the keys).  A producer warp streams units of
-// 16 tokens -- the keys of both maps and the values -- into a ring in shared memory; four consumer warps take units in
-// turn.  The heads are the 8 columns:
+// One CTA per (sequence, kv head and up to 8 of its query heads, split of the keys).  A producer warp streams stages of
+// 64 tokens -- the keys of both maps and the values -- into a ring in shared memory; each of four consumer warps takes
+// 16 tokens of a stage.  The heads are the 8 columns:
 //     S_m^T[16 keys x 8 heads] = K_m[16 x dim] . Q_m^T           per map m
 //     O_m^T[vdim x 8 heads]   += V^T[vdim x 16] . P_m^T          V fragments shared by the two maps
+// Bound by DRAM: 64 sequences of 8192 tokens, 16 / 4 heads, 64 + 64 key and 128 value columns, 1.07 GB: 161 us, 6.7 TB/s; 213 us
+// when the producer copied 16 tokens per map and chunk from a branch on its lane number.
 // At the end the warps add up, and either the head is finished here (one split: difference of the maps, unit norm) or
 // the un-normalised partials go to the workspace for the combine kernel.
+#include "../ktk_umma.cuh"
 #include "ktl_score.cuh"
 
 namespace ktk {
 
 constexpr int kAdConsumers = 4;
 constexpr int kAdThreads = (kAdConsumers + 1) * 32;
-constexpr int kAdStages = 8;          // a multiple of the consumers: a stage belongs to one warp
-constexpr int kAdUnit = 16;           // tokens per stage
-constexpr int kAdTile = kAdUnit * 128;
+constexpr int kAdStages = 2;
+constexpr int kAdUnit = 16;           // tokens of a consumer warp in a stage
+constexpr int kAdTok = kAdUnit * kAdConsumers;               // tokens of a stage
+constexpr int kAdTile = kAdTok * 128; // 64 columns of a stage's tokens
 constexpr int kAdMinKeys = 256;       // a split is not worth less
 constexpr int kAdMaxSplits = 256;
-static_assert(kAdStages % kAdConsumers == 0, "a stage must belong to one consumer warp");
 
 template <int DC, int VC> constexpr int ad_stage_bytes() { return (2 * DC + VC) * kAdTile; }
 template <int DC, int VC> constexpr int ad_smem() {
@@ -55,13 +58,13 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
         if (tid == 0) report(p.status, KTK_STATUS_BAD_TABLE);
         return;
     }
-    const int units = (s.total + kAdUnit - 1) / kAdUnit;
-    const int per = (units + p.splits - 1) / p.splits;
-    const int u0 = split * per, u1 = u0 + per < units ? u0 + per : units;
+    const int tiles = (s.total + kAdTok - 1) / kAdTok;           // stages of the sequence
+    const int per = (tiles + p.splits - 1) / p.splits;
+    const int u0 = split * per, u1 = u0 + per < tiles ? u0 + per : tiles;
     const int n = u1 > u0 ? u1 - u0 : 0;
 
     if (tid == 0) {
-        for (int i = 0; i < kAdStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < kAdStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], kAdConsumers); }
         abort_flag = 0;
         issued_total = 0;
         mbar_init_fence();
@@ -81,36 +84,51 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
     }
 
     if (warp == kAdConsumers) {
-        if (lane == 0) {
-            prefetch_tensormap(&k_map);
-            prefetch_tensormap(&v_map);
-            int i = 0;
-            for (; i < n; ++i) {
-                const int st = i % kAdStages;
-                const int tok = (u0 + i) * kAdUnit;
-                const int64_t page = p.t.kv_indices[s.start + tok / p.t.page_size];
-                if (i >= kAdStages && !mbar_wait(&empty[st], ((i / kAdStages) - 1) & 1, &abort_flag)) break;
-                if (page < 0 || page >= p.t.num_pages) {
-                    report(p.status, KTK_STATUS_BAD_PAGE);
-                    mbar_arrive(&full[st]);              // stale contents: the status word says so
-                    continue;
-                }
-                uint8_t* dst = ring + st * kStage;
-                const int y = tok % p.t.page_size;
-                mbar_arrive_expect_tx(&full[st], kStage);
-#pragma unroll
-                for (int mp = 0; mp < 2; ++mp)
-#pragma unroll
-                    for (int c = 0; c < DC; ++c)
-                        tma_load_3d(dst + (mp * DC + c) * kAdTile, &k_map, &full[st], c * 64, y,
-                                    (int)(page * (2 * a.kv_heads)) + kvh * 2 + mp);
-#pragma unroll
-                for (int c = 0; c < VC; ++c)
-                    tma_load_3d(dst + (2 * DC + c) * kAdTile, &v_map, &full[st], c * 64, y,
-                                (int)(page * a.kv_heads) + kvh);
+        if (lane == 0) { prefetch_tensormap(&k_map); prefetch_tensormap(&v_map); }
+        // page numbers: a lane keeps one of 32, the next 32 on their way.  One wait a stage and straight code with one lane elected
+        // around it: copies in a loop behind a branch on the lane number, 2 KiB each, kept an SM at 17 bytes a clock.
+        const int ps = p.t.page_size, per_tile = kAdTok / ps;
+        const int32_t* list = p.t.kv_indices + s.start + u0 * per_tile;
+        const int pages = min(n * per_tile, s.pages - u0 * per_tile);
+        int ids = lane < pages ? list[lane] : -1, next_ids = 32 + lane < pages ? list[32 + lane] : -1;
+        int i = 0;
+        for (; i < n; ++i) {
+            const int st = i % kAdStages, e0 = i * per_tile;
+            if (i > 0 && (e0 & 31) == 0) {
+                ids = next_ids;
+                next_ids = e0 + 32 + lane < pages ? list[e0 + 32 + lane] : -1;
             }
-            issued_total = i;
+            int z[kAdTok / 16], have = 0;
+#pragma unroll
+            for (int k = 0; k < kAdTok / 16; ++k) {
+                const int pg = __shfl_sync(0xffffffffu, ids, (e0 + k) & 31);
+                z[k] = -1;
+                if (k < per_tile && e0 + k < pages) {
+                    if (pg < 0 || pg >= p.t.num_pages) { if (lane == 0) report(p.status, KTK_STATUS_BAD_PAGE); }   // stale contents
+                    else { z[k] = pg; ++have; }
+                }
+            }
+            if (i >= kAdStages &&
+                !__all_sync(0xffffffffu, mbar_wait(&empty[st], ((i / kAdStages) - 1) & 1, &abort_flag))) break;
+            if (elect_one()) {
+                uint8_t* dst = ring + st * kStage;
+                if (have) mbar_arrive_expect_tx(&full[st], (uint32_t)(have * ps * 128 * (2 * DC + VC)));
+                else mbar_arrive(&full[st]);
+#pragma unroll
+                for (int k = 0; k < kAdTok / 16; ++k) {
+                    if (z[k] < 0) continue;
+#pragma unroll
+                    for (int c = 0; c < 2 * DC; ++c)
+                        tma_load_3d(dst + c * kAdTile + k * ps * 128, &k_map, &full[st], (c % DC) * 64, 0,
+                                    z[k] * (2 * a.kv_heads) + kvh * 2 + c / DC);
+#pragma unroll
+                    for (int c = 0; c < VC; ++c)
+                        tma_load_3d(dst + (2 * DC + c) * kAdTile + k * ps * 128, &v_map, &full[st], c * 64, 0, z[k] * a.kv_heads + kvh);
+                }
+            }
+            __syncwarp();
         }
+        if (lane == 0) issued_total = i;
     } else {
         const float factor = a.scale * query_temperature(a.temp_coef, a.temp_every, s.total - 1);
         CapCoef cap;
@@ -133,12 +151,17 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
         const int mj = lane >> 3, mr = lane & 7;
         const int k_tok = mr + 8 * (mj & 1), k_c = mj >> 1;
         const int v_tok = mr + 8 * (mj >> 1), v_c = mj & 1;
-        for (int i = warp; i < n; i += kAdConsumers) {
+        for (int i = 0; i < n; ++i) {
             const int st = i % kAdStages;
             if (!__all_sync(0xffffffffu, mbar_wait(&full[st], (i / kAdStages) & 1, &abort_flag))) break;
-            uint8_t* stage = ring + st * kStage;
-            const int left = s.total - (u0 + i) * kAdUnit;
+            uint8_t* stage = ring + st * kStage + warp * (kAdUnit * 128);        // this warp's tokens
+            const int left = s.total - (u0 + i) * kAdTok - warp * kAdUnit;
             const int ntok = left < kAdUnit ? left : kAdUnit;
+            if (ntok <= 0) {                             // behind the sequence
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[st]);
+                continue;
+            }
             const uint32_t kt = smem_u32(stage), vt = kt + 2 * DC * kAdTile;
             if (ntok < kAdUnit) {
                 // rows past the end may hold anything: clear them in V so that 0 * x stays 0
@@ -346,7 +369,7 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
     }
 }
 
-// One CTA per (head, row): merges the splits of both maps, takes the difference, unit norm.
+// One CTA per (head, row): merges the splits of both maps, takes the difference, unit norm.  Latency of the parts' loads.
 __global__ void __launch_bounds__(128) attn_combine_kernel(const AttnParams p, int fixed) {
     __shared__ float part[4];
     const ktk_attn& a = p.a;
@@ -354,22 +377,32 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const AttnParams p, i
     const int64_t row = blockIdx.y, head = blockIdx.x;
     const int64_t stride = ad_partial_floats(a.vdim_stride);
     const float* w = p.ws + (row * a.heads + head) * p.splits * stride;
-    float out[2];
-#pragma unroll
-    for (int mp = 0; mp < 2; ++mp) {
-        float M = fixed ? 0.0f : -INFINITY, L = 0.0f, O = 0.0f;
-        if (!fixed)
-            for (int s = 0; s < p.splits; ++s) M = fmaxf(M, w[s * stride + 2 * mp]);
-        const float ref = M == -INFINITY ? 0.0f : M;
+    float M[2] = {0.0f, 0.0f}, L[2] = {0.0f, 0.0f}, O[2] = {0.0f, 0.0f}, out[2];
+    if (!fixed) {
+        M[0] = M[1] = -INFINITY;
 #pragma unroll 4
         for (int s = 0; s < p.splits; ++s) {
-            const float* q = w + s * stride;
-            const float f = fixed ? 1.0f : ex2(q[2 * mp] - ref);
-            L += f * q[2 * mp + 1];
-            if (c < a.vdim_stride) O += f * q[4 + mp * a.vdim_stride + c];
+            const float4 q = *reinterpret_cast<const float4*>(w + s * stride);
+            M[0] = fmaxf(M[0], q.x);
+            M[1] = fmaxf(M[1], q.z);
         }
-        out[mp] = L > 0.0f && c < a.vdim ? O / L : 0.0f;
+        M[0] = M[0] == -INFINITY ? 0.0f : M[0];
+        M[1] = M[1] == -INFINITY ? 0.0f : M[1];
     }
+    const bool on = c < a.vdim_stride;
+#pragma unroll 6
+    for (int s = 0; s < p.splits; ++s) {                 // both maps' parts of several splits in flight
+        const float* q = w + s * stride;
+        const float4 ml = *reinterpret_cast<const float4*>(q);
+        const float o0 = on ? q[4 + c] : 0.0f, o1 = on ? q[4 + a.vdim_stride + c] : 0.0f;
+        const float f0 = fixed ? 1.0f : ex2(ml.x - M[0]), f1 = fixed ? 1.0f : ex2(ml.z - M[1]);
+        L[0] += f0 * ml.y;
+        L[1] += f1 * ml.w;
+        O[0] += f0 * o0;
+        O[1] += f1 * o1;
+    }
+#pragma unroll
+    for (int mp = 0; mp < 2; ++mp) out[mp] = L[mp] > 0.0f && c < a.vdim ? O[mp] / L[mp] : 0.0f;
     const float d = out[0] - a.lambda * out[1];
     const float ss = warp_sum_f(d * d);
     if ((c & 31) == 0) part[c >> 5] = ss;
@@ -387,8 +420,10 @@ static int64_t decode_units(const ktk_attn& a, int64_t batch) {
     return batch * a.kv_heads * ((group + 7) / 8);
 }
 
+// Two to four rounds: enough to even out ragged sequences (64 of 512 .. 8192 tokens: the model's step 267 us, 271 with up to eight
+// rounds), and with fewer partials the combine takes 5 us instead of 9.
 int32_t attn_decode_splits(const ktk_attn& a, int batch, int64_t max_keys) {
-    return fill_rounds(decode_units(a, batch), (int64_t)sm_count() * 3, 2, 8, (max_keys + kAdMinKeys - 1) / kAdMinKeys,
+    return fill_rounds(decode_units(a, batch), (int64_t)sm_count() * 3, 2, 4, (max_keys + kAdMinKeys - 1) / kAdMinKeys,
                        kAdMaxSplits);
 }
 
@@ -414,7 +449,7 @@ int make_cache_maps(const AttnParams& p, CUtensorMap* k_map, CUtensorMap* v_map,
 template <int DC, int VC, bool FIXED, int CTAS> static int decode_launch(const AttnParams& p, cudaStream_t st) {
     const char* who = "ktk_paged_attention";
     CUtensorMap km, vm;
-    const int rc = make_cache_maps(p, &km, &vm, kAdUnit, who);
+    const int rc = make_cache_maps(p, &km, &vm, p.t.page_size, who);
     if (rc != KTK_OK) return rc;
     constexpr int smem = ad_smem<DC, VC>();
     auto kernel = attn_decode_kernel<DC, VC, FIXED, CTAS>;

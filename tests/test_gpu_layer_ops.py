@@ -238,6 +238,15 @@ def test_far_keys_among_many(cuda_device):
     _close(got, want, torch.bfloat16)
 
 
+@pytest.mark.parametrize("page, splits", [(16, 1), (32, 1), (16, 3), (64, 2)])
+def test_far_keys_over_many_pages_of_a_decode_step(cuda_device, page, splits):
+    # the copying warp keeps 32 page numbers and the next 32: stages of 4, 2 and 1 pages across those borders
+    spec = _spec(4, 2, 64, 128, every=500.0)
+    at = [0, 511, 512, 513, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4200]
+    got, want = _run(cuda_device, spec, [4201, 4100, 513], None, page, MMA, torch.bfloat16, splits=splits, strength=6.0, edges=at)
+    _close(got, want, torch.bfloat16)
+
+
 def test_scores_beyond_the_polynomial_range(cuda_device):
     # |score / cap| runs from small to well beyond one: both branches of the softcap, in both kernels
     spec = _spec(2, 1, 64, 64, cap=5.0, lam=0.2)
