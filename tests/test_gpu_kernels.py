@@ -169,6 +169,37 @@ def test_select_many_ragged_items_per_cta(cuda_device, order):
     assert torch.equal(gp, phys)
 
 
+@pytest.mark.parametrize("B, Hkv, dtype, order", [(460, 1, torch.bfloat16, False), (300, 2, torch.bfloat16, True),
+                                                  (500, 1, torch.float32, True), (1500, 1, torch.bfloat16, False)])
+def test_select_takes_items_of_ctas_not_yet_started(cuda_device, B, Hkv, dtype, order):
+    """Long rows and more items than resident CTAs: a CTA goes on with items of CTAs that have not started.  Items of no page, of
+    one, within the budget and of fewer stages than a ring; with and without a sequence order."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(B)
+    stride, topk, G = 520, 20, 2
+    pages = torch.randint(2, 200, (B,), generator=g)
+    pages[torch.arange(0, B, 97)] = stride
+    pages[3], pages[4], pages[5], pages[B - 1] = 0, 1, topk, topk + 2
+    indptr = torch.cat((torch.zeros(1, dtype=torch.long), pages.cumsum(0))).to(torch.int32)
+    indices = torch.randperm(int(indptr[-1]), generator=g).to(torch.int32)
+    last = torch.randint(1, 17, (B,), generator=g).to(torch.int32)
+    summ = torch.randn(B, Hkv, stride, 128, generator=g).to(dtype)
+    q = torch.randn(B, Hkv * G, 128, generator=g).to(dtype)
+    phys, logical = oracle.select(q, summ, indices, indptr, topk)
+    view = None
+    if order:
+        view = ops.PageView(0, 1, None, None, torch.argsort(pages, descending=True, stable=True).to(torch.int32).to(cuda_device))
+    dev = lambda t: t.to(cuda_device)
+    status = ops.new_status(cuda_device)
+    for _ in range(3):                                       # who takes what differs from run to run
+        out_l = torch.full((B, Hkv, topk + 1), -7, dtype=torch.int32, device=cuda_device)
+        out_p = ops.select_pages(dev(q), dev(summ), dev(indices), dev(indptr), dev(last), topk, indices.numel(),
+                                 out_logical=out_l, status=status, view=view)
+        ops.raise_on_status(status)
+        assert torch.equal(out_l.cpu(), logical)
+        assert torch.equal(out_p.cpu(), phys)
+
+
 def test_select_reports_an_order_entry_that_is_no_sequence(cuda_device):
     ops = _ops()
     lens = [100, 200, 300]
