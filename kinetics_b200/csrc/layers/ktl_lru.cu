@@ -253,13 +253,18 @@ __global__ void __launch_bounds__(kLdThreads) lru_step_kernel(const LruParams p)
 }
 
 // ---- one token of every sequence in one launch: convolution, gate products on the tensor cores, recurrence, output gate ----
-// A CTA takes 32 channels of a block and up to 32 rows.  It convolves all channels of the block (the products need them;
-// their inputs lie in L2), multiplies u [32 x block] with the 32 + 32 gate rows by mma.m16n8k16, and finishes its channels.
-// The ring's place that a step writes is read by no other CTA.
-constexpr int kLfRows = 32, kLfChan = 32, kLfThreads = 256, kLfMaxBlock = 512;
+// A CTA takes CHAN channels of a block and up to 32 rows.  It convolves all channels of the block (the products need them;
+// their inputs lie in L2), multiplies u [32 x block] with the CHAN + CHAN gate rows by mma.m16n8k16, and finishes its channels.
+// The ring's place that a step writes is read by no other CTA.  Bound by latency: a chain of loads (slot, window and state), the
+// products, the stores; so a thread keeps to one piece of the channels and loads a tap's weights once, the state and the gate are on their
+// way before the products, and CHAN is what leaves one round of CTAs.
+constexpr int kLfRows = 32, kLfThreads = 256, kLfMaxBlock = 512;
 
 __host__ __device__ inline int lf_ld(int block_stride) { return (block_stride + 15) / 16 * 16 + 8; }      // padded: no bank conflicts
-__host__ __device__ inline int lf_smem(int block_stride) { return (kLfRows + 2 * kLfChan) * lf_ld(block_stride) * 2 + kLfRows * (2 * kLfChan + 1) * 4; }
+__host__ __device__ inline int lf_smem(int block_stride, int chan) { return (kLfRows + 2 * chan) * lf_ld(block_stride) * 2 + kLfRows * (2 * chan + 1) * 4; }
+
+// neighbouring channels of a lane, one access
+template <typename T, int N> struct alignas(N * sizeof(T)) Lanes { T x[N]; };
 
 struct LruDecodeParams {
     LruParams p;
@@ -268,28 +273,20 @@ struct LruDecodeParams {
     __nv_bfloat16* ring;
 };
 
-template <int TAPS> __global__ void __launch_bounds__(kLfThreads) lru_decode_kernel(const LruDecodeParams q) {
+template <int TAPS, int CHAN> __global__ void __launch_bounds__(kLfThreads, 2) lru_decode_kernel(const LruDecodeParams q) {
     extern __shared__ __align__(16) uint8_t lf_raw[];
     __shared__ int row_slot[kLfRows], row_pos[kLfRows];
     const LruParams& p = q.p;
     const int bs = p.a.block_stride, taps = p.a.taps, width = p.a.blocks * bs, ld = lf_ld(bs);
     __nv_bfloat16* su = reinterpret_cast<__nv_bfloat16*>(lf_raw);       // [rows][ld]
-    __nv_bfloat16* sw = su + kLfRows * ld;                              // [32 rows of r, 32 of i][ld]
-    float* sz = reinterpret_cast<float*>(sw + 2 * kLfChan * ld);            // [rows][32 zr | 32 zi | pad]
-    constexpr int kZ = 2 * kLfChan + 1;
+    __nv_bfloat16* sw = su + kLfRows * ld;                              // [CHAN rows of r, CHAN of i][ld]
+    float* sz = reinterpret_cast<float*>(sw + 2 * CHAN * ld);               // [rows][CHAN zr | CHAN zi | pad]
+    constexpr int kZ = 2 * CHAN + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int slices = (bs + kLfChan - 1) / kLfChan, blk = blockIdx.x / slices, n0 = (blockIdx.x - blk * slices) * kLfChan;
+    const int slices = (bs + CHAN - 1) / CHAN, blk = blockIdx.x / slices, n0 = (blockIdx.x - blk * slices) * CHAN;
     const int64_t r0 = (int64_t)blockIdx.y * kLfRows;
     const int rows = p.rows - r0 < kLfRows ? (int)(p.rows - r0) : kLfRows;
     const int c0 = blk * bs, pieces = (ld - 8) / 8;                     // 16-byte pieces of a row
-    // gate weights on their way; rows and columns outside are zero
-    for (int i = tid; i < 2 * kLfChan * pieces; i += kLfThreads) {
-        const int n = i / pieces, k = i - n * pieces, c = n0 + (n & (kLfChan - 1));
-        const bool on = c < bs && k * 8 < bs;
-        const __nv_bfloat16* src = q.gates + (on ? ((int64_t)(2 * blk + n / kLfChan) * bs + c) * bs + k * 8 : 0);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sw + n * ld + k * 8)), "l"(src),
-                     "r"(on ? 16u : 0u) : "memory");
-    }
     if (tid < kLfRows) {
         int slot = -1, pos = 0;
         if (tid < rows) {
@@ -304,96 +301,150 @@ template <int TAPS> __global__ void __launch_bounds__(kLfThreads) lru_decode_ker
         row_slot[tid] = slot;
         row_pos[tid] = pos;
     }
-    __syncthreads();
-    // u of every channel of the block: kBatch pieces per thread with all their loads in flight
-    constexpr int kBatch = TAPS > 0 ? 4 : 1, kTaps = TAPS > 0 ? TAPS : 1;
-    for (int i0 = tid; i0 < kLfRows * pieces; i0 += kLfThreads * kBatch) {
-        uint4 raw[kBatch][kTaps];
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-            const int i = i0 + b * kLfThreads, r = i / pieces, k = i - r * pieces;
-            const bool on = i < kLfRows * pieces && row_slot[r & (kLfRows - 1)] >= 0 && k * 8 < bs;
-            const int slot = on ? row_slot[r] : 0, pos = on ? row_pos[r] : 0, c = c0 + k * 8;
-            const __nv_bfloat16* mine = q.ring + (int64_t)slot * taps * width + c;
-#pragma unroll
-            for (int t = 0; t < kTaps; ++t) {                           // the last is the token's own
-                const int at = pos - (kTaps - 1) + t;
-                raw[b][t] = make_uint4(0u, 0u, 0u, 0u);                 // zeros before the sequence
-                if (t == kTaps - 1) { if (on) raw[b][t] = *reinterpret_cast<const uint4*>(q.x + (r0 + r) * p.row_stride + c); }
-                else if (on && at >= 0) raw[b][t] = *reinterpret_cast<const uint4*>(mine + (int64_t)(at % taps) * width);
-            }
+    // thread: piece k of rows first_row, + row_step, ...
+    int per = 8, shift = 3;                                             // threads of a row: the next power of two
+    while (per < pieces) { per *= 2; ++shift; }
+    const int k = tid & (per - 1), first_row = tid >> shift, row_step = kLfThreads >> shift, c_mine = c0 + k * 8;
+    const bool mine_on = k * 8 < bs;
+    // gate weights on their way; rows and columns outside are zero
+    if (k < pieces) {
+        const __nv_bfloat16* src = q.gates + ((int64_t)2 * blk * bs + n0) * bs + k * 8;
+        const uint32_t dst = smem_u32(sw + k * 8);
+#pragma unroll 4
+        for (int n = first_row; n < 2 * CHAN; n += row_step) {
+            const int c = n & (CHAN - 1);
+            const bool on = mine_on && n0 + c < bs;
+            cp_async16(dst + n * ld * 2, on ? src + (n < CHAN ? c : bs + c) * bs : q.gates, on ? 16u : 0u);
         }
+    }
+    constexpr int kTaps = TAPS > 0 ? TAPS : 1, kBatch = TAPS > 0 ? 2 : 1;
+    __syncthreads();
+    // this CTA's channels, CHAN / 32 neighbours per lane: state and gate of rows warp, + 8, ...
+    constexpr int kCols = CHAN / 32, kMine = kLfRows / (kLfThreads / 32);
+    using Floats = Lanes<float, kCols>;
+    using Halves = Lanes<__nv_bfloat16, kCols>;
+    const int n = n0 + lane * kCols, c = c0 + n;                        // a block's channels are a multiple of 8
+    Floats state0[kMine];
+    Halves gate[kMine];
 #pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-            const int i = i0 + b * kLfThreads, r = i / pieces, k = i - r * pieces, c = c0 + k * 8;
-            if (i >= kLfRows * pieces) continue;
-            float o[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (row_slot[r] >= 0 && k * 8 < bs) {
-                __nv_bfloat16* mine = q.ring + (int64_t)row_slot[r] * taps * width + c;
-                float v[8], w[8];
-                load8(q.conv_b + c, o);
+    for (int i = 0; i < kMine; ++i) {
+        const int r = warp + i * (kLfThreads / 32), slot = n < bs ? row_slot[r] : -1;
+#pragma unroll
+        for (int h = 0; h < kCols; ++h) { state0[i].x[h] = 0.0f; gate[i].x[h] = __float2bfloat16(0.0f); }
+        if (slot >= 0) {
+            if (row_pos[r] > 0) state0[i] = *reinterpret_cast<const Floats*>(p.state + (int64_t)slot * width + c);
+            gate[i] = *reinterpret_cast<const Halves*>((const __nv_bfloat16*)p.y + (r0 + r) * p.row_stride + c);
+        }
+    }
+    // u of every channel of the block: kBatch rows per thread with all their loads in flight
+    if (k < pieces)
+        for (int rb = first_row; rb < kLfRows; rb += row_step * kBatch) {
+            uint4 raw[kBatch][kTaps];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                const int r = rb + b * row_step;
+                const int slot = r < kLfRows && mine_on ? row_slot[r & (kLfRows - 1)] : -1, pos = slot >= 0 ? row_pos[r] : 0;
+                const __nv_bfloat16* mine = q.ring + (int64_t)(slot >= 0 ? slot : 0) * taps * width + c_mine;
+#pragma unroll
+                for (int t = 0; t < kTaps; ++t) {                       // the last is the token's own
+                    const int at = pos - (kTaps - 1) + t;
+                    raw[b][t] = make_uint4(0u, 0u, 0u, 0u);             // zeros before the sequence
+                    if (t == kTaps - 1) { if (slot >= 0) raw[b][t] = *reinterpret_cast<const uint4*>(q.x + (r0 + r) * p.row_stride + c_mine); }
+                    else if (slot >= 0 && at >= 0) raw[b][t] = *reinterpret_cast<const uint4*>(mine + (int64_t)(at % taps) * width);
+                }
+            }
+            float o[kBatch][8], w[8];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) o[b][e] = 0.0f;
+            if (mine_on) {                                              // a tap's weights serve the batch
+                load8(q.conv_b + c_mine, w);
+#pragma unroll
+                for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) o[b][e] = w[e];
                 if (TAPS == 0)
                     for (int t = 0; t + 1 < taps; ++t) {
-                        const int at = row_pos[r] - (taps - 1) + t;
+                        const int slot = rb < kLfRows ? row_slot[rb] : -1, at = slot >= 0 ? row_pos[rb] - (taps - 1) + t : -1;
                         if (at < 0) continue;
-                        Vec8<__nv_bfloat16>::load(mine + (int64_t)(at % taps) * width, v);
-                        load8(q.conv_w + (int64_t)t * width + c, w);
+                        float v[8];
+                        Vec8<__nv_bfloat16>::load(q.ring + ((int64_t)slot * taps + at % taps) * width + c_mine, v);
+                        load8(q.conv_w + (int64_t)t * width + c_mine, w);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) o[e] = fmaf(w[e], v[e], o[e]);
+                        for (int e = 0; e < 8; ++e) o[0][e] = fmaf(w[e], v[e], o[0][e]);
                     }
 #pragma unroll
                 for (int t = 0; t < kTaps; ++t) {
-                    unpack8(raw[b][t], v);
-                    load8(q.conv_w + (int64_t)(taps - kTaps + t) * width + c, w);
+                    load8(q.conv_w + (int64_t)(taps - kTaps + t) * width + c_mine, w);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) o[e] = fmaf(w[e], v[e], o[e]);
+                    for (int b = 0; b < kBatch; ++b) {
+                        float v[8];
+                        unpack8(raw[b][t], v);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[b][e] = fmaf(w[e], v[e], o[b][e]);
+                    }
                 }
-                if (k * 8 >= n0 && k * 8 < n0 + kLfChan)                 // this CTA's channels
-                    *reinterpret_cast<uint4*>(mine + (int64_t)(row_pos[r] % taps) * width) = raw[b][kTaps - 1];
             }
-            Vec8<__nv_bfloat16>::store(su + r * ld + k * 8, o);
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                const int r = rb + b * row_step;
+                if (r >= kLfRows) continue;
+                const int slot = mine_on ? row_slot[r] : -1;
+                if (slot >= 0 && k * 8 >= n0 && k * 8 < n0 + CHAN)      // this CTA's channels
+                    *reinterpret_cast<uint4*>(q.ring + ((int64_t)slot * taps + row_pos[r] % taps) * width + c_mine) = raw[b][kTaps - 1];
+                if (slot < 0)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) o[b][e] = 0.0f;
+                Vec8<__nv_bfloat16>::store(su + r * ld + k * 8, o[b]);
+            }
         }
-    }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     {
-        // warp: 16 rows, 16 of the 64 columns
-        const int gid = lane >> 2, tig = lane & 3, m0 = (warp & 1) * 16, g0 = (warp >> 1) * 16;
-        float acc[2][4] = {};
+        // warp: 16 rows, CHAN / 2 of the 2 CHAN columns
+        constexpr int kTiles = CHAN / 16;
+        const int gid = lane >> 2, tig = lane & 3, m0 = (warp & 1) * 16, g0 = (warp >> 1) * (CHAN / 2);
+        float acc[kTiles][4] = {};
         const __nv_bfloat16* a0 = su + (m0 + gid) * ld + 2 * tig;
         const __nv_bfloat16* b0 = sw + (g0 + gid) * ld + 2 * tig;
 #pragma unroll 4
-        for (int k = 0; k < ld - 8; k += 16) {
+        for (int kk = 0; kk < ld - 8; kk += 16) {
             uint32_t a[4];
-            a[0] = *reinterpret_cast<const uint32_t*>(a0 + k);
-            a[1] = *reinterpret_cast<const uint32_t*>(a0 + 8 * ld + k);
-            a[2] = *reinterpret_cast<const uint32_t*>(a0 + k + 8);
-            a[3] = *reinterpret_cast<const uint32_t*>(a0 + 8 * ld + k + 8);
+            a[0] = *reinterpret_cast<const uint32_t*>(a0 + kk);
+            a[1] = *reinterpret_cast<const uint32_t*>(a0 + 8 * ld + kk);
+            a[2] = *reinterpret_cast<const uint32_t*>(a0 + kk + 8);
+            a[3] = *reinterpret_cast<const uint32_t*>(a0 + 8 * ld + kk + 8);
 #pragma unroll
-            for (int t = 0; t < 2; ++t)
-                mma_bf16(acc[t], a, *reinterpret_cast<const uint32_t*>(b0 + t * 8 * ld + k),
-                         *reinterpret_cast<const uint32_t*>(b0 + t * 8 * ld + k + 8));
+            for (int t = 0; t < kTiles; ++t)
+                mma_bf16(acc[t], a, *reinterpret_cast<const uint32_t*>(b0 + t * 8 * ld + kk),
+                         *reinterpret_cast<const uint32_t*>(b0 + t * 8 * ld + kk + 8));
         }
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
+        for (int t = 0; t < kTiles; ++t)
 #pragma unroll
             for (int e = 0; e < 4; ++e) sz[(m0 + gid + (e >= 2 ? 8 : 0)) * kZ + g0 + t * 8 + 2 * tig + (e & 1)] = acc[t][e];
     }
     __syncthreads();
-    const int n = n0 + lane, c = c0 + n;
     if (n >= bs) return;
-    const float rb = p.rb[c], ib = p.ib[c], decay = p.decay[c];
+    const Floats rb = *reinterpret_cast<const Floats*>(p.rb + c), ib = *reinterpret_cast<const Floats*>(p.ib + c),
+                 decay = *reinterpret_cast<const Floats*>(p.decay + c);
 #pragma unroll
-    for (int r = warp; r < kLfRows; r += kLfThreads / 32) {
-        const int slot = row_slot[r];
+    for (int i = 0; i < kMine; ++i) {
+        const int r = warp + i * (kLfThreads / 32), slot = row_slot[r];
         if (slot < 0) continue;
-        float* state = p.state + (int64_t)slot * width + c;
-        float a, g;
-        gates<true>(sz[r * kZ + lane], sz[r * kZ + kLfChan + lane], __bfloat162float(su[r * ld + n]), rb, ib, decay, a, g);
-        const float S = fmaf(a, row_pos[r] > 0 ? *state : 0.0f, g);
-        *state = S;
-        ((__nv_bfloat16*)p.out)[(r0 + r) * width + c] =
-            __float2bfloat16_rn(S * gelu_tanh<true>(__bfloat162float(((const __nv_bfloat16*)p.y)[(r0 + r) * p.row_stride + c])));
+        Floats S;
+        Halves out;
+#pragma unroll
+        for (int h = 0; h < kCols; ++h) {
+            const int at = lane * kCols + h;
+            float a, g;
+            gates<true>(sz[r * kZ + at], sz[r * kZ + CHAN + at], __bfloat162float(su[r * ld + n + h]), rb.x[h], ib.x[h], decay.x[h], a, g);
+            S.x[h] = fmaf(a, state0[i].x[h], g);
+            out.x[h] = __float2bfloat16_rn(S.x[h] * gelu_tanh<true>(__bfloat162float(gate[i].x[h])));
+        }
+        *reinterpret_cast<Floats*>(p.state + (int64_t)slot * width + c) = S;
+        *reinterpret_cast<Halves*>((__nv_bfloat16*)p.out + (r0 + r) * width + c) = out;
     }
 }
 
@@ -521,11 +572,17 @@ extern "C" int ktk_lru_decode(const void* proj, int64_t row_stride, int64_t y_co
     const LruParams p{*shape, *table, nullptr, nullptr, (const __nv_bfloat16*)proj + y_col, row_stride, nullptr, slots, num_slots,
                       rows, 1, rb, ib, decay, state, out, status};
     const LruDecodeParams q{p, (const __nv_bfloat16*)proj + x_col, (const __nv_bfloat16*)gates, conv_w, conv_b, (__nv_bfloat16*)ring};
-    const int smem = lf_smem(shape->block_stride), slices = (shape->block_stride + kLfChan - 1) / kLfChan;
-    auto kernel = shape->taps == 4 ? lru_decode_kernel<4> : lru_decode_kernel<0>;
+    // 32 channels per CTA while those fit in one round (two CTAs of either form share an SM), 64 beyond that: 16 blocks of 256 channels,
+    // 128 rows: 29 us with 512 CTAs of 32 channels and an element per access, 14.7 with 256 of 64 in pairs
+    const int64_t groups = (rows + kLfRows - 1) / kLfRows;
+    const bool pairs = ((uintptr_t)state & 7u) == 0 && (((uintptr_t)rb | (uintptr_t)ib | (uintptr_t)decay) & 7u) == 0 && ((uintptr_t)out & 3u) == 0;
+    const bool narrow = !pairs || groups * shape->blocks * ((shape->block_stride + 31) / 32) <= 2 * (int64_t)sm_count() ||
+                        lf_smem(shape->block_stride, 64) > 200 * 1024;
+    const int chan = narrow ? 32 : 64, smem = lf_smem(shape->block_stride, chan), slices = (shape->block_stride + chan - 1) / chan;
+    auto kernel = shape->taps == 4 ? (narrow ? lru_decode_kernel<4, 32> : lru_decode_kernel<4, 64>)
+                                   : (narrow ? lru_decode_kernel<0, 32> : lru_decode_kernel<0, 64>);
     KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), who);
-    kernel<<<dim3((unsigned)(shape->blocks * slices), (unsigned)((rows + kLfRows - 1) / kLfRows)), kLfThreads, smem,
-             (cudaStream_t)stream>>>(q);
+    kernel<<<dim3((unsigned)(shape->blocks * slices), (unsigned)groups), kLfThreads, smem, (cudaStream_t)stream>>>(q);
     KTK_CUDA_TRY(cudaGetLastError(), who);
     return KTK_OK;
 }

@@ -440,6 +440,32 @@ def test_fused_steps_of_many_sequences_equal_the_separate_ones(cuda_device):
         assert torch.equal(a.ring, b.ring)
 
 
+@pytest.mark.parametrize("blocks,block,taps,rows,misaligned", [(16, 256, 4, 150, False), (16, 256, 4, 150, True), (20, 200, 3, 70, False),
+                                                               (30, 104, 4, 97, False), (5, 512, 4, 140, False)])
+def test_fused_steps_over_more_than_one_round_of_narrow_ctas(cuda_device, blocks, block, taps, rows, misaligned):
+    # CTAs of 64 channels, whole and partial slices of a block; a state that starts between two pairs keeps the narrow form.
+    # Bounds: as in test_fused_steps_of_many_sequences_equal_the_separate_ones
+    from kinetics_b200.layer_ops import LruSpec
+    spec, dev, g = LruSpec(blocks, block, taps), cuda_device, torch.Generator().manual_seed(rows)
+    c, spread = _lru_case(spec, rows, 4)
+    a, b = (_Lru(spec, [c], spread, BF, dev, rows + 3) for _ in range(2))
+    if misaligned:
+        b.state = torch.empty(b.state.numel() + 1, device=dev)[1:].view(b.state.shape)
+    slots = torch.randperm(rows + 3, generator=g)[:rows].tolist()
+    for lru in (a, b):
+        h = torch.Generator().manual_seed(1)
+        lru.state.copy_(torch.randn(lru.state.shape, generator=h))
+        lru.ring.copy_(torch.randn(lru.ring.shape, generator=h))
+    lens = torch.randint(1, 60, (rows,), generator=g).tolist()
+    lens[:5] = [1, 2, 3, 4, 5]
+    for step in range(2):
+        table = _length_table([n + step for n in lens], dev)
+        one, two = (m.run(spread(c["y"]), spread(c["x"]), table, slots, None, f) for m, f in ((a, False), (b, True)))
+        torch.testing.assert_close(one, two, rtol=2e-2, atol=2e-3)
+    torch.testing.assert_close(a.state, b.state, rtol=1e-3, atol=1e-4)
+    assert torch.equal(a.ring, b.ring)
+
+
 @pytest.mark.parametrize("dtype", [F32, BF])
 def test_long_memory_and_short_memory(cuda_device, dtype):
     # decays from "forgets at once" to "keeps for the whole sequence": the series and the difference in sqrt(1 - a^2)
