@@ -13,8 +13,9 @@
 //                       accumulators hold the output transposed: 16x256b loads give them as 8 x 8 fragments, gate and up
 //                       of a column in one thread, which stmatrix.trans lays down as rows that leave in 16-byte pieces.
 //                       Lanes that swapped neighbours and stored 2 or 4 bytes each held the tensor cores up: 8192 rows,
-//                       8 of 64 experts, 2048 -> 768 columns 415 + 247 us (stages 0 and 1), 381 + 195 this way, 354 + 165
-//                       without any epilogue.
+//                       8 of 64 experts, 2048 -> 768 columns 415 + 247 us (stages 0 and 1), 381 + 195 this way.
+// Now 354 + 166 us, 1.16 and 1.24 PFLOP/s: bound by what an SM reads from L2, 32 KiB per 64 columns (in stage 0 half of it by
+// cp.async).
 // Full tiles (prompts) run on pairs of CTAs (cta_group::2): 256 weight rows x 256 routed rows per item, each CTA with its
 // half of both in shared memory, which takes a third off the traffic from L2.  The second CTA's issuing warp tells the
 // first one's when its part of a stage has landed.
@@ -33,6 +34,13 @@ constexpr int kMuRing = 200 * 1024;                // bytes for the ring
 constexpr int kMuTmemCols = 512;
 constexpr int kMuGatherers = 128;                  // threads
 constexpr int kMuBox = 32;                         // rows per TMA box of the rows in place
+
+// 64-column chunks of a ring stage.  Waits, votes and copies of a stage take the loading warp 600 clocks, the products of one chunk
+// 512: two where it loads both operands (8192 rows, 8 of 64 experts, 768 -> 2048 columns 174 -> 166 us), one where it loads only the
+// weights (354 us, with two 359).
+__host__ __device__ constexpr int mu_chunks(bool pair, int stage) { return pair && stage == 1 ? 2 : 1; }
+// rows of a copy of the rows in place: those of a CTA in a pair, whose tiles are full or nearly so
+__host__ __device__ constexpr int mu_box(bool pair) { return pair ? kMuRows / 2 : kMuBox; }
 
 // Position in a ring of `stages` stages: advanced by one, without a division.
 struct RingPos {
@@ -59,13 +67,14 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int N = STAGE == 0 ? 2 * p.m.ff_stride : p.m.width_stride;       // weight rows
     const int K = STAGE == 0 ? p.m.width_stride : p.m.ff_stride;
-    const int steps = (K + kMuK - 1) / kMuK;
-    constexpr int kCtas = PAIR ? 2 : 1;
+    constexpr int kCtas = PAIR ? 2 : 1, kChunks = mu_chunks(PAIR, STAGE);
+    const int steps = (K + kChunks * kMuK - 1) / (kChunks * kMuK);
+    auto chunks_of = [&](int k) { return kChunks == 2 && (2 * k + 1) * kMuK >= K ? 1 : kChunks; };      // of step k
     constexpr int kPer = kMuRows / kCtas / 16;               // gathered rows per thread
     const int rank = PAIR ? (int)cluster_rank() : 0;
     const int unit = blockIdx.x / kCtas, num_units = gridDim.x / kCtas;
     const int blocks = (N + kCtas * kUmRows - 1) / (kCtas * kUmRows);
-    const int stage_bytes = kMuABytes + cta_rows * 128;
+    const int chunk_bytes = kMuABytes + cta_rows * 128, stage_bytes = kChunks * chunk_bytes;
 
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -118,8 +127,8 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
         for (int w = unit; w < work && alive; w += num_units) {
             const Item it = item(w);
             if (it.n <= 0) continue;
-            const int boxes = STAGE == 0 ? 0 : (it.m + kMuBox - 1) / kMuBox;
-            const uint32_t bytes = (uint32_t)(kMuABytes + boxes * kMuBox * 128);
+            const int box = mu_box(PAIR), boxes = STAGE == 0 ? 0 : (it.m + box - 1) / box;
+            const uint32_t bytes = (uint32_t)(kMuABytes + boxes * box * 128);
             const int row = plan.first_row[it.e] + it.r0 + it.m0;
             for (int k = 0; k < steps; ++k, ++issued, pos.next(stages)) {
                 const int s = pos.stage;
@@ -127,12 +136,21 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
                 if (pos.round > 0) ok = mbar_wait_fast(&empty[s], (pos.round - 1) & 1, &abort_flag);
                 if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                 uint8_t* st = ring + s * stage_bytes;
+                const int chunks = chunks_of(k);
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(&full[s], bytes);
-                    if (STAGE == 0) tma_load_5d(st, &w_map, &full[s], k * kMuK, 0, 0, it.wrow / 16, it.e);
-                    else tma_load_3d(st, &w_map, &full[s], k * kMuK, it.wrow, it.e);
-                    for (int i = 0; i < boxes; ++i)
-                        tma_load_3d(st + kMuABytes + i * kMuBox * 128, &in_map, &full[s], k * kMuK, row + i * kMuBox, 0);
+                    mbar_arrive_expect_tx(&full[s], bytes * chunks);
+#pragma unroll
+                    for (int c = 0; c < kChunks; ++c) {
+                        if (c >= chunks) break;
+                        uint8_t* at = st + c * chunk_bytes;
+                        const int col = (k * kChunks + c) * kMuK;
+                        if (STAGE == 0) tma_load_5d(at, &w_map, &full[s], col, 0, 0, it.wrow / 16, it.e);
+                        else tma_load_3d(at, &w_map, &full[s], col, it.wrow, it.e);
+                        if (STAGE == 1)                      // written out: a copy takes 13 clocks to issue, in a loop 170
+#pragma unroll
+                            for (int i = 0; i < (PAIR ? 1 : kMuRows / kMuBox); ++i)
+                                if (i < boxes) tma_load_3d(at + kMuABytes + i * box * 128, &in_map, &full[s], col, row + i * box, 0);
+                    }
                 }
                 __syncwarp();
             }
@@ -181,14 +199,20 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
                 bool ok = true;
                 if (pos.round > 0) ok = mbar_wait_fast(&empty[s], (pos.round - 1) & 1, &abort_flag);
                 if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
-                const uint32_t dst = dst0 + s * stage_bytes;
-                const bool in_row = k * kMuK + chunk * 8 < K;
-                const char* from = in_row ? base + (int64_t)k * (kMuK * 2) : base;
-                const uint32_t on = in_row ? 16u : 0u;
+                const int chunks = chunks_of(k);
 #pragma unroll
-                for (int i = 0; i < kPer; ++i)
-                    if (16 * i < it.m)                       // uniform
-                        cp_async16(dst + i * 2048, from + (uint64_t)off[i] * 16, bytes[i] & on);
+                for (int c = 0; c < kChunks; ++c) {
+                    if (c >= chunks) break;
+                    const uint32_t dst = dst0 + s * stage_bytes + c * chunk_bytes;
+                    const int col = (k * kChunks + c) * kMuK;
+                    const bool in_row = col + chunk * 8 < K;
+                    const char* from = in_row ? base + (int64_t)col * 2 : base;
+                    const uint32_t on = in_row ? 16u : 0u;
+#pragma unroll
+                    for (int i = 0; i < kPer; ++i)
+                        if (16 * i < it.m)                   // uniform
+                            cp_async16(dst + i * 2048, from + (uint64_t)off[i] * 16, bytes[i] & on);
+                }
                 cp_async_arrive(&full[s]);
             }
         }
@@ -199,6 +223,15 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
         bool alive = true;
         auto landed = [&](uint64_t* bar) {
             return __all_sync(0xffffffffu, mbar_wait_fast(bar, pos.round & 1, &abort_flag)) != 0;
+        };
+        // one look for both, a lane each: two waits one behind the other take longer than the matrix instructions in the queue
+        auto both_landed = [&](uint64_t* a, uint64_t* b) {
+            for (uint32_t i = 0; i < (1u << 24); ++i) {
+                if ((__ballot_sync(0xffffffffu, mbar_test(lane == 0 ? a : b, pos.round & 1)) & 3u) == 3u) return true;
+                if ((i & 63u) == 63u && *(volatile int*)&abort_flag) return false;
+            }
+            abort_flag = 1;
+            return false;
         };
         if (PAIR && rank == 1) {
             // the second CTA of a pair only reports what has landed
@@ -226,16 +259,21 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
                 tc_fence_after();
                 for (int k = 0; k < steps; ++k, pos.next(stages)) {
                     const int s = pos.stage;
-                    if (!landed(&full[s]) || (PAIR && !landed(&peer_full[s]))) { alive = false; break; }
+                    if (PAIR ? !both_landed(&full[s], &peer_full[s]) : !landed(&full[s])) { alive = false; break; }
                     if (STAGE == 0) fence_proxy_async();     // the gathered rows came through the generic proxy
                     tc_fence_after();
                     const uint64_t a = umma_desc_at(a0, s * stage_bytes), b = umma_desc_at(b0, s * stage_bytes);
+                    const int chunks = chunks_of(k);
                     if (elect_one()) {
 #pragma unroll
-                        for (int q = 0; q < kMuK / 16; ++q) {
-                            const uint32_t more = (k > 0 || q > 0) ? 1u : 0u;
-                            if (PAIR) umma_f16_pair(d, umma_desc_at(a, q * 32), umma_desc_at(b, q * 32), idesc, more);
-                            else umma_f16(d, umma_desc_at(a, q * 32), umma_desc_at(b, q * 32), idesc, more);
+                        for (int c = 0; c < kChunks; ++c) {
+                            if (c >= chunks) break;
+#pragma unroll
+                            for (int q = 0; q < kMuK / 16; ++q) {
+                                const uint32_t more = (k > 0 || c > 0 || q > 0) ? 1u : 0u, at = c * chunk_bytes + q * 32;
+                                if (PAIR) umma_f16_pair(d, umma_desc_at(a, at), umma_desc_at(b, at), idesc, more);
+                                else umma_f16(d, umma_desc_at(a, at), umma_desc_at(b, at), idesc, more);
+                            }
                         }
                         if (PAIR) umma_commit_pair(&empty[s]);
                         else umma_commit(&empty[s]);
@@ -366,10 +404,6 @@ template <int STAGE> static int moe_umma(const MoeParams& p, cudaStream_t st) {
         rc = make_tensor_map_3d(&w_map, p.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B, who);
     }
     if (rc != KTK_OK) return rc;
-    const uint64_t id[3] = {K, (uint64_t)(STAGE == 0 ? p.rows : routed), 1}, is[2] = {K * 2, K * id[1] * 2};
-    const uint32_t ib[3] = {kMuK, kMuBox, 1};
-    rc = make_tensor_map_3d(&in_map, p.in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, id, is, ib, CU_TENSOR_MAP_SWIZZLE_128B, who);
-    if (rc != KTK_OK) return rc;
     // tiles for twice the rows that an expert has on average (and never more than all of them): the ring's stages are
     // no larger than they have to be
     int64_t most = 2 * ((routed + p.m.experts - 1) / p.m.experts);
@@ -377,7 +411,11 @@ template <int STAGE> static int moe_umma(const MoeParams& p, cudaStream_t st) {
     const int tile_rows = (int)(most >= kMuRows ? kMuRows : (most + kMuBox - 1) / kMuBox * kMuBox);
     const bool pair = tile_rows == kMuRows;
     const int cta_rows = pair ? tile_rows / 2 : tile_rows;
-    const int stage_bytes = kMuABytes + cta_rows * 128;
+    const uint64_t id[3] = {K, (uint64_t)(STAGE == 0 ? p.rows : routed), 1}, is[2] = {K * 2, K * id[1] * 2};
+    const uint32_t ib[3] = {kMuK, (uint32_t)mu_box(pair), 1};
+    rc = make_tensor_map_3d(&in_map, p.in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, id, is, ib, CU_TENSOR_MAP_SWIZZLE_128B, who);
+    if (rc != KTK_OK) return rc;
+    const int stage_bytes = mu_chunks(pair, STAGE) * (kMuABytes + cta_rows * 128);
     const int stages = kMuRing / stage_bytes < kMuMaxStages ? kMuRing / stage_bytes : kMuMaxStages;
     const int ctas = pair ? 2 : 1;
     const int64_t per = (N + ctas * kUmRows - 1) / (ctas * kUmRows);
