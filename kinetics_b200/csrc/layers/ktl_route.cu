@@ -14,7 +14,6 @@ constexpr int kRtRows = 32;          // rows of a CTA, tensor-core variant
 constexpr int kRtCols = 64;          // experts per pass
 constexpr int kRtByRow = 256;        // up to this many rows: a CTA per row
 constexpr int kRtRowThreads = 512;
-static_assert(kMaxExperts * 2 * 4 <= 4 * (kRtRows + kRtCols) * 72 * 2, "the expert counters fit the ring");
 
 struct RouteParams {
     ktk_moe m;
@@ -122,15 +121,89 @@ __global__ void __launch_bounds__(kRtRowThreads) route_row_kernel(const RoutePar
     }
 }
 
-// A CTA takes 32 rows.  Columns 64 at a time: h [32 x 64] and W [64 experts x 64] through a ring of cp.async stages; warp
-// w accumulates experts 8 w .. 8 w + 7 of the pass for all 32 rows with mma.m16n8k16 (exact products, fp32 sums).
-constexpr int kRtK = 64, kRtStages = 4, kRtLd = kRtK + 8;        // padded rows: no bank conflicts
-constexpr int kRtStageElems = (kRtRows + kRtCols) * kRtLd;
+// The same for the four rows z, z + ld, ... of a warp side by side, whose lookups then share their latency: up to 256 experts, top up
+// to 32, the scores in registers.  The same choice and the same sums in the same order.
+constexpr int kRtPick = 4, kRtPickExperts = 256, kRtPickTop = 32;
+template <int kPer> __device__ __forceinline__ void pick_experts4(const RouteParams& p, float* z, int ld, int64_t row, int32_t* ids_s) {
+    const int lane = threadIdx.x & 31;
+    const int E = p.m.experts, top = p.m.top;
+    uint32_t key[kRtPick][kPer];
+    float denom[kRtPick], val[kRtPick];
+    int id[kRtPick];
+#pragma unroll
+    for (int r = 0; r < kRtPick; ++r) {
+        val[r] = 0.0f;
+        id[r] = 0;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) key[r][i] = lane + 32 * i < E ? score_to_key(z[r * ld + lane + 32 * i]) : 0u;
+        if (p.m.scoring == 1) {
+            float mx = -INFINITY, sum = 0.0f;
+            for (int i = lane; i < E; i += 32) mx = fmaxf(mx, z[r * ld + i]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            for (int i = lane; i < E; i += 32) sum += expf(z[r * ld + i] - mx);
+            denom[r] = warp_sum_f(sum);
+        } else denom[r] = 0.0f;
+    }
+    const uint32_t gone = score_to_key(-INFINITY);
+    for (int j = 0; j < top; ++j) {
+        uint32_t best[kRtPick];
+        int e[kRtPick];
+#pragma unroll
+        for (int r = 0; r < kRtPick; ++r) {
+            best[r] = 0u;
+            e[r] = E - 1;
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+                if (key[r][i] > best[r]) { best[r] = key[r][i]; e[r] = lane + 32 * i; }
+        }
+#pragma unroll
+        for (int r = 0; r < kRtPick; ++r) {
+            const uint32_t most = __reduce_max_sync(0xffffffffu, best[r]);
+            e[r] = (int)__reduce_min_sync(0xffffffffu, best[r] == most ? (uint32_t)e[r] : 0x7fffffffu);
+        }
+#pragma unroll
+        for (int r = 0; r < kRtPick; ++r) {
+            const float v = z[r * ld + e[r]];
+            if (lane == j) { val[r] = v; id[r] = e[r]; }
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+                if (e[r] == lane + 32 * i) key[r][i] = gone;
+        }
+        __syncwarp();
+        if (lane < kRtPick) z[lane * ld + (lane == 0 ? e[0] : lane == 1 ? e[1] : lane == 2 ? e[2] : e[3])] = -INFINITY;
+        __syncwarp();
+    }
+#pragma unroll
+    for (int r = 0; r < kRtPick; ++r) {
+        const float ex = expf(val[r] - __shfl_sync(0xffffffffu, val[r], 0));
+        if (p.m.scoring != 1)
+            for (int j = 0; j < top; ++j) denom[r] += __shfl_sync(0xffffffffu, ex, j);
+        const int64_t at = row + r;
+        if (lane < top && at < p.rows) {
+            ids_s[r * top + lane] = id[r];
+            p.ids[at * top + lane] = id[r];
+            p.weights[at * top + lane] = ex / denom[r];
+        }
+    }
+}
 
-__global__ void __launch_bounds__(kRtThreads) route_mma_kernel(const RouteParams p) {
+// A CTA takes 32 rows.  Columns 128 at a time: h [32 x 128] and W [64 experts x 128] through a ring of cp.async stages; warp
+// w accumulates 16 rows and 16 experts of the pass with mma.m16n8k16 (exact products, fp32 sums).  Bound by latency: 8192 rows of 2048
+// columns, 64 experts, 41 us with stages of 64 columns, a fragment per load and each row's choices one behind the other, 25 us this way (12 of them what W and h
+// take from L2).
+constexpr int kRtK = 128, kRtLd = kRtK + 8;                      // padded rows: no bank conflicts
+constexpr int kRtStageElems = (kRtRows + kRtCols) * kRtLd;
+constexpr int kRtPieces = (kRtRows + kRtCols) * (kRtK / 8) / kRtThreads, kRtPieceRows = kRtThreads / (kRtK / 8);
+static_assert(kMaxExperts * 2 * 4 <= 2 * kRtStageElems * 2, "the expert counters fit the ring");
+constexpr size_t kRtMostRest = 227 * 1024 - 54 * 1024;           // logits and choices; two stages fit beside them
+static_assert(2 * kRtStageElems * 2 <= 54 * 1024, "two stages fit");
+static_assert(kRtRows % kRtPieceRows == 0, "a thread's piece is one of h or one of W");
+
+template <int STAGES> __global__ void __launch_bounds__(kRtThreads) route_mma_kernel(const RouteParams p) {
     extern __shared__ __align__(16) uint8_t rt_raw[];     // ring | logits [32][experts padded to 64] | ids, places [32][top]
     __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(rt_raw);
-    float* rt_z = reinterpret_cast<float*>(rt_raw + kRtStages * kRtStageElems * 2);
+    float* rt_z = reinterpret_cast<float*>(rt_raw + STAGES * kRtStageElems * 2);
     int32_t* ids_s = reinterpret_cast<int32_t*>(rt_z + kRtRows * ((p.m.experts + kRtCols - 1) / kRtCols * kRtCols));
     int32_t* place_s = ids_s + kRtRows * p.m.top;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -138,66 +211,74 @@ __global__ void __launch_bounds__(kRtThreads) route_mma_kernel(const RouteParams
     const int E = p.m.experts, ld = (E + kRtCols - 1) / kRtCols * kRtCols;
     const int64_t row0 = (int64_t)blockIdx.x * kRtRows;
     const int K = p.m.width_stride, steps = (K + kRtK - 1) / kRtK;
-    const __nv_bfloat16* hp = (const __nv_bfloat16*)p.h;
-    const __nv_bfloat16* wp = (const __nv_bfloat16*)p.w;
+    // a thread copies columns `col` .. of every kRtPieceRows-th row, of h first, then of W
+    const int first = tid / (kRtK / 8), col = tid % (kRtK / 8) * 8;
+    const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 16;
     for (int c0 = 0; c0 < E; c0 += kRtCols) {
+        const __nv_bfloat16* src[kRtPieces];
+        bool on[kRtPieces];
+#pragma unroll
+        for (int i = 0; i < kRtPieces; ++i) {
+            const int r = first + i * kRtPieceRows;
+            const bool is_h = i * kRtPieceRows < kRtRows;
+            const int64_t at = is_h ? row0 + r : c0 + r - kRtRows;
+            on[i] = at < (is_h ? p.rows : (int64_t)E);
+            src[i] = (const __nv_bfloat16*)(is_h ? p.h : p.w) + (on[i] ? at * K + col : 0);
+        }
         auto load = [&](int s) {
-            __nv_bfloat16* st = ring + (s % kRtStages) * kRtStageElems;
-            for (int i = tid; i < (kRtRows + kRtCols) * (kRtK / 8); i += kRtThreads) {
-                const int r = i / (kRtK / 8), c = i % (kRtK / 8) * 8, k = s * kRtK + c;
-                const bool is_h = r < kRtRows;
-                const int64_t src_row = is_h ? row0 + r : c0 + r - kRtRows;
-                const bool on = k < K && src_row < (is_h ? p.rows : (int64_t)E);
-                const __nv_bfloat16* src = (is_h ? hp : wp) + (on ? src_row * K + k : 0);
-                const uint32_t bytes = on ? 16u : 0u;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(st + r * kRtLd + c)), "l"(src),
-                             "r"(bytes) : "memory");
-            }
+            const uint32_t dst = smem_u32(ring + (s % STAGES) * kRtStageElems + first * kRtLd + col);
+            const bool in = s * kRtK + col < K;
+#pragma unroll
+            for (int i = 0; i < kRtPieces; ++i)
+                cp_async16(dst + i * kRtPieceRows * kRtLd * 2, in ? src[i] + s * kRtK : (const __nv_bfloat16*)p.h, in && on[i] ? 16u : 0u);
         };
         float acc[2][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
-        for (int s = 0; s < kRtStages - 1; ++s) {
+        for (int s = 0; s < STAGES - 1; ++s) {
             if (s < steps) load(s);
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         for (int s = 0; s < steps; ++s) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(kRtStages - 2) : "memory");
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
             __syncthreads();                              // stage s is in place; everyone is done with stage s - 1
-            if (s + kRtStages - 1 < steps) load(s + kRtStages - 1);
+            if (s + STAGES - 1 < steps) load(s + STAGES - 1);
             asm volatile("cp.async.commit_group;" ::: "memory");
-            const __nv_bfloat16* st = ring + (s % kRtStages) * kRtStageElems;
-            const __nv_bfloat16* w = st + (kRtRows + warp * 8 + gid) * kRtLd + 2 * tig;
+            const __nv_bfloat16* st = ring + (s % STAGES) * kRtStageElems;
+            const uint32_t ha = smem_u32(st + (m0 + (lane & 15)) * kRtLd + (lane >> 4) * 8);
+            const uint32_t wa = smem_u32(st + (kRtRows + n0 + (lane & 7) + (lane >> 4) * 8) * kRtLd + ((lane >> 3) & 1) * 8);
 #pragma unroll
             for (int k = 0; k < kRtK; k += 16) {
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(w + k), b1 = *reinterpret_cast<const uint32_t*>(w + k + 8);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const __nv_bfloat16* h = st + (16 * i + gid) * kRtLd + 2 * tig + k;
-                    uint32_t a[4];
-                    a[0] = *reinterpret_cast<const uint32_t*>(h);
-                    a[1] = *reinterpret_cast<const uint32_t*>(h + 8 * kRtLd);
-                    a[2] = *reinterpret_cast<const uint32_t*>(h + 8);
-                    a[3] = *reinterpret_cast<const uint32_t*>(h + 8 * kRtLd + 8);
-                    mma_bf16(acc[i], a, b0, b1);
-                }
+                uint32_t a[4], b[4];
+                ldmatrix_x4(a, ha + k * 2);
+                ldmatrix_x4(b, wa + k * 2);
+                mma_bf16(acc[0], a, b[0], b[1]);
+                mma_bf16(acc[1], a, b[2], b[3]);
             }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        const int e = c0 + warp * 8 + 2 * tig;
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                const int col = e + (x & 1);
-                rt_z[(16 * i + gid + (x >= 2 ? 8 : 0)) * ld + col] = acc[i][x] + (p.b && col < E ? p.b[col] : 0.0f);
+                const int e = c0 + n0 + 8 * t + 2 * tig + (x & 1);
+                rt_z[(m0 + gid + (x >= 2 ? 8 : 0)) * ld + e] = acc[t][x] + (p.b && e < E ? p.b[e] : 0.0f);
             }
         __syncthreads();
     }
-    for (int r = warp; r < kRtRows; r += kRtWarps)
-        if (row0 + r < p.rows) pick_experts(p, rt_z + r * ld, row0 + r, ids_s + r * p.m.top);
+    static_assert(kRtRows == kRtPick * kRtWarps, "a warp's rows at once");
+    if (E <= kRtPickExperts && p.m.top <= kRtPickTop) {
+        float* z = rt_z + warp * kRtPick * ld;
+        int32_t* ids = ids_s + warp * kRtPick * p.m.top;
+        const int64_t row = row0 + warp * kRtPick;
+        if (E <= 64) pick_experts4<2>(p, z, ld, row, ids);
+        else if (E <= 128) pick_experts4<4>(p, z, ld, row, ids);
+        else pick_experts4<8>(p, z, ld, row, ids);
+    } else
+        for (int r = warp; r < kRtRows; r += kRtWarps)
+            if (row0 + r < p.rows) pick_experts(p, rt_z + r * ld, row0 + r, ids_s + r * p.m.top);
     // places in the buckets: counted in shared memory, one global addition per expert and CTA
     int32_t* count = reinterpret_cast<int32_t*>(ring);    // [experts] | [experts] first place
     for (int e = tid; e < E; e += kRtThreads) count[e] = 0;
@@ -255,16 +336,18 @@ extern "C" int ktk_moe_route(const void* h, const void* w, const float* b, int32
         KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), who);
         kernel<<<(unsigned)rows, kRtRowThreads, smem, st>>>(p);
     } else {
-        const size_t smem = (size_t)kRtStages * kRtStageElems * 2 +
-                            (size_t)kRtRows * ((shape->experts + kRtCols - 1) / kRtCols * kRtCols) * sizeof(float) +
+        const size_t ring = (size_t)kRtStageElems * 2;    // of a stage
+        const size_t rest = (size_t)kRtRows * ((shape->experts + kRtCols - 1) / kRtCols * kRtCols) * sizeof(float) +
                             (size_t)2 * kRtRows * shape->top * sizeof(int32_t);
-        if (smem > 227 * 1024) {
+        const int stages = rest + 3 * ring <= 227 * 1024 ? 3 : 2;
+        const size_t smem = rest + stages * ring;
+        if (rest > kRtMostRest) {
             set_error("%s: top %d of %d experts", who, shape->top, shape->experts);
             return KTK_ERR_UNSUPPORTED;
         }
-        KTK_CUDA_TRY(cudaFuncSetAttribute(route_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                     who);
-        route_mma_kernel<<<(unsigned)((rows + kRtRows - 1) / kRtRows), kRtThreads, smem, st>>>(p);
+        auto kernel = stages == 3 ? route_mma_kernel<3> : route_mma_kernel<2>;
+        KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), who);
+        kernel<<<(unsigned)((rows + kRtRows - 1) / kRtRows), kRtThreads, smem, st>>>(p);
     }
     KTK_CUDA_TRY(cudaGetLastError(), who);
     return KTK_OK;

@@ -371,6 +371,32 @@ def test_router(cuda_device, dtype, variant, rows, experts, top, width, ff):
         assert sorted(bucket[e, :counts[e]].tolist()) == (ids.reshape(-1) == e).nonzero().reshape(-1).tolist()
 
 
+@pytest.mark.parametrize("score_all", [False, True])
+@pytest.mark.parametrize("rows, experts, top, width", [(33, 64, 1, 136), (70, 65, 32, 264), (31, 128, 8, 128), (100, 129, 5, 72),
+                                                       (64, 256, 32, 520), (40, 257, 3, 64), (40, 96, 33, 64)])
+def test_router_by_tiles(cuda_device, rows, experts, top, width, score_all):
+    # every number of scores per lane, the most choices that four rows make side by side, and one more expert and choice
+    from kinetics_b200 import layer_ops as lo
+    c = _moe_case(rows, experts, top, width, 16, torch.bfloat16, seed=experts)
+    c["h"][3], c["b"][5:9] = 0.0, c["b"][5]                 # a row with equal scores among its best: ties to the lower index
+    d = c["dev"](cuda_device)
+    r = lo.moe_route(d["h"], d["router"], d["b"], lo.MoeSpec(experts, top, width, 16, score_all=score_all), variant=MMA)
+    z = c["h"].double() @ c["router"].double().t() + c["b"].double()
+    ids = r.ids.cpu().long()
+    got = z.gather(1, ids)
+    torch.testing.assert_close(got, torch.topk(z, top, dim=1).values, rtol=1e-4, atol=1e-4)
+    assert all(len(set(row.tolist())) == top for row in ids)
+    tied = [e for e in ids[3].tolist() if 5 <= e < 9]
+    assert tied == list(range(5, 5 + len(tied)))
+    weights = torch.softmax(z, dim=1).gather(1, ids) if score_all else torch.softmax(got, dim=1)
+    torch.testing.assert_close(r.weights.cpu().double(), weights, rtol=1e-4, atol=1e-4)
+    counts = torch.bincount(ids.reshape(-1), minlength=experts)
+    assert torch.equal(r.counts.cpu().long(), counts)
+    bucket = r.bucket.cpu()
+    for e in range(experts):
+        assert sorted(bucket[e, :counts[e]].tolist()) == (ids.reshape(-1) == e).nonzero().reshape(-1).tolist()
+
+
 @pytest.mark.parametrize("dtype, variant", [(torch.float32, SIMT), (torch.bfloat16, SIMT), (torch.bfloat16, UMMA)])
 @pytest.mark.parametrize("rows, experts, top, width, ff", MOE)
 @pytest.mark.parametrize("skew", [0.0, 50.0])
