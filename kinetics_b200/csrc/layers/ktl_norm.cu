@@ -2,12 +2,12 @@
 // its parts) is normalised and added, the new stream normalised for the next sublayer.  The stream and everything
 // computed here is fp32; a CTA has one row at a time in registers, 8 elements per access.
 //
-// Bound by DRAM for prompts, by its chain of reductions for few rows: one barrier per sum.  8192 rows of 2048 columns in bf16, 201 MB:
-// 60 us with two barriers per sum, 54 with one, 51 where CTAs walk rows with the next one in flight; eight parts 94, 88.  What keeps
-// rows in flight otherwise is the number of CTAs that the registers allow (rn_resident): half as many, for the registers of a row
-// ahead, made eight parts of 4096 columns 211 us instead of 167, of 5120 columns 178 for 112 (3000 rows).
+// Bound by DRAM for prompts, by its chain of reductions for few rows: one barrier per sum.  What keeps rows in flight is the number of
+// CTAs that the registers allow (rn_resident), and where CTAs walk rows a ring in shared memory (residual_norm_launch): the next row in
+// registers instead, half as many CTAs, made eight parts of 4096 columns 211 us instead of 167.
 #include <type_traits>
 
+#include "../ktk_pipeline.cuh"
 #include "../ktk_vec.cuh"
 #include "ktk_layers.h"
 
@@ -17,10 +17,7 @@ constexpr int kRnThreads = 256;
 constexpr int kRnMaxVec = 8;      // 8 x 8 elements per thread: rows of up to 16384 columns
 // CTAs of full width that an SM's registers have to hold: where each takes a row, and of those that walk rows
 __host__ __device__ constexpr int rn_resident(int nv) { return nv <= 1 ? 4 : nv <= 2 ? 3 : nv <= 4 ? 2 : 1; }
-constexpr int kRnWalkers = 3;
-// CTAs walk from this many rows each: 3000 rows of 2048 bf16 columns 19.7 us with a CTA per row and 20.0 with walkers, 8192 rows 54.3
-// and 50.9.  Not rows of fewer warps (1024 columns: 23.4 and 24.3), of fp32 (61.3 and 62.4) or of several parts.
-constexpr int kRnWalkRows = 8;
+constexpr int kRnStages = 2;       // of a walker: one row at work, one on its way; more take the L1 that holds the weights
 
 struct ResidualNormParams {
     const int64_t* tokens;
@@ -63,21 +60,6 @@ struct RowParts {
     }
 };
 
-// 8 elements as they lie in memory
-template <typename T> struct Raw8;
-template <> struct Raw8<float> {
-    float4 a, b;
-    __device__ __forceinline__ void load(const float* p) { a = *reinterpret_cast<const float4*>(p); b = *(reinterpret_cast<const float4*>(p) + 1); }
-    __device__ __forceinline__ void get(float (&f)[8]) const {
-        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-    }
-};
-template <> struct Raw8<__nv_bfloat16> {
-    uint4 a;
-    __device__ __forceinline__ void load(const __nv_bfloat16* p) { a = *reinterpret_cast<const uint4*>(p); }
-    __device__ __forceinline__ void get(float (&f)[8]) const { unpack8(a, f); }
-};
-
 // v <- norm(v; w, b), in registers; elements past `cols` are zero before and after (their w and b are)
 template <int NV>
 __device__ __forceinline__ void norm_regs(float (&v)[NV][8], const float* w, const float* b, float eps, bool center,
@@ -113,128 +95,195 @@ __device__ __forceinline__ void norm_regs(float (&v)[NV][8], const float* w, con
     }
 }
 
-// TOKENS: the stream starts as embedding rows.  WALK: the CTA walks rows, the next one in flight
-template <typename T, int NV, bool TOKENS, bool WALK>
-__global__ void __launch_bounds__(kRnThreads, WALK ? kRnWalkers : rn_resident(NV)) residual_norm_kernel(const ResidualNormParams p) {
+// The row's own part: x and y (its parts' sum) in registers, the new stream and its norm to memory.  TOKENS: the stream starts as
+// embedding rows, scaled here.
+template <typename T, int NV, bool TOKENS>
+__device__ __forceinline__ void finish_row(const ResidualNormParams& p, int64_t r, float (&x)[NV][8], float (&y)[NV][8], int nvec,
+                                           RowParts& part) {
+    if (TOKENS) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[i][e] *= p.embed_scale;
+    }
+    if (p.y != nullptr) {
+        if (p.post_w != nullptr) norm_regs<NV>(y, p.post_w, p.post_b, p.eps, p.center != 0, p.cols, nvec, part);
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[i][e] += p.mult * y[i][e];
+    }
+    if (TOKENS || p.y != nullptr) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int k = threadIdx.x + i * blockDim.x;
+            if (k < nvec) Vec8<float>::store(p.x + r * p.stride + k * 8, x[i]);
+        }
+    }
+    if (p.h != nullptr) {
+        if (p.pre_w != nullptr) norm_regs<NV>(x, p.pre_w, p.pre_b, p.eps, p.center != 0, p.cols, nvec, part);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int k = threadIdx.x + i * blockDim.x;
+            if (k < nvec) Vec8<T>::store((T*)p.h + r * p.stride + k * 8, x[i]);
+        }
+    }
+}
+
+template <typename T, bool TOKENS> struct RowSource {
     using Stream = typename std::conditional<TOKENS, T, float>::type;
+    const ResidualNormParams& p;
+    // where row r of the stream lies; one thread of the CTA says so if its token is none of the vocabulary
+    __device__ __forceinline__ const Stream* stream(int64_t r, bool tell) const {
+        if (!TOKENS) return (const Stream*)p.x + r * p.stride;
+        const int64_t t = p.tokens[r];
+        if (t >= 0 && t < p.vocab) return (const Stream*)p.embed + t * p.stride;
+        if (tell) report(p.status, KTK_STATUS_BAD_TABLE);
+        return (const Stream*)p.embed;
+    }
+};
+
+__device__ __forceinline__ void clear_counts(const ResidualNormParams& p) {
+    if (p.zero != nullptr && blockIdx.x == 0)
+        for (int i = threadIdx.x; i < p.zero_n; i += blockDim.x) p.zero[i] = 0;
+}
+
+// A CTA per row.
+template <typename T, int NV, bool TOKENS>
+__global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_kernel(const ResidualNormParams p) {
     __shared__ __align__(16) float part_s[2 * (kRnThreads / 32)];
     RowParts part{part_s};
     part.clear();
+    clear_counts(p);
     const int nvec = p.stride / 8;
-    if (p.zero != nullptr && blockIdx.x == 0)
-        for (int i = threadIdx.x; i < p.zero_n; i += blockDim.x) p.zero[i] = 0;
-    auto token = [&](int64_t r) -> int64_t {
-        if (!TOKENS || r >= p.rows) return 0;
-        const int64_t t = p.tokens[r];
-        if (t >= 0 && t < p.vocab) return t;
-        if (threadIdx.x == 0) report(p.status, KTK_STATUS_BAD_TABLE);
-        return 0;
-    };
-    auto stream_row = [&](int64_t r, int64_t tok) {
-        return TOKENS ? (const Stream*)p.embed + tok * p.stride : (const Stream*)p.x + r * p.stride;
-    };
-    Raw8<Stream> xr[WALK ? NV : 1];
-    Raw8<T> yr[WALK ? NV : 1];
-    auto fetch = [&](int64_t r, int64_t tok) {             // WALK
-        if (r >= p.rows) return;
-        const Stream* from = stream_row(r, tok);
+    const int64_t r = blockIdx.x;
+    const auto* from = RowSource<T, TOKENS>{p}.stream(r, threadIdx.x == 0);
+    float x[NV][8], y[NV][8];
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int k = threadIdx.x + i * blockDim.x;
-            if (k >= nvec) continue;
-            xr[WALK ? i : 0].load(from + k * 8);
-            if (p.y != nullptr) yr[WALK ? i : 0].load((const T*)p.y + r * p.stride + k * 8);
-        }
-    };
-    int64_t r = blockIdx.x, ahead = token(r);
-    if (WALK) {
-        fetch(r, ahead);
-        ahead = token(r + gridDim.x);
+    for (int i = 0; i < NV; ++i) {
+        const int k = threadIdx.x + i * blockDim.x;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[i][e] = 0.0f;
+        if (k < nvec) Vec8<typename RowSource<T, TOKENS>::Stream>::load(from + k * 8, x[i]);
     }
-    for (; r < p.rows; r += gridDim.x) {
-        float x[NV][8], y[NV][8];
-        float* xrow = p.x + r * p.stride;
+    if (p.y != nullptr) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int k = threadIdx.x + i * blockDim.x;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[i][e] = 0.0f;
+            for (int e = 0; e < 8; ++e) y[i][e] = 0.0f;
             if (k >= nvec) continue;
-            if (!WALK) xr[0].load(stream_row(r, ahead) + k * 8);
-            xr[WALK ? i : 0].get(x[i]);
-            if (TOKENS) {
+            for (int j = 0; j < p.parts; ++j) {
+                float t[8];
+                Vec8<T>::load((const T*)p.y + (r * p.parts + j) * p.stride + k * 8, t);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) x[i][e] *= p.embed_scale;
+                for (int e = 0; e < 8; ++e) y[i][e] += t[e];
             }
         }
-        if (p.y != nullptr) {
+    }
+    finish_row<T, NV, TOKENS>(p, r, x, y, nvec, part);
+}
+
+// CTAs that walk rows c, c + gridDim.x, ...; a ring in shared memory keeps the next row on its way by bulk copies, a stage holding a row
+// of the stream and its part.  8192 rows of 4096 bf16 columns inside a model 91 -> 72 us (402 MB).
+template <typename T, bool TOKENS>
+__global__ void __launch_bounds__(kRnThreads, rn_resident(2)) residual_norm_walk_kernel(const ResidualNormParams p) {
+    constexpr int NV = 2, stages = kRnStages;
+    extern __shared__ __align__(128) uint8_t rn_ring[];
+    __shared__ __align__(8) uint64_t full[kRnStages];
+    __shared__ __align__(16) float part_s[2 * (kRnThreads / 32)];
+    __shared__ int abort_flag;
+    using Source = RowSource<T, TOKENS>;
+    const Source source{p};
+    RowParts part{part_s};
+    part.clear();
+    clear_counts(p);
+    const int nvec = p.stride / 8, parts = p.y != nullptr ? p.parts : 0;
+    const uint32_t x_bytes = (uint32_t)(p.stride * sizeof(typename Source::Stream)), y_bytes = (uint32_t)(parts * p.stride * sizeof(T));
+    const uint32_t stage_bytes = x_bytes + y_bytes;
+    const bool sums = (p.y != nullptr && p.post_w != nullptr) || (p.h != nullptr && p.pre_w != nullptr);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < stages; ++i) mbar_init(&full[i], 1);
+        abort_flag = 0;
+        mbar_init_fence();
+    }
+    __syncthreads();
+    int issued = 0;                                          // rows asked for, by thread 0
+    auto ask = [&](int64_t r) {
+        if (r >= p.rows) return;
+        const int s = issued++ % stages;
+        uint8_t* at = rn_ring + s * stage_bytes;
+        mbar_arrive_expect_tx(&full[s], stage_bytes);
+        bulk_load(at, source.stream(r, true), x_bytes, &full[s]);
+        if (y_bytes) bulk_load(at + x_bytes, (const T*)p.y + r * parts * p.stride, y_bytes, &full[s]);
+    };
+    const int64_t step = gridDim.x;
+    if (threadIdx.x == 0)
+        for (int i = 0; i < stages; ++i) ask(blockIdx.x + i * step);
+    int s = 0;
+    uint32_t parity = 0;
+    int64_t r = blockIdx.x;
+    for (int i = 0; r < p.rows; ++i, r += step) {
+        if (!mbar_wait(&full[s], parity, &abort_flag)) break;
+        if (threadIdx.x == 0 && i > 0) {                     // everybody has read the row before: its sums had a barrier
+            fence_proxy_async();
+            ask(r + (stages - 1) * step);
+        }
+        const auto* xs = reinterpret_cast<const typename Source::Stream*>(rn_ring + s * stage_bytes);
+        const T* ys = reinterpret_cast<const T*>(rn_ring + s * stage_bytes + x_bytes);
+        float x[NV][8], y[NV][8];
 #pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                const int k = threadIdx.x + i * blockDim.x;
+        for (int v = 0; v < NV; ++v) {
+            const int k = threadIdx.x + v * blockDim.x;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) y[i][e] = 0.0f;
-                if (k >= nvec) continue;
-                if (WALK) {
-                    yr[i].get(y[i]);
-                } else {
-                    for (int j = 0; j < p.parts; ++j) {
-                        float t[8];
-                        Vec8<T>::load((const T*)p.y + (r * p.parts + j) * p.stride + k * 8, t);
+            for (int e = 0; e < 8; ++e) x[v][e] = y[v][e] = 0.0f;
+            if (k >= nvec) continue;
+            Vec8<typename Source::Stream>::load(xs + k * 8, x[v]);       // shared memory: no read-only load
+            for (int j = 0; j < parts; ++j) {
+                float t[8];
+                Vec8<T>::load(ys + j * p.stride + k * 8, t);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) y[i][e] += t[e];
-                    }
-                }
+                for (int e = 0; e < 8; ++e) y[v][e] += t[e];
             }
         }
-        if (WALK) {
-            fetch(r + gridDim.x, ahead);
-            ahead = token(r + 2 * (int64_t)gridDim.x);
-        }
-        if (p.y != nullptr) {
-            if (p.post_w != nullptr) norm_regs<NV>(y, p.post_w, p.post_b, p.eps, p.center != 0, p.cols, nvec, part);
-#pragma unroll
-            for (int i = 0; i < NV; ++i)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[i][e] += p.mult * y[i][e];
-        }
-        if (TOKENS || p.y != nullptr) {
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                const int k = threadIdx.x + i * blockDim.x;
-                if (k < nvec) Vec8<float>::store(xrow + k * 8, x[i]);
-            }
-        }
-        if (p.h != nullptr) {
-            if (p.pre_w != nullptr) norm_regs<NV>(x, p.pre_w, p.pre_b, p.eps, p.center != 0, p.cols, nvec, part);
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                const int k = threadIdx.x + i * blockDim.x;
-                if (k < nvec) Vec8<T>::store((T*)p.h + r * p.stride + k * 8, x[i]);
-            }
-        }
-        if (!WALK) break;
+        if (!sums) __syncthreads();
+        finish_row<T, NV, TOKENS>(p, r, x, y, nvec, part);
+        if (++s == stages) { s = 0; parity ^= 1u; }
+    }
+    if (abort_flag && threadIdx.x == 0) {                    // gave up: the copies in flight still write shared memory
+        report(p.status, KTK_STATUS_TIMEOUT);
+        volatile int never = 0;
+        for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_wait(&full[i % stages], (i / stages) & 1, &never);
     }
 }
 
 template <typename T, bool TOKENS>
 static int residual_norm_launch(const ResidualNormParams& p, cudaStream_t st) {
+    const char* who = "ktk_residual_norm";
     const int nvec = p.stride / 8;
     const int threads = nvec >= kRnThreads ? kRnThreads : (nvec + 31) / 32 * 32;
     const int nv = (nvec + threads - 1) / threads;
-    const int64_t walkers = (int64_t)sm_count() * kRnWalkers;
-    if constexpr (sizeof(T) == 2) {
-        if (threads == kRnThreads && nv == 1 && p.parts == 1 && p.rows >= kRnWalkRows * walkers) {
-            residual_norm_kernel<T, 1, TOKENS, true><<<(unsigned)walkers, threads, 0, st>>>(p);
-            KTK_CUDA_TRY(cudaGetLastError(), "ktk_residual_norm");
-            return KTK_OK;
-        }
+    // Walkers: rows of 1793 to 2048 columns by six CTAs of 128 threads per SM, of up to 4096 by three of 256.  us, a CTA per row /
+    // walkers, next rows not in L2: 8192 x 4096 bf16 98 / 75, 3000 x 4096 37 / 32, 2000 x 4096 24 / 23, 8192 x 2048 56 / 52, 8192 x 4096 fp32
+    // 117 / 109, embedding rows 8192 x 2048 41 / 31 and x 4096 62 / 51; not 3000 x 2048 (21.7 / 23.1), 1024 columns (25 / 28), fp32 of 2048
+    // columns, several parts (8 of 2048 80 / 82, 4 of 4096 110 / 110).
+    const bool narrow = nvec <= kRnThreads;
+    const int walk_threads = narrow ? kRnThreads / 2 : kRnThreads, resident = narrow ? 6 : 3;
+    if (nvec > kRnThreads - 32 && nvec <= 2 * kRnThreads && (p.y == nullptr || p.parts == 1) && (sizeof(T) == 2 || !narrow) &&
+        p.rows >= (narrow ? 8 : 4) * (int64_t)sm_count() * resident) {
+        const size_t stage = (size_t)p.stride * (TOKENS ? sizeof(T) : 4) + (p.y ? (size_t)p.stride * sizeof(T) : 0);
+        auto kernel = residual_norm_walk_kernel<T, TOKENS>;
+        KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRnStages * stage)), who);
+        kernel<<<(unsigned)(sm_count() * resident), walk_threads, kRnStages * stage, st>>>(p);
+        KTK_CUDA_TRY(cudaGetLastError(), who);
+        return KTK_OK;
     }
-    auto kernel = nv <= 1 ? residual_norm_kernel<T, 1, TOKENS, false>
-                : nv <= 2 ? residual_norm_kernel<T, 2, TOKENS, false>
-                : nv <= 4 ? residual_norm_kernel<T, 4, TOKENS, false>
-                          : residual_norm_kernel<T, kRnMaxVec, TOKENS, false>;
+    auto kernel = nv <= 1 ? residual_norm_kernel<T, 1, TOKENS>
+                : nv <= 2 ? residual_norm_kernel<T, 2, TOKENS>
+                : nv <= 4 ? residual_norm_kernel<T, 4, TOKENS>
+                          : residual_norm_kernel<T, kRnMaxVec, TOKENS>;
     kernel<<<(unsigned)p.rows, threads, 0, st>>>(p);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_residual_norm");
+    KTK_CUDA_TRY(cudaGetLastError(), who);
     return KTK_OK;
 }
 

@@ -90,6 +90,33 @@ def test_residual_norm_over_many_rows(cuda_device, dtype, cols):
         torch.testing.assert_close(h[:, :cols].double(), norm(embed[ids].double(), w2, None, False), **tol)
 
 
+@pytest.mark.parametrize("cols", [1793, 2048, 2049, 4096])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_residual_norm_of_walked_rows(cuda_device, dtype, cols):
+    """Rows for walkers of either width and for a ring of two rows, one row over a whole number of each: with a barrier in the sums and
+    without any sum, on a stream and on embedding rows.  Bounds: as in test_residual_norm_over_many_rows."""
+    from kinetics_b200 import layer_ops as lo, ops
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    rows, S, eps, mult = 8 * 6 * sms + 1, lo.pad8(cols), 1e-4, 0.3
+    g = torch.Generator(device=cuda_device).manual_seed(cols)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
+    pad = lambda t: torch.nn.functional.pad(t, (0, S - cols)).contiguous()
+    x0, w, y = rnd(rows, cols) + 2.0, rnd(cols), (rnd(rows, 1, cols) - 1.0).to(dtype)
+    embed, ids = rnd(97, cols).to(dtype), torch.randint(0, 97, (rows,), generator=g, device=cuda_device)
+    unit = lambda v: v / (v.square().mean(1, keepdim=True) + eps).sqrt() * w.double()
+    tol = dict(rtol=1e-5, atol=2e-5) if dtype == torch.float32 else dict(rtol=1e-2, atol=1e-2)
+    for tokens in (False, True):
+        start = embed[ids].double() if tokens else x0.double()
+        for normed in (False, True):
+            x, h, status = pad(x0), torch.full((rows, S), float("nan"), dtype=dtype, device=cuda_device), ops.new_status(cuda_device)
+            lo.residual_norm(x, h, cols, eps, pre=(pad(w), None) if normed else None, y=pad(y), post=(pad(w), None) if normed else None,
+                             mult=mult, center=False, status=status, **(dict(tokens=ids, embed=pad(embed)) if tokens else {}))
+            ops.raise_on_status(status)
+            want = start + mult * (unit(y[:, 0].double()) if normed else y[:, 0].double())
+            torch.testing.assert_close(x[:, :cols].double(), want, rtol=1e-5, atol=2e-5)
+            torch.testing.assert_close(h[:, :cols].double(), unit(want) if normed else want, **tol)
+
+
 def test_residual_norm_reports_a_token_outside_the_vocabulary(cuda_device):
     from kinetics_b200 import layer_ops as lo, ops
     x = torch.empty(1, 8, device=cuda_device)
