@@ -383,6 +383,13 @@ KTK_API int ktk_rank_barrier(const void* flag_ptrs, void* launch_count, int32_t 
 KTK_API int ktk_silu_mul(const void* gate, const void* up, void* out, int64_t n, int32_t dtype,
                  void* stream);
 /*
+ * out [rows, n] = x [rows, k] W^T (+ bias [n]) (+ residual [rows, n]) with W [n, k], or with W2: silu(x W^T) * (x W2^T): the products of
+ * a decode step of few sequences (nn.Linear, benchmark/blocktopk_decoder.py:196,232-239) in one launch, sums in fp32.
+ * At most 16 rows; k a multiple of 8; x, W, W2 16-byte aligned; all contiguous and of one dtype.
+ */
+KTK_API int ktk_linear_rows(const void* x, const void* w, const void* w2, const void* bias, const void* residual, void* out,
+                            int64_t rows, int64_t n, int64_t k, int32_t dtype, void* stream);
+/*
  * The same over [rows, cols] operands whose rows lie in_row_stride elements apart -- the two halves of ONE GEMM
  * output [rows, 2 * cols] when gate_proj and up_proj (benchmark/blocktopk_decoder.py:235, LiteSys qwen3.py:81-83)
  * are multiplied as one stacked weight.  `out` is contiguous [rows, cols]; cols a multiple of 8, rows 16-byte aligned.

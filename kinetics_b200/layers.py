@@ -55,6 +55,29 @@ def random_page_table(batch_size: int, pages_per_req: int, num_pages: int, devic
     return perm.to(torch.int32).view(batch_size, pages_per_req).to(device).contiguous()
 
 
+def _plain(linear) -> bool:
+    """A linear layer whose call is nothing but its product: no subclass, no hook, no other forward."""
+    m = nn.modules.module
+    return type(linear) is nn.Linear and "forward" not in linear.__dict__ and type(linear.weight) is nn.Parameter and not (
+        linear._forward_hooks or linear._forward_pre_hooks or linear._backward_hooks or linear._backward_pre_hooks or
+        m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks)
+
+
+def _by_rows(x, *linears) -> bool:
+    """Whether the product of x with one layer, or the gated product of two, goes to ktk::linear_rows."""
+    w = linears[0].weight
+    return (not torch.compiler.is_compiling() and type(x) is torch.Tensor and x.dim() == 2 and x.is_cuda and
+            ops.linear_rows_wins(x.shape[0], w.shape[0], w.shape[1], x.dtype, len(linears) == 2) and
+            all(_plain(m) and m.weight.dtype == x.dtype and m.weight.is_cuda and m.weight.is_contiguous() and
+                m.weight.shape == w.shape and m.weight.data_ptr() % 16 == 0 for m in linears) and
+            (len(linears) == 1 or all(m.bias is None for m in linears)) and x.is_contiguous() and x.data_ptr() % 16 == 0 and
+            not torch.is_autocast_enabled("cuda"))
+
+
+def _linear(linear, x):
+    return torch.ops.ktk.linear_rows(x, linear.weight, linear.bias, None, None) if _by_rows(x, linear) else linear(x)
+
+
 class _EventPair:
     """Brackets a kernel with CUDA events on the current stream when timing is switched on."""
 
@@ -204,14 +227,19 @@ class _PagedDecoderLayer(nn.Module):
         """SwiGLU MLP.  One rank: the residual add rides in the epilogue of the down projection GEMM.
         Several ranks: the down_proj partials are summed over the ranks and the residual is added once
         (litesys/models/qwen3_dist.py:120-122)."""
-        up = self.up_proj(hidden_states)
-        gate = self.gate_proj(hidden_states)
-        if self.hidden_act == "silu":
-            hidden_states = torch.ops.ktk.silu_mul(gate, up)
+        if self.hidden_act == "silu" and _by_rows(hidden_states, self.gate_proj, self.up_proj):
+            hidden_states = torch.ops.ktk.linear_rows(hidden_states, self.gate_proj.weight, None, None, self.up_proj.weight)
         else:
-            from transformers.activations import ACT2FN
-            hidden_states = ACT2FN[self.hidden_act](gate) * up
+            up = self.up_proj(hidden_states)
+            gate = self.gate_proj(hidden_states)
+            if self.hidden_act == "silu":
+                hidden_states = torch.ops.ktk.silu_mul(gate, up)
+            else:
+                from transformers.activations import ACT2FN
+                hidden_states = ACT2FN[self.hidden_act](gate) * up
         if self.process_group is None:
+            if _by_rows(hidden_states, self.down_proj) and residual.is_contiguous():
+                return torch.ops.ktk.linear_rows(hidden_states, self.down_proj.weight, None, residual, None)
             return torch.addmm(residual, hidden_states, self.down_proj.weight.t())
         if self.fused_down is not None:
             torch.mm(hidden_states, self.down_proj.weight.t(), out=self.fused_down.x)
@@ -241,7 +269,7 @@ class _PagedDecoderLayer(nn.Module):
         # input RMSNorm (mylib::layer_norm of the reference, :192), 16-byte accesses
         hidden_states = torch.ops.ktk.rms_norm(residual, self.input_layernorm_weight,
                                                self.input_layernorm_variance_epsilon)
-        proj = self.wqkv(hidden_states)
+        proj = _linear(self.wqkv, hidden_states)
         # split + q-norm + k-norm (:198-207) in one launch
         query_states, key_states, value_states = torch.ops.ktk.qkv_norm(
             proj, self.qnorm_weight, self.knorm_weight, self.qnorm_variance_epsilon, self.num_heads,
@@ -262,7 +290,7 @@ class _PagedDecoderLayer(nn.Module):
                 residual, hidden_states = self.fused(residual.contiguous(), self.post_attention_layernorm_weight,
                                                      self.post_attention_layernorm_variance_epsilon)
         else:
-            hidden_states = self.wo(o)
+            hidden_states = _linear(self.wo, o)
             if self.process_group is not None:
                 with self._timed("exchange_o_proj"):
                     torch.distributed.all_reduce(hidden_states, group=self.process_group)

@@ -468,6 +468,43 @@ def qkv_norm(proj: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, eps: float,
     return q, k, v
 
 
+LINEAR_ROWS = 16         # most rows of linear_rows
+
+
+def linear_rows_wins(rows: int, n: int, k: int, dtype, gated: bool) -> bool:
+    """Whether linear_rows is faster than the library's products (with two of them and silu_mul if `gated`).  fp32: throughout (16 rows,
+    512 x 512: 7.3 us there, 2.9 here; 12288 x 4096 133 and 119).  bf16, us there / here: 8 rows, 768 x 4096 9.1 / 5.9, 1536 x 4096
+    9.1 / 9.2, 4096 x 1536 6.6 / 11.3; 4 rows, 1536 x 4096 9.4 / 6.3, 2560 x 5120 12.3 / 12.6; gated, 8 rows, 1536 x 4096 20.6 / 14.0,
+    3072 x 4096 25.9 / 25.2, 4 rows, 3200 x 5120 26.2 / 18.5, 6400 x 5120 27.3 / 33.9, 16 rows, 1024 x 1024 10.5 / 7.7."""
+    if rows < 1 or rows > LINEAR_ROWS or k % 8 != 0:
+        return False
+    if dtype == torch.float32:
+        return True
+    if dtype != torch.bfloat16:
+        return False
+    if gated:
+        return n * k <= ((17 << 20) if rows <= 4 else (8 << 20) if rows <= 8 else (1 << 20))
+    return n <= 1536 if rows <= 4 else n <= 1024 and rows <= 8
+
+
+def linear_rows(x: torch.Tensor, w: torch.Tensor, bias=None, residual=None, w2=None) -> torch.Tensor:
+    """x [rows, k] @ w [n, k]^T (+ bias [n]) (+ residual [rows, n]) for at most LINEAR_ROWS rows, or with w2
+    silu(x @ w^T) * (x @ w2^T): one launch, sums in fp32."""
+    _cuda(x, w, bias, residual, w2)
+    rows, k = x.shape
+    n = w.shape[0]
+    if rows > LINEAR_ROWS or w.shape != (n, k) or (w2 is not None and w2.shape != w.shape) or \
+            (bias is not None and bias.shape != (n,)) or (residual is not None and residual.shape != (rows, n)):
+        raise ValueError("linear_rows: x [rows, k], w and w2 [n, k], bias [n], residual [rows, n]")
+    if any(t is not None and t.dtype != x.dtype for t in (w, bias, residual, w2)):
+        raise TypeError("linear_rows: one dtype")
+    out = torch.empty(rows, n, dtype=x.dtype, device=x.device)
+    check(_lib.load().ktk_linear_rows(_ptr(x), _ptr(w), _ptr(w2), _ptr(bias), _ptr(residual), _ptr(out), rows, n, k,
+                                      _dtype_code(x), _stream()))
+    _launched()
+    return out
+
+
 def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     """silu(gate) * up (benchmark/blocktopk_decoder.py:235-236)."""
     if gate.shape != up.shape or gate.dtype != up.dtype:
@@ -763,6 +800,19 @@ def _qkv_norm_fake(proj, wq, wk, eps, num_q_heads, num_kv_heads):
     B = proj.numel() // ((num_q_heads + 2 * num_kv_heads) * HEAD_DIM)
     return (proj.new_empty(B, num_q_heads, HEAD_DIM), proj.new_empty(B, num_kv_heads, HEAD_DIM),
             proj.new_empty(B, num_kv_heads, HEAD_DIM))
+
+
+torch.library.define("ktk::linear_rows", "(Tensor x, Tensor w, Tensor? bias, Tensor? residual, Tensor? w2) -> Tensor")
+
+
+@torch.library.impl("ktk::linear_rows", "cuda")
+def _linear_rows_op(x, w, bias, residual, w2):
+    return linear_rows(x, w, bias, residual, w2)
+
+
+@torch.library.register_fake("ktk::linear_rows")
+def _linear_rows_fake(x, w, bias, residual, w2):
+    return x.new_empty(x.shape[0], w.shape[0])
 
 
 torch.library.define("ktk::silu_mul", "(Tensor gate, Tensor up) -> Tensor")
