@@ -18,9 +18,56 @@ constexpr int kPuPages = kPuKeys / kPageSize;             // of a block
 using PrefillFlash = Flash<kPuKeys, kHeadDim / 64>;
 constexpr int kPuSmem = PrefillFlash::bytes(2, 2);
 
-// TILE_MAJOR: the grid is (kv heads, sequences, tile pairs), so that the last tiles of all heads and sequences, which see most of
-// their own sequence, come first (not the longest histories of sequences that differ); otherwise (tile pairs, kv heads, sequences), for more than 65535 pairs
-template <bool TILE_MAJOR>
+// Which tiles a CTA takes.  A later tile sees more keys, and the work of a launch that leaves SMs idle at its end should end with
+// short ones.
+//   kByLength     grid (kv heads, item): the items of all sequences from the most keys to the fewest
+//   kByTile       grid (kv heads, sequences, tile pairs): the last pairs of all heads and sequences first
+//   kBySequence   grid (tile pairs, kv heads, sequences), for more than 65535 pairs
+enum Order { kBySequence, kByTile, kByLength };
+constexpr int kPuOrdered = 32;                            // sequences that an ordered launch may have: one per lane
+
+// Item `rank` of the launch: a sequence and which `step` of its new tokens.  Its length counts in steps, those of the history rounded
+// up: item p of a sequence with h of history has length p + h.  A warp finds the length at `rank`, 32 probes at a time.  False
+// behind the last item.
+__device__ __forceinline__ bool item_by_length(const PrefillUmmaParams& p, int rank, int step, int& b, int& pair) {
+    const int lane = threadIdx.x & 31;
+    int first = 0, count = 0;
+    if (lane < p.batch) {
+        const int n = p.q_indptr[lane + 1] - p.q_indptr[lane];
+        const SeqPages sp = seq_pages(p.kv_indptr, p.page_count, p.kv_last_page_len, p.sink_tokens, lane);
+        if (n > 0) {
+            count = (n + step - 1) / step;
+            first = sp.bad || sp.total < n ? 0 : (sp.total - n + step - 1) / step;
+        }
+    }
+    // items of length L or more, every lane for its own L; all lanes take part
+    auto at_least = [&](int L) {
+        int have = 0;
+        for (int s = 0; s < p.batch; ++s) {
+            const int f = __shfl_sync(0xffffffffu, first, s), c = __shfl_sync(0xffffffffu, count, s);
+            have += min(max(f + c - L, 0), c);
+        }
+        return have;
+    };
+    int lo = 0, hi = (int)__reduce_max_sync(0xffffffffu, (unsigned)(first + count)), behind = 0;
+    // more than `rank` items have length lo or more, `behind` <= rank of them hi or more
+    for (bool begun = false; hi - lo > 1 || !begun; begun = true) {
+        const int each = (hi - lo + 31) / 32, L = lo + lane * each, seen = at_least(L), have = L < hi ? seen : behind;
+        const unsigned more = __ballot_sync(0xffffffffu, L < hi && have > rank);       // a prefix of the lanes
+        if (more == 0) return false;                       // only of the first probes, which start at 0
+        const int at = 31 - __clz((int)more);
+        const int next = __shfl_sync(0xffffffffu, have, at < 31 ? at + 1 : 31);
+        if (at < 31 && lo + (at + 1) * each < hi) { hi = lo + (at + 1) * each; behind = next; }
+        lo += at * each;
+    }
+    // among the sequences with an item of length lo
+    const unsigned has = __ballot_sync(0xffffffffu, lo >= first && lo < first + count);
+    b = (int)__fns(has, 0, rank - behind + 1);
+    pair = lo - __shfl_sync(0xffffffffu, first, b & 31);
+    return true;
+}
+
+template <Order ORDER>
 __global__ void __launch_bounds__(kFlThreads, 1)
 prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorMap kv_map) {
     extern __shared__ uint8_t um_raw[];
@@ -28,8 +75,13 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(um_raw) + 1023) & ~uintptr_t(1023));
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int b = TILE_MAJOR ? blockIdx.y : blockIdx.z, h = TILE_MAJOR ? blockIdx.x : blockIdx.y;
-    const int pair = TILE_MAJOR ? (int)(gridDim.z - 1 - blockIdx.z) : (int)(gridDim.x - 1 - blockIdx.x);
+    const int h = ORDER == kBySequence ? blockIdx.y : blockIdx.x;
+    int b = ORDER == kByTile ? blockIdx.y : blockIdx.z, pair = 0;
+    if (ORDER == kByLength) {
+        if (!item_by_length(p, blockIdx.y, p.tiles * (kUmRows / p.G), b, pair)) return;
+    } else {
+        pair = ORDER == kByTile ? (int)(gridDim.z - 1 - blockIdx.z) : (int)(gridDim.x - 1 - blockIdx.x);
+    }
     const int G = p.G, Hq = p.Hkv * G;
     const int tpc = kUmRows / G;                    // new tokens per tile
     const int q0 = p.q_indptr[b];
@@ -193,10 +245,18 @@ int launch_prefill_umma(PrefillUmmaParams p, int max_new_tokens, cudaStream_t st
     const int64_t tiles = (p.batch * per_seq < most ? p.batch * per_seq : most) * p.Hkv;
     p.tiles = tiles <= sm_count() ? 1 : 2;
     const unsigned pairs = (unsigned)((per_seq + p.tiles - 1) / p.tiles);
-    const bool tile_major = pairs <= 65535;
-    auto kernel = tile_major ? prefill_umma_kernel<true> : prefill_umma_kernel<false>;
+    // By length where several sequences take between one and four rounds of CTAs: finding its item costs a CTA half a microsecond, and
+    // the more rounds, the less the last one leaves idle.  Six portions of 350 to 1050 tokens behind 2500 to 7500, 16 heads over 8:
+    // 250 us by tile, 203 by length (264 CTAs); eight of 150 to 450 behind 450 to 1350 50 and 47.
+    const int64_t step = (int64_t)tpc * p.tiles, about = p.total_new / step + p.batch / 2;
+    const int64_t items = p.total_new / step + p.batch < (int64_t)p.batch * pairs ? p.total_new / step + p.batch : (int64_t)p.batch * pairs;
+    const bool by_length = p.batch > 1 && p.batch <= kPuOrdered && items <= 65535 && about * p.Hkv > sm_count() &&
+                           about * p.Hkv <= 4 * (int64_t)sm_count();
+    const bool by_tile = !by_length && pairs <= 65535;
+    auto kernel = by_length ? prefill_umma_kernel<kByLength> : by_tile ? prefill_umma_kernel<kByTile> : prefill_umma_kernel<kBySequence>;
     KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPuSmem), who);
-    const dim3 grid = tile_major ? dim3((unsigned)p.Hkv, (unsigned)p.batch, pairs) : dim3(pairs, (unsigned)p.Hkv, (unsigned)p.batch);
+    const dim3 grid = by_length ? dim3((unsigned)p.Hkv, (unsigned)items)
+                    : by_tile ? dim3((unsigned)p.Hkv, (unsigned)p.batch, pairs) : dim3(pairs, (unsigned)p.Hkv, (unsigned)p.batch);
     DecodeParams d{};                               // only what the tensor map needs
     d.cache = p.cache; d.Hkv = p.Hkv; d.num_pages = p.num_pages;
     CUtensorMap map;

@@ -111,3 +111,35 @@ def test_rows_shared_by_all_heads():
         for b, start, n, _ in units:                         # what the joining pass derives from the table alone
             c0, pieces = start // chunk, (start + n - 1) // chunk - start // chunk + 1
             assert (pieces == 1) == (out[b] == "direct") and c0 + pieces - 1 < ctas and pieces <= 256
+
+
+def _item_by_length(first, count, rank):
+    """csrc/ktk_prefill_umma.cu, item_by_length: 32 probes at a time."""
+    at_least = lambda L: sum(min(max(f + c - L, 0), c) for f, c in zip(first, count))
+    lo, hi, behind, begun = 0, max(f + c for f, c in zip(first, count)), 0, False
+    while hi - lo > 1 or not begun:
+        begun = True
+        each = (hi - lo + 31) // 32
+        have = [at_least(lo + i * each) if lo + i * each < hi else behind for i in range(32)]
+        more = [lo + i * each < hi and have[i] > rank for i in range(32)]
+        if not more[0]:
+            return None
+        at = max(i for i in range(32) if more[i])
+        assert all(more[:at + 1])
+        if at < 31 and lo + (at + 1) * each < hi:
+            hi, behind = lo + (at + 1) * each, have[at + 1]
+        lo += at * each
+    has = [s for s, (f, c) in enumerate(zip(first, count)) if f <= lo < f + c]
+    return has[rank - behind], lo - first[has[rank - behind]]
+
+
+def test_prompt_items_by_length():
+    rng = random.Random(4)
+    for _ in range(600):
+        B = rng.randint(1, 32)
+        count = [rng.choice([0, 1, rng.randint(1, 70)]) for _ in range(B)]
+        first = [rng.choice([0, rng.randint(0, 3000)]) if c else 0 for c in count]
+        items = sorted(((-first[s] - p, s, p) for s in range(B) for p in range(count[s])))
+        for rank in {0, len(items) // 3, max(len(items) - 1, 0), len(items), len(items) + 5}:
+            want = items[rank][1:] if rank < len(items) else None
+            assert _item_by_length(first, count, rank) == want

@@ -92,6 +92,30 @@ def test_prefill_long_prompt_many_sequences(cuda_device):
     torch.testing.assert_close(out[n:2 * n].float(), ref, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("G,Hkv,sink,B", [(8, 4, 0, 7), (8, 4, 4, 7), (4, 6, 0, 32), (2, 3, 0, 33)])
+def test_prefill_of_unequal_sequences_over_more_than_one_round(cuda_device, G, Hkv, sink, B):
+    """Portions of very different lengths behind very different histories, some empty: the CTAs take them by length (up to 32
+    sequences).  Every row is written once, with what the row-by-row kernel gives.  Bound: as in the other prompts."""
+    from kinetics_b200 import ops
+    new = ([700, 3, 0, 450, 64, 65, 1200] * 5)[:B]
+    hist = ([100, 2500, 40, 0, 900, 10, 5] * 5)[:B]
+    lens = [h + n for h, n in zip(hist, new)]
+    g = torch.Generator().manual_seed(B)
+    pages = [1 + max(0, -(-(n - sink) // 16)) if sink else -(-n // 16) for n in lens]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)
+    indptr, q_indptr = i32([sum(pages[:i]) for i in range(B + 1)]), i32([sum(new[:i]) for i in range(B + 1)])
+    last = i32([(n - sink - 1) % 16 + 1 if sink and n > sink else n if sink else (n - 1) % 16 + 1 for n in lens])
+    table = torch.randperm(sum(pages), generator=g).to(torch.int32).to(cuda_device)
+    cache = torch.randn(sum(pages), 2, 16, Hkv, 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    q = torch.randn(sum(new), Hkv * G, 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    view, status = ops.PageView(sink_tokens=sink, local_tokens=1) if sink else None, ops.new_status(cuda_device)
+    run = lambda variant: ops.prefill_attention(q, q_indptr, max(new), cache, table, indptr, last, variant=variant, status=status,
+                                                view=view, out=torch.full_like(q, float("nan")))
+    got, want = run(0), run(1)
+    ops.raise_on_status(status)
+    torch.testing.assert_close(got.float(), want.float(), rtol=2e-2, atol=2e-2)
+
+
 @pytest.mark.parametrize("variant", [0, 2])
 @pytest.mark.parametrize("G,sink", [(4, 0), (2, 4), (8, 4)])
 def test_prefill_on_block_and_tile_edges(cuda_device, variant, G, sink):
