@@ -239,13 +239,13 @@ template <int STAGES> __global__ void __launch_bounds__(kRtThreads) route_mma_ke
             for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
         for (int s = 0; s < STAGES - 1; ++s) {
             if (s < steps) load(s);
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            cp_async_commit();
         }
         for (int s = 0; s < steps; ++s) {
             asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
             __syncthreads();                              // stage s is in place; everyone is done with stage s - 1
             if (s + STAGES - 1 < steps) load(s + STAGES - 1);
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            cp_async_commit();
             const __nv_bfloat16* st = ring + (s % STAGES) * kRtStageElems;
             const uint32_t ha = smem_u32(st + (m0 + (lane & 15)) * kRtLd + (lane >> 4) * 8);
             const uint32_t wa = smem_u32(st + (kRtRows + n0 + (lane & 7) + (lane >> 4) * 8) * kRtLd + ((lane >> 3) & 1) * 8);

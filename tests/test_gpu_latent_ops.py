@@ -467,6 +467,38 @@ def test_fused_steps_over_more_than_one_round_of_narrow_ctas(cuda_device, blocks
 
 
 @pytest.mark.parametrize("dtype", [F32, BF])
+@pytest.mark.parametrize("blocks,block,total", [(1, 8, 64), (3, 20, 65), (2, 264, 63), (5, 104, 1100), (40, 256, 700)])
+def test_scan_of_buffers_that_start_anywhere(cuda_device, dtype, blocks, block, total):
+    # whole and partial rounds, with one CTA along the sequence and several; buffers off 16 bytes are not read by pieces of 16.
+    # The loads differ, the arithmetic does not: the same bits
+    from kinetics_b200 import layer_ops as lo, ops
+    spec, dev, g = lo.LruSpec(blocks, block, 4), cuda_device, torch.Generator().manual_seed(total)
+    cols, table = spec.cols, _length_table([total + 3], cuda_device)
+    f32 = lambda *size: torch.randn(*size, generator=g).to(dev)
+    proj, u, z = f32(total, 2 * cols).to(dtype), f32(total, cols).to(dtype), f32(blocks, total, 2 * (cols // blocks))
+    rb, ib, decay, state0 = f32(cols), f32(cols), f32(cols).abs(), f32(2, cols)
+    new, slots = torch.tensor([0, total], dtype=torch.int32, device=dev), torch.tensor([1], dtype=torch.int32, device=dev)
+
+    def run(shift):
+        moved = lambda t: torch.cat([t.new_zeros(shift), t.flatten()])[shift:].view(t.shape)
+        state, status = state0.clone(), ops.new_status(dev)
+        out = lo.lru_scan(moved(z), moved(u), moved(proj), spec, table, slots, rb, ib, decay, state, new_indptr=new, max_new=total, status=status)
+        ops.raise_on_status(status)
+        return out, state
+    (a, sa), (b, sb) = run(0), run(1)
+    assert torch.equal(a, b) and torch.equal(sa, sb) and torch.equal(sa[0], state0[0])
+    halves = z.double().view(blocks, total, 2, -1).permute(2, 1, 0, 3).reshape(2, total, cols).cpu()
+    gate = [torch.sigmoid(h + w.double().cpu()) for h, w in zip(halves, (rb, ib))]
+    S, want, x = state0[1].double().cpu(), [], gate[0] * decay.double().cpu()
+    for t in range(total):
+        S = torch.exp(-x[t]) * S + torch.sqrt(-torch.expm1(-2 * x[t])) * gate[1][t] * u[t].double().cpu()
+        want.append(S * plain.gelu_tanh(proj[t, :cols].double().cpu()))
+    want = torch.stack(want)
+    # as in test_recurrence_in_portions: fp32 rounding over the tokens that the decays keep; bf16's of the result
+    assert (a.double().cpu() - want).pow(2).mean().sqrt() / rms(want) < (2e-5 if dtype == F32 else 4e-3)
+
+
+@pytest.mark.parametrize("dtype", [F32, BF])
 def test_long_memory_and_short_memory(cuda_device, dtype):
     # decays from "forgets at once" to "keeps for the whole sequence": the series and the difference in sqrt(1 - a^2)
     from kinetics_b200.layer_ops import LruSpec
