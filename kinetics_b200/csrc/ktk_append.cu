@@ -19,6 +19,7 @@ append_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ 
               const int32_t* __restrict__ kv_indices, const int32_t* __restrict__ kv_indptr,
               const int32_t* __restrict__ kv_last_page_len, const int32_t* __restrict__ page_count,
               const int32_t* __restrict__ slot_index, int Hkv, int64_t num_pages, int32_t* status) {
+    wait_for_front();
     const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
     const int beg = kv_indptr[b];
     const int n_pages = page_count ? page_count[b] : kv_indptr[b + 1] - beg;
@@ -257,10 +258,10 @@ static int append_impl(const void* k, const void* v, void* cache, void* summarie
                        const int32_t* kv_indptr, const int32_t* kv_last_page_len, const View& view,
                        const ktk_shape* s, int32_t* status, cudaStream_t st) {
     dim3 grid(s->batch, s->num_kv_heads);
-    append_kernel<T><<<grid, kHeadDim, 0, st>>>(
-        (const T*)k, (const T*)v, (T*)cache, (T*)summaries, summary_stride, kv_indices, kv_indptr,
-        kv_last_page_len, view.page_count, view.slot_index, s->num_kv_heads, s->num_pages, status);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_append");
+    KTK_CUDA_TRY(launch_behind(append_kernel<T>, grid, kHeadDim, 0, st, (const T*)k, (const T*)v, (T*)cache, (T*)summaries,
+                               summary_stride, kv_indices, kv_indptr, kv_last_page_len, view.page_count, view.slot_index,
+                               s->num_kv_heads, s->num_pages, status),
+                 "ktk_append");
     return KTK_OK;
 }
 

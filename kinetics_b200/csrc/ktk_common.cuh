@@ -53,6 +53,32 @@ inline int view_row_width(int topk, const View& v) {
         if (_e != cudaSuccess) return cuda_fail(_e, who); \
     } while (0)
 
+// ---- launches that overlap their start with the end of the kernel in front ----
+// The small kernels of a decode step last about as long as it takes to get one going.  A kernel launched by launch_behind is
+// sent to the device while the kernel in front of it in the stream still runs, and its CTAs wait in wait_for_front until
+// that one has ended and its writes are visible; nothing but registers and shared memory is touched before.  A kernel that
+// has called wait_for_front lets its own successor come as soon as all its CTAs have begun.  Every CTA calls it, also one
+// without work: then the end of a kernel implies the end of all in front of it.  Replayed from a graph, us: the fp32 layer
+// step of 4 sequences (11 such kernels) 33.4 -> 31.5, 256 sequences of 8192 tokens (9 of 14) 106.4 -> 104.7.
+__device__ __forceinline__ void wait_for_front() {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // ---- element access -------------------------------------------------------
 __device__ __forceinline__ float to_f32(float x) { return x; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 x) { return __bfloat162float(x); }

@@ -49,6 +49,7 @@ decode_simt_kernel(const DecodeParams p) {
     __shared__ __align__(16) float red_o[kSimtWarps][G][kHeadDim];
     __shared__ float red_m[kSimtWarps][G], red_l[kSimtWarps][G];
 
+    wait_for_front();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = p.num_splits;
     const int64_t bh = blockIdx.x / S;
@@ -221,6 +222,7 @@ template <typename T>
 __global__ void __launch_bounds__(kHeadDim)
 combine_kernel(const float* __restrict__ ws_ml, const float* __restrict__ ws_o, T* __restrict__ o,
                int S) {
+    wait_for_front();
     const int64_t qh = blockIdx.x;
     const int d = threadIdx.x;
     float M = -INFINITY;
@@ -241,8 +243,7 @@ combine_kernel(const float* __restrict__ ws_ml, const float* __restrict__ ws_o, 
 template <typename T, int G>
 static int simt_launch(const DecodeParams& p, cudaStream_t st) {
     const int64_t ctas = (int64_t)p.batch * p.Hkv * p.num_splits;
-    decode_simt_kernel<T, G><<<(unsigned)ctas, kSimtWarps * 32, 0, st>>>(p);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk decode (simt)");
+    KTK_CUDA_TRY(launch_behind(decode_simt_kernel<T, G>, (unsigned)ctas, kSimtWarps * 32, 0, st, p), "ktk decode (simt)");
     return KTK_OK;
 }
 
@@ -262,11 +263,11 @@ int launch_decode_simt(const DecodeParams& p, int dtype, int G, cudaStream_t st)
 
 int launch_combine(const DecodeParams& p, int dtype, int G, cudaStream_t st) {
     const int64_t rows = (int64_t)p.batch * p.Hkv * G;
-    if (dtype == KTK_F32)
-        combine_kernel<float><<<(unsigned)rows, kHeadDim, 0, st>>>(p.ws_ml, p.ws_o, (float*)p.o, p.num_splits);
-    else
-        combine_kernel<__nv_bfloat16><<<(unsigned)rows, kHeadDim, 0, st>>>(p.ws_ml, p.ws_o, (__nv_bfloat16*)p.o, p.num_splits);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk decode (combine)");
+    const auto go = [&](auto kernel, auto* o) {
+        return launch_behind(kernel, (unsigned)rows, kHeadDim, 0, st, p.ws_ml, p.ws_o, o, p.num_splits);
+    };
+    KTK_CUDA_TRY(dtype == KTK_F32 ? go(combine_kernel<float>, (float*)p.o) : go(combine_kernel<__nv_bfloat16>, (__nv_bfloat16*)p.o),
+                 "ktk decode (combine)");
     return KTK_OK;
 }
 

@@ -37,6 +37,7 @@ decode_mma_kernel(const MmaParams p, const __grid_constant__ CUtensorMap kv_map)
 
     const DecodeParams& d = p.d;
     const int G = p.G;
+    wait_for_front();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = d.num_splits;
     const int64_t bh = blockIdx.x / S;
@@ -203,8 +204,7 @@ int launch_decode_mma(const DecodeParams& p, int G, cudaStream_t st) {
     mp.d = p;
     mp.G = G;
     const int64_t ctas = (int64_t)p.batch * p.Hkv * p.num_splits;
-    decode_mma_kernel<<<(unsigned)ctas, kMmaThreads, smem, st>>>(mp, map);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk decode (mma)");
+    KTK_CUDA_TRY(launch_behind(decode_mma_kernel, (unsigned)ctas, kMmaThreads, smem, st, mp, map), "ktk decode (mma)");
     return KTK_OK;
 }
 

@@ -174,6 +174,7 @@ decode_stream_kernel(const StreamParams p, const __grid_constant__ CUtensorMap k
     const int G = p.G;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Hq = d.Hkv * G;
+    wait_for_front();
     const Range rg = cta_range(p, blockIdx.x);
     if (rg.p1 <= rg.p0) return;                            // nothing left for this CTA (exact mode, small batches)
     const int64_t p0 = rg.p0, p1 = rg.p1;
@@ -336,6 +337,7 @@ __global__ void __launch_bounds__(kHeadDim)
 stream_combine_kernel(const StreamParams p) {
     const DecodeParams& d = p.d;
     const int G = p.G, dd = threadIdx.x;
+    wait_for_front();
     if (p.exact) {
         for (int b = blockIdx.x; b < d.batch; b += gridDim.x) {
             if (d.kv_indptr[b + 1] - d.kv_indptr[b] > 0) continue;
@@ -463,11 +465,10 @@ int launch_decode_stream(const DecodeParams& p, int G, int max_entries, cudaStre
     const int smem = stream_smem(var.stages);
     KTK_CUDA_TRY(cudaFuncSetAttribute(var.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                  "ktk decode (balanced)");
-    var.kernel<<<grid, kMmaThreads, smem, st>>>(sp, map);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk decode (balanced)");
+    KTK_CUDA_TRY(launch_behind(var.kernel, grid, kMmaThreads, smem, st, sp, map), "ktk decode (balanced)");
     if (grid > 1 || sp.exact) {
-        stream_combine_kernel<<<dim3(grid, (unsigned)sp.G), kHeadDim, 0, st>>>(sp);
-        KTK_CUDA_TRY(cudaGetLastError(), "ktk decode (balanced, combine)");
+        KTK_CUDA_TRY(launch_behind(stream_combine_kernel, dim3(grid, (unsigned)sp.G), kHeadDim, 0, st, sp),
+                     "ktk decode (balanced, combine)");
     }
     return KTK_OK;
 }

@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(kNormThreads)
 add_rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ w, float eps,
                    T* __restrict__ out_sum, T* __restrict__ out_norm, int cols) {
     __shared__ float part[kNormThreads / 32];
+    wait_for_front();
     const int64_t r = blockIdx.x;
     const int nvec = cols / 8;
     float v[kNormMaxVec][8];
@@ -68,6 +69,7 @@ qkv_norm_kernel(const T* __restrict__ proj, const T* __restrict__ wq, const T* _
                 T* __restrict__ q, T* __restrict__ k, T* __restrict__ v, int64_t rows, int Hq, int Hkv,
                 const T* __restrict__ cos_tab, const T* __restrict__ sin_tab,
                 const int64_t* __restrict__ position_ids, int64_t max_positions) {
+    wait_for_front();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -112,6 +114,7 @@ qkv_norm_kernel(const T* __restrict__ proj, const T* __restrict__ wq, const T* _
 template <typename T>
 __global__ void __launch_bounds__(256)
 silu_mul_vec_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ out, int64_t nvec) {
+    wait_for_front();
     const int64_t stride = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += stride) {
         float g[8], u[8], o[8];
@@ -129,6 +132,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 silu_mul_rows_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ out, int64_t rows,
                      int64_t vec_per_row, int64_t in_stride) {
+    wait_for_front();
     const int64_t nvec = rows * vec_per_row;
     const int64_t stride = (int64_t)gridDim.x * 256;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += stride) {
@@ -145,9 +149,9 @@ silu_mul_rows_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __
 template <typename T>
 static int add_rmsnorm_launch(const void* x, const void* residual, const void* w, float eps, void* out_sum,
                               void* out_norm, int64_t rows, int cols, cudaStream_t st) {
-    add_rmsnorm_kernel<T><<<(unsigned)rows, kNormThreads, 0, st>>>((const T*)x, (const T*)residual, (const T*)w,
-                                                                   eps, (T*)out_sum, (T*)out_norm, cols);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_add_rmsnorm");
+    KTK_CUDA_TRY(launch_behind(add_rmsnorm_kernel<T>, (unsigned)rows, kNormThreads, 0, st, (const T*)x, (const T*)residual,
+                               (const T*)w, eps, (T*)out_sum, (T*)out_norm, cols),
+                 "ktk_add_rmsnorm");
     return KTK_OK;
 }
 
@@ -156,14 +160,11 @@ static int qkv_norm_launch(const void* proj, const void* wq, const void* wk, flo
                            int64_t rows, int Hq, int Hkv, const void* cos_tab, const void* sin_tab,
                            const int64_t* position_ids, int64_t max_positions, cudaStream_t st) {
     const unsigned grid = (unsigned)((rows + 3) / 4);
-    if (cos_tab != nullptr)
-        qkv_norm_kernel<T, true><<<grid, 128, 0, st>>>((const T*)proj, (const T*)wq, (const T*)wk, eps, (T*)q, (T*)k,
-                                                       (T*)v, rows, Hq, Hkv, (const T*)cos_tab, (const T*)sin_tab,
-                                                       position_ids, max_positions);
-    else
-        qkv_norm_kernel<T, false><<<grid, 128, 0, st>>>((const T*)proj, (const T*)wq, (const T*)wk, eps, (T*)q, (T*)k,
-                                                        (T*)v, rows, Hq, Hkv, nullptr, nullptr, nullptr, 0);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_qkv_norm");
+    const bool turn = cos_tab != nullptr;
+    KTK_CUDA_TRY(launch_behind(turn ? qkv_norm_kernel<T, true> : qkv_norm_kernel<T, false>, grid, 128, 0, st, (const T*)proj,
+                               (const T*)wq, (const T*)wk, eps, (T*)q, (T*)k, (T*)v, rows, Hq, Hkv, (const T*)cos_tab,
+                               (const T*)sin_tab, turn ? position_ids : nullptr, turn ? max_positions : 0),
+                 "ktk_qkv_norm");
     return KTK_OK;
 }
 
@@ -172,8 +173,8 @@ static int silu_vec_launch(const void* gate, const void* up, void* out, int64_t 
     int64_t blocks = (nvec + 255) / 256;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    silu_mul_vec_kernel<T><<<(unsigned)blocks, 256, 0, st>>>((const T*)gate, (const T*)up, (T*)out, nvec);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_silu_mul");
+    KTK_CUDA_TRY(launch_behind(silu_mul_vec_kernel<T>, (unsigned)blocks, 256, 0, st, (const T*)gate, (const T*)up, (T*)out, nvec),
+                 "ktk_silu_mul");
     return KTK_OK;
 }
 
@@ -184,9 +185,9 @@ static int silu_rows_launch(const void* gate, const void* up, void* out, int64_t
     int64_t blocks = (nvec + 255) / 256;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    silu_mul_rows_kernel<T><<<(unsigned)blocks, 256, 0, st>>>((const T*)gate, (const T*)up, (T*)out, rows, cols / 8,
-                                                               in_stride);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_silu_mul_rows");
+    KTK_CUDA_TRY(launch_behind(silu_mul_rows_kernel<T>, (unsigned)blocks, 256, 0, st, (const T*)gate, (const T*)up, (T*)out, rows,
+                               cols / 8, in_stride),
+                 "ktk_silu_mul_rows");
     return KTK_OK;
 }
 

@@ -74,6 +74,7 @@ template <typename T, int ROWS, int COLS, bool GATED>
 __global__ void __launch_bounds__(kLrThreads) linear_rows_kernel(const LinearParams p) {
     constexpr int kVec = LrVec<T>::kN, kSums = ROWS * COLS, kOwn = GATED ? COLS / 2 : COLS, kLeft = kSums > 32 ? kSums / 32 : 1;
     __shared__ float part[kLrWarps][kSums];
+    wait_for_front();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n0 = blockIdx.x * kOwn;
     const T* wrow[COLS];
@@ -124,15 +125,15 @@ __global__ void __launch_bounds__(kLrThreads) linear_rows_kernel(const LinearPar
 
 template <typename T, bool GATED> static int linear_rows_launch(const LinearParams& p, cudaStream_t st) {
     auto go = [&](auto kernel, int own) {
-        kernel<<<(unsigned)((p.n + own - 1) / own), kLrThreads, 0, st>>>(p);
+        return launch_behind(kernel, (unsigned)((p.n + own - 1) / own), kLrThreads, 0, st, p);
     };
     constexpr int kHalf = GATED ? 2 : 1;
-    if (p.rows <= 1) go(linear_rows_kernel<T, 1, 8, GATED>, 8 / kHalf);
-    else if (p.rows <= 2) go(linear_rows_kernel<T, 2, 8, GATED>, 8 / kHalf);
-    else if (p.rows <= 4) go(linear_rows_kernel<T, 4, 8, GATED>, 8 / kHalf);
-    else if (p.rows <= 8) go(linear_rows_kernel<T, 8, 8, GATED>, 8 / kHalf);
-    else go(linear_rows_kernel<T, 16, 4, GATED>, 4 / kHalf);
-    KTK_CUDA_TRY(cudaGetLastError(), "ktk_linear_rows");
+    KTK_CUDA_TRY(p.rows <= 1   ? go(linear_rows_kernel<T, 1, 8, GATED>, 8 / kHalf)
+                 : p.rows <= 2 ? go(linear_rows_kernel<T, 2, 8, GATED>, 8 / kHalf)
+                 : p.rows <= 4 ? go(linear_rows_kernel<T, 4, 8, GATED>, 8 / kHalf)
+                 : p.rows <= 8 ? go(linear_rows_kernel<T, 8, 8, GATED>, 8 / kHalf)
+                               : go(linear_rows_kernel<T, 16, 4, GATED>, 4 / kHalf),
+                 "ktk_linear_rows");
     return KTK_OK;
 }
 
