@@ -258,7 +258,7 @@ static int append_impl(const void* k, const void* v, void* cache, void* summarie
                        const int32_t* kv_indptr, const int32_t* kv_last_page_len, const View& view,
                        const ktk_shape* s, int32_t* status, cudaStream_t st) {
     dim3 grid(s->batch, s->num_kv_heads);
-    KTK_CUDA_TRY(launch_behind(append_kernel<T>, grid, kHeadDim, 0, st, (const T*)k, (const T*)v, (T*)cache, (T*)summaries,
+    KTK_CUDA_TRY(launch_behind(true, append_kernel<T>, grid, kHeadDim, 0, st, (const T*)k, (const T*)v, (T*)cache, (T*)summaries,
                                summary_stride, kv_indices, kv_indptr, kv_last_page_len, view.page_count, view.slot_index,
                                s->num_kv_heads, s->num_pages, status),
                  "ktk_append");

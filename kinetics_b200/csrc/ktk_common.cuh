@@ -59,13 +59,17 @@ inline int view_row_width(int topk, const View& v) {
 // that one has ended and its writes are visible; nothing but registers and shared memory is touched before.  A kernel that
 // has called wait_for_front lets its own successor come as soon as all its CTAs have begun.  Every CTA calls it, also one
 // without work: then the end of a kernel implies the end of all in front of it.  Replayed from a graph, us: the fp32 layer
-// step of 4 sequences (11 such kernels) 33.4 -> 31.5, 256 sequences of 8192 tokens (9 of 14) 106.4 -> 104.7.
+// step of 4 sequences (11 such kernels) 33.4 -> 31.5.
+// `early` says whether the CTAs may come before the front's end.  A kernel with much shared memory per CTA comes early only with at
+// most one CTA per SM: while CTAs of either kernel run on an SM its shared memory keeps the share it was given for the front, fewer
+// CTAs fit, and the rest of a grid that was sized for one round waits for a second one (decode of 700 short ragged lists, 592 CTAs,
+// 45 -> 64 us).
 __device__ __forceinline__ void wait_for_front() {
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
 }
 template <typename... P, typename... A>
-inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+inline cudaError_t launch_behind(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -75,7 +79,7 @@ inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, si
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 

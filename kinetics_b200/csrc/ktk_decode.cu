@@ -243,7 +243,7 @@ combine_kernel(const float* __restrict__ ws_ml, const float* __restrict__ ws_o, 
 template <typename T, int G>
 static int simt_launch(const DecodeParams& p, cudaStream_t st) {
     const int64_t ctas = (int64_t)p.batch * p.Hkv * p.num_splits;
-    KTK_CUDA_TRY(launch_behind(decode_simt_kernel<T, G>, (unsigned)ctas, kSimtWarps * 32, 0, st, p), "ktk decode (simt)");
+    KTK_CUDA_TRY(launch_behind(ctas <= sm_count(), decode_simt_kernel<T, G>, (unsigned)ctas, kSimtWarps * 32, 0, st, p), "ktk decode (simt)");
     return KTK_OK;
 }
 
@@ -264,7 +264,7 @@ int launch_decode_simt(const DecodeParams& p, int dtype, int G, cudaStream_t st)
 int launch_combine(const DecodeParams& p, int dtype, int G, cudaStream_t st) {
     const int64_t rows = (int64_t)p.batch * p.Hkv * G;
     const auto go = [&](auto kernel, auto* o) {
-        return launch_behind(kernel, (unsigned)rows, kHeadDim, 0, st, p.ws_ml, p.ws_o, o, p.num_splits);
+        return launch_behind(true, kernel, (unsigned)rows, kHeadDim, 0, st, p.ws_ml, p.ws_o, o, p.num_splits);
     };
     KTK_CUDA_TRY(dtype == KTK_F32 ? go(combine_kernel<float>, (float*)p.o) : go(combine_kernel<__nv_bfloat16>, (__nv_bfloat16*)p.o),
                  "ktk decode (combine)");

@@ -204,7 +204,7 @@ int launch_decode_mma(const DecodeParams& p, int G, cudaStream_t st) {
     mp.d = p;
     mp.G = G;
     const int64_t ctas = (int64_t)p.batch * p.Hkv * p.num_splits;
-    KTK_CUDA_TRY(launch_behind(decode_mma_kernel, (unsigned)ctas, kMmaThreads, smem, st, mp, map), "ktk decode (mma)");
+    KTK_CUDA_TRY(launch_behind(ctas <= sm_count(), decode_mma_kernel, (unsigned)ctas, kMmaThreads, smem, st, mp, map), "ktk decode (mma)");
     return KTK_OK;
 }
 

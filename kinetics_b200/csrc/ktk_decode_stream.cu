@@ -465,9 +465,9 @@ int launch_decode_stream(const DecodeParams& p, int G, int max_entries, cudaStre
     const int smem = stream_smem(var.stages);
     KTK_CUDA_TRY(cudaFuncSetAttribute(var.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                  "ktk decode (balanced)");
-    KTK_CUDA_TRY(launch_behind(var.kernel, grid, kMmaThreads, smem, st, sp, map), "ktk decode (balanced)");
+    KTK_CUDA_TRY(launch_behind(grid <= sm_count(), var.kernel, grid, kMmaThreads, smem, st, sp, map), "ktk decode (balanced)");
     if (grid > 1 || sp.exact) {
-        KTK_CUDA_TRY(launch_behind(stream_combine_kernel, dim3(grid, (unsigned)sp.G), kHeadDim, 0, st, sp),
+        KTK_CUDA_TRY(launch_behind(true, stream_combine_kernel, dim3(grid, (unsigned)sp.G), kHeadDim, 0, st, sp),
                      "ktk decode (balanced, combine)");
     }
     return KTK_OK;

@@ -149,7 +149,7 @@ silu_mul_rows_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __
 template <typename T>
 static int add_rmsnorm_launch(const void* x, const void* residual, const void* w, float eps, void* out_sum,
                               void* out_norm, int64_t rows, int cols, cudaStream_t st) {
-    KTK_CUDA_TRY(launch_behind(add_rmsnorm_kernel<T>, (unsigned)rows, kNormThreads, 0, st, (const T*)x, (const T*)residual,
+    KTK_CUDA_TRY(launch_behind(true, add_rmsnorm_kernel<T>, (unsigned)rows, kNormThreads, 0, st, (const T*)x, (const T*)residual,
                                (const T*)w, eps, (T*)out_sum, (T*)out_norm, cols),
                  "ktk_add_rmsnorm");
     return KTK_OK;
@@ -161,7 +161,7 @@ static int qkv_norm_launch(const void* proj, const void* wq, const void* wk, flo
                            const int64_t* position_ids, int64_t max_positions, cudaStream_t st) {
     const unsigned grid = (unsigned)((rows + 3) / 4);
     const bool turn = cos_tab != nullptr;
-    KTK_CUDA_TRY(launch_behind(turn ? qkv_norm_kernel<T, true> : qkv_norm_kernel<T, false>, grid, 128, 0, st, (const T*)proj,
+    KTK_CUDA_TRY(launch_behind(true, turn ? qkv_norm_kernel<T, true> : qkv_norm_kernel<T, false>, grid, 128, 0, st, (const T*)proj,
                                (const T*)wq, (const T*)wk, eps, (T*)q, (T*)k, (T*)v, rows, Hq, Hkv, (const T*)cos_tab,
                                (const T*)sin_tab, turn ? position_ids : nullptr, turn ? max_positions : 0),
                  "ktk_qkv_norm");
@@ -173,7 +173,7 @@ static int silu_vec_launch(const void* gate, const void* up, void* out, int64_t 
     int64_t blocks = (nvec + 255) / 256;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    KTK_CUDA_TRY(launch_behind(silu_mul_vec_kernel<T>, (unsigned)blocks, 256, 0, st, (const T*)gate, (const T*)up, (T*)out, nvec),
+    KTK_CUDA_TRY(launch_behind(true, silu_mul_vec_kernel<T>, (unsigned)blocks, 256, 0, st, (const T*)gate, (const T*)up, (T*)out, nvec),
                  "ktk_silu_mul");
     return KTK_OK;
 }
@@ -185,7 +185,7 @@ static int silu_rows_launch(const void* gate, const void* up, void* out, int64_t
     int64_t blocks = (nvec + 255) / 256;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    KTK_CUDA_TRY(launch_behind(silu_mul_rows_kernel<T>, (unsigned)blocks, 256, 0, st, (const T*)gate, (const T*)up, (T*)out, rows,
+    KTK_CUDA_TRY(launch_behind(true, silu_mul_rows_kernel<T>, (unsigned)blocks, 256, 0, st, (const T*)gate, (const T*)up, (T*)out, rows,
                                cols / 8, in_stride),
                  "ktk_silu_mul_rows");
     return KTK_OK;

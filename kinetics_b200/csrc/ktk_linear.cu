@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kLrThreads) linear_rows_kernel(const LinearPar
 
 template <typename T, bool GATED> static int linear_rows_launch(const LinearParams& p, cudaStream_t st) {
     auto go = [&](auto kernel, int own) {
-        return launch_behind(kernel, (unsigned)((p.n + own - 1) / own), kLrThreads, 0, st, p);
+        return launch_behind(true, kernel, (unsigned)((p.n + own - 1) / own), kLrThreads, 0, st, p);
     };
     constexpr int kHalf = GATED ? 2 : 1;
     KTK_CUDA_TRY(p.rows <= 1   ? go(linear_rows_kernel<T, 1, 8, GATED>, 8 / kHalf)

@@ -185,7 +185,7 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
         issued_total = 0;
         mbar_init_fence();
     }
-    if (!TAKE) wait_for_front();
+    if (!TAKE) wait_for_front();                         // a kernel that takes its items is launched plainly: its CTAs come and go
     __syncthreads();
 
     if (warp == kSelWarps) {
@@ -575,13 +575,9 @@ static int select_launch(const void* q, const void* summaries, int64_t summary_s
     KTK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                  "ktk_select");
     const unsigned grid = (unsigned)(take || items < slots ? items : slots);
-    const auto go = [&](auto... args) {
-        if (!take) return launch_behind(kern, grid, kSelCtaThreads, smem, st, args...);
-        kern<<<grid, kSelCtaThreads, smem, st>>>(args...);    // its CTAs come and go as they are taken
-        return cudaGetLastError();
-    };
-    KTK_CUDA_TRY(go((const T*)q, (const T*)summaries, summary_stride, kv_indices, kv_indptr, kv_last_page_len, topk, key_cap, kp,
-                    view, out_pages, out_logical, out_scores, items, s->num_kv_heads, s->num_pages, status),
+    KTK_CUDA_TRY(launch_behind(items <= sm_count(), kern, grid, kSelCtaThreads, smem, st, (const T*)q, (const T*)summaries,
+                               summary_stride, kv_indices, kv_indptr, kv_last_page_len, topk, key_cap, kp, view, out_pages,
+                               out_logical, out_scores, items, s->num_kv_heads, s->num_pages, status),
                  "ktk_select");
     return KTK_OK;
 }

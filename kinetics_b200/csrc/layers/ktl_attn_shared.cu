@@ -10,8 +10,8 @@
 // Else, and for portions: one CTA per (split of a sequence's tokens, chunk of heads, group of rows).  Roles:
 //     loading warp     TMA: tiles of 64 tokens into a ring
 //     issuing warps    one for each product
-//     softmax warps    warp w holds tokens 16 w .., two per thread; exponentials against a reference per column, at first the largest of its sink and the first tile's scores, that moves
-//                      only when a score exceeds it by 2^8
+//     softmax warps    warp w holds tokens 16 w .., two per thread; exponentials against a reference per column, at first
+//                      the largest of its sink and the first tile's scores, that moves only when a score exceeds it by 2^8
 // The sum of a column's weights stays spread over the threads until the end.  Tensor memory: S of two tiles, then
 // O^T in blocks of 128 columns of V.  Every wait is bounded.
 #include "ktl_score.cuh"
