@@ -636,3 +636,20 @@ def test_append_tokens_by_pieces_bit_exact(cuda_device, dtype, shift, Hkv):
     want = oracle.summaries_v(st["kv_cache"], st["kv_indices"], st["kv_indptr"], st["kv_last_page_len"], st["summary_stride"], 0)
     for b, n in enumerate(st["npages"]):
         assert torch.equal(_bits(summ.cpu()[b, :, :n]), _bits(want[b, :, :n]))
+
+
+@pytest.mark.parametrize("batch, pages", [(1, 40), (1, 700), (1, 9000), (3, 2100), (37, 300), (150, 70)])
+def test_lists_cut_into_many_pieces(cuda_device, batch, pages):
+    # 2 to several hundred pieces per list, whole and partial rounds of the merge, against one piece per list: either side's
+    # weights are rounded to bf16 (2^-9 of a term), its result once more
+    from kinetics_b200 import ops
+    g = torch.Generator().manual_seed(pages)
+    put = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).to(cuda_device)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda_device)
+    q, cache = put(batch, 8, 128), put(batch * pages, 2, 16, 1, 128)
+    table = (i32(torch.randperm(batch * pages, generator=g).tolist()), i32([b * pages for b in range(batch + 1)]),
+             i32([1 + b % 16 for b in range(batch)]))
+    one = ops.dense_decode(q, cache, *table, pages, num_splits=1)
+    got = ops.dense_decode(q, cache, *table, pages)
+    scale = one.double().pow(2).mean().sqrt()
+    assert (got.double() - one.double()).abs().max() < 0.03 * scale
