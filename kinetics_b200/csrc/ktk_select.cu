@@ -44,6 +44,15 @@ __device__ __forceinline__ unsigned long long composite(uint32_t key, int page) 
 __device__ __forceinline__ void consumer_sync() {
     asm volatile("bar.sync 1, %0;" ::"n"(kSelThreads) : "memory");
 }
+// The same, and whether any consumer thread brings x.  A consumer leaves the item loop by this answer alone, which is one for all: a warp
+// that left by a wait or by a look at abort_flag of its own would leave the others in a barrier for good.
+__device__ __forceinline__ bool consumer_any(bool x) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any) : "r"((uint32_t)x), "n"(kSelThreads) : "memory");
+    return any != 0;
+}
 
 // eight consecutive elements (one chunk) of a staged row as fp32
 __device__ __forceinline__ void lds8(const float* p, float (&out)[8]) {
@@ -237,6 +246,7 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
                 fence_proxy_async();                         // read before the next answer overwrites it
                 const int slot = k % kSelAhead;
                 if (k >= kSelAhead && !mbar_wait(&item_free[slot], (k / kSelAhead - 1) & 1, &abort_flag)) break;
+                if (*(volatile int*)&abort_flag) break;      // the wait may have ended after somebody gave up: nothing more is handed out
                 item_ring[slot] = rank;
                 mbar_arrive(&item_full[slot]);
                 if (rank < 0) break;
@@ -253,7 +263,7 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
                 if (rank < 0) break;
             } else if (k >= 0) {
                 const int slot = k % kSelAhead;
-                if (!__all_sync(0xffffffffu, mbar_wait(&item_full[slot], (k / kSelAhead) & 1, &abort_flag))) break;
+                if (consumer_any(!mbar_wait(&item_full[slot], (k / kSelAhead) & 1, &abort_flag))) break;
                 rank = item_ring[slot];
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&item_free[slot]);
@@ -357,8 +367,7 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
                     if (lane == 0) mbar_arrive(&empty_bar[s]);
                 }
                 ibase += it.n_stages;
-                consumer_sync();            // every key of the item is in shared memory (or the CTA gave up)
-                if (!ok || abort_flag) break;
+                if (consumer_any(!ok)) break;            // every key of the item is in shared memory, or the CTA gives up
             }
 
             if (!it.need_select) {

@@ -1,0 +1,46 @@
+"""What the kernels' sources have to keep to where a bounded wait runs out, which no test can make happen on a GPU: the threads
+that meet in a barrier go on together or leave together."""
+import itertools
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "kinetics_b200" / "csrc"
+
+
+def _consumers_of_selection():
+    text = (CSRC / "ktk_select.cu").read_text()
+    return text[text.index("// ---------------- consumer warps ----------------"):text.index("// ---- the k-th largest")]
+
+
+def _stuck(vote):
+    """Two warps and what each sees at its two points of leaving (its wait for the item, then the flag behind the item's barrier, raised
+    in between): the cases in which one has left and the other stands in a barrier."""
+    cases = []
+    for item_a, item_b, flag_a, flag_b in itertools.product((True, False), repeat=4):
+        left = []
+        for mine, flag in ((item_a, flag_a), (item_b, flag_b)):
+            if vote:
+                left.append(not (item_a and item_b) or flag_a or flag_b)
+            else:
+                left.append(not mine or flag)
+        if left[0] != left[1]:
+            cases.append((item_a, item_b, flag_a, flag_b))
+    return cases
+
+
+def test_consumers_of_the_selection_leave_together():
+    assert _stuck(vote=False) and not _stuck(vote=True)
+    body = _consumers_of_selection()
+    # every way out of the item loop: behind a vote of all consumers, or behind a rank that is the same for all of them
+    for line in (x.strip() for x in body.splitlines()):
+        if re.search(r"\bbreak;", line) and line != "break;":
+            assert "consumer_any(" in line or line == "if (rank < 0) break;", line
+    alone = re.findall(r"\{\s*ok = false;\s*break;\s*\}", body)            # out of the loop over an item's stages, to the vote behind it
+    assert len(re.findall(r"^\s*break;", body, re.M)) == len(alone) == 1
+    assert "abort_flag)" not in body.replace("&abort_flag)", "")             # no look of a warp's own
+
+
+def test_the_producer_of_the_selection_hands_out_nothing_after_giving_up():
+    text = (CSRC / "ktk_select.cu").read_text()
+    wait, hand_out = text.index("mbar_wait(&item_free[slot]"), text.index("mbar_arrive(&item_full[slot])")
+    assert "*(volatile int*)&abort_flag) break;" in text[wait:hand_out]
