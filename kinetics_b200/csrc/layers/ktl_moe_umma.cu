@@ -224,10 +224,14 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
         auto landed = [&](uint64_t* bar) {
             return __all_sync(0xffffffffu, mbar_wait_fast(bar, pos.round & 1, &abort_flag)) != 0;
         };
-        // one look for both, a lane each: two waits one behind the other take longer than the matrix instructions in the queue
+        // One look for both, a lane each: two waits one behind the other take longer than the matrix instructions in the queue.  What a lane
+        // saw land is ordered before the other lanes' instructions by the __syncwarp; the ballot orders no memory.
         auto both_landed = [&](uint64_t* a, uint64_t* b) {
             for (uint32_t i = 0; i < (1u << 24); ++i) {
-                if ((__ballot_sync(0xffffffffu, mbar_test(lane == 0 ? a : b, pos.round & 1)) & 3u) == 3u) return true;
+                if ((__ballot_sync(0xffffffffu, mbar_test(lane == 0 ? a : b, pos.round & 1)) & 3u) == 3u) {
+                    __syncwarp();
+                    return true;
+                }
                 if ((i & 63u) == 63u && *(volatile int*)&abort_flag) return false;
             }
             abort_flag = 1;

@@ -1,5 +1,5 @@
-"""What the kernels' sources have to keep to where a bounded wait runs out, which no test can make happen on a GPU: the threads
-that meet in a barrier go on together or leave together."""
+"""What the kernels' sources have to keep to around their bounded waits and no run can show: where a wait runs out, the threads that
+meet in a barrier leave together; what one lane has seen land is ordered before what another lane issues."""
 import itertools
 import re
 from pathlib import Path
@@ -44,3 +44,11 @@ def test_the_producer_of_the_selection_hands_out_nothing_after_giving_up():
     text = (CSRC / "ktk_select.cu").read_text()
     wait, hand_out = text.index("mbar_wait(&item_free[slot]"), text.index("mbar_arrive(&item_full[slot])")
     assert "*(volatile int*)&abort_flag) break;" in text[wait:hand_out]
+
+
+def test_a_lane_that_looks_for_another_hands_on_what_it_saw():
+    """Two lanes look at a barrier each and any lane may issue the products: a vote orders control flow, __syncwarp memory."""
+    text = (CSRC / "layers" / "ktl_moe_umma.cu").read_text()
+    look = text[text.index("auto both_landed"):]
+    look = look[:look.index("return true;")]
+    assert look.index("__ballot_sync(") < look.index("__syncwarp();")
