@@ -232,7 +232,7 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
                     __syncwarp();
                     return true;
                 }
-                if ((i & 63u) == 63u && *(volatile int*)&abort_flag) return false;
+                if ((i & 63u) == 63u && __any_sync(0xffffffffu, *(volatile int*)&abort_flag)) return false;
             }
             abort_flag = 1;
             return false;

@@ -224,7 +224,8 @@ __global__ void __launch_bounds__(kRnThreads, rn_resident(2)) residual_norm_walk
     uint32_t parity = 0;
     int64_t r = blockIdx.x;
     for (int i = 0; r < p.rows; ++i, r += step) {
-        if (!mbar_wait(&full[s], parity, &abort_flag)) break;
+        // the vote keeps the warp together should a single lane give up: the sums below shuffle over all of it
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], parity, &abort_flag))) break;
         if (threadIdx.x == 0 && i > 0) {                     // everybody has read the row before: its sums had a barrier
             fence_proxy_async();
             ask(r + (stages - 1) * step);

@@ -52,3 +52,13 @@ def test_a_lane_that_looks_for_another_hands_on_what_it_saw():
     look = text[text.index("auto both_landed"):]
     look = look[:look.index("return true;")]
     assert look.index("__ballot_sync(") < look.index("__syncwarp();")
+
+
+def test_lanes_of_a_warp_give_up_together():
+    """Behind these waits stand shuffles and votes over the whole warp: one lane alone may not leave."""
+    look = (CSRC / "layers" / "ktl_moe_umma.cu").read_text()
+    look = look[look.index("auto both_landed"):look.index("if (PAIR && rank == 1)")]
+    assert re.findall(r"if \((.*)\) return false;", look) == ["(i & 63u) == 63u && __any_sync(0xffffffffu, *(volatile int*)&abort_flag)"]
+    walk = (CSRC / "layers" / "ktl_norm.cu").read_text()
+    walk = walk[walk.index("residual_norm_walk_kernel(const"):]
+    assert re.findall(r"if \((.*mbar_wait.*)\) break;", walk) == ["!__all_sync(0xffffffffu, mbar_wait(&full[s], parity, &abort_flag))"]
