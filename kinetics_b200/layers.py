@@ -64,13 +64,17 @@ def _plain(linear) -> bool:
 
 
 def _by_rows(x, *linears) -> bool:
-    """Whether the product of x with one layer, or the gated product of two, goes to ktk::linear_rows."""
-    w = linears[0].weight
+    """Whether the product of x with one layer, or the gated product of two, goes to ktk::linear_rows.  What that op would refuse and the
+    library takes (or refuses in its own words) stays with the library."""
+    w, bias = linears[0].weight, linears[0].bias
     return (not torch.compiler.is_compiling() and type(x) is torch.Tensor and x.dim() == 2 and x.is_cuda and
+            x.shape[1] == w.shape[1] and
             ops.linear_rows_wins(x.shape[0], w.shape[0], w.shape[1], x.dtype, len(linears) == 2) and
-            all(_plain(m) and m.weight.dtype == x.dtype and m.weight.is_cuda and m.weight.is_contiguous() and
+            all(_plain(m) and m.weight.dtype == x.dtype and m.weight.device == x.device and m.weight.is_contiguous() and
                 m.weight.shape == w.shape and m.weight.data_ptr() % 16 == 0 for m in linears) and
-            (len(linears) == 1 or all(m.bias is None for m in linears)) and x.is_contiguous() and x.data_ptr() % 16 == 0 and
+            (bias is None or len(linears) == 1 and type(bias) is nn.Parameter and bias.dtype == x.dtype and
+             bias.device == x.device and bias.is_contiguous()) and
+            (len(linears) == 1 or linears[1].bias is None) and x.is_contiguous() and x.data_ptr() % 16 == 0 and
             not torch.is_autocast_enabled("cuda"))
 
 

@@ -53,3 +53,15 @@ def test_a_hooked_layer_is_called(cuda_device):
     assert not layers._by_rows(x.half(), lin) and not layers._by_rows(x.t(), lin)
     with torch.autocast("cuda", dtype=torch.bfloat16):
         assert not layers._by_rows(x, lin)
+
+
+def test_a_bias_that_is_not_contiguous_stays_with_the_library(cuda_device):
+    from kinetics_b200 import layers
+    lin = torch.nn.Linear(64, 32, device=cuda_device).requires_grad_(False)
+    x, plain = torch.randn(4, 64, device=cuda_device), lin.bias.detach().clone()
+    lin.bias = torch.nn.Parameter(torch.stack((plain, plain + 1), dim=1)[:, 0], requires_grad=False)
+    assert not lin.bias.is_contiguous()
+    want = x.double() @ lin.weight.double().t() + plain.double()
+    torch.testing.assert_close(layers._linear(lin, x).double(), want, rtol=1e-5, atol=1e-5)
+    with pytest.raises(RuntimeError):                        # refused as the library refuses it
+        layers._linear(lin, torch.randn(4, 72, device=cuda_device))
