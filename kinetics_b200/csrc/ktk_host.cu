@@ -16,7 +16,10 @@ void set_error(const char* fmt, ...) {
     va_end(ap);
 }
 
+// Takes the runtime's last error with it (a call that returns its own error leaves it there): the check behind the next launch, of
+// another operation, would report it again.
 int cuda_fail(cudaError_t e, const char* who) {
+    (void)cudaGetLastError();
     set_error("%s: CUDA error %d (%s)", who, (int)e, cudaGetErrorString(e));
     return KTK_ERR_CUDA;
 }

@@ -1,4 +1,6 @@
 """Kernels that are sent to the device while the one in front of them still runs: each sees all that was written before it."""
+import ctypes
+
 import pytest
 import torch
 
@@ -55,3 +57,21 @@ def test_chains_equal_synchronised_ones(cuda_device, dtype, rows, batch, pages):
         graph.replay()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     ops.raise_on_status(status)
+
+
+def test_a_launch_that_fails_leaves_no_error_behind(cuda_device):
+    # a capture that was ended by a forbidden call refuses launches on its stream; the next operation, elsewhere, is none the wiser
+    from kinetics_b200 import _lib, ops
+    lib, runtime, stream = _lib.load(), ctypes.CDLL("libcudart.so.12"), torch.cuda.Stream()
+    x, w = torch.randn(4, 64, device=cuda_device), torch.randn(32, 64, device=cuda_device)
+    out, on = torch.empty(4, 32, device=cuda_device), ctypes.c_void_p(stream.cuda_stream)
+    torch.cuda.synchronize()
+    assert runtime.cudaStreamBeginCapture(on, 2) == 0
+    assert runtime.cudaStreamSynchronize(on) != 0
+    rc = lib.ktk_linear_rows(x.data_ptr(), w.data_ptr(), None, None, None, out.data_ptr(), 4, 32, 64, _lib.KTK_F32, on)
+    text, graph = lib.ktk_last_error(), ctypes.c_void_p()
+    assert runtime.cudaStreamEndCapture(on, ctypes.byref(graph)) != 0
+    runtime.cudaGetLastError()                               # the test's own calls
+    assert rc != 0 and b"CUDA error" in text
+    torch.testing.assert_close(ops.rmsnorm(x, torch.ones(64, device=cuda_device), 1e-6),
+                               torch.nn.functional.rms_norm(x, (64,), eps=1e-6), rtol=1e-5, atol=1e-5)
