@@ -82,7 +82,8 @@ KTK_API int ktk_kv_append(const void* proj, int64_t row_stride, int64_t k_col, i
  * variant: KTK_VARIANT_AUTO, _SIMT (any size, fp32 math), _MMA (bf16, one row per sequence), _UMMA (bf16 on tcgen05).
  * splits: parts that a sequence's keys are cut into (0: policy); with new_indptr only where values lie in the keys.
  * KTK_SPLITS_BALANCED (one row per sequence, values in the keys): the page lists of all sequences are cut into equal parts instead;
- * ktk_paged_attention_splits gives it where that is faster.  With less workspace than it needs, the policy's parts are used.
+ * ktk_paged_attention_splits gives it where that is faster.  With less workspace than it needs, the policy's parts are used,
+ * as many as the workspace holds (one needs none).
  * The policy's new_rows: 0 for one row per sequence, else the rows of each.
  * sink fp32 [heads] (nullable, maps = 1): exp(sink) joins each row's denominator, without key, value or scale.
  * gate (nullable, maps = 1), in `dtype`: head h of row r is multiplied by sigmoid(gate[r * gate_stride + h]).

@@ -131,6 +131,10 @@ extern "C" int ktk_paged_attention(const void* q, int64_t q_stride, const int32_
         const bool balanced = splits == KTK_SPLITS_BALANCED && !new_indptr &&
                               workspace_bytes >= attn_shared_workspace(*shape, rows, splits) && workspace;
         if (p.splits <= 0 && !balanced) p.splits = attn_shared_splits(*shape, table->batch, new_indptr ? max_new : 0, 1 << 20);
+        if (splits == KTK_SPLITS_BALANCED && !new_indptr && !balanced) {       // as many of those parts as the workspace holds
+            const size_t each = attn_shared_workspace(*shape, rows, 2) / 2, hold = workspace ? workspace_bytes / each : 0;
+            if ((size_t)p.splits > hold) p.splits = hold < 1 ? 1 : (int32_t)hold;
+        }
         const size_t need = attn_shared_workspace(*shape, rows, p.splits);
         if (need && (!workspace || workspace_bytes < need)) {
             set_error("%s: workspace of %zu bytes needed, got %zu", who, need, workspace ? workspace_bytes : (size_t)0);

@@ -17,12 +17,12 @@ def _spec(heads, cols, vdim, scale):
     return AttentionSpec(heads=heads, kv_heads=1, dim=cols, vdim=vdim, scale=scale, values_in_keys=True)
 
 
-def _attend(dev, spec, q, pages, dtype, sink, gate, indptr, max_new, variant=0, splits=1):
+def _attend(dev, spec, q, pages, dtype, sink, gate, indptr, max_new, variant=0, splits=1, workspace=None):
     from kinetics_b200 import layer_ops as lo, ops
     status = ops.new_status(dev)
     out = lo.paged_attention(q.flatten(1).to(dtype).to(dev).contiguous(), pages.pages, pages.pages, pages.table, spec,
                              None if indptr is None else torch.tensor(indptr, dtype=torch.int32, device=dev), max_new,
-                             splits, variant=variant, status=status, sink=sink.float().to(dev),
+                             splits, workspace, variant=variant, status=status, sink=sink.float().to(dev),
                              gate=gate.to(dtype).to(dev).contiguous())
     ops.raise_on_status(status)
     return out.view(q.shape[0], spec.heads, -1)[:, :, :spec.vdim].double().cpu()
@@ -438,6 +438,23 @@ def test_fused_steps_of_many_sequences_equal_the_separate_ones(cuda_device):
             torch.testing.assert_close(one, two, rtol=2e-2, atol=2e-3)
         torch.testing.assert_close(a.state, b.state, rtol=1e-3, atol=1e-4)
         assert torch.equal(a.ring, b.ring)
+
+
+@pytest.mark.parametrize("batch", [1, 40, 130])
+def test_balanced_rows_with_little_workspace(cuda_device, batch):
+    """What the workspace holds decides the parts: none, two, all but one of the policy's, one byte less than the balanced form's.
+    Bound: either side's weights and result are rounded to bf16, as in test_decode_rows."""
+    from kinetics_b200 import layer_ops as lo, ops
+    heads, cols, vdim = 16, 576, 512
+    spec, lens = _spec(heads, cols, vdim, 1.1 / cols ** 0.5), [1 + 391 * i % 900 for i in range(batch)]
+    g = torch.Generator().manual_seed(batch)
+    pages = RowPages([torch.randn(n, cols, generator=g) for n in lens], BF, 64, cuda_device, 1)
+    q, sink, gate = torch.randn(batch, heads, cols, generator=g), torch.randn(heads, generator=g), torch.randn(batch, heads, generator=g)
+    run = lambda splits, ws=None: _attend(cuda_device, spec, q, pages, BF, sink, gate, None, 1, 0, splits, ws)
+    want, size = run(1), lambda s: lo.attention_workspace(spec, batch, s, BF)
+    for need in (16, size(2), size(9) - 16, size(ops.SPLITS_BALANCED) - 16):
+        got = run(ops.SPLITS_BALANCED, torch.empty(need, dtype=torch.uint8, device=cuda_device))
+        assert rms(got - want) / rms(want) < 1.2e-2, need
 
 
 @pytest.mark.parametrize("blocks,block,taps,rows,misaligned", [(16, 256, 4, 150, False), (16, 256, 4, 150, True), (20, 200, 3, 70, False),
