@@ -29,7 +29,6 @@ template <typename T> struct SelStage;              // rows per stage: a multipl
 template <> struct SelStage<__nv_bfloat16> { static constexpr int kRows = 24; };   // 6 KiB
 template <> struct SelStage<float> { static constexpr int kRows = 16; };           // 8 KiB
 constexpr int kSelCtasPerSm = 3;
-constexpr int kSelAhead = 4;                        // items that the producer may be ahead
 constexpr int kMaxTopk = 1024;
 constexpr int kSelBins = 2048;                      // first radix digit: the top 11 bits of a key
 constexpr int kSelBinShift = 21;
@@ -44,6 +43,7 @@ __device__ __forceinline__ unsigned long long composite(uint32_t key, int page) 
 __device__ __forceinline__ void consumer_sync() {
     asm volatile("bar.sync 1, %0;" ::"n"(kSelThreads) : "memory");
 }
+
 // The same, and whether any consumer thread brings x.  A consumer leaves the item loop by this answer alone, which is one for all: a warp
 // that left by a wait or by a look at abort_flag of its own would leave the others in a barrier for good.
 __device__ __forceinline__ bool consumer_any(bool x) {
@@ -63,23 +63,6 @@ __device__ __forceinline__ void lds8(const float* p, float (&out)[8]) {
 }
 __device__ __forceinline__ void lds8(const __nv_bfloat16* p, float (&out)[8]) {
     unpack8(*reinterpret_cast<const uint4*>(p), out);
-}
-
-// Asks for a CTA of the grid that has not started yet: it is then not launched, and its work is the caller's.  The answer, 16 bytes,
-// lands in shared memory and is counted on the barrier.
-__device__ __forceinline__ void take_pending_cta(uint4* answer, uint64_t* bar) {
-    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
-                 ::"r"(smem_u32(answer)), "r"(smem_u32(bar)) : "memory");
-}
-// its index, or -1: there is none left, and no more may be asked for
-__device__ __forceinline__ int64_t taken_cta(const uint4* answer) {
-    uint32_t x, got;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\tld.shared.b128 a, [%2];\n\t"
-        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\tselp.u32 %1, 1, 0, p;\n\tmov.u32 %0, 0;\n\t"
-        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n\t}"
-        : "=&r"(x), "=&r"(got) : "r"(smem_u32(answer)) : "memory");
-    return got ? (int64_t)x : -1;
 }
 
 // The view of the page table a launch works under (ktk_view with defaults filled in) and the
@@ -119,32 +102,33 @@ __device__ __forceinline__ SelItem sel_item(int b, const int32_t* kv_indptr, con
     return it;
 }
 
-// Position `round` of CTA blockIdx.x in the queue of items, dealt out beforehand: -1 behind the last.  With an order the rounds
-// alternate in direction, so that the CTA that got the longest sequences of one round gets the shortest of the next.
-__device__ __forceinline__ int64_t dealt_rank(int64_t round, int64_t n_items, const SelView& view) {
+// The item CTA `cta` handles in its round `round`, or -1 when that round has none for it.  Without an order: item
+// round * grid + cta.  With one (sequences sorted from the longest to the shortest) the rounds alternate in
+// direction, so that the CTA that got the longest sequences of one round gets the shortest of the next, and the
+// item is (seq_order[rank / Hkv], rank % Hkv); -2 for an entry that is no sequence of the batch.  us without / with an order: 1024
+// lists of 64 to 1024 pages 46.6 / 37.1, 1024 of 30 .. 500 30.5 / 26.5, 4096 of 128 .. 2048 226 / 206, 500 of 200 .. 1000 32.4 / 22.9.
+// CTAs that take the next list of the grid when they are nearly through (cluster launch control) were slower than a deal in order (38.4,
+// 29.6, 209, 23.5) and, without one, for even lists (600 of 1024 pages 39.4 dealt, 42.7 taken; 1024 59.2, 62.6; 4096 188.7, 195.8).
+__device__ __forceinline__ int64_t sel_item_of(int64_t round, int64_t n_items, int Hkv, const int32_t* seq_order) {
     const int64_t grid = gridDim.x, cta = blockIdx.x;
-    const int64_t rank = round * grid + (view.seq_order && (round & 1) ? grid - 1 - cta : cta);
-    return round * grid >= n_items ? -1 : rank < n_items ? rank : n_items;
-}
-// The item at a position: (seq_order[rank / Hkv], rank % Hkv) with an order (sequences sorted from the longest to the shortest),
-// -2 for an entry that is no sequence of the batch, -1 behind the last.
-__device__ __forceinline__ int64_t sel_item_of(int64_t rank, int64_t n_items, int Hkv, const int32_t* seq_order) {
+    if (seq_order == nullptr) {
+        const int64_t bh = round * grid + cta;
+        return bh < n_items ? bh : -1;
+    }
+    const int64_t rank = round * grid + ((round & 1) ? grid - 1 - cta : cta);
     if (rank >= n_items) return -1;
-    if (seq_order == nullptr) return rank;
     const int64_t b = seq_order[rank / Hkv];
     if (b < 0 || b >= n_items / Hkv) return -2;
     return b * Hkv + rank % Hkv;
 }
 
-// Persistent kernel over the (sequence, kv head) items.  TAKE: the grid has a CTA for each, and one that is nearly through with
-// its streaming takes the item of a CTA that has not started yet in that one's place (cluster launch control), so that
-// ragged items even out; else CTA c handles the items c, c + gridDim.x, ...
+// Persistent kernel: CTA c handles the (sequence, kv head) items c, c + gridDim.x, ... (see sel_item_of)
 // A producer warp streams the summaries of its items, one after the other without a gap,
 // through a ring of shared-memory stages with bulk asynchronous copies (the rows of one item
 // are contiguous); stage i of the stream is scored by consumer warp i mod 8, sixteen lanes per
 // row.  While the consumers run the selection of one item, the producer is already filling the
 // ring with the rows of the next.  The first radix pass is histogrammed while scoring.
-template <typename T, int G, bool TAKE>
+template <typename T, int G>
 __global__ void __launch_bounds__(kSelCtaThreads, kSelCtasPerSm)
 select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t summary_stride,
               const int32_t* __restrict__ kv_indices, const int32_t* __restrict__ kv_indptr,
@@ -162,10 +146,6 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
     __shared__ unsigned int s_wsum[kSelWarps];
     __shared__ int s_digit, s_greater, s_bincount, s_count, s_ccount;
     __shared__ int abort_flag, issued_total;
-    // the items of this CTA in order, -1 behind the last: written by the producer, read by the consumers
-    __shared__ int64_t item_ring[kSelAhead];
-    __shared__ __align__(8) uint64_t item_full[kSelAhead], item_free[kSelAhead], next_bar;
-    __shared__ __align__(16) uint4 next_answer;
 
     constexpr int kRowBytes = kHeadDim * (int)sizeof(T);
     constexpr int kRowsPerStage = SelStage<T>::kRows;
@@ -183,18 +163,11 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
-        if (TAKE) {
-            for (int k = 0; k < kSelAhead; ++k) {
-                mbar_init(&item_full[k], 1);
-                mbar_init(&item_free[k], kSelWarps);
-            }
-            mbar_init(&next_bar, 1);
-        }
         abort_flag = 0;
         issued_total = 0;
         mbar_init_fence();
     }
-    if (!TAKE) wait_for_front();                         // a kernel that takes its items is launched plainly: its CTAs come and go
+    wait_for_front();
     __syncthreads();
 
     if (warp == kSelWarps) {
@@ -202,25 +175,16 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
         if (lane == 0) {
             int i = 0;           // stages issued so far, over all items of this CTA
             bool alive = true;
-            int64_t rank = blockIdx.x;
-            for (int k = 0;; ++k) {                          // items taken so far; the first is known without the ring
-                // the item after this one is asked for a ring's length before this one's last rows (all items asked for at
-                // their predecessors' start were dealt out as unevenly as beforehand) and looked at behind them
-                bool asked = false;
-                auto ask = [&] {
-                    mbar_arrive_expect_tx(&next_bar, 16);
-                    take_pending_cta(&next_answer, &next_bar);
-                    asked = true;
-                };
-                const int64_t bh = sel_item_of(rank, n_items, Hkv, view.seq_order);
-                if (bh >= 0) {
+            const int64_t rounds = (n_items + gridDim.x - 1) / gridDim.x;
+            for (int64_t round = 0; round < rounds && alive; ++round) {
+                const int64_t bh = sel_item_of(round, n_items, Hkv, view.seq_order);
+                if (bh < 0) continue;
                 const int b = (int)(bh / Hkv);
                 const int h = (int)(bh % Hkv);
                 const SelItem it = sel_item<kRowsPerStage>(b, kv_indptr, kv_last_page_len, view, summary_stride,
                                                            key_cap, topk, want_scores);
                 const T* sbase = summaries + (((int64_t)it.slot * Hkv + h) * summary_stride + it.front) * kHeadDim;
                 for (int st = 0; st < it.n_stages; ++st, ++i) {
-                    if (TAKE && !asked && st + kSelStages + 4 >= it.n_stages) ask();
                     const int s = i % kSelStages;
                     if (i >= kSelStages && !mbar_wait(&empty_bar[s], ((i / kSelStages) - 1) & 1, &abort_flag)) {
                         alive = false;
@@ -232,44 +196,15 @@ select_kernel(const T* __restrict__ q, const T* __restrict__ summaries, int64_t 
                     mbar_arrive_expect_tx(&full_bar[s], bytes);
                     bulk_load(sel_smem + s * kSelStageBytes, sbase + (int64_t)r0 * kHeadDim, bytes, &full_bar[s]);
                 }
-                }
-                if (!TAKE) {
-                    rank = dealt_rank(k + 1, n_items, view);
-                    if (!alive || rank < 0) break;
-                    continue;
-                }
-                if (!asked) ask();
-                volatile int never = 0;                      // the answer still writes shared memory: no leaving before it
-                if (!mbar_wait(&next_bar, k & 1, &never)) abort_flag = 1;
-                if (!alive || abort_flag) break;
-                rank = taken_cta(&next_answer);
-                fence_proxy_async();                         // read before the next answer overwrites it
-                const int slot = k % kSelAhead;
-                if (k >= kSelAhead && !mbar_wait(&item_free[slot], (k / kSelAhead - 1) & 1, &abort_flag)) break;
-                if (*(volatile int*)&abort_flag) break;      // the wait may have ended after somebody gave up: nothing more is handed out
-                item_ring[slot] = rank;
-                mbar_arrive(&item_full[slot]);
-                if (rank < 0) break;
             }
             issued_total = i;
         }
     } else {
         // ---------------- consumer warps ----------------
         int ibase = 0;           // stream position of the current item's first stage
-        for (int k = -1;; ++k) {                             // -1: this CTA's own item
-            int64_t rank = blockIdx.x;
-            if (k >= 0 && !TAKE) {
-                rank = dealt_rank(k + 1, n_items, view);
-                if (rank < 0) break;
-            } else if (k >= 0) {
-                const int slot = k % kSelAhead;
-                if (consumer_any(!mbar_wait(&item_full[slot], (k / kSelAhead) & 1, &abort_flag))) break;
-                rank = item_ring[slot];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&item_free[slot]);
-                if (rank < 0) break;
-            }
-            const int64_t bh = sel_item_of(rank, n_items, Hkv, view.seq_order);
+        const int64_t rounds = (n_items + gridDim.x - 1) / gridDim.x;
+        for (int64_t round = 0; round < rounds; ++round) {
+            const int64_t bh = sel_item_of(round, n_items, Hkv, view.seq_order);
             if (bh < 0) {
                 if (bh == -2 && tid == 0) report(status, KTK_STATUS_BAD_TABLE);
                 continue;
@@ -574,17 +509,13 @@ static int select_launch(const void* q, const void* summaries, int64_t summary_s
     while (kp < topk) kp <<= 1;
     const size_t smem = (size_t)kSelStages * SelStage<T>::kRows * kHeadDim * sizeof(T) + (size_t)kp * 8 +
                         (size_t)key_cap * sizeof(uint32_t);
-    const int64_t items = (int64_t)s->batch * s->num_kv_heads;
-    // Items that outnumber the CTAs and are long enough for a look at the next one: us dealt out / taken, 1024 ragged lists of 64 to
-    // 1024 pages 50 / 42, 4096 ragged of 128 .. 2048 226 / 202, 2048 even of 2048 195 / 192, 4096 even of 1024 189 / 193;
-    // 3000 ragged of 6 to 100 33 / 35, 256 of 512 (one round) 12.4 / 12.7.
-    const int64_t slots = (int64_t)sm_count() * kSelCtasPerSm;
-    const bool take = items > slots && summary_stride >= 512;
-    auto kern = take ? select_kernel<T, G, true> : select_kernel<T, G, false>;
+    auto kern = select_kernel<T, G>;
     KTK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                  "ktk_select");
-    const unsigned grid = (unsigned)(take || items < slots ? items : slots);
-    KTK_CUDA_TRY(launch_behind(items <= sm_count(), kern, grid, kSelCtaThreads, smem, st, (const T*)q, (const T*)summaries,
+    const int64_t items = (int64_t)s->batch * s->num_kv_heads;
+    int64_t grid = (int64_t)sm_count() * kSelCtasPerSm;
+    if (grid > items) grid = items;
+    KTK_CUDA_TRY(launch_behind(items <= sm_count(), kern, (unsigned)grid, kSelCtaThreads, smem, st, (const T*)q, (const T*)summaries,
                                summary_stride, kv_indices, kv_indptr, kv_last_page_len, topk, key_cap, kp, view, out_pages,
                                out_logical, out_scores, items, s->num_kv_heads, s->num_pages, status),
                  "ktk_select");

@@ -831,15 +831,16 @@ def _silu_mul_fake(gate, up):
 torch.library.define(
     "ktk::select_pages_into",
     "(Tensor q, Tensor summaries, Tensor kv_indices, Tensor kv_indptr, Tensor kv_last_page_len, int topk, "
-    "int num_pages, Tensor(a!) out, Tensor(b!) status) -> ()",
+    "int num_pages, Tensor(a!) out, Tensor(b!) status, Tensor? seq_order=None) -> ()",
 )
 
 
 @torch.library.impl("ktk::select_pages_into", "cuda")
-def _select_pages_into(q, summaries, kv_indices, kv_indptr, kv_last_page_len, topk, num_pages, out, status):
-    select_pages(q, summaries, kv_indices, kv_indptr, kv_last_page_len, topk, num_pages, out=out, status=status)
+def _select_pages_into(q, summaries, kv_indices, kv_indptr, kv_last_page_len, topk, num_pages, out, status, seq_order=None):
+    select_pages(q, summaries, kv_indices, kv_indptr, kv_last_page_len, topk, num_pages, out=out, status=status,
+                 view=None if seq_order is None else PageView(seq_order=seq_order))
 
 
 @torch.library.register_fake("ktk::select_pages_into")
-def _select_pages_into_fake(q, summaries, kv_indices, kv_indptr, kv_last_page_len, topk, num_pages, out, status):
+def _select_pages_into_fake(q, summaries, kv_indices, kv_indptr, kv_last_page_len, topk, num_pages, out, status, seq_order=None):
     return None

@@ -13,37 +13,26 @@ def _consumers_of_selection():
 
 
 def _stuck(vote):
-    """Two warps and what each sees at its two points of leaving (its wait for the item, then the flag behind the item's barrier, raised
-    in between): the cases in which one has left and the other stands in a barrier."""
+    """Two warps at the point of leaving: whether the waits of each came through, and what a look at the flag shows each of them, which may
+    be raised in between.  The cases in which one leaves and the other goes on to the next barrier."""
     cases = []
-    for item_a, item_b, flag_a, flag_b in itertools.product((True, False), repeat=4):
-        left = []
-        for mine, flag in ((item_a, flag_a), (item_b, flag_b)):
-            if vote:
-                left.append(not (item_a and item_b) or flag_a or flag_b)
-            else:
-                left.append(not mine or flag)
+    for came_a, came_b, flag_a, flag_b in itertools.product((True, False), repeat=4):
+        alone = [not came or flag for came, flag in ((came_a, flag_a), (came_b, flag_b))]
+        left = [not came_a or not came_b] * 2 if vote else alone
         if left[0] != left[1]:
-            cases.append((item_a, item_b, flag_a, flag_b))
+            cases.append((came_a, came_b, flag_a, flag_b))
     return cases
 
 
 def test_consumers_of_the_selection_leave_together():
     assert _stuck(vote=False) and not _stuck(vote=True)
     body = _consumers_of_selection()
-    # every way out of the item loop: behind a vote of all consumers, or behind a rank that is the same for all of them
-    for line in (x.strip() for x in body.splitlines()):
-        if re.search(r"\bbreak;", line) and line != "break;":
-            assert "consumer_any(" in line or line == "if (rank < 0) break;", line
+    # the one way out of the item loop: behind a vote of all consumers
+    outs = [x.strip() for x in body.splitlines() if re.search(r"\bbreak;", x) and x.strip() != "break;"]
+    assert len(outs) == 1 and outs[0].startswith("if (consumer_any(!ok)) break;")
     alone = re.findall(r"\{\s*ok = false;\s*break;\s*\}", body)            # out of the loop over an item's stages, to the vote behind it
     assert len(re.findall(r"^\s*break;", body, re.M)) == len(alone) == 1
     assert "abort_flag)" not in body.replace("&abort_flag)", "")             # no look of a warp's own
-
-
-def test_the_producer_of_the_selection_hands_out_nothing_after_giving_up():
-    text = (CSRC / "ktk_select.cu").read_text()
-    wait, hand_out = text.index("mbar_wait(&item_free[slot]"), text.index("mbar_arrive(&item_full[slot])")
-    assert "*(volatile int*)&abort_flag) break;" in text[wait:hand_out]
 
 
 def test_a_lane_that_looks_for_another_hands_on_what_it_saw():

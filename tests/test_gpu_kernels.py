@@ -171,8 +171,8 @@ def test_select_many_ragged_items_per_cta(cuda_device, order):
 
 @pytest.mark.parametrize("B, Hkv, dtype, order", [(460, 1, torch.bfloat16, False), (300, 2, torch.bfloat16, True),
                                                   (500, 1, torch.float32, True), (1500, 1, torch.bfloat16, False)])
-def test_select_takes_items_of_ctas_not_yet_started(cuda_device, B, Hkv, dtype, order):
-    """Long rows and more items than resident CTAs: a CTA goes on with items of CTAs that have not started.  Items of no page, of
+def test_select_of_more_items_than_resident_ctas(cuda_device, B, Hkv, dtype, order):
+    """Long rows and more items than resident CTAs: a CTA goes on from one item to the next.  Items of no page, of
     one, within the budget and of fewer stages than a ring; with and without a sequence order."""
     ops = _ops()
     g = torch.Generator().manual_seed(B)
@@ -191,7 +191,7 @@ def test_select_takes_items_of_ctas_not_yet_started(cuda_device, B, Hkv, dtype, 
         view = ops.PageView(0, 1, None, None, torch.argsort(pages, descending=True, stable=True).to(torch.int32).to(cuda_device))
     dev = lambda t: t.to(cuda_device)
     status = ops.new_status(cuda_device)
-    for _ in range(3):                                       # who takes what differs from run to run
+    for _ in range(3):
         out_l = torch.full((B, Hkv, topk + 1), -7, dtype=torch.int32, device=cuda_device)
         out_p = ops.select_pages(dev(q), dev(summ), dev(indices), dev(indptr), dev(last), topk, indices.numel(),
                                  out_logical=out_l, status=status, view=view)

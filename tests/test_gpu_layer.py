@@ -128,6 +128,26 @@ def test_ragged_contexts_select_like_the_oracle(cuda_device):
     torch.testing.assert_close(got.float().cpu(), ref, rtol=2e-2, atol=2e-2)
 
 
+def test_a_ragged_layer_hands_the_selection_its_order(cuda_device):
+    # the sequences from the longest to the shortest go with the op; the selection is the one without an order
+    import kinetics_b200 as kb
+    dtype, B = torch.bfloat16, 6
+    for lens, want in (([40 * 16, 17, 16, 0, 333, 100], [0, 4, 5, 1, 2, 3]), ([300, 310, 297, 400, 352, 300], None)):
+        layer = kb.BlockTopkDecoderLayer(config=Cfg, world_size=1, batch_size=B, prefix_len=640, max_len=704, page_size=16, topk_page=8,
+                                         device=cuda_device, dtype=dtype, page_table="random", seed=5, context_lens=lens)
+        assert (None if layer.seq_order is None else layer.seq_order.tolist()) == want
+        q = torch.randn(B, layer.num_heads, 128, device=cuda_device, dtype=dtype)
+        out = [torch.empty(B, layer.num_kv_heads, 9, dtype=torch.int32, device=cuda_device) for _ in range(2)]
+        for o, order in zip(out, (None, layer.seq_order)):
+            args = (q, layer.compressed_key_cache, layer.paged_kv_indices, layer.full_kv_indptr, layer.last_kv_lens, 8,
+                    layer.total_pages, o, layer.status, order)
+            torch.library.opcheck(torch.ops.ktk.select_pages_into.default, args,
+                                  test_utils=("test_schema", "test_autograd_registration", "test_faketensor"))
+            torch.ops.ktk.select_pages_into(*args)
+        layer.check_status()
+        assert torch.equal(*out)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_qkv_norm_with_rotary_embedding(cuda_device, dtype):
     # split + q-norm + k-norm + rotary embedding in one launch, against the reference's statements in fp32
