@@ -317,11 +317,24 @@ __global__ void __launch_bounds__(kLdThreads) lru_step_kernel(const LruParams p)
 // their inputs lie in L2), multiplies u [32 x block] with the CHAN + CHAN gate rows by mma.m16n8k16, and finishes its channels.
 // The ring's place that a step writes is read by no other CTA.  Bound by latency: a chain of loads (slot, window and state), the
 // products, the stores; so a thread keeps to one piece of the channels and loads a tap's weights once, the state and the gate are on their
-// way before the products, and CHAN is what leaves one round of CTAs.
+// way before the products, and CHAN is what leaves the shorter rounds of CTAs (lf_wide).
 constexpr int kLfRows = 32, kLfThreads = 256, kLfMaxBlock = 512;
 
 __host__ __device__ inline int lf_ld(int block_stride) { return (block_stride + 15) / 16 * 16 + 8; }      // padded: no bank conflicts
 __host__ __device__ inline int lf_smem(int block_stride, int chan) { return (kLfRows + 2 * chan) * lf_ld(block_stride) * 2 + kLfRows * (2 * chan + 1) * 4; }
+
+// 64 channels per CTA instead of 32: where two such CTAs share an SM as two of the others do (blocks of up to 288 channels), and their
+// rounds, of 5/4 the length, are fewer by more than that.  16 blocks of 256 channels, 128 rows: 29 us with an element per access, 22.8
+// with 32 channels in two rounds, 16.8 with 64 in one.  us of 32 / 64 channels elsewhere: 40 x 64, 256 rows 19.4 / 18.3, 64 x 96, 128 rows
+// 22.7 / 21.8, 20 x 200, 256 rows 41.7 / 38.1; but 20 x 200, 128 rows 22.8 / 24.9 (two rounds either way), blocks of one slice 64 x 32,
+// 256 rows 14.5 / 18.6 and 128 x 24 24.5 / 32.3, one CTA per SM 8 x 512, 256 rows 59.9 / 64.6 and 12 x 304 55.4 / 60.0.
+static bool lf_wide(const ktk_lru& a, int64_t groups) {
+    const auto rounds = [&](int chan) {
+        const int64_t ctas = groups * a.blocks * ((a.block_stride + chan - 1) / chan), slots = 2 * (int64_t)sm_count();
+        return (ctas + slots - 1) / slots;
+    };
+    return 2 * (lf_smem(a.block_stride, 64) + 2048) <= 228 * 1024 && 5 * rounds(64) < 4 * rounds(32);
+}
 
 // neighbouring channels of a lane, one access
 template <typename T, int N> struct alignas(N * sizeof(T)) Lanes { T x[N]; };
@@ -637,12 +650,9 @@ extern "C" int ktk_lru_decode(const void* proj, int64_t row_stride, int64_t y_co
     const LruParams p{*shape, *table, nullptr, nullptr, (const __nv_bfloat16*)proj + y_col, row_stride, nullptr, slots, num_slots,
                       rows, 1, rb, ib, decay, state, out, status};
     const LruDecodeParams q{p, (const __nv_bfloat16*)proj + x_col, (const __nv_bfloat16*)gates, conv_w, conv_b, (__nv_bfloat16*)ring};
-    // 32 channels per CTA while those fit in one round (two CTAs of either form share an SM), 64 beyond that: 16 blocks of 256 channels,
-    // 128 rows: 29 us with 512 CTAs of 32 channels and an element per access, 14.7 with 256 of 64 in pairs
     const int64_t groups = (rows + kLfRows - 1) / kLfRows;
     const bool pairs = ((uintptr_t)state & 7u) == 0 && (((uintptr_t)rb | (uintptr_t)ib | (uintptr_t)decay) & 7u) == 0 && ((uintptr_t)out & 3u) == 0;
-    const bool narrow = !pairs || groups * shape->blocks * ((shape->block_stride + 31) / 32) <= 2 * (int64_t)sm_count() ||
-                        lf_smem(shape->block_stride, 64) > 200 * 1024;
+    const bool narrow = !pairs || !lf_wide(*shape, groups);
     const int chan = narrow ? 32 : 64, smem = lf_smem(shape->block_stride, chan), slices = (shape->block_stride + chan - 1) / chan;
     auto kernel = shape->taps == 4 ? (narrow ? lru_decode_kernel<4, 32> : lru_decode_kernel<4, 64>)
                                    : (narrow ? lru_decode_kernel<0, 32> : lru_decode_kernel<0, 64>);

@@ -1,0 +1,41 @@
+"""Rules by which the host picks a kernel's form, run here as they stand in the sources."""
+import re
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "kinetics_b200" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def wide(tmp_path_factory):
+    """lf_wide of the recurrent step as a program: block, blocks and rows to 0 or 1, and the shared memory of either form."""
+    text = (CSRC / "layers" / "ktl_lru.cu").read_text()
+    parts = [re.search(p, text, re.S | re.M).group(0) for p in (
+        r"^constexpr int kLfRows = [^\n]*\n", r"^[^\n]* int lf_ld\([^\n]*\n", r"^[^\n]* int lf_smem\([^\n]*\n", r"^static bool lf_wide\(.*?^}\n")]
+    source = ("#include <cstdint>\n#include <cstdio>\n#define __host__\n#define __device__\nstruct ktk_lru { int blocks, block_stride; };\n"
+              "static int sm_count() { return 148; }\n" + "".join(parts) +
+              'int main() { int b, n, r; while (scanf("%d %d %d", &b, &n, &r) == 3) {\n'
+              '    const ktk_lru a{n, b};\n    printf("%d %d %d\\n", (int)lf_wide(a, (r + kLfRows - 1) / kLfRows), lf_smem(b, 32), lf_smem(b, 64)); } }\n')
+    d = tmp_path_factory.mktemp("rule")
+    (d / "rule.cpp").write_text(source)
+    subprocess.run(["g++", "-std=c++17", "-o", str(d / "rule"), str(d / "rule.cpp")], check=True)
+
+    def ask(cases):
+        out = subprocess.run([str(d / "rule")], input="\n".join("%d %d %d" % c for c in cases), capture_output=True, text=True, check=True)
+        return [tuple(map(int, line.split())) for line in out.stdout.splitlines()]
+    return ask
+
+
+def test_wide_recurrent_steps_only_where_they_take_less(wide):
+    cases = [(block, blocks, rows) for block in range(8, 513, 8) for blocks in (1, 3, 16, 40, 128) for rows in (1, 33, 128, 256, 1000)]
+    for (block, blocks, rows), (chosen, narrow_smem, wide_smem) in zip(cases, wide(cases)):
+        assert 2 * (narrow_smem + 1024) <= 228 * 1024                        # the narrow form always has two CTAs on an SM
+        if chosen:
+            groups = (rows + 31) // 32
+            ctas = [groups * blocks * -(-block // chan) for chan in (32, 64)]
+            assert 2 * (wide_smem + 1024) <= 228 * 1024 and ctas[1] < ctas[0] and ctas[0] > 2 * 148, (block, blocks, rows)
+    # measured: block, blocks, rows
+    assert [c for c, _, _ in wide([(256, 16, 128), (128, 32, 256), (64, 40, 256), (96, 64, 128), (200, 20, 256)])] == [1] * 5
+    assert [c for c, _, _ in wide([(512, 8, 256), (304, 12, 256), (32, 64, 256), (24, 128, 256), (200, 20, 128), (256, 16, 64)])] == [0] * 6

@@ -458,7 +458,8 @@ def test_balanced_rows_with_little_workspace(cuda_device, batch):
 
 
 @pytest.mark.parametrize("blocks,block,taps,rows,misaligned", [(16, 256, 4, 150, False), (16, 256, 4, 150, True), (20, 200, 3, 70, False),
-                                                               (30, 104, 4, 97, False), (5, 512, 4, 140, False)])
+                                                               (30, 104, 4, 97, False), (5, 512, 4, 140, False), (9, 288, 4, 230, False),
+                                                               (128, 24, 4, 130, False), (20, 200, 4, 250, False)])
 def test_fused_steps_over_more_than_one_round_of_narrow_ctas(cuda_device, blocks, block, taps, rows, misaligned):
     # CTAs of 64 channels, whole and partial slices of a block; a state that starts between two pairs keeps the narrow form.
     # Bounds: as in test_fused_steps_of_many_sequences_equal_the_separate_ones
