@@ -472,19 +472,34 @@ LINEAR_ROWS = 16         # most rows of linear_rows
 
 
 def linear_rows_wins(rows: int, n: int, k: int, dtype, gated: bool) -> bool:
-    """Whether linear_rows is faster than the library's products (with two of them and silu_mul if `gated`).  fp32: throughout (16 rows,
-    512 x 512: 7.3 us there, 2.9 here; 12288 x 4096 133 and 119).  bf16, us there / here: 8 rows, 768 x 4096 9.1 / 5.9, 1536 x 4096
-    9.1 / 9.2, 4096 x 1536 6.6 / 11.3; 4 rows, 1536 x 4096 9.4 / 6.3, 2560 x 5120 12.3 / 12.6; gated, 8 rows, 1536 x 4096 20.6 / 14.0,
-    3072 x 4096 25.9 / 25.2, 4 rows, 3200 x 5120 26.2 / 18.5, 6400 x 5120 27.3 / 33.9, 16 rows, 1024 x 1024 10.5 / 7.7."""
-    if rows < 1 or rows > LINEAR_ROWS or k % 8 != 0:
+    """Whether linear_rows is faster than the library's products (with two of them and silu_mul if `gated`).  A CTA takes 8 (from 9 rows
+    on 4) columns, half as many if gated, over all of k: few columns of a long k leave SMs idle, many of a short k are more rounds of
+    CTAs that hardly begin.  us, library / here, weights not in L2.
+    fp32, 16 rows: 512 x 512 7.3 / 2.9, 12288 x 2048 as fast, 8192 x 1024 28.6 / 30.8, 4096 x 256 1.42 times the library's time, 128 x
+    12288 0.90, x 16384 1.09.  One row, where the library has kernels of its own: 1024 x 1024 6.3 / 3.8, x 2560 6.2 / 7.7, 3072 x 4096
+    16.0 / 12.5, 512 x 4096 1.56 times its time, 32 x 16384 4.6.
+    bf16: 8 rows, 768 x 4096 9.1 / 5.9, 512 x 1024 0.88, x 256 0.94 to 1.25, 1536 x 4096 9.1 / 9.2; 4 rows, 1536 x 4096 9.4 / 6.3, 2560 x 5120
+    12.3 / 12.6, any n x 16384 1.02 to 1.36; gated, 8 rows, 1536 x 4096 20.6 / 14.0, 4096 x 1024 1.14, 4 rows, 3200 x 5120 26.2 / 18.5,
+    6144 x 1024 13.2 / 14.2, 6400 x 5120 27.3 / 33.9, 16 rows, 1024 x 1024 10.5 / 7.7, 1024 x 256 1.08, 1536 x 512 1.34."""
+    if rows < 1 or rows > LINEAR_ROWS or k % 8 != 0 or k > 16384:
         return False
     if dtype == torch.float32:
-        return True
+        if n > (12 if rows == 1 else 16 if rows <= 8 else 6) * k:
+            return False
+        if rows == 1:
+            return n >= 512 or k <= 6144 if gated else 256 <= k <= 1024 or n >= 2048 and k <= 8192
+        return n >= 512 or k <= (8192 if rows <= 8 or gated else 6144)
     if dtype != torch.bfloat16:
         return False
     if gated:
-        return n * k <= ((17 << 20) if rows <= 4 else (8 << 20) if rows <= 8 else (1 << 20))
-    return n <= 1536 if rows <= 4 else n <= 1024 and rows <= 8
+        if rows <= 4:
+            return n * k <= 17 << 20 and n <= 4096
+        if rows <= 8:
+            return n * k <= 8 << 20 and n <= 2048
+        return n * k <= 1 << 20 and n <= min(1024, max(512, k))
+    if k > 12288 or rows > 8:
+        return False
+    return n <= 1536 if rows <= 2 else k >= 1024 and n <= (1536 if rows <= 4 else 1024)
 
 
 def linear_rows(x: torch.Tensor, w: torch.Tensor, bias=None, residual=None, w2=None) -> torch.Tensor:

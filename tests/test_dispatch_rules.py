@@ -4,6 +4,7 @@ import subprocess
 from pathlib import Path
 
 import pytest
+import torch
 
 CSRC = Path(__file__).resolve().parent.parent / "kinetics_b200" / "csrc"
 
@@ -39,3 +40,25 @@ def test_wide_recurrent_steps_only_where_they_take_less(wide):
     # measured: block, blocks, rows
     assert [c for c, _, _ in wide([(256, 16, 128), (128, 32, 256), (64, 40, 256), (96, 64, 128), (200, 20, 256)])] == [1] * 5
     assert [c for c, _, _ in wide([(512, 8, 256), (304, 12, 256), (32, 64, 256), (24, 128, 256), (200, 20, 128), (256, 16, 64)])] == [0] * 6
+
+
+# rows, columns, inner size, gated: measured with weights that are not in L2
+FASTER_HERE = {
+    torch.float32: [(1, 512, 512, False), (4, 768, 512, False), (4, 1024, 512, True), (4, 512, 1024, False), (16, 512, 512, False),
+                    (4, 4096, 4096, False), (16, 4096, 4096, False), (16, 12288, 4096, False), (8, 12288, 4096, True), (1, 4096, 4096, True)],
+    torch.bfloat16: [(4, 768, 4096, False), (4, 1536, 4096, False), (8, 768, 4096, False), (1, 1536, 1024, False), (4, 1536, 4096, True),
+                     (4, 3200, 5120, True), (8, 1536, 4096, True), (16, 1024, 1024, True), (16, 512, 512, True)]}
+FASTER_THERE = {
+    torch.float32: [(1, 8, 16384, False), (1, 64, 16384, False), (1, 512, 4096, False), (1, 1024, 2560, False), (1, 32, 16384, True),
+                    (1, 128, 8192, True), (2, 32, 16384, False), (16, 32, 12288, False), (16, 4096, 256, False), (16, 8192, 1024, True),
+                    (12, 12288, 1024, False), (8, 12288, 256, False), (8, 4096, 128, False)],
+    torch.bfloat16: [(4, 8, 256, False), (4, 128, 16384, False), (8, 64, 256, False), (8, 1536, 4096, False), (8, 1024, 16384, False),
+                     (8, 4096, 1024, True), (4, 6144, 1024, True), (4, 8192, 640, True), (16, 1024, 256, True), (16, 1536, 512, True)]}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_products_by_rows_only_where_they_are_faster(dtype):
+    from kinetics_b200 import ops
+    assert [c for c in FASTER_HERE[dtype] if not ops.linear_rows_wins(c[0], c[1], c[2], dtype, c[3])] == []
+    assert [c for c in FASTER_THERE[dtype] if ops.linear_rows_wins(c[0], c[1], c[2], dtype, c[3])] == []
+    assert not any(ops.linear_rows_wins(r, 512, k, dtype, g) for r, k in ((0, 512), (17, 512), (4, 500)) for g in (False, True))
