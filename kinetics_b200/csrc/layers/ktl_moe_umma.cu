@@ -199,20 +199,15 @@ moe_umma_kernel(const MoeParams p, const int tile_rows, const int cta_rows, cons
                 bool ok = true;
                 if (pos.round > 0) ok = mbar_wait_fast(&empty[s], (pos.round - 1) & 1, &abort_flag);
                 if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
-                const int chunks = chunks_of(k);
+                static_assert(STAGE == 1 || kChunks == 1, "a stage of gathered rows is one chunk");
+                const uint32_t dst = dst0 + s * stage_bytes;
+                const bool in_row = k * kMuK + chunk * 8 < K;
+                const char* from = in_row ? base + (int64_t)k * (kMuK * 2) : base;
+                const uint32_t on = in_row ? 16u : 0u;
 #pragma unroll
-                for (int c = 0; c < kChunks; ++c) {
-                    if (c >= chunks) break;
-                    const uint32_t dst = dst0 + s * stage_bytes + c * chunk_bytes;
-                    const int col = (k * kChunks + c) * kMuK;
-                    const bool in_row = col + chunk * 8 < K;
-                    const char* from = in_row ? base + (int64_t)col * 2 : base;
-                    const uint32_t on = in_row ? 16u : 0u;
-#pragma unroll
-                    for (int i = 0; i < kPer; ++i)
-                        if (16 * i < it.m)                   // uniform
-                            cp_async16(dst + i * 2048, from + (uint64_t)off[i] * 16, bytes[i] & on);
-                }
+                for (int i = 0; i < kPer; ++i)
+                    if (16 * i < it.m)                       // uniform
+                        cp_async16(dst + i * 2048, from + (uint64_t)off[i] * 16, bytes[i] & on);
                 cp_async_arrive(&full[s]);
             }
         }
