@@ -33,8 +33,8 @@ template <> struct LrVec<__nv_bfloat16> {
     static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&f)[8]) { load8(p, f); }
 };
 
-// N sums over the warp's 32 lanes at once, N a power of two: afterwards lane l holds in v[0] .. those of the sums i with
-// i % min(N, 32) == l % min(N, 32) (v[j]: sum j * 32 + l)
+// N sums over the warp's 32 lanes at once, N a power of two.  Afterwards lane l holds, for N >= 32, sum l * (N / 32) + j in v[j], for
+// fewer sum l / (32 / N) in v[0]
 template <int N> __device__ __forceinline__ void fold_lanes(float (&v)[N]) {
     const int lane = threadIdx.x & 31;
     int have = N;
