@@ -78,8 +78,9 @@ constexpr int kAtWarps = 4, kAtBatch = 4;
 // Several tokens per sequence (prefill, chunked append): token j of the packed k / v belongs to the
 // sequence b with append_indptr[b] <= j < append_indptr[b+1] and is the (j - append_indptr[b])-th of the
 // sequence's n_app newest tokens.  A warp per token, all heads, E elements per access (16 bytes; 1 element where a pointer is
-// not aligned) and kAtBatch of keys and of values in flight: bound by DRAM.  8192 tokens of 8 heads: 40 us with a CTA per token and
-// head, an element per thread.
+// not aligned) and kAtBatch of keys and of values in flight.  Bound by the latency of its loads (0.55
+// instructions a clock, 28 of 64 warps resident).  8192 tokens of 8 heads, 67 MB: 18.6 us with k and v in DRAM, 7.6 with them and the pages
+// in L2; with a CTA per token and head, an element per thread, 40 where this form took 11.5, behind the kernels that wrote k and v.
 template <typename T, int E>
 __global__ void __launch_bounds__(kAtWarps * 32)
 append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ append_indptr, int total,
@@ -133,7 +134,8 @@ append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int
 }
 
 // grid (B, Hkv, Z): a CTA rebuilds the summaries of E logical pages at a time, E elements of one per thread with all its tokens'
-// keys in flight (512 pages of 8 heads, all touched by one prompt: 15 us with an element per thread, 9 with eight).
+// keys in flight.  512 pages of 8 heads behind the prompt that wrote them: 15 us with an element per thread, 7.4 with four (102 registers,
+// 14 of 64 warps resident).
 template <typename T, int E>
 __global__ void __launch_bounds__(kHeadDim)
 build_summaries_kernel(const T* __restrict__ cache, T* __restrict__ summaries,

@@ -159,7 +159,8 @@ struct LruParams {
 // 32 channels of one sequence: lane = channel, a warp runs 8 consecutive tokens, a CTA 64, the CTAs of a cluster consecutive
 // tiles of 64.  Per round of the cluster: local products and end states, joined over the CTA's warps in shared memory and
 // over the cluster's CTAs through theirs; then every warp replays its tokens from the state in front of them.
-// Bound by memory (14 bytes per token and channel) and, close behind, by the eight special functions of each: so a warp's
+// Bound by what it issues and by the rounds' barriers (8192 tokens of 2048 channels: 2.6 instructions a clock and SM, DRAM at a third of
+// its rate), eight special functions per token and channel first; the bytes, 14 of each, take half the time.  So a warp's
 // next round is on its way into shared memory while it computes this one, the output gate is worked out between the two
 // halves of the cluster's barrier, and a CTA writes its totals into its peers' memory, where each warp folds them by itself.
 // 8192 tokens of 4096 channels, bf16: 139 us (3.4 TB/s; the output gate's functions 16 of them), with loads into registers at

@@ -14,8 +14,9 @@
 //                       of a column in one thread, which stmatrix.trans lays down as rows that leave in 16-byte pieces.
 //                       Lanes that swapped neighbours and stored 2 or 4 bytes each held the tensor cores up: 8192 rows,
 //                       8 of 64 experts, 2048 -> 768 columns 415 + 247 us (stages 0 and 1), 381 + 195 this way.
-// Now 354 + 166 us, 1.16 and 1.24 PFLOP/s: bound by what an SM reads from L2, 32 KiB per 64 columns (in stage 0 half of it by
-// cp.async).
+// Now 354 + 166 us, 1.16 and 1.24 PFLOP/s.  By the counters no unit is full: the tensor pipe is busy 62 and 69 % of the cycles, an SM
+// reads 42 and 51 bytes a clock from L2 (of 64; 32 KiB per 64 columns, in stage 0 half of it by cp.async), L2 as a whole runs at 40
+// and 45 %.
 // Full tiles (prompts) run on pairs of CTAs (cta_group::2): 256 weight rows x 256 routed rows per item, each CTA with its
 // half of both in shared memory, which takes a third off the traffic from L2.  The second CTA's issuing warp tells the
 // first one's when its part of a stage has landed.

@@ -190,8 +190,8 @@ template <int kPer> __device__ __forceinline__ void pick_experts4(const RoutePar
 
 // A CTA takes 32 rows.  Columns 128 at a time: h [32 x 128] and W [64 experts x 128] through a ring of cp.async stages; warp
 // w accumulates 16 rows and 16 experts of the pass with mma.m16n8k16 (exact products, fp32 sums).  Bound by latency: 8192 rows of 2048
-// columns, 64 experts, 41 us with stages of 64 columns, a fragment per load and each row's choices one behind the other, 25 us this way (12 of them what W and h
-// take from L2).
+// columns, 64 experts, 41 us with stages of 64 columns, a fragment per load and each row's choices one behind the other, 25 us this way;
+// 13 of 64 warps resident, an SM reads 26 bytes a clock from L2, tensor pipe 18 %.
 constexpr int kRtK = 128, kRtLd = kRtK + 8;                      // padded rows: no bank conflicts
 constexpr int kRtStageElems = (kRtRows + kRtCols) * kRtLd;
 constexpr int kRtPieces = (kRtRows + kRtCols) * (kRtK / 8) / kRtThreads, kRtPieceRows = kRtThreads / (kRtK / 8);
