@@ -713,16 +713,18 @@ static int balanced_ctas(const ktk_attn& a) {
 }
 
 // Whether a decode step is cut over all sequences instead of sequence by sequence.  Its CTAs run the mean of the tiles, which for
-// lengths that differ is well under that of the longest sequence's (counted here as three quarters of it; the host knows no more),
-// but pay for each change of sequence and for a second launch.  Measured at 32 heads, 576 columns, us by sequence / balanced:
-// 128 x 4096 tokens 127 / 123, 128 of 256 .. 4096 118 / 85, 64 x 16384 246 / 224, 64 of 1024 .. 16384 221 / 131;
-// 128 x 600 31 / 38, 128 x 150 16 / 29, 1 x 16384 27 / 49.
+// lengths that differ is well under that of the longest sequence's (counted here as four fifths of it; the host knows no more), but pay for each
+// sequence (13 tiles' time) and for a second launch that joins the pieces of a sequence one behind the other.  So never below 25 tiles a CTA,
+// where few sequences are cut into many pieces.  Fitted to 412 shapes of 8 to 128 heads, 576 columns; us by sequence / balanced, 32 heads:
+// 128 x 4000 tokens 121 / 120, ragged (a sixteenth of it upwards) 116 / 92; 32 x 16384 122 / 119, ragged 117 / 89; 150 x 2000 139 / 103;
+// 100 x 4000 116 / 102; but 1 x 16384 34 / 56, 4 x 4000 27 / 38, 16 x 4000 33 / 37, 48 x 2000 38 / 44, 128 x 600 31 / 39.
 bool attn_shared_balanced(const ktk_attn& a, int batch, int64_t max_keys) {
     const int64_t tiles = (max_keys + kAsTok - 1) / kAsTok, ctas = balanced_ctas(a);
     int64_t splits;
     const int64_t cost = splits_cost((int64_t)batch * packing_of(a.heads, true).chunks, tiles, &splits);
-    return batch > 0 && batch <= 65535 &&
-           (3 * batch * tiles / 4 + 3 * batch) / ctas + kAsStartTiles + 7 < cost;
+    if (batch <= 0 || batch > 65535 || batch * tiles < 25 * ctas) return false;
+    const double pieces = batch < ctas ? (double)ctas / batch : 1.0;             // of a sequence
+    return (0.8 * (double)tiles + 13.0) * batch / (double)ctas + 10.0 + 2.0 * pieces < (double)cost;
 }
 
 size_t attn_shared_workspace(const ktk_attn& a, int64_t rows, int splits) {

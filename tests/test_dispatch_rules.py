@@ -9,6 +9,17 @@ import torch
 CSRC = Path(__file__).resolve().parent.parent / "kinetics_b200" / "csrc"
 
 
+def _program(folder, source):
+    (folder / "rule.cpp").write_text(source)
+    subprocess.run(["g++", "-std=c++17", "-o", str(folder / "rule"), str(folder / "rule.cpp")], check=True)
+
+    def ask(cases):
+        text = "\n".join(" ".join(map(str, c)) for c in cases)
+        out = subprocess.run([str(folder / "rule")], input=text, capture_output=True, text=True, check=True)
+        return [tuple(map(int, line.split())) for line in out.stdout.splitlines()]
+    return ask
+
+
 @pytest.fixture(scope="module")
 def wide(tmp_path_factory):
     """lf_wide of the recurrent step as a program: block, blocks and rows to 0 or 1, and the shared memory of either form."""
@@ -19,14 +30,7 @@ def wide(tmp_path_factory):
               "static int sm_count() { return 148; }\n" + "".join(parts) +
               'int main() { int b, n, r; while (scanf("%d %d %d", &b, &n, &r) == 3) {\n'
               '    const ktk_lru a{n, b};\n    printf("%d %d %d\\n", (int)lf_wide(a, (r + kLfRows - 1) / kLfRows), lf_smem(b, 32), lf_smem(b, 64)); } }\n')
-    d = tmp_path_factory.mktemp("rule")
-    (d / "rule.cpp").write_text(source)
-    subprocess.run(["g++", "-std=c++17", "-o", str(d / "rule"), str(d / "rule.cpp")], check=True)
-
-    def ask(cases):
-        out = subprocess.run([str(d / "rule")], input="\n".join("%d %d %d" % c for c in cases), capture_output=True, text=True, check=True)
-        return [tuple(map(int, line.split())) for line in out.stdout.splitlines()]
-    return ask
+    return _program(tmp_path_factory.mktemp("wide"), source)
 
 
 def test_wide_recurrent_steps_only_where_they_take_less(wide):
@@ -40,6 +44,26 @@ def test_wide_recurrent_steps_only_where_they_take_less(wide):
     # measured: block, blocks, rows
     assert [c for c, _, _ in wide([(256, 16, 128), (128, 32, 256), (64, 40, 256), (96, 64, 128), (200, 20, 256)])] == [1] * 5
     assert [c for c, _, _ in wide([(512, 8, 256), (304, 12, 256), (32, 64, 256), (24, 128, 256), (200, 20, 128), (256, 16, 64)])] == [0] * 6
+
+
+def test_decode_steps_over_shared_rows_are_balanced_only_where_that_is_faster(tmp_path):
+    text = (CSRC / "layers" / "ktl_attn_shared.cu").read_text()
+    parts = [re.search(p, text, re.S | re.M).group(0) for p in (
+        r"^constexpr int kAsTok = [^\n]*\n", r"^constexpr int kAsMinTiles = [^\n]*\n", r"^constexpr int kAsMaxSplits = [^\n]*\n",
+        r"^struct Packing [^\n]*\n", r"^__host__ __device__ inline Packing packing_of\(.*?^}\n", r"^static int64_t splits_cost\(.*?^}\n",
+        r"^static int balanced_ctas\(.*?^}\n", r"^bool attn_shared_balanced\(.*?^}\n")]
+    ask = _program(tmp_path, "#include <cstdint>\n#include <cstdio>\n#define __host__\n#define __device__\nstruct ktk_attn { int heads; };\n"
+                   "static int sm_count() { return 148; }\n" + "".join(parts) +
+                   'int main() { int h, b, k; while (scanf("%d %d %d", &h, &b, &k) == 3) printf("%d\\n", '
+                   "(int)attn_shared_balanced(ktk_attn{h}, b, k)); }\n")
+    # heads, sequences, longest: measured at 576 columns, even and ragged lists
+    by_sequence = [(8, 1, 16384), (16, 1, 600), (16, 1, 16384), (16, 4, 5000), (16, 16, 600), (16, 16, 5000), (16, 48, 2000), (32, 1, 16384),
+                   (32, 4, 4000), (32, 16, 4000), (32, 128, 600), (32, 1, 32768), (128, 8, 8192), (128, 150, 1000), (128, 128, 2000),
+                   (128, 64, 2000), (32, 0, 100), (32, 70000, 4000)]
+    balanced = [(16, 32, 16384), (16, 128, 4096), (32, 100, 4000), (32, 128, 4096), (32, 150, 2000), (32, 64, 16384), (128, 64, 16384),
+                (128, 150, 4000)]
+    assert [c for c, (x,) in zip(by_sequence, ask(by_sequence)) if x] == []
+    assert [c for c, (x,) in zip(balanced, ask(balanced)) if not x] == []
 
 
 # rows, columns, inner size, gated: measured with weights that are not in L2
