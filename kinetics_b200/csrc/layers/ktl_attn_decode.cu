@@ -43,7 +43,7 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
     extern __shared__ uint8_t ad_raw[];
     __shared__ __align__(8) uint64_t full[kAdStages], empty[kAdStages];
     __shared__ int abort_flag, issued_total;
-    __shared__ float red_m[kAdConsumers][2][8], red_l[kAdConsumers][2][8];
+    __shared__ float red_m[kAdConsumers][2][8], red_l[kAdConsumers][2][8], red_f[kAdConsumers][2][8], all_m[2][8], all_l[2][8];
     constexpr int kStage = ad_stage_bytes<DC, VC>();
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ad_raw) + 1023) & ~uintptr_t(1023));
     const ktk_attn& a = p.a;
@@ -278,6 +278,22 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
     }
 
     // ---- the four warps' parts, one map at a time through the ring's memory ----
+    // what each warp's part counts for, and the sum, worked out once per map and head
+    if (tid < 16) {
+        const int mp = tid >> 3, h = tid & 7;
+        float M = red_m[0][mp][h], L = 0.0f;
+#pragma unroll
+        for (int w = 1; w < kAdConsumers; ++w) M = fmaxf(M, red_m[w][mp][h]);
+        const float ref = M == -INFINITY ? 0.0f : M;
+#pragma unroll
+        for (int w = 0; w < kAdConsumers; ++w) {
+            const float f = FIXED ? 1.0f : ex2(red_m[w][mp][h] - ref);
+            red_f[w][mp][h] = f;
+            L += f * red_l[w][mp][h];
+        }
+        all_m[mp][h] = M;
+        all_l[mp][h] = L;
+    }
     float* merge = reinterpret_cast<float*>(ring);       // [warp][8 heads][VC * 64]
     constexpr int kVt = VC * 64;
     float o[2][8 * kVt / 128];                           // thread tid (of 128): elements tid, tid + 128, ... of [heads][kVt]
@@ -298,28 +314,15 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
 #pragma unroll
             for (int i = 0; i < 8 * kVt / 128; ++i) {
                 const int x = tid + i * 128, h = x / kVt;
-                float M = 0.0f, v = 0.0f;
-                if (!FIXED) {
-                    M = red_m[0][mp][h];
-                    for (int w = 1; w < kAdConsumers; ++w) M = fmaxf(M, red_m[w][mp][h]);
-                    if (M == -INFINITY) M = 0.0f;
-                }
+                float v = 0.0f;
 #pragma unroll
-                for (int w = 0; w < kAdConsumers; ++w)
-                    v += (FIXED ? 1.0f : ex2(red_m[w][mp][h] - M)) * merge[w * 8 * kVt + x];
+                for (int w = 0; w < kAdConsumers; ++w) v += (FIXED ? 1.0f : red_f[w][mp][h]) * merge[w * 8 * kVt + x];
                 o[mp][i] = v;
             }
         }
         __syncthreads();
     }
     if (warp >= kAdConsumers) return;
-    auto merged = [&](int mp, int h, float& M, float& L) {
-        M = red_m[0][mp][h];
-        for (int w = 1; w < kAdConsumers; ++w) M = fmaxf(M, red_m[w][mp][h]);
-        const float ref = M == -INFINITY ? 0.0f : M;
-        L = 0.0f;
-        for (int w = 0; w < kAdConsumers; ++w) L += (FIXED ? 1.0f : ex2(red_m[w][mp][h] - ref)) * red_l[w][mp][h];
-    };
     if (p.splits > 1) {
 #pragma unroll
         for (int i = 0; i < 8 * kVt / 128; ++i) {
@@ -333,10 +336,8 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
             if (c == 0) {
 #pragma unroll
                 for (int mp = 0; mp < 2; ++mp) {
-                    float M, L;
-                    merged(mp, h, M, L);
-                    w[2 * mp] = M;
-                    w[2 * mp + 1] = L;
+                    w[2 * mp] = all_m[mp][h];
+                    w[2 * mp + 1] = all_l[mp][h];
                 }
             }
         }
@@ -348,9 +349,7 @@ attn_decode_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k_map
 #pragma unroll
     for (int i = 0; i < 8 * kVt / 128; ++i) {
         const int x = tid + i * 128, h = x / kVt, c = x % kVt;
-        float M, L1, L2;
-        merged(0, h, M, L1);
-        merged(1, h, M, L2);
+        const float L1 = all_l[0][h], L2 = all_l[1][h];
         d[i] = L1 > 0.0f && L2 > 0.0f && c < a.vdim ? o[0][i] / L1 - a.lambda * (o[1][i] / L2) : 0.0f;
         const float ss = warp_sum_f(d[i] * d[i]);        // a warp's 32 columns lie in one head
         if (lane == 0) sq[i * kAdConsumers + warp] = ss;
