@@ -148,7 +148,8 @@ __device__ __forceinline__ void clear_counts(const ResidualNormParams& p) {
         for (int i = threadIdx.x; i < p.zero_n; i += blockDim.x) p.zero[i] = 0;
 }
 
-// A CTA per row.
+// A CTA per row.  56 registers with NV = 1: two more would cost an SM a sixth of its CTAs of 192 threads (bf16, 8192 x 1536, the part
+// normalised: 38.8 us, 40.9 with 58 registers, which is what r as a 64-bit index gives).
 template <typename T, int NV, bool TOKENS>
 __global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_kernel(const ResidualNormParams p) {
     __shared__ __align__(16) float part_s[2 * (kRnThreads / 32)];
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_ker
     part.clear();
     clear_counts(p);
     const int nvec = p.stride / 8;
-    const int64_t r = blockIdx.x;
+    const unsigned r = blockIdx.x;
     const auto* from = RowSource<T, TOKENS>{p}.stream(r, threadIdx.x == 0);
     float x[NV][8], y[NV][8];
 #pragma unroll
@@ -186,9 +187,9 @@ __global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_ker
 
 // CTAs that walk rows c, c + gridDim.x, ...; a ring in shared memory keeps the next row on its way by bulk copies, a stage holding a row
 // of the stream and its part.  8192 rows of 4096 bf16 columns inside a model 91 -> 72 us (402 MB).
-template <typename T, bool TOKENS>
-__global__ void __launch_bounds__(kRnThreads, rn_resident(2)) residual_norm_walk_kernel(const ResidualNormParams p) {
-    constexpr int NV = 2, stages = kRnStages;
+template <typename T, bool TOKENS, int NV>
+__global__ void __launch_bounds__(kRnThreads, rn_resident(NV)) residual_norm_walk_kernel(const ResidualNormParams p) {
+    constexpr int stages = kRnStages;
     extern __shared__ __align__(128) uint8_t rn_ring[];
     __shared__ __align__(8) uint64_t full[kRnStages];
     __shared__ __align__(16) float part_s[2 * (kRnThreads / 32)];
@@ -264,20 +265,29 @@ static int residual_norm_launch(const ResidualNormParams& p, cudaStream_t st) {
     const int nvec = p.stride / 8;
     const int threads = nvec >= kRnThreads ? kRnThreads : (nvec + 31) / 32 * 32;
     const int nv = (nvec + threads - 1) / threads;
-    // Walkers: rows of 1793 to 2048 columns by six CTAs of 128 threads per SM, of up to 4096 by three of 256.  us, a CTA per row /
-    // walkers, next rows not in L2: 8192 x 4096 bf16 98 / 75, 3000 x 4096 37 / 32, 2000 x 4096 24 / 23, 8192 x 2048 56 / 52, 8192 x 4096 fp32
-    // 117 / 109, embedding rows 8192 x 2048 41 / 31 and x 4096 62 / 51; not 3000 x 2048 (21.7 / 23.1), 1024 columns (25 / 28), fp32 of 2048
-    // columns, several parts (8 of 2048 80 / 82, 4 of 4096 110 / 110).
-    const bool narrow = nvec <= kRnThreads;
-    const int walk_threads = narrow ? kRnThreads / 2 : kRnThreads, resident = narrow ? 6 : 3;
-    if (nvec > kRnThreads - 32 && nvec <= 2 * kRnThreads && (p.y == nullptr || p.parts == 1) && (sizeof(T) == 2 || !narrow) &&
-        p.rows >= (narrow ? 8 : 4) * (int64_t)sm_count() * resident) {
+    // Walkers: rows of up to 4096 columns by three CTAs of 256 threads per SM; bf16 rows of 1793 to 2048 columns by six of 128, or by four of 256
+    // (from 1921 columns on, whose threads are all busy) where only the part is normalised.  us, a CTA per row / walkers, next rows not in L2, part and next sublayer normed: 8192 x 4096 bf16
+    // 111 / 94, 1776 x 4096 33 / 30.5, 8192 x 2048 bf16 58 / 54, 2400 x 2048 24 / 23, 8192 x 4096 fp32 129 / 112; the part alone 8192 x 4096
+    // 96 / 79, 4100 x 2048 29.9 / 29.4 (six of 128: 30.4); embedding rows 8192 x 2048 48 / 41 and x 4096 90 / 68.  Not fp32 of 2048 columns
+    // (68 / 70), sums of neither (2048 columns 24.4 / 25.4, fp32 4096 102 / 105), 1024 columns (25 / 28), several parts (8 of 2048 80 / 82, 4 of
+    // 4096 110 / 110).
+    const bool narrow = nvec <= kRnThreads, pre = p.h != nullptr && p.pre_w != nullptr, post = p.y != nullptr && p.post_w != nullptr;
+    const bool fits = nvec > kRnThreads - 32 && nvec <= 2 * kRnThreads && (p.y == nullptr || p.parts == 1);
+    if (fits && (pre || post || TOKENS || (!narrow && sizeof(T) == 2)) && (sizeof(T) == 2 || !narrow) &&
+        p.rows >= (narrow ? 16 : 12) * (int64_t)sm_count()) {
         const size_t stage = (size_t)p.stride * (TOKENS ? sizeof(T) : 4) + (p.y ? (size_t)p.stride * sizeof(T) : 0);
-        auto kernel = residual_norm_walk_kernel<T, TOKENS>;
-        KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRnStages * stage)), who);
-        kernel<<<(unsigned)(sm_count() * resident), walk_threads, kRnStages * stage, st>>>(p);
-        KTK_CUDA_TRY(cudaGetLastError(), who);
-        return KTK_OK;
+        const auto walk = [&](auto kernel, int threads_of, int resident) {
+            KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRnStages * stage)), who);
+            kernel<<<(unsigned)(sm_count() * resident), threads_of, kRnStages * stage, st>>>(p);
+            KTK_CUDA_TRY(cudaGetLastError(), who);
+            return (int)KTK_OK;
+        };
+        if (!narrow) return walk(residual_norm_walk_kernel<T, TOKENS, 2>, kRnThreads, 3);
+        if constexpr (sizeof(T) == 2) {
+            if constexpr (!TOKENS)
+                if (!pre && nvec > kRnThreads - 16) return walk(residual_norm_walk_kernel<T, false, 1>, kRnThreads, 4);
+            return walk(residual_norm_walk_kernel<T, TOKENS, 2>, kRnThreads / 2, 6);
+        }
     }
     auto kernel = nv <= 1 ? residual_norm_kernel<T, 1, TOKENS>
                 : nv <= 2 ? residual_norm_kernel<T, 2, TOKENS>

@@ -117,6 +117,28 @@ def test_residual_norm_of_walked_rows(cuda_device, dtype, cols):
             torch.testing.assert_close(h[:, :cols].double(), unit(want) if normed else want, **tol)
 
 
+@pytest.mark.parametrize("cols", [1920, 1921, 2048])
+def test_walked_rows_whose_part_alone_is_normalised(cuda_device, cols):
+    # bf16, on either side of where whole CTAs walk; one row over a whole number of rounds.  Bounds: as in test_residual_norm_over_many_rows
+    from kinetics_b200 import layer_ops as lo, ops
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    rows, S, eps, mult = 16 * sms + 1, lo.pad8(cols), 1e-4, 0.3
+    g = torch.Generator(device=cuda_device).manual_seed(cols)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
+    pad = lambda t: torch.nn.functional.pad(t, (0, S - cols)).contiguous()
+    x0, w, b, y = rnd(rows, cols) + 2.0, rnd(cols), rnd(cols), (rnd(rows, 1, cols) - 1.0).to(torch.bfloat16)
+    v = y[:, 0].double() - y[:, 0].double().mean(1, keepdim=True)
+    want = x0.double() + mult * (v / (v.square().mean(1, keepdim=True) + eps).sqrt() * w.double() + b.double())
+    for copied in (False, True):
+        x, h, status = pad(x0), torch.empty(rows, S, dtype=torch.bfloat16, device=cuda_device), ops.new_status(cuda_device)
+        lo.residual_norm(x, h if copied else None, cols, eps, y=pad(y), post=(pad(w), pad(b)), mult=mult, status=status)
+        ops.raise_on_status(status)
+        torch.testing.assert_close(x[:, :cols].double(), want, rtol=1e-5, atol=2e-5)
+        assert x[:, cols:].abs().sum() == 0
+        if copied:
+            torch.testing.assert_close(h[:, :cols].double(), want, rtol=1e-2, atol=1e-2)
+
+
 def test_residual_norm_reports_a_token_outside_the_vocabulary(cuda_device):
     from kinetics_b200 import layer_ops as lo, ops
     x = torch.empty(1, 8, device=cuda_device)
