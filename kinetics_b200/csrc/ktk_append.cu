@@ -81,7 +81,8 @@ constexpr int kAtWarps = 4, kAtBatch = 4;
 // not aligned) and kAtBatch of keys and of values in flight.  Bound by the latency of its loads (0.55
 // instructions a clock, 28 of 64 warps resident).  8192 tokens of 8 heads, 67 MB: 18.6 us with k and v in DRAM, 7.6 with them and the pages
 // in L2; with a CTA per token and head, an element per thread, 40 where this form took 11.5, behind the kernels that wrote k and v.
-template <typename T, int E>
+// SPLIT: a warp per batch of a token (blockIdx.y).
+template <typename T, int E, bool SPLIT>
 __global__ void __launch_bounds__(kAtWarps * 32)
 append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int32_t* __restrict__ append_indptr, int total,
                      int B, T* __restrict__ cache, const int32_t* __restrict__ kv_indices,
@@ -122,7 +123,7 @@ append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int
     P* vp = kp + kPageSize * row;
     const P* ks = reinterpret_cast<const P*>(k) + j * row;
     const P* vs = reinterpret_cast<const P*>(v) + j * row;
-    for (int64_t i0 = lane; i0 < row; i0 += 32 * kAtBatch) {
+    for (int64_t i0 = SPLIT ? lane + 32 * kAtBatch * blockIdx.y : lane; i0 < row; i0 += 32 * kAtBatch) {
         P kk[kAtBatch], vv[kAtBatch];
 #pragma unroll
         for (int i = 0; i < kAtBatch; ++i)
@@ -130,6 +131,7 @@ append_tokens_kernel(const T* __restrict__ k, const T* __restrict__ v, const int
 #pragma unroll
         for (int i = 0; i < kAtBatch; ++i)
             if (i0 + 32 * i < row) { kp[i0 + 32 * i] = kk[i]; vp[i0 + 32 * i] = vv[i]; }
+        if (SPLIT) break;
     }
 }
 
@@ -271,16 +273,21 @@ template <typename T>
 static int build_impl(const void* cache, void* summaries, int64_t summary_stride,
                       const int32_t* kv_indices, const int32_t* kv_indptr,
                       const int32_t* kv_last_page_len, const View& view, const ktk_shape* s, int32_t* status,
-                      cudaStream_t st, const int32_t* append_indptr = nullptr) {
-    // CTAs for all pages a list can have, no more than keep the device busy; four elements a thread, whose 16 tokens fit more warps
-    // than those of eight
+                      cudaStream_t st, const int32_t* append_indptr = nullptr, int64_t appended = 0) {
+    // Pages to rebuild, at most: of a list, and of all of them.
+    const int64_t touched = append_indptr != nullptr ? appended / kPageSize + 2 : summary_stride;
+    const int64_t of_list = touched < summary_stride ? touched : summary_stride;
+    const int64_t of_all = append_indptr != nullptr ? appended / kPageSize + 2 * (int64_t)s->batch : s->batch * summary_stride;
+    // CTAs for all pages a list can have, no more than keep the device busy.  Four elements a thread, whose 16 tokens fit more warps than
+    // those of eight; one where there is a CTA for every page and head, so that only its latency counts.  us, one / four elements a thread:
+    // 32 pages of a head 4.9 / 6.3, one or two pages of each of 64 lists of 8 heads with the append 9.2 / 10.8; 512 pages of 8 heads 15 / 7.4.
     constexpr int kPiece = 4;
-    const bool aligned = ((((uintptr_t)cache) | (uintptr_t)summaries) & 15u) == 0;
-    const int64_t bh = (int64_t)s->batch * s->num_kv_heads, each = aligned ? kPiece : 1;
+    const bool wide = ((((uintptr_t)cache) | (uintptr_t)summaries) & 15u) == 0 && of_all * s->num_kv_heads > 16LL * sm_count();
+    const int64_t bh = (int64_t)s->batch * s->num_kv_heads, each = wide ? kPiece : 1;
     int64_t z = (16LL * sm_count() + bh - 1) / bh;
-    if (z > (summary_stride + each - 1) / each) z = (summary_stride + each - 1) / each;
+    if (z > (of_list + each - 1) / each) z = (of_list + each - 1) / each;
     dim3 grid(s->batch, s->num_kv_heads, (unsigned)(z < 1 ? 1 : z));
-    auto kernel = aligned ? build_summaries_kernel<T, kPiece> : build_summaries_kernel<T, 1>;
+    auto kernel = wide ? build_summaries_kernel<T, kPiece> : build_summaries_kernel<T, 1>;
     kernel<<<grid, kHeadDim, 0, st>>>(
         (const T*)cache, (T*)summaries, summary_stride, kv_indices, kv_indptr, kv_last_page_len,
         view.page_count, view.slot_index, append_indptr, view.sink_tokens, s->num_kv_heads, s->num_pages, status);
@@ -294,8 +301,13 @@ static int append_tokens_impl(const void* k, const void* v, const int32_t* appen
                               const ktk_shape* s, int32_t* status, cudaStream_t st) {
     constexpr int kPiece = 16 / (int)sizeof(T);
     const bool aligned = (((uintptr_t)k | (uintptr_t)v | (uintptr_t)cache) & 15u) == 0;
-    auto kernel = aligned ? append_tokens_kernel<T, kPiece> : append_tokens_kernel<T, 1>;
-    kernel<<<(unsigned)((total + kAtWarps - 1) / kAtWarps), kAtWarps * 32, 0, st>>>(
+    // few tokens: a warp for each batch of pieces of a token (17 tokens of 16 heads, fp32: 4.4 us, 6.5 with a warp for its four batches)
+    const int64_t batches = ((int64_t)s->num_kv_heads * kHeadDim / (aligned ? kPiece : 1) + 32 * kAtBatch - 1) / (32 * kAtBatch);
+    const bool split = total <= 512 && batches > 1 && batches <= 64;
+    auto kernel = split ? (aligned ? append_tokens_kernel<T, kPiece, true> : append_tokens_kernel<T, 1, true>)
+                        : (aligned ? append_tokens_kernel<T, kPiece, false> : append_tokens_kernel<T, 1, false>);
+    const dim3 grid((unsigned)((total + kAtWarps - 1) / kAtWarps), (unsigned)(split ? batches : 1));
+    kernel<<<grid, kAtWarps * 32, 0, st>>>(
         (const T*)k, (const T*)v, append_indptr, (int)total, s->batch, (T*)cache, kv_indices, kv_indptr, kv_last_page_len,
         view.page_count, view.sink_tokens, s->num_kv_heads, s->num_pages, status);
     KTK_CUDA_TRY(cudaGetLastError(), "ktk_append_tokens");
@@ -399,9 +411,9 @@ extern "C" int ktk_append_tokens(const void* k, const void* v, const int32_t* ap
     if (summaries == nullptr) return KTK_OK;
     if (shape->dtype == KTK_F32)
         return build_impl<float>(kv_cache, summaries, summary_stride, kv_indices, kv_indptr, kv_last_page_len, view,
-                                 shape, status, st, append_indptr);
+                                 shape, status, st, append_indptr, total_tokens);
     return build_impl<__nv_bfloat16>(kv_cache, summaries, summary_stride, kv_indices, kv_indptr, kv_last_page_len,
-                                     view, shape, status, st, append_indptr);
+                                     view, shape, status, st, append_indptr, total_tokens);
 }
 
 extern "C" int ktk_build_summaries(const void* kv_cache, void* summaries, int64_t summary_stride,

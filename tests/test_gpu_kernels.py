@@ -610,11 +610,11 @@ def test_append_tokens_chunks_bit_exact(cuda_device, dtype, sink):
 
 @pytest.mark.parametrize("shift", [0, 1])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("Hkv", [1, 9])
-def test_append_tokens_by_pieces_bit_exact(cuda_device, dtype, shift, Hkv):
-    # a token's heads in less and in more than one batch of 16-byte pieces; tensors that start between two of them
+@pytest.mark.parametrize("Hkv, lens", [(1, [300, 16, 1]), (9, [300, 16, 1]), (9, [511, 1]), (9, [512, 1]), (48, [600, 250, 40])])
+def test_append_tokens_by_pieces_bit_exact(cuda_device, dtype, shift, Hkv, lens):
+    # a token's heads in less and in more than one batch of 16-byte pieces, each batch with a warp of its own or all with one; fewer and
+    # more pages than a CTA each; tensors that start between two pieces
     ops = _ops()
-    lens = [300, 16, 1]
     q, k, v = random_case(7, len(lens), Hkv, 1, lens, dtype)
     st = paged_state(k, v, lens, dtype, seed=3, fill=0.0)
     pack = lambda x: torch.cat([x[b, :, :n].transpose(0, 1) for b, n in enumerate(lens)]).to(dtype).contiguous()
