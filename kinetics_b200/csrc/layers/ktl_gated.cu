@@ -21,24 +21,27 @@ gated_rows_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t rows, i
     }
 }
 
-// Eight elements a thread in two accesses (single ones at the end, and where z does not start on 16 bytes): 128 x 32768 logits 10 us with
-// one element at a time and a step over the grid, 7.4 us this way (5.2 by the bytes).
-__global__ void __launch_bounds__(kGtThreads) scale_cap_kernel(float* z, int64_t n, float scale, float cap, const bool wide) {
+// WIDE: eight elements a thread in two accesses (single ones at the end): 128 x 32768 logits 10 us with one element at a time and a step
+// over the grid, 7.4 us this way (5.2 by the bytes).  Fewer elements, and a z that does not start on 16 bytes, one a thread: 32768 of
+// them 2.5 us, 3.1 with eight.
+template <bool WIDE> __global__ void __launch_bounds__(kGtThreads) scale_cap_kernel(float* z, int64_t n, float scale, float cap) {
     auto one = [&](float x) {
         const float v = x * scale;
         return cap > 0.0f ? cap * tanhf(v / cap) : v;
     };
     const int64_t at = (int64_t)blockIdx.x * kGtThreads + threadIdx.x, step = (int64_t)gridDim.x * kGtThreads;
-    const int64_t eights = wide ? n / 8 : 0;
-    for (int64_t i = at; i < eights; i += step) {
-        float v[8];
-        Vec8<float>::load(z + i * 8, v);
+    const int64_t eights = WIDE ? n / 8 : 0;
+    if (WIDE)
+        for (int64_t i = at; i < eights; i += step) {
+            float v[8];
+            Vec8<float>::load(z + i * 8, v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = one(v[e]);
-        Vec8<float>::store(z + i * 8, v);
-    }
+            for (int e = 0; e < 8; ++e) v[e] = one(v[e]);
+            Vec8<float>::store(z + i * 8, v);
+        }
     for (int64_t i = eights * 8 + at; i < n; i += step) z[i] = one(z[i]);
 }
+constexpr int64_t kCapWide = 160 * 1024;      // us, one / eight elements a thread: 131072 elements 3.15 / 3.4, 200000 3.5 / 3.3
 
 static unsigned rows_grid(int64_t work) {
     const int64_t blocks = (work + kGtThreads - 1) / kGtThreads, cap = (int64_t)sm_count() * 16;
@@ -77,8 +80,9 @@ extern "C" int ktk_scale_cap(float* z, int64_t n, float scale, float cap, void* 
     const char* who = "ktk_scale_cap";
     if (n < 0 || (n > 0 && !z)) { set_error("%s: n=%lld", who, (long long)n); return KTK_ERR_ARG; }
     if (n == 0) return KTK_OK;
-    const bool wide = ((uintptr_t)z & 15u) == 0;
-    scale_cap_kernel<<<rows_grid(wide ? (n + 7) / 8 : n), kGtThreads, 0, (cudaStream_t)stream>>>(z, n, scale, cap, wide);
+    const bool wide = ((uintptr_t)z & 15u) == 0 && n >= kCapWide;
+    auto kernel = wide ? scale_cap_kernel<true> : scale_cap_kernel<false>;
+    kernel<<<rows_grid(wide ? (n + 7) / 8 : n), kGtThreads, 0, (cudaStream_t)stream>>>(z, n, scale, cap);
     KTK_CUDA_TRY(cudaGetLastError(), who);
     return KTK_OK;
 }

@@ -547,6 +547,19 @@ def test_gated_rows_and_scale_cap(cuda_device, dtype):
     torch.testing.assert_close(lo.scale_cap(z.clone().to(cuda_device), 0.3, 0.0).cpu(), z * 0.3)
 
 
+@pytest.mark.parametrize("n", [160 * 1024 - 1, 160 * 1024, 160 * 1024 + 5])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_scale_cap_of_many(cuda_device, n, shift):
+    # an element a thread and eight, a rest, a start between two pieces.  Bound: fp32 rounding of the argument and of the result
+    from kinetics_b200 import layer_ops as lo
+    z = 50 * torch.randn(n + shift, generator=torch.Generator().manual_seed(n))
+    for cap, want in ((9.0, 9 * torch.tanh(z[shift:].double() * 0.3 / 9)), (0.0, z[shift:].double() * 0.3)):
+        got = z.to(cuda_device)
+        lo.scale_cap(got[shift:], 0.3, cap)
+        torch.testing.assert_close(got[shift:].double().cpu(), want, rtol=1e-5, atol=1e-5)
+        assert torch.equal(got[:shift].cpu(), z[:shift])
+
+
 @pytest.mark.parametrize("dtype", [F32, BF])
 def test_experts_with_clamped_gates_and_shares_of_the_whole_softmax(cuda_device, dtype):
     from kinetics_b200 import layer_ops as lo
