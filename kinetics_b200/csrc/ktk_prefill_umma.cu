@@ -20,30 +20,22 @@ constexpr int kPuSmem = PrefillFlash::bytes(2, 2);
 
 // Which tiles a CTA takes.  A later tile sees more keys, and the work of a launch that leaves SMs idle at its end should end with
 // short ones.
-//   kByLength     grid (kv heads, item): the items of all sequences from the most keys to the fewest
 //   kByTile       grid (kv heads, sequences, tile pairs): the last pairs of all heads and sequences first
+//   kByEither     the same grid; where histories differ, the items of all sequences from the most keys to the fewest
 //   kBySequence   grid (tile pairs, kv heads, sequences), for more than 65535 pairs
-enum Order { kBySequence, kByTile, kByLength };
+enum Order { kBySequence, kByTile, kByEither };
 constexpr int kPuOrdered = 32;                            // sequences that an ordered launch may have: one per lane
 
 // Item `rank` of the launch: a sequence and which `step` of its new tokens.  Its length counts in steps, those of the history rounded
-// up: item p of a sequence with h of history has length p + h.  A warp finds the length at `rank`, 32 probes at a time.  False
-// behind the last item.
-__device__ __forceinline__ bool item_by_length(const PrefillUmmaParams& p, int rank, int step, int& b, int& pair) {
-    const int lane = threadIdx.x & 31;
-    int first = 0, count = 0;
-    if (lane < p.batch) {
-        const int n = p.q_indptr[lane + 1] - p.q_indptr[lane];
-        const SeqPages sp = seq_pages(p.kv_indptr, p.page_count, p.kv_last_page_len, p.sink_tokens, lane);
-        if (n > 0) {
-            count = (n + step - 1) / step;
-            first = sp.bad || sp.total < n ? 0 : (sp.total - n + step - 1) / step;
-        }
-    }
+// up: item p of a sequence with h of history has length p + h.  Lane s brings sequence s: its new tokens (0 behind the last) and its history.
+// A warp finds the length at `rank`, 32 probes at a time.  The sequence * 65536 + the step, or -1 behind the last item.  A call, so that
+// launches without it do not fetch it (one to two us a CTA: 32 portions of 40 tokens 23.2 us, 27 with it).
+__device__ __noinline__ int item_by_length(int rank, int step, int batch, int n, int history) {
+    const int lane = threadIdx.x & 31, count = (n + step - 1) / step, first = n > 0 ? (history + step - 1) / step : 0;
     // items of length L or more, every lane for its own L; all lanes take part
     auto at_least = [&](int L) {
         int have = 0;
-        for (int s = 0; s < p.batch; ++s) {
+        for (int s = 0; s < batch; ++s) {
             const int f = __shfl_sync(0xffffffffu, first, s), c = __shfl_sync(0xffffffffu, count, s);
             have += min(max(f + c - L, 0), c);
         }
@@ -54,7 +46,7 @@ __device__ __forceinline__ bool item_by_length(const PrefillUmmaParams& p, int r
     for (bool begun = false; hi - lo > 1 || !begun; begun = true) {
         const int each = (hi - lo + 31) / 32, L = lo + lane * each, seen = at_least(L), have = L < hi ? seen : behind;
         const unsigned more = __ballot_sync(0xffffffffu, L < hi && have > rank);       // a prefix of the lanes
-        if (more == 0) return false;                       // only of the first probes, which start at 0
+        if (more == 0) return -1;                          // only of the first probes, which start at 0
         const int at = 31 - __clz((int)more);
         const int next = __shfl_sync(0xffffffffu, have, at < 31 ? at + 1 : 31);
         if (at < 31 && lo + (at + 1) * each < hi) { hi = lo + (at + 1) * each; behind = next; }
@@ -62,8 +54,23 @@ __device__ __forceinline__ bool item_by_length(const PrefillUmmaParams& p, int r
     }
     // among the sequences with an item of length lo
     const unsigned has = __ballot_sync(0xffffffffu, lo >= first && lo < first + count);
-    b = (int)__fns(has, 0, rank - behind + 1);
-    pair = lo - __shfl_sync(0xffffffffu, first, b & 31);
+    const bool mine = (has >> lane & 1u) && __popc(has & ((1u << lane) - 1u)) == rank - behind;
+    const int b = __ffs((int)__ballot_sync(0xffffffffu, mine)) - 1;
+    return b * 65536 + lo - __shfl_sync(0xffffffffu, first, b);
+}
+
+// Whether a launch in either order goes by length, and the CTA's item if so.  Histories, counted in whole pages, that lie within a
+// quarter of the longest sequence are left in the order of the tiles, which is that of the lengths or close to it.
+__device__ __forceinline__ bool item_of_either(const PrefillUmmaParams& p, int& item) {
+    const int lane = threadIdx.x & 31, seq = lane < p.batch ? lane : p.batch - 1;
+    const int n = p.q_indptr[seq + 1] - p.q_indptr[seq];
+    const int tokens = (p.page_count ? p.page_count[seq] : p.kv_indptr[seq + 1] - p.kv_indptr[seq]) * kPageSize;
+    const int history = tokens > n ? tokens - n : 0;
+    const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)(n > 0 ? history + n : 0));
+    const int spread = (int)(__reduce_max_sync(0xffffffffu, n > 0 ? (unsigned)history : 0u) -
+                             __reduce_min_sync(0xffffffffu, n > 0 ? (unsigned)history : 0x7fffffffu));
+    if (spread <= longest / 4) return false;               // the same for all CTAs
+    item = item_by_length(blockIdx.z * gridDim.y + blockIdx.y, p.tiles * (kUmRows / p.G), p.batch, lane < p.batch && n > 0 ? n : 0, history);
     return true;
 }
 
@@ -76,20 +83,21 @@ prefill_umma_kernel(const PrefillUmmaParams p, const __grid_constant__ CUtensorM
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int h = ORDER == kBySequence ? blockIdx.y : blockIdx.x;
-    int b = ORDER == kByTile ? blockIdx.y : blockIdx.z, pair = 0;
-    if (ORDER == kByLength) {
-        if (!item_by_length(p, blockIdx.y, p.tiles * (kUmRows / p.G), b, pair)) return;
-    } else {
-        pair = ORDER == kByTile ? (int)(gridDim.z - 1 - blockIdx.z) : (int)(gridDim.x - 1 - blockIdx.x);
+    int b = ORDER == kBySequence ? blockIdx.z : blockIdx.y;
+    int pair = ORDER == kBySequence ? (int)(gridDim.x - 1 - blockIdx.x) : (int)(gridDim.z - 1 - blockIdx.z);
+    int item;
+    if (ORDER == kByEither && item_of_either(p, item)) {
+        if (item < 0) return;
+        b = item >> 16;
+        pair = item & 65535;
     }
+    const int q0 = p.q_indptr[b], n_new = p.q_indptr[b + 1] - q0;
+    const SeqPages sp = seq_pages(p.kv_indptr, p.page_count, p.kv_last_page_len, p.sink_tokens, b);
     const int G = p.G, Hq = p.Hkv * G;
     const int tpc = kUmRows / G;                    // new tokens per tile
-    const int q0 = p.q_indptr[b];
-    const int n_new = p.q_indptr[b + 1] - q0;
     const int tok0 = pair * p.tiles * tpc;
     if (tok0 >= n_new) return;                      // uniform for the CTA: nothing allocated yet
 
-    const SeqPages sp = seq_pages(p.kv_indptr, p.page_count, p.kv_last_page_len, p.sink_tokens, b);
     const int base_pos = sp.total - n_new;          // position of the sequence's first new token
     if (sp.bad || base_pos < 0) {
         if (tid == 0) report(p.status, KTK_STATUS_BAD_TABLE);
@@ -245,18 +253,16 @@ int launch_prefill_umma(PrefillUmmaParams p, int max_new_tokens, cudaStream_t st
     const int64_t tiles = (p.batch * per_seq < most ? p.batch * per_seq : most) * p.Hkv;
     p.tiles = tiles <= sm_count() ? 1 : 2;
     const unsigned pairs = (unsigned)((per_seq + p.tiles - 1) / p.tiles);
-    // By length where several sequences take between one and four rounds of CTAs: finding its item costs a CTA half a microsecond, and
-    // the more rounds, the less the last one leaves idle.  Six portions of 350 to 1050 tokens behind 2500 to 7500, 16 heads over 8:
-    // 250 us by tile, 203 by length (264 CTAs); eight of 150 to 450 behind 450 to 1350 50 and 47.
-    const int64_t step = (int64_t)tpc * p.tiles, about = p.total_new / step + p.batch / 2;
-    const int64_t items = p.total_new / step + p.batch < (int64_t)p.batch * pairs ? p.total_new / step + p.batch : (int64_t)p.batch * pairs;
-    const bool by_length = p.batch > 1 && p.batch <= kPuOrdered && items <= 65535 && about * p.Hkv > sm_count() &&
-                           about * p.Hkv <= 4 * (int64_t)sm_count();
-    const bool by_tile = !by_length && pairs <= 65535;
-    auto kernel = by_length ? prefill_umma_kernel<kByLength> : by_tile ? prefill_umma_kernel<kByTile> : prefill_umma_kernel<kBySequence>;
+    // By length, if histories differ, where several sequences take between one round of CTAs and two and a half: the more rounds, the less
+    // the last one leaves idle.  Six portions of 350 to 1050 tokens behind 2500 to 7500, 16 heads over 8: 255 us by tile, 229 by length
+    // (280 CTAs); eight of 150 to 450 behind 450 to 1350 59 and 56; the first with 32 heads (544 CTAs) 446 either way.  Where histories do
+    // not differ the look costs a CTA half a microsecond: 16 portions of 300 behind 300 60 us, 62 with it.
+    const int64_t about = p.total_new / (tpc * p.tiles) + p.batch / 2;
+    const bool by_tile = pairs <= 65535;
+    const bool either = by_tile && p.batch > 1 && p.batch <= kPuOrdered && about * p.Hkv > sm_count() && 2 * about * p.Hkv <= 5 * (int64_t)sm_count();
+    auto kernel = either ? prefill_umma_kernel<kByEither> : by_tile ? prefill_umma_kernel<kByTile> : prefill_umma_kernel<kBySequence>;
     KTK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPuSmem), who);
-    const dim3 grid = by_length ? dim3((unsigned)p.Hkv, (unsigned)items)
-                    : by_tile ? dim3((unsigned)p.Hkv, (unsigned)p.batch, pairs) : dim3(pairs, (unsigned)p.Hkv, (unsigned)p.batch);
+    const dim3 grid = by_tile ? dim3((unsigned)p.Hkv, (unsigned)p.batch, pairs) : dim3(pairs, (unsigned)p.Hkv, (unsigned)p.batch);
     DecodeParams d{};                               // only what the tensor map needs
     d.cache = p.cache; d.Hkv = p.Hkv; d.num_pages = p.num_pages;
     CUtensorMap map;

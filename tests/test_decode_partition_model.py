@@ -114,7 +114,7 @@ def test_rows_shared_by_all_heads():
 
 
 def _item_by_length(first, count, rank):
-    """csrc/ktk_prefill_umma.cu, item_by_length: 32 probes at a time."""
+    """csrc/ktk_prefill_umma.cu, item_of_either where histories differ: 32 probes at a time."""
     at_least = lambda L: sum(min(max(f + c - L, 0), c) for f, c in zip(first, count))
     lo, hi, behind, begun = 0, max(f + c for f, c in zip(first, count)), 0, False
     while hi - lo > 1 or not begun:

@@ -92,10 +92,10 @@ def test_prefill_long_prompt_many_sequences(cuda_device):
     torch.testing.assert_close(out[n:2 * n].float(), ref, rtol=2e-2, atol=2e-2)
 
 
-@pytest.mark.parametrize("G,Hkv,sink,B", [(8, 4, 0, 7), (8, 4, 4, 7), (4, 6, 0, 32), (2, 3, 0, 33)])
+@pytest.mark.parametrize("G,Hkv,sink,B", [(8, 4, 0, 7), (8, 4, 4, 7), (4, 6, 0, 32), (4, 1, 0, 32), (8, 1, 4, 16), (2, 3, 0, 33)])
 def test_prefill_of_unequal_sequences_over_more_than_one_round(cuda_device, G, Hkv, sink, B):
     """Portions of very different lengths behind very different histories, some empty: the CTAs take them by length (up to 32
-    sequences).  Every row is written once, with what the row-by-row kernel gives.  Bound: as in the other prompts."""
+    sequences in one to two and a half rounds of CTAs).  Every row is written once, with what the row-by-row kernel gives.  Bound: as in the other prompts."""
     from kinetics_b200 import ops
     new = ([700, 3, 0, 450, 64, 65, 1200] * 5)[:B]
     hist = ([100, 2500, 40, 0, 900, 10, 5] * 5)[:B]
